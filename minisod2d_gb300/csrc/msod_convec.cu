@@ -9,357 +9,537 @@
 //   Rener  += gpvol [ 1/4 (div(rho H u) + H div q + rho H div u + rho div(H u))
 //                     + 1/4 sum_i (q_i d_i H + u_i d_i(rho H) + H u_i d_i rho) ]
 //
-// with F = q (x) u, Fuu = u (x) u, k = |u|^2/2 and H = E + k.  The energy
-// residual uses the sums E+k, rho E + rho k, rho E u + rho k u and E u + k u
-// of the reference's separate E and k terms (elem_convec.f90:810-817): the
-// derivatives are linear, so the sums are differentiated once.
+// with F = q (x) u, Fuu = u (x) u, k = |u|^2/2 and H = E + k (the reference's
+// separate E and k terms, elem_convec.f90:810-817, are linear in them).
 //
-// Design (one group of NE elements per block at porders 2-5; a persistent
-// form that loops over groups, below, at porders 1, 6, 7 and 8 in FP32):
-//   * the block copies the node permutations of the call's tables (prepared
-//     once per call from the caller's invAtoIJK / gmshAtoI/J/K, msod_tables.cu)
-//     into shared memory while its connec entries load; the 1-D derivative
-//     matrices are constant-bank operands (shared memory when S > 1);
-//   * connec is read coalesced along elements (it is element-fastest), node
-//     fields are gathered into a per-element (I,J,K) lattice in shared memory;
-//   * each thread owns one GLL line (S threads share a line at high order).
-//     Three passes (xi, eta, zeta) load the line's nodal values into
-//     registers once, form every differentiated product on the fly and apply
-//     the 1-D derivative matrix held in registers (sum factorisation).  The
-//     residual is linear in the iso-parametric derivatives, so each pass adds
-//     its direction's contribution -- through the He column of that direction
-//     and the point's own nodal values -- to seven per-point accumulators kept
-//     in shared memory;
-//   * the last pass multiplies by gpvol and scatter-adds with red.global.add.
-#include "msod_convec.cuh"
+// Pairwise form.  Along a line of direction d, with D its 1-D derivative matrix,
+// h = He(:,d) at the output point r, and for a point s of the line
+// U_s = h.u_s, Q_s = h.q_s, direction d's share of the bracket above at r is
+//
+//   4 mom_i = sum_s D_rs [ u_i,r (U_r rho_s + Q_s) + u_i,s (Q_r + rho_r U_s)
+//                        + q_i,s (U_r + U_s) + q_i,r U_s + 4 h_i p_s ]
+//   4 ener  = the same with u_i -> H, q_i -> rho H and without p
+//   2 mass  = sum_s D_rs [ U_r rho_s + Q_s + rho_r U_s ]
+//
+// (the metric is taken at r in every term, as the reference does, so nothing
+// else of the metric enters).  Writing every value at s as the value at r plus
+// a difference turns it into, with t = h.(u_s - u_r),
+//
+//   4 mom_i = sum_s D_rs [ (u_i,s - u_i,r)(Q_r + rho_r U_r + rho_r t) + (q_i,s - q_i,r)(2 U_r + t) ]
+//             + u_i,r S + 2 q_i,r div u + 4 h_i dp      (S = U_r drho + h.dq + rho_r div u)
+//   2 mass  = S
+//
+// with drho, dp, dq, div u the sums of D_rs times the differences, plus the row
+// sum of D (zero but for the table's rounding) times the bracket at s = r.
+// The 31 products of the bracket's own form, each differentiated in three
+// directions, become 12 multiply-adds per pair of points beside the ten
+// differences and six linear sums; no product field is formed; and since only
+// differences are summed, the constant part of every field, which a derivative
+// cancels, no longer leaves its rounding behind (momentum residual against 64
+// bits on 64^3 smooth fields: 8e-8 instead of 6e-6 relative).
+//
+// Design (one group of NE elements per block, one thread per GLL line,
+// msod_group.cuh):
+//   * one thread issues the bulk copies of the group's He and gpvol spans;
+//     meanwhile each thread gathers the points of its zeta line through connec,
+//     forms H and rho H once per point and stores the records (u, H), (q, rho H)
+//     and (rho, p) of its points to the shared-memory lattice;
+//   * three passes (zeta, xi, eta) evaluate the pairwise form along the lines of
+//     a direction, point after point of the line: the line's records sit in
+//     registers (the zeta pass has them from the gather), the derivative matrix
+//     is a constant-bank operand, and the five sums of a point (momentum,
+//     energy, mass) pass from one direction's thread to the next through
+//     shared memory;
+//   * the last pass applies gpvol and scatter-adds with red.global.add.
+#include <cuda_runtime.h>
+
+#include "msod_group.cuh"
 
 namespace msod {
 namespace {
 
-template <typename real, int P>
-__global__ void __launch_bounds__(ConvecGeom<real, P>::NT, convec_minb<real, P>())
-    convec_kernel(int nelem, int npoin, const int *__restrict__ connec, const real *__restrict__ He,
-                  const real *__restrict__ gpvol, const real *__restrict__ dlxigp_ip,
-                  const int *__restrict__ invAtoIJK, const int *__restrict__ AtoI,
-                  const int *__restrict__ AtoJ, const int *__restrict__ AtoK, const real *__restrict__ u,
-                  const real *__restrict__ q, const real *__restrict__ rho, const real *__restrict__ pr,
-                  const real *__restrict__ E, const TableScratch *__restrict__ tabs, real *__restrict__ Rmass,
-                  real *__restrict__ Rmom, real *__restrict__ Rener)
+// 1-D derivative matrices and their row sums of the current call, per porder
+// (copied from the per-call table area before the launch).
+__constant__ float c_CDf[MSOD_MAX_PORDER + 1][kTableDSMax];
+__constant__ double c_CDd[MSOD_MAX_PORDER + 1][kTableDSMax];
+template <typename real>
+__device__ __forceinline__ real cCD(int P, int i);
+template <>
+__device__ __forceinline__ float cCD<float>(int P, int i)
 {
-    using G = ConvecGeom<real, P>;
-    constexpr int Q = G::Q, N = G::N, QP = G::QP, ES = G::ES, NE = G::NE, NT = G::NT;
-    constexpr int NPL = NE * ES;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr bool STAGED = convec_staged<real>();
-    constexpr size_t HEB = ((size_t)NE * N * 9 * sizeof(real) + 31) / 16 * 16;
-    constexpr size_t GPB = ((size_t)NE * N * sizeof(real) + 31) / 16 * 16;
-    char *sHeB = reinterpret_cast<char *>(smem_raw);
-    char *sGpB = sHeB + HEB;
-    unsigned long long *sBar = reinterpret_cast<unsigned long long *>(sGpB + GPB);
-    real *sF = reinterpret_cast<real *>(smem_raw + convec_stage_bytes<real, P>());
-    real *sA = sF + NFIELD * NPL;
-    real *sD = sA + NACC * NPL;
-    int *sNode = reinterpret_cast<int *>(sD + 3 * Q * Q);
-    int *sPerm = sNode + NPL;
-    int *sLat = sPerm + N;
+    return c_CDf[P][i];
+}
+template <>
+__device__ __forceinline__ double cCD<double>(int P, int i)
+{
+    return c_CDd[P][i];
+}
 
-    const int tid = threadIdx.x;
-    const int e0 = blockIdx.x * NE;
-    // The compact pass when the call's tables allow it (uniform over the grid).
-    bool compact = false;
-    if constexpr (convec_compact_capable<real, P>()) compact = ldg(&tabs->eo_ok) != 0;
-    // The group's He and gpvol spans: bulk copies issued first, so that they
-    // land while the node fields are gathered.
-    const real *Hs = He, *Gs = gpvol;
-    if constexpr (STAGED) {
-        const int e1 = min(e0 + NE, nelem);
-        const SpanPlan ph(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(real));
-        const SpanPlan pg(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(real));
-        if (tid == 0) {
-            mbar_init(sBar, 1);
-            mbar_arrive_expect_tx(sBar, ph.bulk + pg.bulk);
-            ph.issue(sHeB, sBar);
-            pg.issue(sGpB, sBar);
-        } else if (tid >= 32 && tid < 38) {
-            ph.plain(sHeB, tid - 32);
-        } else if (tid >= 64 && tid < 70) {
-            pg.plain(sGpB, tid - 64);
+// Elements per block, threads per line, blocks per SM that the register budget
+// allows for, and the form of the passes, measured per porder (FP32, ms).
+// Whole warps of lines count most (5 x 25 lines at porder 4: 125 of 128
+// threads): on 64^3 porder-4 hexes 5 elements take 0.944 (1.044 before the pitch
+// search, where 4, with 100 of 128 threads, took 1.15, 6 1.17, 8 1.13, 9 1.10).  A fourth block per SM (12 bytes per point less
+// through kSlots, 128 registers) gains nothing: 1.04.
+template <typename real, int P>
+constexpr int convec_ne()
+{
+    constexpr int nf[9] = {0, 32, 16, 8, 5, 4, 2, 2, 2}, nd[9] = {0, 32, 14, 8, 5, 3, 2, 1, 1};
+    return sizeof(real) == 4 ? nf[P] : nd[P];
+}
+// Two threads share a line where one would spill (porder 8; FP64 from 7 up).
+// At lower porders they lose what the second load of the line costs (porder 4
+// 1.30, porder 3 1.01 against 0.71 on 80^3).
+template <typename real, int P>
+constexpr int convec_s()
+{
+    return P >= (sizeof(real) == 4 ? 8 : 7) ? 2 : 1;
+}
+template <typename real, int P>
+constexpr int convec_minb()
+{
+    constexpr int nb[9] = {0, 1, 1, 4, 3, 2, 2, 1, 1};
+    return sizeof(real) == 4 ? nb[P] : 1;
+}
+// All points of a line at once (the pairs' differences shared) or one point
+// after the other (fewer registers): porder 3 0.711 / 0.738, 4 0.944 / 1.05, 6
+// 1.052 / 1.149 (40^3), but 5 1.169 / 1.143 (51^3) and 7 0.855 / 0.786 (32^3),
+// where the sums of all points no longer fit beside the line.
+template <typename real, int P>
+constexpr bool convec_all_points()
+{
+    return sizeof(real) == 4 && P <= 6 && P != 5;
+}
+// The three directions as one copy of the pass with run-time strides (porders
+// 6 to 8, whose unrolled passes overrun the instruction cache: porder 6 1.052 /
+// 1.148) or unrolled (porder 4 0.944 / 1.05, porder 3 0.711 / 0.911).
+template <int P>
+constexpr bool convec_rolled()
+{
+    return P >= 6;
+}
+// Sums kept in the spent part of the He records (ConvecShared::kSlots): where
+// it makes room for another block (porder 7: 0.786 / 0.860; porder 5 1.143 /
+// 1.155); elsewhere the records' bank conflicts cost more than the room gives.
+template <typename real, int P>
+constexpr bool convec_slots()
+{
+    return sizeof(real) == 4 && (P == 5 || P == 7);
+}
+template <typename real, int P>
+using ConvecGeom = GroupGeom<real, P, convec_ne<real, P>(), convec_s<real, P>()>;
+
+// Shared memory of a block.
+template <class G>
+struct ConvecShared {
+    using real = typename G::real;
+    static constexpr size_t kW = G::HEB + G::GPB + 16;
+    static constexpr size_t kV = kW + G::NREC * sizeof(Four<real>);
+    static constexpr size_t kA = kV + G::NREC * sizeof(Four<real>);
+    static constexpr bool kSlots = convec_slots<real, G::P>();
+    static constexpr size_t kZ = kA + G::NREC * (kSlots ? sizeof(Two<real>) : sizeof(Four<real>));
+    static constexpr size_t kM = kZ + G::NREC * sizeof(real);
+    static constexpr size_t kNode = kM + G::NREC * sizeof(real);
+    static constexpr size_t kPerm = kNode + (kSlots ? 0 : G::NREC * sizeof(int));
+    static constexpr size_t kBytes = kPerm + G::N * sizeof(int);
+    unsigned char *base;
+    __device__ __forceinline__ unsigned long long *bar() const
+    {
+        return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
+    }
+    __device__ __forceinline__ Four<real> *W() const { return reinterpret_cast<Four<real> *>(base + kW); }  // u, H
+    __device__ __forceinline__ Four<real> *V() const { return reinterpret_cast<Four<real> *>(base + kV); }  // q, p
+    __device__ __forceinline__ Four<real> *A() const { return reinterpret_cast<Four<real> *>(base + kA); }  // 4 mom, 4 ener
+    __device__ __forceinline__ real *Z() const { return reinterpret_cast<real *>(base + kZ); }              // rho
+    __device__ __forceinline__ real *M() const { return reinterpret_cast<real *>(base + kM); }              // 2 mass
+    __device__ __forceinline__ int *node() const { return reinterpret_cast<int *>(base + kNode); }
+    // The sums of a point (record o, its He record at he) between the passes.
+    // kSlots: the zeta column of a point's He record is read in the zeta pass
+    // only, by the thread that owns the point's zeta line; from then on it holds
+    // the mass and energy sums and the point's node.
+    __device__ __forceinline__ void put(int o, real *he, const Two<real> &a, const Two<real> &b, real m) const
+    {
+        if constexpr (kSlots) {
+            reinterpret_cast<Two<real> *>(base + kA)[o] = a;
+            M()[o] = b.x;
+            he[6] = b.y;
+            he[7] = m;
+        } else {
+            Four<real> p;
+            p.a = a;
+            p.b = b;
+            A()[o] = p;
+            M()[o] = m;
         }
-        Hs = reinterpret_cast<const real *>(sHeB + ph.shift);
-        Gs = reinterpret_cast<const real *>(sGpB + pg.shift);
-    } else if (CONVEC_PREFETCH != 0 && tid == 0) {
-        // The group's He and gpvol spans into L2 while the node fields are
-        // gathered: the passes' first He loads then hit L2.  (Also
-        // prefetching the spans of the block a wave later -- the grid's
-        // resident blocks on -- measured slower: 1.489 against 1.468 ms.)
-        const int e1 = min(e0 + NE, nelem);
-        prefetch_span_l2(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(real));
-        prefetch_span_l2(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(real));
     }
-    // Node ids of the group's elements (connec is element-fastest), loaded
-    // while the per-call tables are copied into shared memory.
-    constexpr int IPT = (NE * N + NT - 1) / NT;
-    int ids[IPT];
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = tid + k * NT;
-        const int el = i % NE, a = i / NE, e = e0 + el;
-        ids[k] = (i < NE * N && e < nelem) ? ldg(connec + (size_t)a * nelem + e) - 1 : -1;
-    }
-    for (int i = tid; i < N; i += NT) {
-        sPerm[i] = tabs->perm[i];
-        sLat[i] = tabs->lat[i];
-    }
-    if (G::S > 1)
-        for (int i = tid; i < 3 * Q * Q; i += NT) sD[i] = table_D<real>(tabs)[i];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = tid + k * NT;
-        if (i < NE * N) {
-            const int v = ids[k];
-            sNode[(i % NE) * ES + sLat[i / NE]] = (v >= 0 && v < npoin) ? v : -1;
+    __device__ __forceinline__ void add(int o, const real *he, Two<real> &a, Two<real> &b, real &m) const
+    {
+        if constexpr (kSlots) {
+            a = add2(a, reinterpret_cast<const Two<real> *>(base + kA)[o]);
+            b = add2(b, two(M()[o], he[6]));
+            m += he[7];
+        } else {
+            const Four<real> p = A()[o];
+            a = add2(a, p.a);
+            b = add2(b, p.b);
+            m += M()[o];
         }
     }
-    __syncthreads();
-    // Gather node fields into the lattice: asynchronous copies, all of a
-    // thread's in flight at once (a missing node reads as zeros).
-    const size_t np = (size_t)npoin;
-    for (int i = tid; i < NE * N; i += NT) {
-        const int el = i / N, l = i - el * N;
-        const int I = l % Q, J = (l / Q) % Q, K = l / (Q * Q);
-        const int o = el * ES + (K * Q + J) * QP + I;
-        const int p = sNode[o];
-        const bool ok = p >= 0;
-        const size_t pp = ok ? (size_t)p : 0;
-        cp_async_elem(sF + F_RHO * NPL + o, rho + pp, ok);
-        cp_async_elem(sF + F_P * NPL + o, pr + pp, ok);
-        cp_async_elem(sF + F_E * NPL + o, E + pp, ok);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            cp_async_elem(sF + (F_U0 + c) * NPL + o, u + c * np + pp, ok);
-            cp_async_elem(sF + (F_Q0 + c) * NPL + o, q + c * np + pp, ok);
-        }
+    __device__ __forceinline__ int node_at(int o, const real *he) const
+    {
+        if constexpr (kSlots)
+            return __float_as_int(he[8]);
+        else
+            return node()[o];
     }
-    cp_async_commit();
-    cp_async_wait_all();
-    if constexpr (STAGED) {
-        // Bounded wait for the bulk copies; every thread learns the outcome.
-        const bool ok = mbar_wait(sBar, 0);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) report_wait_fault(tabs);
-            return;
-        }
+    __device__ __forceinline__ int *perm() const { return reinterpret_cast<int *>(base + kPerm); }
+};
+
+// The records of one line.
+template <class G>
+struct ConvecLine {
+    Four<typename G::real> w[G::Q], v[G::Q];  // (u, H), (q, rho H)
+    Two<typename G::real> z[G::Q];            // (rho, p)
+    __device__ __forceinline__ void set(int s, const Four<typename G::real> &uH, const Four<typename G::real> &qp,
+                                        typename G::real rho)
+    {
+        w[s] = uH;
+        v[s].a = qp.a;
+        v[s].b = two(qp.b.x, rho * uH.b.y);
+        z[s] = two(rho, qp.b.y);
+    }
+};
+
+// One direction of a pass: the line's record and lattice strides, and where its
+// coefficients lie.
+template <class G>
+struct ConvecDir {
+    int dir, base, step, lat, lstep;
+    bool first, last;
+    __device__ __forceinline__ ConvecDir(const GroupThread<G> &t, int ip)
+    {
+        dir = ip == 0 ? 2 : ip - 1;
+        first = ip == 0;
+        last = ip == 2;
+        step = dir == 0 ? 1 : (dir == 1 ? G::RP : G::PP);
+        lstep = dir == 0 ? 1 : (dir == 1 ? G::Q : G::L);
+        base = t.rec0(dir);
+        lat = t.lat0(dir);
+    }
+};
+// Coefficient i of direction dir; SAME: the three directions share one matrix
+// (as every table of the reference does), and the coefficient is an immediate
+// operand from the constant bank.
+template <class G, bool SAME>
+__device__ __forceinline__ typename G::real convec_D(int dir, int i)
+{
+    return cCD<typename G::real>(G::P, SAME ? i : dir * G::Q * G::Q + i);
+}
+template <class G, bool SAME>
+__device__ __forceinline__ typename G::real convec_rowsum(int dir, int r)
+{
+    return cCD<typename G::real>(G::P, 3 * G::Q * G::Q + (SAME ? r : dir * G::Q + r));
+}
+
+template <class G>
+__device__ __forceinline__ void convec_finish(const ConvecDir<G> &d, const ConvecShared<G> &sm,
+                                              const GroupMetric<G> &gm, int el, int o, int pt, int node0,
+                                              Two<typename G::real> a, Two<typename G::real> b, typename G::real m,
+                                              int npoin, typename G::real *__restrict__ Rmass,
+                                              typename G::real *__restrict__ Rmom,
+                                              typename G::real *__restrict__ Rener)
+{
+    using real = typename G::real;
+    real *he = gm.he(el, pt);
+    if (!d.first) sm.add(o, he, a, b, m);
+    if (!d.last) {
+        sm.put(o, he, a, b, m);
+        if constexpr (ConvecShared<G>::kSlots)
+            if (d.first) he[8] = __int_as_float(node0);
     } else {
-        __syncthreads();
-    }
-    if constexpr (convec_compact_capable<real, P>()) {
-        if (compact) {
-#if CONVEC_RTDIR
-#pragma unroll 1
-#else
-#pragma unroll
-#endif
-            for (int dir = 0; dir < 3; ++dir) {
-                if (dir > 0) __syncthreads();
-                convec_pass_compact<P>(dir, sF, sA, sNode, sPerm, He, gpvol, e0, nelem, npoin, Rmass, Rmom, Rener);
-            }
-            return;
+        const int node = sm.node_at(o, he);
+        if (node >= 0) {
+            const real g = *gm.vol(el, pt), g4 = (real)0.25 * g;
+            red_add(Rmass + node, (real)0.5 * g * m);
+            red_add(Rmom + node, g4 * a.x);
+            red_add(Rmom + (size_t)npoin + node, g4 * a.y);
+            red_add(Rmom + 2 * (size_t)npoin + node, g4 * b.x);
+            red_add(Rener + node, g4 * b.y);
         }
     }
-    convec_dir<real, P, 0, STAGED>(sF, sA, sD, sNode, sPerm, Hs, Gs, e0, nelem, npoin, Rmass, Rmom, Rener);
-    __syncthreads();
-    convec_dir<real, P, 1, STAGED>(sF, sA, sD, sNode, sPerm, Hs, Gs, e0, nelem, npoin, Rmass, Rmom, Rener);
-    __syncthreads();
-    convec_dir<real, P, 2, STAGED>(sF, sA, sD, sNode, sPerm, Hs, Gs, e0, nelem, npoin, Rmass, Rmom, Rener);
 }
 
-// Persistent form: blocks loop over element groups, the block's tables are
-// copied once and a group's He and gpvol spans are prefetched into L2 a group
-// ahead.  FP32 at the porders whose bit is set in CONVEC_PERSIST_PORDERS.
-// Measured (16.8 M-node meshes, CUDA events, persistent against one-shot):
-// porder 1 4.68 / 4.96 ms, 6 1.73 / 1.77, 7 1.53 / 1.72, 8 2.33 / 2.48 (few
-// elements per block, or very many blocks, and the one-shot blocks' prologue
-// and first He loads weigh on little work each); porder 2 2.40 / 2.13, 3
-// 1.65 / 1.52, 4 1.78 / 1.47 (a 264-byte spill at 128 registers; 1.54 ms at
-// 168 registers, three blocks per SM), 5 1.73 / 1.53.
-// CONVEC_PERSIST: 1 = the next group's node ids load after the passes, 2 =
-// during them (porder 7: 1.58 ms).
-#ifndef CONVEC_PERSIST_PORDERS
-#define CONVEC_PERSIST_PORDERS ((1 << 1) | (1 << 6) | (1 << 7) | (1 << 8))
-#endif
-#ifndef CONVEC_PERSIST
-#define CONVEC_PERSIST 1
-#endif
-template <typename real, int P>
-constexpr bool convec_persist()
+// Points R0 .. R0+R-1 of a line, one after the other.
+template <class G, bool SAME, int SEG>
+__device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const GroupThread<G> &t, const ConvecDir<G> &d,
+                                              const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                              const int (&id)[G::R], int npoin,
+                                              typename G::real *__restrict__ Rmass,
+                                              typename G::real *__restrict__ Rmom,
+                                              typename G::real *__restrict__ Rener)
 {
-    return sizeof(real) == 4 && ((CONVEC_PERSIST_PORDERS >> P) & 1) != 0 && !convec_staged<real>();
+    using real = typename G::real;
+    using R2 = Two<real>;
+    constexpr int Q = G::Q, R0 = SEG * G::R, R1 = R0 + G::R < Q ? R0 + G::R : Q;
+    constexpr real k2 = (real)2, k3 = (real)3, k4 = (real)4;
+#pragma unroll
+    for (int r = R0; r < R1; ++r) {
+        const int pt = sm.perm()[d.lat + r * d.lstep];
+        const real *hp = gm.he(t.el, pt) + d.dir * 3;
+        const real h0 = hp[0], h1 = hp[1], h2 = hp[2];
+        const Four<real> wr = ln.w[r], vr = ln.v[r];
+        const real rr = ln.z[r].x;
+        const real U = fma(wr.b.x, h2, fma(wr.a.y, h1, wr.a.x * h0));
+        const real Qc = fma(vr.b.x, h2, fma(vr.a.y, h1, vr.a.x * h0));
+        const real X0 = U + U, Y0 = fma(rr, U, Qc);
+        R2 A = two((real)0, (real)0), B = A, dz = A, dq = A;  // momentum 1-2; momentum 3, energy; drho, dp; dq 1-2
+        real dq3 = (real)0, divu = (real)0;
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            if (s == r) continue;
+            const real D = convec_D<G, SAME>(d.dir, r * Q + s);
+            const R2 D2 = two(D, D);
+            const R2 wa = sub2(ln.w[s].a, wr.a), wb = sub2(ln.w[s].b, wr.b);
+            const R2 va = sub2(ln.v[s].a, vr.a), vb = sub2(ln.v[s].b, vr.b);
+            const R2 dzs = sub2(ln.z[s], ln.z[r]);
+            const real tt = fma(wb.x, h2, fma(wa.y, h1, wa.x * h0));
+            const real X = D * (X0 + tt), Y = D * fma(rr, tt, Y0);
+            A = fma2(va, two(X, X), fma2(wa, two(Y, Y), A));
+            B = fma2(vb, two(X, X), fma2(wb, two(Y, Y), B));
+            dz = fma2(D2, dzs, dz);
+            dq = fma2(D2, va, dq);
+            dq3 = fma(D, vb.x, dq3);
+            divu = fma(D, tt, divu);
+        }
+        const real sg = convec_rowsum<G, SAME>(d.dir, r);
+        const real divq = fma(dq3, h2, fma(dq.y, h1, dq.x * h0));
+        const real S = fma(rr, divu, fma(U, dz.x, divq));
+        const real cw = fma(k2 * sg, Y0, S), cv = fma(k3 * sg, U, k2 * divu);
+        const real dp = k4 * fma(sg, ln.z[r].y, dz.y);
+        A = fma2(wr.a, two(cw, cw), fma2(vr.a, two(cv, cv), A));
+        B = fma2(wr.b, two(cw, cw), fma2(vr.b, two(cv, cv), B));
+        A = fma2(two(h0, h1), two(dp, dp), A);
+        B.x = fma(h2, dp, B.x);
+        convec_finish<G>(d, sm, gm, t.el, d.base + r * d.step, pt, id[r - R0], A, B, fma(sg, fma(rr, U, Y0), S), npoin, Rmass, Rmom,
+                         Rener);
+    }
 }
-template <typename real, int P>
-__global__ void __launch_bounds__(ConvecGeom<real, P>::NT, convec_minb<real, P>())
-    convec_kernel_persist(int nelem, int npoin, int ngroups, const int *__restrict__ connec,
-                          const real *__restrict__ He, const real *__restrict__ gpvol, const real *__restrict__ u,
-                          const real *__restrict__ q, const real *__restrict__ rho, const real *__restrict__ pr,
-                          const real *__restrict__ E, const TableScratch *__restrict__ tabs, real *__restrict__ Rmass,
-                          real *__restrict__ Rmom, real *__restrict__ Rener)
+
+// All points of a line at once: the differences of a pair of points serve both
+// of its rows.
+template <class G, bool SAME>
+__device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const GroupThread<G> &t, const ConvecDir<G> &d,
+                                             const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                              const int (&id)[G::R], int npoin,
+                                             typename G::real *__restrict__ Rmass, typename G::real *__restrict__ Rmom,
+                                             typename G::real *__restrict__ Rener)
 {
-    using G = ConvecGeom<real, P>;
-    constexpr int Q = G::Q, N = G::N, QP = G::QP, ES = G::ES, NE = G::NE, NT = G::NT;
-    constexpr int NPL = NE * ES;
-    constexpr int IPT = (NE * N + NT - 1) / NT;
+    using real = typename G::real;
+    using R2 = Two<real>;
+    constexpr int Q = G::Q;
+    constexpr real k2 = (real)2, k3 = (real)3, k4 = (real)4;
+    const R2 zero = two((real)0, (real)0);
+    int pt[Q];
+    real h[Q][3], U[Q], Y0[Q], dq3[Q], divu[Q];
+    R2 A[Q], B[Q], dz[Q], dq[Q];
+#pragma unroll
+    for (int r = 0; r < Q; ++r) pt[r] = sm.perm()[d.lat + r * d.lstep];
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+        const real *hp = gm.he(t.el, pt[r]) + d.dir * 3;
+        h[r][0] = hp[0];
+        h[r][1] = hp[1];
+        h[r][2] = hp[2];
+    }
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+        U[r] = fma(ln.w[r].b.x, h[r][2], fma(ln.w[r].a.y, h[r][1], ln.w[r].a.x * h[r][0]));
+        Y0[r] = fma(ln.z[r].x, U[r], fma(ln.v[r].b.x, h[r][2], fma(ln.v[r].a.y, h[r][1], ln.v[r].a.x * h[r][0])));
+        A[r] = B[r] = dz[r] = dq[r] = zero;
+        dq3[r] = divu[r] = (real)0;
+    }
+#pragma unroll
+    for (int r = 0; r < Q; ++r)
+#pragma unroll
+        for (int s = r + 1; s < Q; ++s) {
+            const R2 wa = sub2(ln.w[s].a, ln.w[r].a), wb = sub2(ln.w[s].b, ln.w[r].b);
+            const R2 va = sub2(ln.v[s].a, ln.v[r].a), vb = sub2(ln.v[s].b, ln.v[r].b);
+            const R2 zz = sub2(ln.z[s], ln.z[r]);
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                // Row m, its partner's values minus its own = sign * the differences.
+                const int m = side ? s : r, o = side ? r : s;
+                const real D0 = convec_D<G, SAME>(d.dir, m * Q + o), D = side ? -D0 : D0;
+                const real tt = fma(wb.x, h[m][2], fma(wa.y, h[m][1], wa.x * h[m][0]));
+                const real x0 = U[m] + U[m];
+                const real X = D * (side ? x0 - tt : x0 + tt), Y = D * fma(side ? -ln.z[m].x : ln.z[m].x, tt, Y0[m]);
+                A[m] = fma2(va, two(X, X), fma2(wa, two(Y, Y), A[m]));
+                B[m] = fma2(vb, two(X, X), fma2(wb, two(Y, Y), B[m]));
+                dz[m] = fma2(two(D, D), zz, dz[m]);
+                dq[m] = fma2(two(D, D), va, dq[m]);
+                dq3[m] = fma(D, vb.x, dq3[m]);
+                divu[m] = fma(D, tt, divu[m]);
+            }
+        }
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+        const real rr = ln.z[r].x, Ur = U[r];
+        const real sg = convec_rowsum<G, SAME>(d.dir, r);
+        const real divq = fma(dq3[r], h[r][2], fma(dq[r].y, h[r][1], dq[r].x * h[r][0]));
+        const real S = fma(rr, divu[r], fma(Ur, dz[r].x, divq));
+        const real cw = fma(k2 * sg, Y0[r], S), cv = fma(k3 * sg, Ur, k2 * divu[r]);
+        const real dp = k4 * fma(sg, ln.z[r].y, dz[r].y);
+        R2 a = fma2(ln.w[r].a, two(cw, cw), fma2(ln.v[r].a, two(cv, cv), A[r]));
+        R2 b = fma2(ln.w[r].b, two(cw, cw), fma2(ln.v[r].b, two(cv, cv), B[r]));
+        a = fma2(two(h[r][0], h[r][1]), two(dp, dp), a);
+        b.x = fma(h[r][2], dp, b.x);
+        convec_finish<G>(d, sm, gm, t.el, d.base + r * d.step, pt[r], id[r], a, b, fma(sg, fma(rr, Ur, Y0[r]), S), npoin, Rmass,
+                         Rmom, Rener);
+    }
+}
+
+template <class G, bool SAME>
+__device__ __forceinline__ void convec_pass(ConvecLine<G> &ln, const GroupThread<G> &t, int ip,
+                                            const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                              const int (&id)[G::R], int npoin,
+                                            typename G::real *__restrict__ Rmass,
+                                            typename G::real *__restrict__ Rmom,
+                                            typename G::real *__restrict__ Rener)
+{
+    if (!t.active) return;
+    const ConvecDir<G> d(t, ip);
+    if (!d.first || G::S > 1) {
+#pragma unroll
+        for (int s = 0; s < G::Q; ++s) {
+            const int o = d.base + s * d.step;
+            ln.set(s, sm.W()[o], sm.V()[o], sm.Z()[o]);
+        }
+    }
+    if constexpr (G::S == 1 && convec_all_points<typename G::real, G::P>()) {
+        convec_pairs<G, SAME>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+    } else if constexpr (G::S == 1) {
+        convec_points<G, SAME, 0>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+    } else {
+        if (t.seg == 0)
+            convec_points<G, SAME, 0>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        else
+            convec_points<G, SAME, 1>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+    }
+}
+
+template <class G, int MINB>
+__global__ void __launch_bounds__(G::NT, MINB)
+    convec_kernel(int nelem, int npoin, int ngroups, const int *__restrict__ connec,
+                  const typename G::real *__restrict__ He, const typename G::real *__restrict__ gpvol,
+                  const typename G::real *__restrict__ u, const typename G::real *__restrict__ q,
+                  const typename G::real *__restrict__ rho, const typename G::real *__restrict__ pr,
+                  const typename G::real *__restrict__ E, const TableScratch *__restrict__ tabs,
+                  typename G::real *__restrict__ Rmass, typename G::real *__restrict__ Rmom,
+                  typename G::real *__restrict__ Rener)
+{
+    using real = typename G::real;
+    constexpr int Q = G::Q, N = G::N, R = G::R;
+    static_assert(G::S <= 2, "one or two segments per line");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    real *sF = reinterpret_cast<real *>(smem_raw);
-    real *sA = sF + NFIELD * NPL;
-    real *sD = sA + NACC * NPL;
-    int *sNode = reinterpret_cast<int *>(sD + 3 * Q * Q);
-    int *sPerm = sNode + NPL;
-    int *sLat = sPerm + N;
+    const ConvecShared<G> sm{smem_raw};
     const int tid = threadIdx.x;
-    bool compact = false;
-    if constexpr (convec_compact_capable<real, P>()) compact = ldg(&tabs->eo_ok) != 0;
-    for (int i = tid; i < N; i += NT) {
-        sPerm[i] = tabs->perm[i];
-        sLat[i] = tabs->lat[i];
+    const GroupThread<G> t(tid);
+    const int r0 = t.seg * R;
+    const int e0 = blockIdx.x * G::NE;
+    const GroupMetric<G> gm(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);
+    for (int i = tid; i < N; i += G::NT) sm.perm()[i] = ldg(&tabs->perm[i]);
+    ConvecLine<G> ln;
+    int id[R];  // the nodes of the thread's points of its zeta line (-1: none)
+    {
+        const int e = e0 + t.el;
+        const size_t np = (size_t)npoin;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const bool ok = t.active && e < nelem && (R * G::S == Q || r0 + k < Q);
+            const int row = ok ? ldg(&tabs->perm[t.template lat<2>(r0 + k)]) : 0;
+            const int v = ok ? ldg(connec + (size_t)row * nelem + e) - 1 : -1;
+            id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
+        }
+        real f[R][9];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const bool ok = id[k] >= 0;  // a missing node reads as zeros
+            const size_t p = ok ? (size_t)id[k] : 0;
+            f[k][0] = ok ? ldg(u + p) : (real)0;
+            f[k][1] = ok ? ldg(u + np + p) : (real)0;
+            f[k][2] = ok ? ldg(u + 2 * np + p) : (real)0;
+            f[k][3] = ok ? ldg(E + p) : (real)0;
+            f[k][4] = ok ? ldg(q + p) : (real)0;
+            f[k][5] = ok ? ldg(q + np + p) : (real)0;
+            f[k][6] = ok ? ldg(q + 2 * np + p) : (real)0;
+            f[k][7] = ok ? ldg(rho + p) : (real)0;
+            f[k][8] = ok ? ldg(pr + p) : (real)0;
+        }
+        const int base = t.rec0(2);
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const real H = f[k][3] + (real)0.5 * fma(f[k][2], f[k][2], fma(f[k][1], f[k][1], f[k][0] * f[k][0]));
+            Four<real> w, v;
+            w.a = two(f[k][0], f[k][1]);
+            w.b = two(f[k][2], H);
+            v.a = two(f[k][4], f[k][5]);
+            v.b = two(f[k][6], f[k][8]);
+            if (t.active && (R * G::S == Q || r0 + k < Q)) {
+                const int o = base + (r0 + k) * G::template step<2>();
+                sm.W()[o] = w;
+                sm.V()[o] = v;
+                sm.Z()[o] = f[k][7];
+                if constexpr (!ConvecShared<G>::kSlots) sm.node()[o] = id[k];
+            }
+            if (G::S == 1) ln.set(k, w, v, f[k][7]);
+        }
     }
-    if (G::S > 1)
-        for (int i = tid; i < 3 * Q * Q; i += NT) sD[i] = table_D<real>(tabs)[i];
-    auto load_ids = [&](int g, int(&ids)[IPT]) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int i = tid + k * NT;
-            const int el = i % NE, a = i / NE, e = g * NE + el;
-            ids[k] = (i < NE * N && e < nelem) ? ldg(connec + (size_t)a * nelem + e) - 1 : -1;
+    __syncthreads();
+    // Bounded wait for the bulk copies; a wait that ran out is reported and
+    // nothing is assembled (every thread learns it at the barrier below).
+    const bool ok = gm.wait(sm.bar());
+    const bool same = ldg(&tabs->same_dirs) != 0;  // uniform over the grid
+    auto pass = [&](int ip) {
+        if (same)
+            convec_pass<G, true>(ln, t, ip, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        else
+            convec_pass<G, false>(ln, t, ip, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        if (ip < 2 && __syncthreads_or(!ok)) {
+            if (tid == 0) report_wait_fault(tabs);
+            return false;
         }
+        return true;
     };
-    auto prefetch_group = [&](int g) {
-        if (CONVEC_PREFETCH != 0 && tid == 0 && g < ngroups) {
-            const int e0 = g * NE, e1 = min(e0 + NE, nelem);
-            prefetch_span_l2(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(real));
-            prefetch_span_l2(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(real));
-        }
-    };
-    int g = blockIdx.x;
-    const int stride = gridDim.x;
-    prefetch_group(g);
-    int ids[IPT];
-    load_ids(g, ids);
-    __syncthreads();  // sLat ready
-    const size_t np = (size_t)npoin;
-    for (;;) {
-        const int e0 = g * NE;
+    if constexpr (convec_rolled<G::P>()) {
+#pragma unroll 1
+        for (int ip = 0; ip < 3; ++ip)
+            if (!pass(ip)) return;
+    } else {
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int i = tid + k * NT;
-            if (i < NE * N) {
-                const int v = ids[k];
-                sNode[(i % NE) * ES + sLat[i / NE]] = (v >= 0 && v < npoin) ? v : -1;
-            }
-        }
-        __syncthreads();
-        for (int i = tid; i < NE * N; i += NT) {
-            const int el = i / N, l = i - el * N;
-            const int I = l % Q, J = (l / Q) % Q, K = l / (Q * Q);
-            const int o = el * ES + (K * Q + J) * QP + I;
-            const int p = sNode[o];
-            const bool ok = p >= 0;
-            const size_t pp = ok ? (size_t)p : 0;
-            cp_async_elem(sF + F_RHO * NPL + o, rho + pp, ok);
-            cp_async_elem(sF + F_P * NPL + o, pr + pp, ok);
-            cp_async_elem(sF + F_E * NPL + o, E + pp, ok);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                cp_async_elem(sF + (F_U0 + c) * NPL + o, u + c * np + pp, ok);
-                cp_async_elem(sF + (F_Q0 + c) * NPL + o, q + c * np + pp, ok);
-            }
-        }
-        cp_async_commit();
-        const int gn = g + stride;
-        prefetch_group(gn);
-        if (CONVEC_PERSIST == 2 && gn < ngroups) load_ids(gn, ids);
-        cp_async_wait_all();
-        __syncthreads();
-        bool done = false;
-        if constexpr (convec_compact_capable<real, P>()) {
-            if (compact) {
-#pragma unroll
-                for (int dir = 0; dir < 3; ++dir) {
-                    if (dir > 0) __syncthreads();
-                    convec_pass_compact<P>(dir, sF, sA, sNode, sPerm, He, gpvol, e0, nelem, npoin, Rmass, Rmom,
-                                           Rener);
-                }
-                done = true;
-            }
-        }
-        if (!done) {
-            convec_dir<real, P, 0, false>(sF, sA, sD, sNode, sPerm, He, gpvol, e0, nelem, npoin, Rmass, Rmom, Rener);
-            __syncthreads();
-            convec_dir<real, P, 1, false>(sF, sA, sD, sNode, sPerm, He, gpvol, e0, nelem, npoin, Rmass, Rmom, Rener);
-            __syncthreads();
-            convec_dir<real, P, 2, false>(sF, sA, sD, sNode, sPerm, He, gpvol, e0, nelem, npoin, Rmass, Rmom, Rener);
-        }
-        if (gn >= ngroups) break;
-        if (CONVEC_PERSIST != 2) load_ids(gn, ids);
-        g = gn;
-        __syncthreads();  // the passes are done with sNode and the lattice
+        for (int ip = 0; ip < 3; ++ip)
+            if (!pass(ip)) return;
     }
-}
-
-template <typename real, int P>
-constexpr size_t convec_smem()
-{
-    using G = ConvecGeom<real, P>;
-    return convec_stage_bytes<real, P>() + (size_t)(NFIELD + NACC) * G::NE * G::ES * sizeof(real) +
-           3 * G::Q * G::Q * sizeof(real) + (size_t)(G::NE * G::ES + 2 * G::N) * sizeof(int);
 }
 
 template <typename real, int P>
 cudaError_t launch_convec_p(const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st)
 {
     using G = ConvecGeom<real, P>;
-    constexpr size_t smem = convec_smem<real, P>();
+    constexpr size_t smem = ConvecShared<G>::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    cudaError_t err = cudaFuncSetAttribute(convec_kernel<real, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
     if (!tabs) return cudaErrorInvalidValue;
-    if (G::S == 1) {
-        if (sizeof(real) == 4)
-            err = cudaMemcpyToSymbolAsync(c_CDf, table_D<float>(tabs), sizeof(float) * 3 * G::Q * G::Q,
-                                          sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
-        else
-            err = cudaMemcpyToSymbolAsync(c_CDd, table_D<double>(tabs), sizeof(double) * 3 * G::Q * G::Q,
-                                          sizeof(double) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
-        if (err != cudaSuccess) return err;
-        if (convec_compact_capable<real, P>()) {
-            err = cudaMemcpyToSymbolAsync(c_CEO, tabs->EO, sizeof(float) * kTableEOMax, sizeof(float) * kTableEOMax * P,
-                                          cudaMemcpyDeviceToDevice, st);
-            if (err == cudaSuccess)
-                err = cudaMemcpyToSymbolAsync(c_CEOp, tabs->EOp, sizeof(float) * kTableEOMax,
-                                              sizeof(float) * kTableEOMax * P, cudaMemcpyDeviceToDevice, st);
-            if (err != cudaSuccess) return err;
-        }
-        if (convec_packed<real, P>()) {
-            constexpr int H = (G::Q + 1) / 2;
-            err = cudaMemcpyToSymbolAsync(c_CDp, tabs->Dp, sizeof(float2) * 3 * G::Q * H,
-                                          sizeof(float2) * (kTableDPairMax / 2) * P, cudaMemcpyDeviceToDevice, st);
-            if (err != cudaSuccess) return err;
-        }
-    }
-    if constexpr (convec_persist<real, P>()) {
-        auto kern = convec_kernel_persist<real, P>;
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) return err;
-        const int ngroups = (a.nelem + G::NE - 1) / G::NE;
-        const int pgrid = persistent_grid(kern, G::NT, smem, ngroups);
-        if (pgrid <= 0) return cudaErrorInvalidConfiguration;
-        kern<<<pgrid, G::NT, smem, st>>>(a.nelem, a.npoin, ngroups, a.connec, a.He, a.gpvol, a.u, a.q, a.rho, a.pr,
-                                         a.E, tabs, a.Rmass, a.Rmom, a.Rener);
-        return cudaGetLastError();
-    }
-    const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
-    convec_kernel<real, P><<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.dlxigp_ip,
-                                                      a.invAtoIJK, a.AtoI, a.AtoJ, a.AtoK, a.u, a.q, a.rho,
-                                                      a.pr, a.E, tabs, a.Rmass, a.Rmom, a.Rener);
+    auto kern = convec_kernel<G, convec_minb<real, P>()>;
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    constexpr size_t nb = sizeof(real) * (3 * G::Q * G::Q + 3 * G::Q), off = sizeof(real) * kTableDSMax * P;
+    if (sizeof(real) == 4)
+        err = cudaMemcpyToSymbolAsync(c_CDf, tabs->Df, nb, off, cudaMemcpyDeviceToDevice, st);
+    else
+        err = cudaMemcpyToSymbolAsync(c_CDd, tabs->Dd, nb, off, cudaMemcpyDeviceToDevice, st);
+    if (err != cudaSuccess) return err;
+    const int ngroups = (a.nelem + G::NE - 1) / G::NE;
+    kern<<<ngroups, G::NT, smem, st>>>(a.nelem, a.npoin, ngroups, a.connec, a.He, a.gpvol, a.u, a.q, a.rho, a.pr, a.E,
+                                    tabs, a.Rmass, a.Rmom, a.Rener);
     return cudaGetLastError();
 }
 

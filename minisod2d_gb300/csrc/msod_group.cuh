@@ -1,0 +1,241 @@
+// msod_group.cuh -- element groups for the line-parallel hex kernels: the
+// thread-to-line map, the shared-memory lattice of vector records, the bulk
+// staging of He and gpvol, and pairwise (f32x2) arithmetic.
+//
+// What bounds these kernels is the L1 / shared-memory pipe (the wavefronts of
+// every load, store and reduction of an SM) beside FP32 issue, so the layout
+// is chosen by wavefronts per element point:
+//   * a block takes NE consecutive elements, and the lanes of a warp run along
+//     the elements first.  connec, mu_e and mu_sgs are element-fastest, and on
+//     meshes numbered along x the same local node of consecutive elements, for
+//     neighbouring local nodes, fills whole sectors: a gather or reduction of
+//     a node field touches 1-3 cache lines per warp, where lanes that run over
+//     one element's lattice touch seven or eight;
+//   * He and gpvol of a group are contiguous (He(3,3,ngaus,nelem)): one bulk
+//     copy each brings them to shared memory.  Read by the line threads from
+//     global memory, a point's three He values cost one L1 tag lookup per lane
+//     and value (9 x ~28 cycles per warp and point), from shared memory ~2
+//     wavefronts each;
+//   * node fields are stored as 16-byte records, so a point takes three loads.
+//     With lanes along elements the records of an 8-lane phase differ by
+//     multiples of the element stride ES: ES is padded so that they, and the
+//     lines beside them, fall on distinct banks.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "msod_device.cuh"
+#include "msod_kernels.h"
+
+namespace msod {
+namespace {
+
+// ---- pairs ---------------------------------------------------------------
+template <typename real>
+struct Pair;
+template <>
+struct Pair<float> {
+    using T = float2;
+};
+template <>
+struct Pair<double> {
+    using T = double2;
+};
+template <typename real>
+using Two = typename Pair<real>::T;
+
+__device__ __forceinline__ float2 two(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 two(double a, double b) { return make_double2(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c)
+{
+    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    return __fadd2_rn(a, make_float2(-b.x, -b.y));
+}
+__device__ __forceinline__ double2 sub2(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+
+// Four reals of one shared-memory record.
+template <typename real>
+struct alignas(16) Four {
+    Two<real> a, b;
+};
+
+// ---- geometry ------------------------------------------------------------
+// Pitches of the record lattice, by porder and elements per block, searched for
+// the fewest wavefronts of the 16- and 4-byte accesses of the three directions'
+// line passes (lanes along elements, then lines) at little padding.  An access
+// of 16 bytes per lane takes four wavefronts per warp without conflicts; with
+// rows and planes packed (5, 25, 125) the xi lines of porder 4 take 7.75, with
+// the xi lines run through along K first 4.0.
+struct GroupPitch {
+    int row, plane, elem;
+    bool swap;
+};
+constexpr GroupPitch group_pitch(int P, int NE)
+{
+    switch (P * 100 + NE) {
+    case 132: return {2, 4, 9, false};
+    case 308: return {4, 16, 67, false};
+    case 405: return {5, 25, 125, true};
+    case 409: return {5, 25, 129, true};
+    case 503: return {6, 36, 219, false};
+    case 504: return {6, 37, 222, true};
+    case 507: return {6, 38, 231, false};
+    case 602: return {7, 49, 348, false};
+    case 603: return {7, 49, 347, true};
+    case 604: return {7, 49, 346, false};
+    case 701: return {8, 67, 533, true};
+    case 702: return {8, 65, 524, true};
+    case 703: return {8, 65, 523, true};
+    case 802: return {9, 81, 732, false};
+    case 803: return {9, 81, 731, true};
+    default: break;
+    }
+    const int Q = P + 1, RP = Q % 2 ? Q : Q + 1;
+    return {RP, Q * RP, Q * Q * RP, false};
+}
+
+// Q points per line, L lines per direction, N points per element, NE elements
+// per block, S threads per line (each owns R consecutive points; the split is
+// by warp, so that a warp's code and coefficients are uniform).
+template <typename real_t, int P_, int NE_, int S_ = 1>
+struct GroupGeom {
+    using real = real_t;
+    static constexpr int P = P_, NE = NE_, S = S_;
+    static constexpr int Q = P + 1, L = Q * Q, N = Q * Q * Q;
+    static constexpr int R = (Q + S - 1) / S;
+    // Record of point (I, J, K) of element el: I + RP J + PP K + ES el.
+    static constexpr GroupPitch PITCH = group_pitch(P, NE);
+    static constexpr int RP = PITCH.row, PP = PITCH.plane, ES = PITCH.elem;
+    static constexpr bool SWAP = PITCH.swap;
+    static constexpr int NREC = NE * ES;
+    static constexpr int LT = ((NE * L + 31) / 32) * 32;  // threads of one segment
+    static constexpr int NT = S * LT;
+    // Pitch of an element's He and gpvol in shared memory.  Where an element's
+    // span is a multiple of 16 bytes (odd porders) it is copied by itself, to a
+    // pitch of 16 bytes more than a multiple of all banks, so that the elements
+    // of a warp do not fall on one bank (64 x 9 and 512 x 9 words are multiples
+    // of 32); the other spans have odd lengths and are copied as one.
+    static constexpr bool STAGED = sizeof(real) == 4;  // FP64: read in place (bound by FP64 issue, short of shared memory)
+    static constexpr bool SPLIT = STAGED && N >= 64 && (N * sizeof(real)) % 16 == 0;
+    static constexpr int BANKS = 128 / (int)sizeof(real), OFF = 16 / (int)sizeof(real);
+    static constexpr int pitch(int n) { return SPLIT ? n + (BANKS + OFF - n % BANKS) % BANKS : n; }
+    static constexpr int HEP = pitch(9 * N), GPP = pitch(N);
+    static constexpr size_t HEB = STAGED ? ((size_t)NE * HEP * sizeof(real) + 31) / 16 * 16 : 0;
+    static constexpr size_t GPB = STAGED ? ((size_t)NE * GPP * sizeof(real) + 31) / 16 * 16 : 0;
+    template <int DIR>
+    static constexpr int step()
+    {
+        return DIR == 0 ? 1 : (DIR == 1 ? RP : PP);
+    }
+};
+
+// The thread's element and its line (q0, q1) of each direction: the line
+// through (J, K) = (q0, q1) along xi (swapped where SWAP), (I, K) along eta,
+// (I, J) along zeta.
+template <class G>
+struct GroupThread {
+    int el, q0, q1, seg;
+    bool active;
+    __device__ __forceinline__ GroupThread(int tid)
+    {
+        seg = G::S == 1 ? 0 : tid / G::LT;
+        const int t = tid - seg * G::LT;
+        active = t < G::NE * G::L;
+        const int line = active ? t / G::NE : 0;
+        el = active ? t - line * G::NE : 0;
+        q1 = line / G::Q;
+        q0 = line - q1 * G::Q;
+    }
+    // Record of the line's first point and its lattice index (K Q + J) Q + I.
+    __device__ __forceinline__ int rec0(int dir) const
+    {
+        const bool sw = dir == 0 && G::SWAP;
+        const int a = dir == 0 ? G::RP : 1, b = dir == 2 ? G::RP : G::PP;
+        return el * G::ES + (sw ? q1 * a + q0 * b : q0 * a + q1 * b);
+    }
+    __device__ __forceinline__ int lat0(int dir) const
+    {
+        const bool sw = dir == 0 && G::SWAP;
+        const int a = dir == 0 ? G::Q : 1, b = dir == 2 ? G::Q : G::L;
+        return sw ? q1 * a + q0 * b : q0 * a + q1 * b;
+    }
+    // Lattice index of point r of the line.
+    template <int DIR>
+    __device__ __forceinline__ int lat(int r) const
+    {
+        return lat0(DIR) + r * (DIR == 0 ? 1 : (DIR == 1 ? G::Q : G::L));
+    }
+};
+
+// Bulk copies of a group's He and gpvol spans into shared memory (one
+// mbarrier phase), a span per lane of the first warp; the unaligned ends, if
+// any, by plain loads.
+template <class G>
+struct GroupMetric {
+    using real = typename G::real;
+    // He(i, dir, a) of element el at He[el HEP + 9 a + 3 dir + i], gpvol(a) at gp[el GPP + a].
+    real *He;
+    const real *gp;
+    int last;  // the group's last element
+    __device__ __forceinline__ real *he(int el, int a) const
+    {
+        return He + (G::STAGED ? el : min(el, last)) * G::HEP + a * 9;
+    }
+    __device__ __forceinline__ const real *vol(int el, int a) const
+    {
+        return gp + (G::STAGED ? el : min(el, last)) * G::GPP + a;
+    }
+    // Bounded wait for the bulk copies (false: the limit ran out).
+    __device__ __forceinline__ bool wait(unsigned long long *bar) const { return G::STAGED ? mbar_wait(bar, 0) : true; }
+    __device__ __forceinline__ GroupMetric(unsigned char *heb, unsigned char *gpb, unsigned long long *bar,
+                                           const real *gHe, const real *ggp, int e0, int nelem, int tid)
+    {
+        last = min(G::NE, nelem - e0) - 1;
+        if constexpr (!G::STAGED) {
+            He = const_cast<real *>(gHe) + (size_t)e0 * G::N * 9;
+            gp = ggp + (size_t)e0 * G::N;
+            return;
+        }
+        constexpr int SPANS = G::SPLIT ? G::NE : 1;
+        static_assert(SPANS <= 32, "one lane of the first warp per span");
+        char *hs = reinterpret_cast<char *>(heb), *gs = reinterpret_cast<char *>(gpb);
+        const int ne = min(G::NE, nelem - e0), spans = G::SPLIT ? ne : 1;
+        const size_t n = (size_t)(G::SPLIT ? 1 : ne) * G::N;
+        const unsigned hsh = (unsigned)(reinterpret_cast<size_t>(gHe + (size_t)e0 * G::N * 9) & 15);
+        const unsigned gsh = (unsigned)(reinterpret_cast<size_t>(ggp + (size_t)e0 * G::N) & 15);
+        if (tid < 32) {
+            const int k = tid < spans ? tid : 0;  // the lane's span (the spans are alike modulo 16 bytes)
+            const size_t off = ((size_t)e0 + k) * G::N;
+            const SpanPlan ph(gHe + off * 9, n * 9 * sizeof(real)), pg(ggp + off, n * sizeof(real));
+            if (tid == 0) {
+                mbar_init(bar, 1);
+                mbar_arrive_expect_tx(bar, (unsigned)spans * (ph.bulk + pg.bulk));
+            }
+            __syncwarp();
+            if (tid < spans) {
+                ph.issue(hs + (size_t)k * G::HEP * sizeof(real), bar);
+                pg.issue(gs + (size_t)k * G::GPP * sizeof(real), bar);
+            }
+            if (ph.head + ph.tail + pg.head + pg.tail != 0)
+                for (int s = 0; s < spans; ++s) {
+                    const size_t o = ((size_t)e0 + s) * G::N;
+                    const SpanPlan qh(gHe + o * 9, n * 9 * sizeof(real)), qg(ggp + o, n * sizeof(real));
+                    if (tid >= 8 && tid < 14) qh.plain(hs + (size_t)s * G::HEP * sizeof(real), tid - 8);
+                    if (tid >= 16 && tid < 22) qg.plain(gs + (size_t)s * G::GPP * sizeof(real), tid - 16);
+                }
+        }
+        He = reinterpret_cast<real *>(hs + hsh);
+        gp = reinterpret_cast<const real *>(gs + gsh);
+    }
+};
+
+}  // namespace
+}  // namespace msod

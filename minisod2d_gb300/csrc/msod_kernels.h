@@ -13,6 +13,8 @@ namespace msod {
 // FP64 copies), lattice -> gmsh node (perm) and gmsh node -> padded lattice
 // offset (lat).
 constexpr int kTableDMax = 3 * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
+// D[d][r][c] at [(d*Q + r)*Q + c], followed at 3*Q*Q by its row sums [d*Q + r].
+constexpr int kTableDSMax = kTableDMax + 3 * (MSOD_MAX_PORDER + 1);
 constexpr int kTableNMax = (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
 // Row pairs of the FP32 matrices for packed (f32x2) contractions:
 // Dp[((d*Q + c)*H + m)*2 + t] = D[d][2m+t][c] (zero for 2m+t = Q), H = (Q+1)/2.
@@ -36,13 +38,14 @@ __host__ __device__ constexpr int sod_left(int i) { return i == 0 ? 0 : i + 1; }
 __host__ __device__ constexpr int sod_centre(int Q) { return (Q + 1) / 2; }
 constexpr int kTableEOMax = 2 * (MSOD_MAX_PORDER / 2 + 1) * (MSOD_MAX_PORDER / 2 + 1) + 2 * (MSOD_MAX_PORDER / 2 + 1);
 struct TableScratch {
-    float Df[kTableDMax];
+    float Df[kTableDSMax];
     float EO[kTableEOMax];
     int eo_ok;  // 1 when EO represents all three directions' matrices
+    int same_dirs;  // 1 when the three directions' matrices are equal
     // The even-odd A and B entries side by side, for packed (f32x2)
     // contractions: EOp[2*(i*M + j)] = A[i][j], EOp[2*(i*M + j) + 1] = B[i][j].
     alignas(8) float EOp[kTableEOMax];
-    double Dd[kTableDMax];
+    double Dd[kTableDSMax];
     alignas(8) float Dp[kTableDPairMax];
     int perm[kTableNMax];
     int lat[kTableNMax];

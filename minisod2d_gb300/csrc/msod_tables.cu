@@ -44,8 +44,18 @@ __global__ void table_prep_kernel(const int *__restrict__ invAtoIJK, const int *
         const int l = d == 0 ? r : (d == 1 ? r * Q : r * Q * Q);
         D[i] = dlxigp_ip[(size_t)(c * 3 + d) * N + sperm[l]];
     }
+    __syncthreads();  // D complete
+    for (int i = threadIdx.x; i < 3 * Q; i += blockDim.x) {
+        double sum = 0.0;
+        for (int c = 0; c < Q; ++c) sum += (double)D[i * Q + c];
+        D[3 * Q * Q + i] = (real)sum;
+    }
+    if (threadIdx.x == 0) {
+        bool same = true;
+        for (int i = 0; i < Q * Q; ++i) same = same && D[Q * Q + i] == D[i] && D[2 * Q * Q + i] == D[i];
+        out->same_dirs = same ? 1 : 0;
+    }
     if (sizeof(real) == 4) {
-        __syncthreads();  // D complete
         // Even-odd form and its validity: the directions' matrices equal, the
         // matrix centro-antisymmetric to within 1e-6 of its largest entry.
         constexpr int M = Q / 2, mc = sod_centre(Q);
