@@ -211,7 +211,7 @@ static int diffu_impl(int porder, int nelem, int npoin, const int *connec, const
     return rc;
 }
 
-static int fused_impl(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
+static int both_impl(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                       const float *dlx, const int *inv, const int *ai, const int *aj, const int *ak, float Cp,
                       float Pr, const float *u, const float *q, const float *rho, const float *pr, const float *E,
                       const float *Tem, const float *mu_fluid, const float *mu_e, const float *mu_sgs,
@@ -249,7 +249,8 @@ static int fused_impl(int porder, int nelem, int npoin, const int *connec, const
     d.Cp = Cp; d.Pr = Pr; d.rho = rho; d.u = u; d.Tem = Tem; d.mu_fluid = mu_fluid; d.mu_e = mu_e;
     d.mu_sgs = mu_sgs; d.nu_elem = nullptr; d.Rmass = Rmass_d; d.Rmom = Rmom_d; d.Rener = Rener_d;
     rc = cuda_status(launch_table_prep<float>(porder, c, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_fused(porder, c, d, tabs, st), "convection + diffusion kernel launch");
+    if (!rc) rc = cuda_status(launch_convec_plain<float>(porder, c, tabs, st), "convection kernel launch");
+    if (!rc) rc = cuda_status(launch_diffu_plain<float>(porder, d, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection + diffusion kernel");
     return rc;
 }
@@ -392,7 +393,7 @@ int msod_convec_diffusion_ijk(int porder, int nelem, int npoin, const int *conne
                                   Rmass_d, Rmom_d, Rener_d, stream);
     }
     (void)Ngp; (void)dNgp; (void)xgp;
-    return fused_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
+    return both_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
                       Cp, Pr, u, q, rho, pr, E, Tem, mu_fluid, mu_e, mu_sgs, Rmass_c, Rmom_c, Rener_c, Rmass_d,
                       Rmom_d, Rener_d, stream);
 }

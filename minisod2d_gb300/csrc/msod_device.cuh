@@ -54,10 +54,6 @@ struct LineGeom {
     static constexpr int NPL = NE * ES;  // words per shared-memory plane
 };
 
-// Largest element count per block whose `planes` shared-memory planes of
-// `bytes` bytes per word fit in `budget` bytes.
-constexpr int necap_for(int planes, int es, int bytes, int budget) { return budget / (planes * es * bytes); }
-
 // Thread -> (element, line, segment) of the line-parallel passes.
 template <class G>
 struct LineThread {
@@ -75,15 +71,6 @@ struct LineThread {
         lb = line / G::Q;
         r0 = seg * G::R;
     }
-    // The line of a bank-aware map entry (LineMap), one thread per line.
-    __device__ __forceinline__ LineThread(unsigned code, bool)
-    {
-        active = code != 0xFFFFu;
-        el = active ? (int)(code >> 8) : 0;
-        lb = active ? (int)((code >> 4) & 15u) : 0;
-        la = active ? (int)(code & 15u) : 0;
-        r0 = 0;
-    }
     __device__ __forceinline__ bool owns(int rr) const { return (G::R * G::S == G::Q) || r0 + rr < G::Q; }
     __device__ __forceinline__ int rc(int rr) const { return owns(rr) ? r0 + rr : 0; }
 };
@@ -96,82 +83,6 @@ __host__ __device__ constexpr int line_off(int la, int lb, int r)
     return DIR == 0 ? (lb * Q + la) * QP + r : (DIR == 1 ? (lb * Q + r) * QP + la : (r * Q + lb) * QP + la);
 }
 
-// Bank-aware assignment of threads to the block's GLL lines, one per
-// direction (one thread per line).  Shared-memory accesses of a line pass
-// address point r of every line at (line base + r * stride), so a warp's
-// lanes conflict exactly when their lines' bases fall in the same bank (mod
-// 32).  Warps are filled one after the other with lines of distinct banks,
-// taking from the banks with the most lines left first, so that the lines a
-// bank has beyond one per warp end up together in the last warps.  At porder 4
-// (5 elements per 128-thread block) this turns the 2-way conflicts of every
-// eta and zeta access of the natural order (lines of consecutive elements
-// side by side) into one extra wavefront on one or two of the four warps
-// (counted from the index arithmetic: 100 -> 75 wavefronts per point step of
-// the three directions, 60 without conflicts).
-// code = (el << 8) | (lb << 4) | la; 0xFFFF marks an idle thread.
-template <class G>
-struct LineMap {
-    unsigned short code[3][G::NT];
-};
-template <class G, int DIR>
-constexpr int line_bank(int l)
-{
-    return (l / G::L * G::ES + line_off<DIR, G::Q, G::QP>(l % G::L % G::Q, l % G::L / G::Q, 0)) % 32;
-}
-template <class G, int DIR>
-constexpr void fill_line_map(LineMap<G> &m)
-{
-    constexpr int NL = G::NE * G::L, NW = G::NT / 32;
-    int start[33] = {}, left_b[32] = {}, order[NL] = {};
-    for (int l = 0; l < NL; ++l) ++start[line_bank<G, DIR>(l) + 1];
-    for (int b = 0; b < 32; ++b) {
-        left_b[b] = start[b + 1];
-        start[b + 1] += start[b];
-    }
-    {
-        int fill[32] = {};
-        for (int b = 0; b < 32; ++b) fill[b] = start[b];
-        for (int l = 0; l < NL; ++l) order[fill[line_bank<G, DIR>(l)]++] = l;
-    }
-    for (int t = 0; t < G::NT; ++t) m.code[DIR][t] = 0xFFFF;
-    int left = NL;
-    for (int w = 0; w < NW; ++w) {
-        const int want = left < 32 ? left : 32;
-        int taken = 0;
-        while (taken < want) {
-            // One pass over distinct banks, most lines left first (ties: lower bank).
-            bool used[32] = {};
-            bool progress = false;
-            while (taken < want) {
-                int best = -1;
-                for (int b = 0; b < 32; ++b)
-                    if (!used[b] && left_b[b] > 0 && (best < 0 || left_b[b] > left_b[best])) best = b;
-                if (best < 0) break;
-                used[best] = true;
-                const int l = order[start[best]++];
-                --left_b[best];
-                const int el = l / G::L, line = l % G::L;
-                m.code[DIR][32 * w + taken] = (unsigned short)((el << 8) | ((line / G::Q) << 4) | (line % G::Q));
-                ++taken;
-                progress = true;
-            }
-            if (!progress) break;
-        }
-        left -= taken;
-    }
-}
-template <class G>
-constexpr LineMap<G> make_line_map()
-{
-    static_assert(G::S == 1 && G::NE < 256 && G::Q <= 16, "one thread per line");
-    LineMap<G> m{};
-    fill_line_map<G, 0>(m);
-    fill_line_map<G, 1>(m);
-    fill_line_map<G, 2>(m);
-    return m;
-}
-template <class G>
-__device__ const LineMap<G> kLineMap = make_line_map<G>();
 template <int DIR, int Q>
 __device__ __forceinline__ int line_lat(int la, int lb, int r)
 {
@@ -275,12 +186,6 @@ __device__ __forceinline__ void prefetch_element_l2(const float *He, const float
 {
     prefetch_span_l2(He + (size_t)e * ngaus * 9, (size_t)ngaus * 9 * sizeof(float));
     prefetch_span_l2(gpvol + (size_t)e * ngaus, (size_t)ngaus * sizeof(float));
-}
-
-// L2 prefetch of the sector at p (a hint).
-__device__ __forceinline__ void prefetch_l2(const void *p)
-{
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 struct SpanPlan {

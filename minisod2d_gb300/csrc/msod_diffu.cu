@@ -12,446 +12,351 @@
 //   kappa_e(a) = mu_fluid Cp/Pr + mu_e Cp/Pr + Cp rho mu_sgs / 0.9 evaluated at
 //   the output node (elem_diffu.f90:143-146).
 //
-// Design (persistent blocks, groups of NE elements, one thread per GLL line):
-//   0. the node ids of the next group are loaded into registers while the
-//      current group is computed; after it, the next group's node fields
-//      (rho, T, u, mu_fluid) and element-layout mu_e, mu_sgs are gathered with
-//      cp.async into the shared-memory lattice (single-buffered: measured 6 %
-//      faster than a double-buffered lattice, whose shared memory held the
-//      kernel to two blocks per SM instead of three; DIFFU_NBUF = 2 selects
-//      it); the He and gpvol values of the point pass are loaded into
-//      registers before pass 1;
-//   1. three line passes store the 15 iso-parametric derivatives per point;
-//   2. a point pass turns them into physical gradients and stress and stores,
-//      per direction d, the contravariant fluxes gpvol * He(:,d)^T X for the
-//      six vectors X = grad rho, tauU, grad T, tau rows 1..3 (18 per point),
-//      plus nu_e and kappa_e per output node;
-//   3. three line passes apply the transposed 1-D derivative matrix along the
-//      lines (the weak divergence), accumulating five sums per node through
-//      shared memory; the last pass scatter-adds with red.global.add.
-// With one thread per line from porder 3 up, the zeta derivative pass, the
-// point pass and the zeta divergence pass run as one pass over each zeta line
-// (the zeta derivatives and fluxes never reach shared memory, the He rows are
-// loaded there one point ahead), and the flux region shrinks from 18 planes to
-// 12: porder 4 then takes 53.8 KB of shared memory per block instead of 68.8 KB,
-// three blocks leave ~88 KB of L1 instead of ~28 KB for the He and node-field
-// loads, and the kernel runs 1.50 ms instead of 1.82 ms on 64^3 hexes (the same
-// fusion with the 18-plane region: 1.79 ms; four blocks per SM at 128
-// registers, which fill the shared memory again: 1.90 ms).
-// The 1-D derivative matrices are constant-bank operands.
-#include "msod_diffu.cuh"
+// Design (one group of NE elements per block, one thread per GLL line,
+// msod_group.cuh):
+//   0. bulk copies bring the group's He and gpvol; each thread gathers the
+//      points of its zeta line (node fields through connec, mu_e and mu_sgs in
+//      the element layout) and keeps them in registers; rho, T and u go to the
+//      shared-memory lattice as records;
+//   1. xi and eta passes store the iso-parametric derivatives of the five
+//      fields;
+//   2. zeta stage, at the points of the thread's zeta line: zeta derivatives
+//      from the line's registers, physical gradients and stress, and the
+//      contravariant fluxes gpvol He(:,d)^T X of the six vectors X = grad rho,
+//      tauU, grad T, tau rows 1..3; the xi and eta fluxes go to shared memory
+//      (over the derivatives), the zeta divergence stays in registers;
+//   3. xi and eta passes apply the transposed 1-D derivative matrix to their
+//      fluxes, in place;
+//   4. the thread of the zeta line adds the three divergences of its points,
+//      forms the residuals and scatter-adds them with red.global.add.
+// The viscosities, nu_e, kappa_e and the node ids never leave the registers of
+// the zeta line's thread.  The 1-D derivative matrices are constant-bank
+// operands.
+#include <cuda_runtime.h>
+
+#include "msod_group.cuh"
 
 namespace msod {
 namespace {
 
-template <class G, int VISC>
-__global__ void __launch_bounds__(G::NT, diffu_minb<G>())
-    diffu_kernel(int nelem, int npoin, int ngroups, const int *__restrict__ connec,
-                 const typename G::real *__restrict__ He, const typename G::real *__restrict__ gpvol,
-                 const TableScratch *__restrict__ tabs, typename G::real Cp, typename G::real Pr,
-                 const typename G::real *__restrict__ rho, const typename G::real *__restrict__ u,
-                 const typename G::real *__restrict__ Tem, const typename G::real *__restrict__ mu_fluid,
-                 const typename G::real *__restrict__ mu_e, const typename G::real *__restrict__ mu_sgs,
-                 const typename G::real *__restrict__ nu_elem, typename G::real *__restrict__ Rmass,
-                 typename G::real *__restrict__ Rmom, typename G::real *__restrict__ Rener, int linemap)
+__constant__ float c_Df[MSOD_MAX_PORDER + 1][kTableDMax];
+__constant__ double c_Dd[MSOD_MAX_PORDER + 1][kTableDMax];
+template <typename real>
+__device__ __forceinline__ real cD(int P, int i);
+template <>
+__device__ __forceinline__ float cD<float>(int P, int i)
+{
+    return c_Df[P][i];
+}
+template <>
+__device__ __forceinline__ double cD<double>(int P, int i)
+{
+    return c_Dd[P][i];
+}
+
+// Viscosity source of the diffusion kernel: the mu_e array, or one value per
+// element (mu_e(e, a) = rho(a) nu_elem(e)).
+enum { VISC_MU_E = 0, VISC_NU_ELEM = 1 };
+
+// Elements per block and blocks per SM that the register budget allows for.
+// Whole warps of lines (5 x 25 lines at porder 4: 125 of 128 threads) count
+// most; the FP64 kernels, bound by FP64 issue, which a warp pays for its idle
+// lanes too, take the same groups.  Measured in FP32 (ms, 64^3 hexes at porder
+// 4): 5 elements at four blocks 1.141, at three 1.152, 8 elements at two 1.302,
+// 9 at two 1.284, 4 at four 1.236.  Porder 5 (51^3): 3 elements at three blocks
+// 1.162, at four 1.409 (spills), 4 at two 1.250, 7 at one 1.546.  Porder 6
+// (40^3): 3 at one 1.229, 2 at two 1.266, 4 at one 1.394.  Porder 7 (32^3): 2
+// at two 0.991, 1 at three 1.142, 3 at one 1.043.  Porder 8 (26^3): 1 0.922, 2
+// 1.007, 3 0.950.  Porder 2 (100^3): 16 at four 0.707, at the compiler's choice
+// 0.738; porder 3 (80^3): 8 at four 0.922, at the compiler's choice 0.937.
+template <typename real, int P>
+constexpr int diffu_ne()
+{
+    constexpr int nf[9] = {0, 32, 16, 8, 5, 3, 3, 2, 1}, nd[9] = {0, 32, 14, 8, 5, 3, 2, 1, 1};
+    return sizeof(real) == 4 ? nf[P] : nd[P];
+}
+template <typename real, int P>
+constexpr int diffu_minb()
+{
+    constexpr int nb[9] = {0, 1, 4, 4, 4, 3, 1, 2, 1};
+    return sizeof(real) == 4 ? nb[P] : 1;
+}
+template <typename real, int P>
+using DiffuGeom = GroupGeom<real, P, diffu_ne<real, P>()>;
+
+// Shared memory of a block.  X1 and X3 hold the xi and eta derivatives of
+// (rho, T, u1, u2), then the fluxes (and divergences) of grad rho, tauU, grad T
+// and tau_1; X2 holds the node fields (rho, T, u1, u2), then the fluxes of
+// tau_2, tau_3 (xi, eta).
+template <class G>
+struct DiffuShared {
+    using real = typename G::real;
+    static constexpr size_t k1 = G::HEB + G::GPB + 16;
+    static constexpr size_t k2 = k1 + G::NREC * sizeof(Four<real>);
+    static constexpr size_t k3 = k2 + G::NREC * sizeof(Four<real>);
+    static constexpr size_t kU = k3 + G::NREC * sizeof(Four<real>);
+    static constexpr size_t kE1 = kU + G::NREC * sizeof(real);
+    static constexpr size_t kE3 = kE1 + G::NREC * sizeof(real);
+    static constexpr size_t kBytes = kE3 + G::NREC * sizeof(real);
+    unsigned char *base;
+    __device__ __forceinline__ unsigned long long *bar() const
+    {
+        return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
+    }
+    __device__ __forceinline__ Four<real> *X1() const { return reinterpret_cast<Four<real> *>(base + k1); }
+    __device__ __forceinline__ Four<real> *X2() const { return reinterpret_cast<Four<real> *>(base + k2); }
+    __device__ __forceinline__ Four<real> *X3() const { return reinterpret_cast<Four<real> *>(base + k3); }
+    __device__ __forceinline__ real *U3() const { return reinterpret_cast<real *>(base + kU); }   // u3
+    __device__ __forceinline__ real *E1() const { return reinterpret_cast<real *>(base + kE1); }  // its xi derivative
+    __device__ __forceinline__ real *E3() const { return reinterpret_cast<real *>(base + kE3); }  // its eta derivative
+};
+
+// Derivatives of the five fields along the thread's line in direction DIR.
+template <class G, int DIR>
+__device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuShared<G> &sm)
 {
     using real = typename G::real;
-    constexpr int Q = G::Q, N = G::N, QP = G::QP, ES = G::ES, NE = G::NE, NT = G::NT, NPL = G::NPL;
-    constexpr int IPT = (NE * N + NT - 1) / NT;  // items (node ids, points) per thread
+    using R2 = Two<real>;
+    constexpr int Q = G::Q, P = G::P;
+    const int base = t.rec0(DIR);
+    Four<real> f[Q];
+    real u3[Q];
+#pragma unroll
+    for (int c = 0; c < Q; ++c) {
+        f[c] = sm.X2()[base + c * G::template step<DIR>()];
+        u3[c] = sm.U3()[base + c * G::template step<DIR>()];
+    }
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+        Four<real> g;
+        g.a = g.b = two((real)0, (real)0);
+        real g3 = (real)0;
+#pragma unroll
+        for (int c = 0; c < Q; ++c) {
+            const real D = cD<real>(P, (DIR * Q + r) * Q + c);
+            g.a = fma2(two(D, D), f[c].a, g.a);
+            g.b = fma2(two(D, D), f[c].b, g.b);
+            g3 = fma(D, u3[c], g3);
+        }
+        const int o = base + r * G::template step<DIR>();
+        (DIR == 0 ? sm.X1() : sm.X3())[o] = g;
+        (DIR == 0 ? sm.E1() : sm.E3())[o] = g3;
+    }
+}
+
+// Weak divergence of the thread's line in direction DIR, in place.
+template <class G, int DIR>
+__device__ __forceinline__ void diffu_div(const GroupThread<G> &t, const DiffuShared<G> &sm)
+{
+    using real = typename G::real;
+    using R2 = Two<real>;
+    constexpr int Q = G::Q, P = G::P;
+    const int base = t.rec0(DIR);
+    Four<real> *X = DIR == 0 ? sm.X1() : sm.X3();
+    {
+        Four<real> f[Q];
+#pragma unroll
+        for (int c = 0; c < Q; ++c) f[c] = X[base + c * G::template step<DIR>()];
+#pragma unroll
+        for (int r = 0; r < Q; ++r) {
+            Four<real> s;
+            s.a = s.b = two((real)0, (real)0);
+#pragma unroll
+            for (int c = 0; c < Q; ++c) {
+                const real D = cD<real>(P, (DIR * Q + c) * Q + r);
+                s.a = fma2(two(D, D), f[c].a, s.a);
+                s.b = fma2(two(D, D), f[c].b, s.b);
+            }
+            X[base + r * G::template step<DIR>()] = s;
+        }
+    }
+    R2 f[Q];
+#pragma unroll
+    for (int c = 0; c < Q; ++c) {
+        const Four<real> *x = sm.X2() + base + c * G::template step<DIR>();
+        f[c] = DIR == 0 ? x->a : x->b;
+    }
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+        R2 s = two((real)0, (real)0);
+#pragma unroll
+        for (int c = 0; c < Q; ++c) {
+            const real D = cD<real>(P, (DIR * Q + c) * Q + r);
+            s = fma2(two(D, D), f[c], s);
+        }
+        Four<real> *x = sm.X2() + base + r * G::template step<DIR>();
+        (DIR == 0 ? x->a : x->b) = s;
+    }
+}
+
+template <class G, int VISC, int MINB>
+__global__ void __launch_bounds__(G::NT, MINB)
+    diffu_kernel(int nelem, int npoin, const int *__restrict__ connec, const typename G::real *__restrict__ He,
+                 const typename G::real *__restrict__ gpvol, const TableScratch *__restrict__ tabs,
+                 typename G::real Cp, typename G::real Pr, const typename G::real *__restrict__ rho,
+                 const typename G::real *__restrict__ u, const typename G::real *__restrict__ Tem,
+                 const typename G::real *__restrict__ mu_fluid, const typename G::real *__restrict__ mu_e,
+                 const typename G::real *__restrict__ mu_sgs, const typename G::real *__restrict__ nu_elem,
+                 typename G::real *__restrict__ Rmass, typename G::real *__restrict__ Rmom,
+                 typename G::real *__restrict__ Rener)
+{
+    using real = typename G::real;
+    using R2 = Two<real>;
+    constexpr int Q = G::Q, P = G::P, N = G::N;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int NBUF = DIFFU_NBUF;
-    constexpr bool STAGED = diffu_staged<G>();
-    char *sHeB = reinterpret_cast<char *>(smem_raw);  // staged He / gpvol spans, then the mbarrier
-    char *sGpB = sHeB + diffu_he_bytes<G>();
-    unsigned long long *sBar = reinterpret_cast<unsigned long long *>(sGpB + diffu_gp_bytes<G>());
-    real *sF = reinterpret_cast<real *>(smem_raw + diffu_stage_bytes<G>());  // [NBUF][NDF][NPL]
-    real *sX = sF + NBUF * NDF * NPL;                // [2 or 3 NX][NPL]
-    real *sD = sX + diffu_xplanes<G>() * NPL;        // [3][Q][Q] (several threads per line)
-    int *sNode = reinterpret_cast<int *>(sD + 3 * Q * Q);  // [NBUF][NPL]
-    int *sPerm = sNode + NBUF * NPL;
-    int *sLat = sPerm + N;
+    const DiffuShared<G> sm{smem_raw};
+    const int tid = threadIdx.x, e0 = blockIdx.x * G::NE;
+    const GroupThread<G> t(tid);
+    const GroupMetric<G> gm(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);
+    const int e = e0 + t.el, base = t.rec0(2);
+    const bool in = t.active && e < nelem;
+    const size_t np = (size_t)npoin;
 
-    const int tid = threadIdx.x;
-    const LineThread<G> lt0 = diffu_line<G>(tid, 0, linemap), lt1 = diffu_line<G>(tid, 1, linemap),
-                        lt2 = diffu_line<G>(tid, 2, linemap);
-    constexpr bool FUSEZ = diffu_fusez<G>();
-    constexpr bool LATE = FUSEZ && DIFFU_HE_LATE != 0;
-    // The xi and eta passes in even-odd form when the call's tables allow it
-    // (uniform over the grid).
-    constexpr bool EOK = ((DIFFU_EO >> G::P) & 1) != 0 && FUSEZ && sizeof(real) == 4;
-    bool eo = false;
-    if constexpr (EOK) eo = ldg(&tabs->eo_ok) != 0;
-    constexpr int MP = LATE ? 1 : (FUSEZ ? Q : IPT);  // points whose He and gpvol a thread holds
-    for (int i = tid; i < N; i += NT) {
-        sPerm[i] = tabs->perm[i];
-        sLat[i] = tabs->lat[i];
+    // The points of the thread's zeta line (a missing node reads as zeros).
+    int id[Q], pt[Q];
+    R2 rT[Q], u12[Q];
+    real u3[Q], muf[Q], ms[Q], me[Q];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) pt[k] = ldg(&tabs->perm[t.template lat<2>(k)]);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        const int v = in ? ldg(connec + (size_t)pt[k] * nelem + e) - 1 : -1;
+        id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
     }
-    if (G::S > 1)
-        for (int i = tid; i < 3 * Q * Q; i += NT) sD[i] = table_D<real>(tabs)[i];
-    // Group-invariant parts of the gathers (GOFF), per item k of the thread: the
-    // lattice offset of its point in the node-field gather (go), and for the
-    // element-layout loads (node ids, mu_e, mu_sgs) the row offset a nelem + el
-    // (mr) and the element el in bits 20.. of mo, whose low bits take the
-    // lattice offset el ES + lat(a) once sLat is in shared memory; -1 for no item.
-    constexpr bool GOFF = ((DIFFU_GOFF >> G::P) & 1) != 0 && NBUF == 1 && DIFFU_GATHER_LDG == 0;
-    constexpr int KG = GOFF ? IPT : 1;
-    int go[KG], mr[KG], mo[KG];
-    if constexpr (GOFF) {
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int i = tid + k * NT;
-            const bool in = i < NE * N;
-            const int el = i / N, l = i - el * N;
-            const int I = l % Q, J = (l / Q) % Q, K = l / (Q * Q);
-            go[k] = in ? el * ES + (K * Q + J) * QP + I : -1;
-            const int el2 = i % NE, a = i / NE;
-            mr[k] = in ? a * nelem + el2 : 0;
-            mo[k] = in ? (el2 << 20) : -1;
-        }
+    for (int k = 0; k < Q; ++k) {
+        const bool ok = id[k] >= 0;
+        const size_t p = ok ? (size_t)id[k] : 0, i = in ? (size_t)pt[k] * nelem + e : 0;
+        rT[k] = two(ok ? ldg(rho + p) : (real)0, ok ? ldg(Tem + p) : (real)0);
+        u12[k] = two(ok ? ldg(u + p) : (real)0, ok ? ldg(u + np + p) : (real)0);
+        u3[k] = ok ? ldg(u + 2 * np + p) : (real)0;
+        muf[k] = ok ? ldg(mu_fluid + p) : (real)0;
+        ms[k] = in ? ldg(mu_sgs + i) : (real)0;
+        me[k] = (VISC == VISC_MU_E && in) ? ldg(mu_e + i) : (real)0;
     }
-    auto load_ids = [&](int g, int (&ids)[IPT]) {
+    if (VISC == VISC_NU_ELEM) {
+        const real nu = in ? ldg(nu_elem + e) : (real)0;
 #pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            if constexpr (GOFF) {
-                const bool ok = mo[k] >= 0 && g * NE + (mo[k] >> 20) < nelem;
-                ids[k] = ok ? ldg(connec + (size_t)(mr[k] + g * NE)) : 0;
-            } else {
-                const int i = tid + k * NT;
-                const int el = i % NE, a = i / NE, e = g * NE + el;
-                ids[k] = (i < NE * N && e < nelem) ? ldg(connec + (size_t)a * nelem + e) : 0;
-            }
-        }
-    };
-    auto store_ids = [&](const int (&ids)[IPT], int *dst) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int v = ids[k] - 1;
-            if constexpr (GOFF) {
-                if (mo[k] >= 0) dst[mo[k] & 0xFFFFF] = (v >= 0 && v < npoin) ? v : -1;
-            } else {
-                const int i = tid + k * NT;
-                if (i < NE * N) dst[(i % NE) * ES + sLat[i / NE]] = (v >= 0 && v < npoin) ? v : -1;
-            }
-        }
-    };
-    // Node fields in lattice order; mu_e / mu_sgs along elements (coalesced).
-    auto gather = [&](int g, const int *ids_s, real *dst) {
-        if constexpr (DIFFU_GATHER_LDG != 0) {
-            // Loads of all of a thread's items first, then the stores.
-            real v[IPT][6], w[IPT][2];
-            int ov[IPT], ow[IPT];
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const int i = tid + k * NT;
-                const bool in = i < NE * N;
-                const int el = in ? i / N : 0, l = in ? i - el * N : 0;
-                const int I = l % Q, J = (l / Q) % Q, K = l / (Q * Q);
-                const int o = el * ES + (K * Q + J) * QP + I;
-                ov[k] = in ? o : -1;
-                const int p = in ? ids_s[o] : -1;
-                const bool ok = (unsigned)p < (unsigned)npoin;
-                const size_t pp = ok ? (size_t)p : 0, np = (size_t)npoin;
-                v[k][0] = ok ? ldg(rho + pp) : (real)0;
-                v[k][1] = ok ? ldg(Tem + pp) : (real)0;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) v[k][2 + c] = ok ? ldg(u + c * np + pp) : (real)0;
-                v[k][5] = ok ? ldg(mu_fluid + pp) : (real)0;
-                const int el2 = i % NE, a = i / NE, e = g * NE + el2;
-                ow[k] = in ? el2 * ES + sLat[in ? a : 0] : -1;
-                const bool ok2 = in && e < nelem;
-                const size_t idx = ok2 ? (size_t)a * nelem + e : 0;
-                w[k][0] = (VISC == VISC_MU_E && ok2) ? ldg(mu_e + idx) : (real)0;
-                w[k][1] = ok2 ? ldg(mu_sgs + idx) : (real)0;
-            }
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                if (ov[k] < 0) continue;
-                dst[D_RHO * NPL + ov[k]] = v[k][0];
-                dst[D_T * NPL + ov[k]] = v[k][1];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) dst[(D_U0 + c) * NPL + ov[k]] = v[k][2 + c];
-                dst[D_MUF * NPL + ov[k]] = v[k][5];
-                if (VISC == VISC_MU_E) dst[D_MUE * NPL + ow[k]] = w[k][0];
-                dst[D_MUS * NPL + ow[k]] = w[k][1];
-            }
-            return;
-        }
-        if constexpr (GOFF) {
-            const size_t np = (size_t)npoin;
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const int o = go[k];
-                if (o >= 0) {
-                    const int p = ids_s[o];
-                    const bool ok = (unsigned)p < (unsigned)npoin;
-                    const size_t pp = ok ? (size_t)p : 0;
-                    cp_async_elem(dst + D_RHO * NPL + o, rho + pp, ok);
-                    cp_async_elem(dst + D_T * NPL + o, Tem + pp, ok);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) cp_async_elem(dst + (D_U0 + c) * NPL + o, u + c * np + pp, ok);
-                    cp_async_elem(dst + D_MUF * NPL + o, mu_fluid + pp, ok);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                if (mo[k] >= 0) {
-                    const bool ok = g * NE + (mo[k] >> 20) < nelem;
-                    const size_t idx = ok ? (size_t)(mr[k] + g * NE) : 0;
-                    const int o = mo[k] & 0xFFFFF;
-                    if (VISC == VISC_MU_E) cp_async_elem(dst + D_MUE * NPL + o, mu_e + idx, ok);
-                    cp_async_elem(dst + D_MUS * NPL + o, mu_sgs + idx, ok);
-                }
-            }
-            cp_async_commit();
-            return;
-        }
-        for (int i = tid; i < NE * N; i += NT) {
-            const int el = i / N, l = i - el * N;
-            const int I = l % Q, J = (l / Q) % Q, K = l / (Q * Q);
-            const int o = el * ES + (K * Q + J) * QP + I;
-            const int p = ids_s[o];
-            const bool ok = (unsigned)p < (unsigned)npoin;
-            const size_t pp = ok ? (size_t)p : 0, np = (size_t)npoin;
-            cp_async_elem(dst + D_RHO * NPL + o, rho + pp, ok);
-            cp_async_elem(dst + D_T * NPL + o, Tem + pp, ok);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) cp_async_elem(dst + (D_U0 + c) * NPL + o, u + c * np + pp, ok);
-            cp_async_elem(dst + D_MUF * NPL + o, mu_fluid + pp, ok);
-        }
-        for (int i = tid; i < NE * N; i += NT) {
-            const int el = i % NE, a = i / NE, e = g * NE + el;
-            const int o = el * ES + sLat[a];
-            const bool ok = e < nelem;
-            const size_t idx = ok ? (size_t)a * nelem + e : 0;
-            if (VISC == VISC_MU_E) cp_async_elem(dst + D_MUE * NPL + o, mu_e + idx, ok);
-            cp_async_elem(dst + D_MUS * NPL + o, mu_sgs + idx, ok);
-        }
-        cp_async_commit();
-    };
-    // He(:,:) and gpvol of the thread's point-pass points: items tid + k NT
-    // (lattice order), or the points of its zeta line in the zeta stage.
-    auto load_metric = [&](int g, real (&Hm)[MP][9], real (&gv)[MP]) {
-#pragma unroll
-        for (int k = 0; k < MP; ++k) {
-            const int i = tid + k * NT;
-            const int el = FUSEZ ? lt2.el : i / N;
-            const int l = FUSEZ ? line_lat<2, Q>(lt2.la, lt2.lb, k) : i - el * N, e = g * NE + el;
-            const bool ok = (FUSEZ ? lt2.active : i < NE * N) && e < nelem;
-            const int a = ok ? sPerm[l] : 0;
-            const real *hp = He + (ok ? ((size_t)e * N + a) * 9 : 0);
-#pragma unroll
-            for (int j = 0; j < 9; ++j) Hm[k][j] = ok ? ldg(hp + j) : (real)0;
-            gv[k] = ok ? ldg(gpvol + (size_t)e * N + a) : (real)0;
-        }
-    };
-
-    // mu_e at a point of element el of group g (lattice offset o, density r).
-    auto point_mu_e = [&](int g, int el, int o, real r, const real *sFs) -> real {
-        const int ee = g * NE + el;
-        return VISC == VISC_NU_ELEM ? (ee < nelem ? r * ldg(nu_elem + ee) : (real)0) : sFs[D_MUE * NPL + o];
-    };
-
-    // Staged He / gpvol: bulk copies of group g's spans (thread 0), the
-    // unaligned ends by plain loads (threads 32..37, 64..69).  Offsets of the
-    // spans' first words in the staging area.
-    int he_off = 0, gp_off = 0;
-    auto stage = [&](int g) {
-        if constexpr (STAGED) {
-            const int e0 = g * NE, e1 = min(e0 + NE, nelem);
-            const SpanPlan ph(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(real));
-            const SpanPlan pg(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(real));
-            if (tid == 0) {
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(sBar, ph.bulk + pg.bulk);
-                ph.issue(sHeB, sBar);
-                pg.issue(sGpB, sBar);
-            } else if (tid >= 32 && tid < 38) {
-                ph.plain(sHeB, tid - 32);
-            } else if (tid >= 64 && tid < 70) {
-                pg.plain(sGpB, tid - 64);
-            }
-            he_off = (int)(ph.shift / sizeof(real));
-            gp_off = (int)(pg.shift / sizeof(real));
-        }
-    };
-    unsigned phase = 0;
-
-    int g = blockIdx.x;
-    const int stride = gridDim.x;
-    if constexpr (STAGED) {
-        if (tid == 0) mbar_init(sBar, 1);
-        __syncthreads();
-        stage(g);
+        for (int k = 0; k < Q; ++k) me[k] = rT[k].x * nu;
     }
-    // Group g's He and gpvol spans into L2 (one thread), a group ahead of
-    // their loads in the zeta stage.
-    auto prefetch_group = [&](int gg) {
-        if constexpr (DIFFU_PREFETCH != 0 && !STAGED) {
-            if (tid == 0 && gg < ngroups) {
-                const int e0 = gg * NE, e1 = min(e0 + NE, nelem);
-                prefetch_span_l2(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(real));
-                prefetch_span_l2(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(real));
-            }
-        }
-    };
-    // Group gg's gathered inputs into L2 (ids: its node ids), a group ahead of
-    // the gather: the node fields of its element points and its mu_e, mu_sgs
-    // rows (N rows of NE consecutive values).
-    auto prefetch_nodes = [&](int gg, const int(&ids_g)[IPT]) {
-        if constexpr (DIFFU_PREFETCH >= 3 && NBUF == 1) {
-            const size_t np = (size_t)npoin;
+    if (t.active)
 #pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const int i = tid + k * NT, v = ids_g[k] - 1;
-                if (i < NE * N && (unsigned)v < (unsigned)npoin) {
-                    prefetch_l2(rho + v);
-                    prefetch_l2(Tem + v);
-                    prefetch_l2(mu_fluid + v);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) prefetch_l2(u + c * np + v);
-                }
-            }
+        for (int k = 0; k < Q; ++k) {
+            Four<real> f;
+            f.a = rT[k];
+            f.b = u12[k];
+            sm.X2()[base + k * G::template step<2>()] = f;
+            sm.U3()[base + k * G::template step<2>()] = u3[k];
         }
-        if constexpr (DIFFU_PREFETCH >= 2 && NBUF == 1) {
-            if (tid < N) {
-                const size_t row = (size_t)tid * nelem + (size_t)gg * NE;
-                if (VISC == VISC_MU_E) prefetch_l2(mu_e + row);
-                prefetch_l2(mu_sgs + row);
-            }
-        }
-    };
-    prefetch_group(g);
-    int ids[IPT];
-    load_ids(g, ids);
-    __syncthreads();  // sLat ready
-    if constexpr (GOFF) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k)
-            if (mo[k] >= 0) mo[k] |= (mo[k] >> 20) * ES + sLat[(tid + k * NT) / NE];
-    }
-    store_ids(ids, sNode);
     __syncthreads();
-    gather(g, sNode, sF);
-    int gn = g + stride;
-    if (gn < ngroups) load_ids(gn, ids);
-
-    int s = 0;
-    for (; g < ngroups; g = gn, gn += stride, s = NBUF == 2 ? s ^ 1 : 0) {
-        prefetch_group(gn);
-        real *sFs = sF + s * NDF * NPL;
-        int *sNs = sNode + s * NPL;
-        real Hm[MP][9], gv[MP];
-        if (!LATE) load_metric(g, Hm, gv);
-        if (NBUF == 2 && gn < ngroups) store_ids(ids, sNode + (s ^ 1) * NPL);
-        cp_async_wait_all();
-        __syncthreads();
-        if (gn < ngroups) prefetch_nodes(gn, ids);
-        if (NBUF == 2 && gn < ngroups) {
-            gather(gn, sNode + (s ^ 1) * NPL, sF + (s ^ 1) * NDF * NPL);
-            if (gn + stride < ngroups) load_ids(gn + stride, ids);
+    if (t.active) {
+        diffu_grad<G, 0>(t, sm);
+        diffu_grad<G, 1>(t, sm);
+    }
+    // Bounded wait for the bulk copies; a wait that ran out is reported and
+    // nothing is assembled.
+    const bool ok = gm.wait(sm.bar());
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) report_wait_fault(tabs);
+        return;
+    }
+    // Zeta stage: acc[r][0..2] = the zeta divergence at point r of the fluxes of
+    // (grad rho, tauU), (grad T, tau_1), (tau_2, tau_3).
+    const real CpPr = Cp / Pr, Cp09 = Cp / (real)0.9;
+    R2 acc[Q][3];
+    real nu[Q], kap[Q];
+#pragma unroll
+    for (int r = 0; r < Q; ++r) acc[r][0] = acc[r][1] = acc[r][2] = two((real)0, (real)0);
+    if (t.active) {
+#pragma unroll
+        for (int c = 0; c < Q; ++c) {
+            const int o = base + c * G::template step<2>();
+            real H[9];
+            const real *hp = gm.he(t.el, pt[c]);
+#pragma unroll
+            for (int j = 0; j < 9; ++j) H[j] = hp[j];
+            const real gv = *gm.vol(t.el, pt[c]);
+            const Four<real> gx = sm.X1()[o], ge = sm.X3()[o];
+            R2 za = two((real)0, (real)0), zb = za;
+            real z3 = (real)0;
+#pragma unroll
+            for (int j = 0; j < Q; ++j) {
+                const real D = cD<real>(P, (2 * Q + c) * Q + j);
+                za = fma2(two(D, D), rT[j], za);
+                zb = fma2(two(D, D), u12[j], zb);
+                z3 = fma(D, u3[j], z3);
+            }
+            const R2 xa = gx.a, xb = gx.b, ea = ge.a, eb = ge.b;
+            const real x3 = sm.E1()[o], e3 = sm.E3()[o];
+            // Physical gradients: (grad rho, grad T)_i and (grad u1, grad u2)_i as pairs.
+            R2 gRT[3], gU[3];
+            real gU3[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const R2 h0 = two(H[i], H[i]), h1 = two(H[3 + i], H[3 + i]), h2 = two(H[6 + i], H[6 + i]);
+                gRT[i] = fma2(h2, za, fma2(h1, ea, mul2(h0, xa)));
+                gU[i] = fma2(h2, zb, fma2(h1, eb, mul2(h0, xb)));
+                gU3[i] = fma(H[6 + i], z3, fma(H[3 + i], e3, H[i] * x3));
+            }
+            const real r = rT[c].x;
+            const real mf = muf[c] + r * ms[c], mt = mf + me[c];
+            const real cut = mf * ((real)2 / (real)3) * (gU[0].x + gU[1].y + gU3[2]);
+            const real t00 = mt * (gU[0].x + gU[0].x) - cut, t11 = mt * (gU[1].y + gU[1].y) - cut,
+                       t22 = mt * (gU3[2] + gU3[2]) - cut;
+            const real t01 = mt * (gU[1].x + gU[0].y), t02 = mt * (gU[2].x + gU3[0]), t12 = mt * (gU[2].y + gU3[1]);
+            const real v0 = u12[c].x, v1 = u12[c].y, v2 = u3[c];
+            const real q0 = fma(t02, v2, fma(t01, v1, t00 * v0)), q1 = fma(t12, v2, fma(t11, v1, t01 * v0)),
+                       q2 = fma(t22, v2, fma(t12, v1, t02 * v0));
+            // The six vectors as pairs: (grad rho, tauU), (grad T, tau_1), (tau_2, tau_3).
+            const R2 v[3][3] = {{two(gRT[0].x, q0), two(gRT[1].x, q1), two(gRT[2].x, q2)},
+                                {two(gRT[0].y, t00), two(gRT[1].y, t01), two(gRT[2].y, t02)},
+                                {two(t01, t02), two(t11, t12), two(t12, t22)}};
+            R2 F[3][3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const real w0 = gv * H[d * 3], w1 = gv * H[d * 3 + 1], w2 = gv * H[d * 3 + 2];
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    F[d][x] = fma2(two(w2, w2), v[x][2], fma2(two(w1, w1), v[x][1], mul2(two(w0, w0), v[x][0])));
+            }
+            Four<real> s;
+            s.a = F[0][0];
+            s.b = F[0][1];
+            sm.X1()[o] = s;
+            s.a = F[1][0];
+            s.b = F[1][1];
+            sm.X3()[o] = s;
+            s.a = F[0][2];
+            s.b = F[1][2];
+            sm.X2()[o] = s;
+#pragma unroll
+            for (int rr = 0; rr < Q; ++rr) {
+                const real D = cD<real>(P, (2 * Q + c) * Q + rr);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) acc[rr][x] = fma2(two(D, D), F[2][x], acc[rr][x]);
+            }
+            nu[c] = me[c] / r;
+            kap[c] = fma(muf[c] + me[c], CpPr, Cp09 * (r * ms[c]));
         }
-        if constexpr (FUSEZ) {
-            if (eo) {
-                if (lt0.active) grad_pass<G, 0, EOK>(lt0, sFs, sX, sD);
-                if (lt1.active) grad_pass<G, 1, EOK>(lt1, sFs, sX, sD);
-            } else {
-                if (lt0.active) grad_pass<G, 0>(lt0, sFs, sX, sD);
-                if (lt1.active) grad_pass<G, 1>(lt1, sFs, sX, sD);
-            }
-            if constexpr (STAGED) {
-                // Bounded wait for group g's spans; every thread learns the outcome.
-                const bool ok = mbar_wait(sBar, phase);
-                phase ^= 1u;
-                if (__syncthreads_or(!ok)) {
-                    if (tid == 0) report_wait_fault(tabs);
-                    return;
-                }
-            } else {
-                __syncthreads();
-            }
-            if (lt2.active) {
-                const int ee = g * NE + lt2.el;
-                const bool eok = ee < nelem;
-                // Point c's He row and gpvol: staged, in registers from the
-                // start of the group, or loaded here (one point ahead).
-                auto he_row = [&](int c, real(&h)[9], real &gp) {
-                    const int a = sPerm[line_lat<2, Q>(lt2.la, lt2.lb, c)];
-                    if constexpr (!LATE) {
+    }
+    __syncthreads();
+    if (t.active) {
+        diffu_div<G, 0>(t, sm);
+        diffu_div<G, 1>(t, sm);
+    }
+    __syncthreads();
 #pragma unroll
-                        for (int j = 0; j < 9; ++j) h[j] = Hm[c < MP ? c : 0][j];
-                        gp = gv[c < MP ? c : 0];
-                    } else if constexpr (STAGED) {
-                        const real *hp = reinterpret_cast<const real *>(sHeB) + he_off + (lt2.el * N + a) * 9;
-#pragma unroll
-                        for (int j = 0; j < 9; ++j) h[j] = hp[j];
-                        gp = reinterpret_cast<const real *>(sGpB)[gp_off + lt2.el * N + a];
-                    } else {
-                        const real *hp = He + (eok ? ((size_t)ee * N + a) * 9 : 0);
-#pragma unroll
-                        for (int j = 0; j < 9; ++j) h[j] = eok ? ldg(hp + j) : (real)0;
-                        gp = eok ? ldg(gpvol + (size_t)ee * N + a) : (real)0;
-                    }
-                };
-                auto mu_at = [&](int o, real r) -> real { return point_mu_e(g, lt2.el, o, r, sFs); };
-                zeta_stage<G>(lt2, sFs, sX, he_row, mu_at, Cp, Pr);
-            }
-            __syncthreads();
-            if constexpr (STAGED) {
-                if (gn < ngroups) stage(gn);  // the spans of the next group, during the divergence
-            }
-            if (eo) {
-                if (lt0.active) div_pass<G, 0, false, false, EOK>(lt0, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-                __syncthreads();
-                if (lt1.active) div_pass<G, 1, false, true, EOK>(lt1, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-            } else {
-                if (lt0.active) div_pass<G, 0, false, false>(lt0, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-                __syncthreads();
-                if (lt1.active) div_pass<G, 1, false, true>(lt1, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-            }
-        } else {
-            if (lt0.active) grad_pass<G, 0>(lt0, sFs, sX, sD);
-            if (lt1.active) grad_pass<G, 1>(lt1, sFs, sX, sD);
-            if (lt2.active) grad_pass<G, 2>(lt2, sFs, sX, sD);
-            __syncthreads();
-            // Point pass: physical gradients, stress and contravariant fluxes.
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const int i = tid + k * NT;
-                if (i >= NE * N) break;
-                const int el = i / N, l = i - el * N;
-                const int o = el * ES + (l / (Q * Q) * Q + (l / Q) % Q) * QP + l % Q;
-                real gi[3][5];
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) gi[d][f] = sX[(d * 5 + f) * NPL + o];
-                const real r = sFs[D_RHO * NPL + o];
-                const real uu[3] = {sFs[D_U0 * NPL + o], sFs[D_U1 * NPL + o], sFs[D_U2 * NPL + o]};
-                const real muf = sFs[D_MUF * NPL + o], ms = sFs[D_MUS * NPL + o];
-                const real me = point_mu_e(g, el, o, r, sFs);
-                real F[3][NX];
-                point_flux(gi, r, uu, muf, ms, me, Hm[k], gv[k], F);
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-#pragma unroll
-                    for (int x = 0; x < NX; ++x) sX[(d * NX + x) * NPL + o] = F[d][x];
-                sFs[P_NUE * NPL + o] = me / r;
-                sFs[P_KAP * NPL + o] = kappa_e(muf, me, ms, r, Cp, Pr);
-            }
-            __syncthreads();
-            if (lt0.active) div_pass<G, 0, true, false>(lt0, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-            __syncthreads();
-            if (lt1.active) div_pass<G, 1, false, false>(lt1, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-            __syncthreads();
-            if (lt2.active) div_pass<G, 2, false, true>(lt2, sFs, sX, sD, sNs, npoin, Rmass, Rmom, Rener);
-        }
-        __syncthreads();
-        if (NBUF == 1 && gn < ngroups) {  // the next group's node ids, then its fields
-            store_ids(ids, sNode);
-            __syncthreads();
-            gather(gn, sNode, sF);
-            if (gn + stride < ngroups) load_ids(gn + stride, ids);
-        }
+    for (int k = 0; k < Q; ++k) {
+        if (id[k] < 0) continue;
+        const int o = base + k * G::template step<2>();
+        const Four<real> x1 = sm.X1()[o], x2 = sm.X2()[o], x3 = sm.X3()[o];
+        const R2 s0 = add2(add2(acc[k][0], x1.a), x3.a), s1 = add2(add2(acc[k][1], x1.b), x3.b),
+                 s2 = add2(add2(acc[k][2], x2.a), x2.b);
+        red_add(Rmass + id[k], nu[k] * s0.x);
+        red_add(Rener + id[k], fma(kap[k], s1.x, s0.y));
+        red_add(Rmom + id[k], s1.y);
+        red_add(Rmom + np + id[k], s2.x);
+        red_add(Rmom + 2 * np + id[k], s2.y);
     }
 }
 
@@ -459,34 +364,20 @@ template <typename real, int P, int VISC>
 cudaError_t launch_diffu_pn(const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st)
 {
     using G = DiffuGeom<real, P>;
-    constexpr size_t smem = diffu_smem_bytes<G>();
+    constexpr size_t smem = DiffuShared<G>::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    static_assert(G::NE >= 1, "element group");
-    auto kern = diffu_kernel<G, VISC>;
+    auto kern = diffu_kernel<G, VISC, diffu_minb<real, P>()>;
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    if (sizeof(real) == 4) {
-        err = cudaMemcpyToSymbolAsync(c_Df, table_D<float>(tabs), sizeof(float) * 3 * G::Q * G::Q,
-                                      sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
-        constexpr bool eo = ((DIFFU_EO >> P) & 1) != 0 && diffu_fusez<G>();
-        if (err == cudaSuccess && eo)
-            err = cudaMemcpyToSymbolAsync(c_DEO, tabs->EO, sizeof(float) * kTableEOMax,
-                                          sizeof(float) * kTableEOMax * P, cudaMemcpyDeviceToDevice, st);
-        if (err == cudaSuccess && eo)
-            err = cudaMemcpyToSymbolAsync(c_DEOp, tabs->EOp, sizeof(float) * kTableEOMax,
-                                          sizeof(float) * kTableEOMax * P, cudaMemcpyDeviceToDevice, st);
-    }
+    constexpr size_t nb = sizeof(real) * 3 * G::Q * G::Q, off = sizeof(real) * kTableDMax * P;
+    if (sizeof(real) == 4)
+        err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, nb, off, cudaMemcpyDeviceToDevice, st);
     else
-        err = cudaMemcpyToSymbolAsync(c_Dd, table_D<double>(tabs), sizeof(double) * 3 * G::Q * G::Q,
-                                      sizeof(double) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
+        err = cudaMemcpyToSymbolAsync(c_Dd, tabs->Dd, nb, off, cudaMemcpyDeviceToDevice, st);
     if (err != cudaSuccess) return err;
-    const int ngroups = (a.nelem + G::NE - 1) / G::NE;
-    const int grid = persistent_grid(kern, G::NT, smem, ngroups);
-    if (grid <= 0) return cudaErrorInvalidConfiguration;
-    const int linemap = DIFFU_LINEMAP_MODE == 2 ? (a.npoin < (long long)a.nelem * G::N ? 1 : 0) : DIFFU_LINEMAP_MODE;
-    kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, ngroups, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u,
-                                    a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem, a.Rmass, a.Rmom, a.Rener,
-                                    linemap);
+    const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
+    kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem,
+                                    a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem, a.Rmass, a.Rmom, a.Rener);
     return cudaGetLastError();
 }
 

@@ -16,37 +16,10 @@ constexpr int kTableDMax = 3 * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
 // D[d][r][c] at [(d*Q + r)*Q + c], followed at 3*Q*Q by its row sums [d*Q + r].
 constexpr int kTableDSMax = kTableDMax + 3 * (MSOD_MAX_PORDER + 1);
 constexpr int kTableNMax = (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
-// Row pairs of the FP32 matrices for packed (f32x2) contractions:
-// Dp[((d*Q + c)*H + m)*2 + t] = D[d][2m+t][c] (zero for 2m+t = Q), H = (Q+1)/2.
-constexpr int kTableDPairMax = 3 * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 2);
-// Even-odd form of the FP32 matrix (one direction), valid when the three
-// directions' matrices are equal and centro-antisymmetric, as the GLL
-// derivative matrix is: D[s'(r)][s'(c)] = -D[r][c] where s' mirrors a node
-// through the element centre.  Lines are stored in the reference's SOD 1-D
-// order (the two ends first, then the interior: natural indices 0, P, 1, ...,
-// P-1), where the mirror is sod_mirror.  With M = Q/2 mirror pairs (L_i,
-// s'(L_i)), L_i = sod_left(i), and for odd Q the centre node m:
-//   EO[i*M + j]           A = (D[L_i][L_j] - D[L_i][s'(L_j)]) / 2
-//   EO[M*M + i*M + j]     B = (D[L_i][L_j] + D[L_i][s'(L_j)]) / 2
-//   EO[2*M*M + i]         D[L_i][m]                         (odd Q)
-//   EO[2*M*M + M + j]     D[m][L_j]                         (odd Q)
-// so that, with e_j = v[L_j] + v[s'(L_j)] and o_j = v[L_j] - v[s'(L_j)],
-// d[L_i] = S_i + T_i and d[s'(L_i)] = S_i - T_i for S_i = sum_j A o_j and
-// T_i = sum_j B e_j (+ D[L_i][m] v[m]), and d[m] = sum_j D[m][L_j] o_j.
-__host__ __device__ constexpr int sod_mirror(int Q, int s) { return s == 0 ? 1 : (s == 1 ? 0 : Q + 1 - s); }
-__host__ __device__ constexpr int sod_left(int i) { return i == 0 ? 0 : i + 1; }
-__host__ __device__ constexpr int sod_centre(int Q) { return (Q + 1) / 2; }
-constexpr int kTableEOMax = 2 * (MSOD_MAX_PORDER / 2 + 1) * (MSOD_MAX_PORDER / 2 + 1) + 2 * (MSOD_MAX_PORDER / 2 + 1);
 struct TableScratch {
     float Df[kTableDSMax];
-    float EO[kTableEOMax];
-    int eo_ok;  // 1 when EO represents all three directions' matrices
     int same_dirs;  // 1 when the three directions' matrices are equal
-    // The even-odd A and B entries side by side, for packed (f32x2)
-    // contractions: EOp[2*(i*M + j)] = A[i][j], EOp[2*(i*M + j) + 1] = B[i][j].
-    alignas(8) float EOp[kTableEOMax];
     double Dd[kTableDSMax];
-    alignas(8) float Dp[kTableDPairMax];
     int perm[kTableNMax];
     int lat[kTableNMax];
     // Set (sticky, zero at allocation) by a kernel whose bounded wait for a
@@ -111,13 +84,6 @@ template <typename real>
 cudaError_t launch_convec_plain(int porder, const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
 template <typename real>
 cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
-// Both plain FP32 kernels on the same inputs (outputs zeroed by the caller;
-// tables prepared): one kernel where fused_porder(porder), else the two
-// kernels in turn.  The convection and diffusion outputs must not overlap.
-bool fused_porder(int porder);
-cudaError_t launch_fused(int porder, const ConvecArgs<float> &c, const DiffuArgs<float> &d, const TableScratch *tabs,
-                         cudaStream_t st);
-
 // Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by the
 // caller; tables prepared).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
 struct MixedConvecArgs {
