@@ -139,13 +139,20 @@ static int check_wait_fault(TableScratch *tabs, cudaStream_t st, const char *wha
 }
 
 template <typename real>
-static int zero_outputs(real *Rmass, real *Rmom, real *Rener, int npoin, cudaStream_t st)
+static void add_outputs(ZeroSpans &z, real *Rmass, real *Rmom, real *Rener, int npoin)
 {
     const size_t b = sizeof(real) * (size_t)npoin;
-    int rc = cuda_status(cudaMemsetAsync(Rmass, 0, b, st), "cudaMemsetAsync(Rmass)");
-    if (!rc) rc = cuda_status(cudaMemsetAsync(Rmom, 0, 3 * b, st), "cudaMemsetAsync(Rmom)");
-    if (!rc) rc = cuda_status(cudaMemsetAsync(Rener, 0, b, st), "cudaMemsetAsync(Rener)");
-    return rc;
+    z.add(Rmass, b);
+    z.add(Rmom, 3 * b);
+    z.add(Rener, b);
+}
+
+template <typename real>
+static int zero_outputs(real *Rmass, real *Rmom, real *Rener, int npoin, cudaStream_t st)
+{
+    ZeroSpans z;
+    add_outputs(z, Rmass, Rmom, Rener, npoin);
+    return cuda_status(launch_zero(z, st), "residual zeroing launch");
 }
 
 template <typename real>
@@ -172,8 +179,7 @@ static int convec_impl(int porder, int nelem, int npoin, const int *connec, cons
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlx;
     a.invAtoIJK = inv; a.AtoI = ai; a.AtoJ = aj; a.AtoK = ak;
     a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E; a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
-    rc = cuda_status(launch_table_prep<real>(porder, a, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_convec_plain<real>(porder, a, tabs, st), "convection kernel launch");
+    rc = cuda_status(launch_convec_plain<real>(porder, a, tabs, st), "convection kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection kernel");
     return rc;
 }
@@ -205,8 +211,7 @@ static int diffu_impl(int porder, int nelem, int npoin, const int *connec, const
     a.invAtoIJK = inv; a.AtoI = ai; a.AtoJ = aj; a.AtoK = ak; a.Cp = Cp; a.Pr = Pr;
     a.rho = rho; a.u = u; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mu_e = mu_e; a.mu_sgs = mu_sgs; a.nu_elem = nu_elem;
     a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
-    rc = cuda_status(launch_table_prep<real>(porder, a, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_diffu_plain<real>(porder, a, tabs, st), "diffusion kernel launch");
+    rc = cuda_status(launch_diffu_plain<real>(porder, a, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "diffusion kernel");
     return rc;
 }
@@ -237,8 +242,10 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     }
     TableScratch *tabs = device_tables(porder);
     if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
-    rc = zero_outputs(Rmass_c, Rmom_c, Rener_c, npoin, st);
-    if (!rc) rc = zero_outputs(Rmass_d, Rmom_d, Rener_d, npoin, st);
+    ZeroSpans z;
+    add_outputs(z, Rmass_c, Rmom_c, Rener_c, npoin);
+    add_outputs(z, Rmass_d, Rmom_d, Rener_d, npoin);
+    rc = cuda_status(launch_zero(z, st), "residual zeroing launch");
     if (rc) return rc;
     ConvecArgs<float> c;
     c.nelem = nelem; c.npoin = npoin; c.connec = connec; c.He = He; c.gpvol = gpvol; c.dlxigp_ip = dlx;
@@ -248,8 +255,7 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     static_cast<ElementArgs<float> &>(d) = c;
     d.Cp = Cp; d.Pr = Pr; d.rho = rho; d.u = u; d.Tem = Tem; d.mu_fluid = mu_fluid; d.mu_e = mu_e;
     d.mu_sgs = mu_sgs; d.nu_elem = nullptr; d.Rmass = Rmass_d; d.Rmom = Rmom_d; d.Rener = Rener_d;
-    rc = cuda_status(launch_table_prep<float>(porder, c, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_convec_plain<float>(porder, c, tabs, st), "convection kernel launch");
+    rc = cuda_status(launch_convec_plain<float>(porder, c, tabs, st), "convection kernel launch");
     if (!rc) rc = cuda_status(launch_diffu_plain<float>(porder, d, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection + diffusion kernel");
     return rc;

@@ -58,33 +58,19 @@
 namespace msod {
 namespace {
 
-// 1-D derivative matrices and their row sums of the current call, per porder
-// (copied from the per-call table area before the launch).
-__constant__ float c_CDf[MSOD_MAX_PORDER + 1][kTableDSMax];
-__constant__ double c_CDd[MSOD_MAX_PORDER + 1][kTableDSMax];
-template <typename real>
-__device__ __forceinline__ real cCD(int P, int i);
-template <>
-__device__ __forceinline__ float cCD<float>(int P, int i)
-{
-    return c_CDf[P][i];
-}
-template <>
-__device__ __forceinline__ double cCD<double>(int P, int i)
-{
-    return c_CDd[P][i];
-}
-
 // Elements per block, threads per line, blocks per SM that the register budget
 // allows for, and the form of the passes, measured per porder (FP32, ms).
 // Whole warps of lines count most (5 x 25 lines at porder 4: 125 of 128
-// threads): on 64^3 porder-4 hexes 5 elements take 0.944 (1.044 before the pitch
-// search, where 4, with 100 of 128 threads, took 1.15, 6 1.17, 8 1.13, 9 1.10).  A fourth block per SM (12 bytes per point less
-// through kSlots, 128 registers) gains nothing: 1.04.
+// threads), then what is left of the L1 beside the blocks' shared memory, where
+// the gathers' lines are in flight: three blocks of 64 KB stay within a 196 KB
+// carveout.  On 64^3 porder-4 hexes 5 elements take 0.944 (1.044 before the
+// pitch search, where 4, with 100 of 128 threads, took 1.15, 6 1.17, 8 1.13, 9
+// 1.10).  A fourth block per SM (12 bytes per point less through kSlots, 128
+// registers) gains nothing: 1.04.
 template <typename real, int P>
 constexpr int convec_ne()
 {
-    constexpr int nf[9] = {0, 32, 16, 8, 5, 4, 2, 2, 2}, nd[9] = {0, 32, 14, 8, 5, 3, 2, 1, 1};
+    constexpr int nf[9] = {0, 32, 14, 8, 5, 4, 2, 2, 2}, nd[9] = {0, 32, 14, 8, 5, 3, 2, 1, 1};
     return sizeof(real) == 4 ? nf[P] : nd[P];
 }
 // Two threads share a line where one would spill (porder 8; FP64 from 7 up).
@@ -98,17 +84,18 @@ constexpr int convec_s()
 template <typename real, int P>
 constexpr int convec_minb()
 {
-    constexpr int nb[9] = {0, 1, 1, 4, 3, 2, 2, 1, 1};
+    constexpr int nb[9] = {0, 1, 4, 4, 3, 2, 2, 1, 1};
     return sizeof(real) == 4 ? nb[P] : 1;
 }
 // All points of a line at once (the pairs' differences shared) or one point
 // after the other (fewer registers): porder 3 0.711 / 0.738, 4 0.944 / 1.05, 6
-// 1.052 / 1.149 (40^3), but 5 1.169 / 1.143 (51^3) and 7 0.855 / 0.786 (32^3),
-// where the sums of all points no longer fit beside the line.
+// 1.052 / 1.149 (40^3), but 2 0.565 / 0.557 (100^3), 5 1.169 / 1.143 (51^3) and 7
+// 0.855 / 0.786 (32^3), where the sums of all points no longer fit beside the
+// line.
 template <typename real, int P>
 constexpr bool convec_all_points()
 {
-    return sizeof(real) == 4 && P <= 6 && P != 5;
+    return sizeof(real) == 4 && (P == 1 || P == 3 || P == 4 || P == 6);
 }
 // The three directions as one copy of the pass with run-time strides (porders
 // 6 to 8, whose unrolled passes overrun the instruction cache: porder 6 1.052 /
@@ -140,8 +127,8 @@ struct ConvecShared {
     static constexpr size_t kZ = kA + G::NREC * (kSlots ? sizeof(Two<real>) : sizeof(Four<real>));
     static constexpr size_t kM = kZ + G::NREC * sizeof(real);
     static constexpr size_t kNode = kM + G::NREC * sizeof(real);
-    static constexpr size_t kPerm = kNode + (kSlots ? 0 : G::NREC * sizeof(int));
-    static constexpr size_t kBytes = kPerm + G::N * sizeof(int);
+    static constexpr size_t kTab = (kNode + (kSlots ? 0 : G::NREC * sizeof(int)) + 15) / 16 * 16;
+    static constexpr size_t kBytes = kTab + GroupTables<G, true>::kBytes;
     unsigned char *base;
     __device__ __forceinline__ unsigned long long *bar() const
     {
@@ -192,7 +179,7 @@ struct ConvecShared {
         else
             return node()[o];
     }
-    __device__ __forceinline__ int *perm() const { return reinterpret_cast<int *>(base + kPerm); }
+    __device__ __forceinline__ GroupTables<G, true> tab() const { return GroupTables<G, true>{base + kTab}; }
 };
 
 // The records of one line.
@@ -227,20 +214,6 @@ struct ConvecDir {
         lat = t.lat0(dir);
     }
 };
-// Coefficient i of direction dir; SAME: the three directions share one matrix
-// (as every table of the reference does), and the coefficient is an immediate
-// operand from the constant bank.
-template <class G, bool SAME>
-__device__ __forceinline__ typename G::real convec_D(int dir, int i)
-{
-    return cCD<typename G::real>(G::P, SAME ? i : dir * G::Q * G::Q + i);
-}
-template <class G, bool SAME>
-__device__ __forceinline__ typename G::real convec_rowsum(int dir, int r)
-{
-    return cCD<typename G::real>(G::P, 3 * G::Q * G::Q + (SAME ? r : dir * G::Q + r));
-}
-
 template <class G>
 __device__ __forceinline__ void convec_finish(const ConvecDir<G> &d, const ConvecShared<G> &sm,
                                               const GroupMetric<G> &gm, int el, int o, int pt, int node0,
@@ -270,9 +243,9 @@ __device__ __forceinline__ void convec_finish(const ConvecDir<G> &d, const Conve
 }
 
 // Points R0 .. R0+R-1 of a line, one after the other.
-template <class G, bool SAME, int SEG>
+template <class G, int SEG>
 __device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const GroupThread<G> &t, const ConvecDir<G> &d,
-                                              const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                              const ConvecShared<G> &sm, const GroupRows<G, true> &tab, const GroupMetric<G> &gm,
                                               const int (&id)[G::R], int npoin,
                                               typename G::real *__restrict__ Rmass,
                                               typename G::real *__restrict__ Rmom,
@@ -284,7 +257,7 @@ __device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const Gro
     constexpr real k2 = (real)2, k3 = (real)3, k4 = (real)4;
 #pragma unroll
     for (int r = R0; r < R1; ++r) {
-        const int pt = sm.perm()[d.lat + r * d.lstep];
+        const int pt = tab.node(d.lat + r * d.lstep);
         const real *hp = gm.he(t.el, pt) + d.dir * 3;
         const real h0 = hp[0], h1 = hp[1], h2 = hp[2];
         const Four<real> wr = ln.w[r], vr = ln.v[r];
@@ -293,11 +266,12 @@ __device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const Gro
         const real Qc = fma(vr.b.x, h2, fma(vr.a.y, h1, vr.a.x * h0));
         const real X0 = U + U, Y0 = fma(rr, U, Qc);
         R2 A = two((real)0, (real)0), B = A, dz = A, dq = A;  // momentum 1-2; momentum 3, energy; drho, dp; dq 1-2
-        real dq3 = (real)0, divu = (real)0;
+        real dq3 = (real)0, divu = (real)0, Dr[Q];
+        tab.row(Dr, d.dir, r);
 #pragma unroll
         for (int s = 0; s < Q; ++s) {
             if (s == r) continue;
-            const real D = convec_D<G, SAME>(d.dir, r * Q + s);
+            const real D = Dr[s];
             const R2 D2 = two(D, D);
             const R2 wa = sub2(ln.w[s].a, wr.a), wb = sub2(ln.w[s].b, wr.b);
             const R2 va = sub2(ln.v[s].a, vr.a), vb = sub2(ln.v[s].b, vr.b);
@@ -311,7 +285,7 @@ __device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const Gro
             dq3 = fma(D, vb.x, dq3);
             divu = fma(D, tt, divu);
         }
-        const real sg = convec_rowsum<G, SAME>(d.dir, r);
+        const real sg = tab.sum(d.dir, r);
         const real divq = fma(dq3, h2, fma(dq.y, h1, dq.x * h0));
         const real S = fma(rr, divu, fma(U, dz.x, divq));
         const real cw = fma(k2 * sg, Y0, S), cv = fma(k3 * sg, U, k2 * divu);
@@ -327,9 +301,9 @@ __device__ __forceinline__ void convec_points(const ConvecLine<G> &ln, const Gro
 
 // All points of a line at once: the differences of a pair of points serve both
 // of its rows.
-template <class G, bool SAME>
+template <class G>
 __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const GroupThread<G> &t, const ConvecDir<G> &d,
-                                             const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                             const ConvecShared<G> &sm, const GroupRows<G, true> &tab, const GroupMetric<G> &gm,
                                               const int (&id)[G::R], int npoin,
                                              typename G::real *__restrict__ Rmass, typename G::real *__restrict__ Rmom,
                                              typename G::real *__restrict__ Rener)
@@ -343,7 +317,7 @@ __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const Grou
     real h[Q][3], U[Q], Y0[Q], dq3[Q], divu[Q];
     R2 A[Q], B[Q], dz[Q], dq[Q];
 #pragma unroll
-    for (int r = 0; r < Q; ++r) pt[r] = sm.perm()[d.lat + r * d.lstep];
+    for (int r = 0; r < Q; ++r) pt[r] = tab.node(d.lat + r * d.lstep);
 #pragma unroll
     for (int r = 0; r < Q; ++r) {
         const real *hp = gm.he(t.el, pt[r]) + d.dir * 3;
@@ -359,7 +333,10 @@ __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const Grou
         dq3[r] = divu[r] = (real)0;
     }
 #pragma unroll
-    for (int r = 0; r < Q; ++r)
+    for (int r = 0; r < Q - 1; ++r) {
+        real Dr[Q], Dc[Q];  // row and column r
+        tab.row(Dr, d.dir, r);
+        tab.col(Dc, d.dir, r);
 #pragma unroll
         for (int s = r + 1; s < Q; ++s) {
             const R2 wa = sub2(ln.w[s].a, ln.w[r].a), wb = sub2(ln.w[s].b, ln.w[r].b);
@@ -368,8 +345,8 @@ __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const Grou
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
                 // Row m, its partner's values minus its own = sign * the differences.
-                const int m = side ? s : r, o = side ? r : s;
-                const real D0 = convec_D<G, SAME>(d.dir, m * Q + o), D = side ? -D0 : D0;
+                const int m = side ? s : r;
+                const real D = side ? -Dc[s] : Dr[s];
                 const real tt = fma(wb.x, h[m][2], fma(wa.y, h[m][1], wa.x * h[m][0]));
                 const real x0 = U[m] + U[m];
                 const real X = D * (side ? x0 - tt : x0 + tt), Y = D * fma(side ? -ln.z[m].x : ln.z[m].x, tt, Y0[m]);
@@ -381,10 +358,11 @@ __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const Grou
                 divu[m] = fma(D, tt, divu[m]);
             }
         }
+    }
 #pragma unroll
     for (int r = 0; r < Q; ++r) {
         const real rr = ln.z[r].x, Ur = U[r];
-        const real sg = convec_rowsum<G, SAME>(d.dir, r);
+        const real sg = tab.sum(d.dir, r);
         const real divq = fma(dq3[r], h[r][2], fma(dq[r].y, h[r][1], dq[r].x * h[r][0]));
         const real S = fma(rr, divu[r], fma(Ur, dz[r].x, divq));
         const real cw = fma(k2 * sg, Y0[r], S), cv = fma(k3 * sg, Ur, k2 * divu[r]);
@@ -398,9 +376,9 @@ __device__ __forceinline__ void convec_pairs(const ConvecLine<G> &ln, const Grou
     }
 }
 
-template <class G, bool SAME>
+template <class G>
 __device__ __forceinline__ void convec_pass(ConvecLine<G> &ln, const GroupThread<G> &t, int ip,
-                                            const ConvecShared<G> &sm, const GroupMetric<G> &gm,
+                                            const ConvecShared<G> &sm, const GroupRows<G, true> &tab, const GroupMetric<G> &gm,
                                               const int (&id)[G::R], int npoin,
                                             typename G::real *__restrict__ Rmass,
                                             typename G::real *__restrict__ Rmom,
@@ -416,24 +394,25 @@ __device__ __forceinline__ void convec_pass(ConvecLine<G> &ln, const GroupThread
         }
     }
     if constexpr (G::S == 1 && convec_all_points<typename G::real, G::P>()) {
-        convec_pairs<G, SAME>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        convec_pairs<G>(ln, t, d, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
     } else if constexpr (G::S == 1) {
-        convec_points<G, SAME, 0>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        convec_points<G, 0>(ln, t, d, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
     } else {
         if (t.seg == 0)
-            convec_points<G, SAME, 0>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+            convec_points<G, 0>(ln, t, d, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
         else
-            convec_points<G, SAME, 1>(ln, t, d, sm, gm, id, npoin, Rmass, Rmom, Rener);
+            convec_points<G, 1>(ln, t, d, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
     }
 }
 
 template <class G, int MINB>
 __global__ void __launch_bounds__(G::NT, MINB)
-    convec_kernel(int nelem, int npoin, int ngroups, const int *__restrict__ connec,
+    convec_kernel(int nelem, int npoin, const int *__restrict__ connec,
                   const typename G::real *__restrict__ He, const typename G::real *__restrict__ gpvol,
                   const typename G::real *__restrict__ u, const typename G::real *__restrict__ q,
                   const typename G::real *__restrict__ rho, const typename G::real *__restrict__ pr,
-                  const typename G::real *__restrict__ E, const TableScratch *__restrict__ tabs,
+                  const typename G::real *__restrict__ E, const int *__restrict__ inv,
+                  const typename G::real *__restrict__ dlxigp_ip, const TableScratch *__restrict__ tabs,
                   typename G::real *__restrict__ Rmass, typename G::real *__restrict__ Rmom,
                   typename G::real *__restrict__ Rener)
 {
@@ -447,7 +426,6 @@ __global__ void __launch_bounds__(G::NT, MINB)
     const int r0 = t.seg * R;
     const int e0 = blockIdx.x * G::NE;
     const GroupMetric<G> gm(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);
-    for (int i = tid; i < N; i += G::NT) sm.perm()[i] = ldg(&tabs->perm[i]);
     ConvecLine<G> ln;
     int id[R];  // the nodes of the thread's points of its zeta line (-1: none)
     {
@@ -456,24 +434,25 @@ __global__ void __launch_bounds__(G::NT, MINB)
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const bool ok = t.active && e < nelem && (R * G::S == Q || r0 + k < Q);
-            const int row = ok ? ldg(&tabs->perm[t.template lat<2>(r0 + k)]) : 0;
-            const int v = ok ? ldg(connec + (size_t)row * nelem + e) - 1 : -1;
+            const int row = ok ? GroupTables<G, true>::node(inv, t.template lat<2>(r0 + k)) : 0;
+            const int v = ok ? ldg_once(connec + (size_t)row * nelem + e) - 1 : -1;
             id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
         }
+        sm.tab().build(inv, dlxigp_ip, tid);
         real f[R][9];
 #pragma unroll
         for (int k = 0; k < R; ++k) {
             const bool ok = id[k] >= 0;  // a missing node reads as zeros
             const size_t p = ok ? (size_t)id[k] : 0;
-            f[k][0] = ok ? ldg(u + p) : (real)0;
-            f[k][1] = ok ? ldg(u + np + p) : (real)0;
-            f[k][2] = ok ? ldg(u + 2 * np + p) : (real)0;
-            f[k][3] = ok ? ldg(E + p) : (real)0;
-            f[k][4] = ok ? ldg(q + p) : (real)0;
-            f[k][5] = ok ? ldg(q + np + p) : (real)0;
-            f[k][6] = ok ? ldg(q + 2 * np + p) : (real)0;
-            f[k][7] = ok ? ldg(rho + p) : (real)0;
-            f[k][8] = ok ? ldg(pr + p) : (real)0;
+            f[k][0] = ok ? ldg_once(u + p) : (real)0;
+            f[k][1] = ok ? ldg_once(u + np + p) : (real)0;
+            f[k][2] = ok ? ldg_once(u + 2 * np + p) : (real)0;
+            f[k][3] = ok ? ldg_once(E + p) : (real)0;
+            f[k][4] = ok ? ldg_once(q + p) : (real)0;
+            f[k][5] = ok ? ldg_once(q + np + p) : (real)0;
+            f[k][6] = ok ? ldg_once(q + 2 * np + p) : (real)0;
+            f[k][7] = ok ? ldg_once(rho + p) : (real)0;
+            f[k][8] = ok ? ldg_once(pr + p) : (real)0;
         }
         const int base = t.rec0(2);
 #pragma unroll
@@ -497,13 +476,11 @@ __global__ void __launch_bounds__(G::NT, MINB)
     __syncthreads();
     // Bounded wait for the bulk copies; a wait that ran out is reported and
     // nothing is assembled (every thread learns it at the barrier below).
+    const GroupRows<G, true> tab(sm.tab());
     const bool ok = gm.wait(sm.bar());
-    const bool same = ldg(&tabs->same_dirs) != 0;  // uniform over the grid
     auto pass = [&](int ip) {
-        if (same)
-            convec_pass<G, true>(ln, t, ip, sm, gm, id, npoin, Rmass, Rmom, Rener);
-        else
-            convec_pass<G, false>(ln, t, ip, sm, gm, id, npoin, Rmass, Rmom, Rener);
+        if (ip == 2) grid_dependency_wait();  // the residuals are zeroed
+        convec_pass<G>(ln, t, ip, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
         if (ip < 2 && __syncthreads_or(!ok)) {
             if (tid == 0) report_wait_fault(tabs);
             return false;
@@ -529,18 +506,12 @@ cudaError_t launch_convec_p(const ConvecArgs<real> &a, const TableScratch *tabs,
     static_assert(smem <= 227 * 1024, "shared memory budget");
     if (!tabs) return cudaErrorInvalidValue;
     auto kern = convec_kernel<G, convec_minb<real, P>()>;
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
-    constexpr size_t nb = sizeof(real) * (3 * G::Q * G::Q + 3 * G::Q), off = sizeof(real) * kTableDSMax * P;
-    if (sizeof(real) == 4)
-        err = cudaMemcpyToSymbolAsync(c_CDf, tabs->Df, nb, off, cudaMemcpyDeviceToDevice, st);
-    else
-        err = cudaMemcpyToSymbolAsync(c_CDd, tabs->Dd, nb, off, cudaMemcpyDeviceToDevice, st);
-    if (err != cudaSuccess) return err;
-    const int ngroups = (a.nelem + G::NE - 1) / G::NE;
-    kern<<<ngroups, G::NT, smem, st>>>(a.nelem, a.npoin, ngroups, a.connec, a.He, a.gpvol, a.u, a.q, a.rho, a.pr, a.E,
-                                    tabs, a.Rmass, a.Rmom, a.Rener);
-    return cudaGetLastError();
+    const unsigned ngroups = (unsigned)((a.nelem + G::NE - 1) / G::NE);
+    return launch_after(kern, ngroups, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.u, a.q, a.rho,
+                        a.pr, a.E, a.invAtoIJK, a.dlxigp_ip, tabs, a.Rmass, a.Rmom, a.Rener);
 }
 
 }  // namespace

@@ -20,11 +20,28 @@ __device__ __forceinline__ void red_add(double *addr, double v)
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(addr), "d"(v) : "memory");
 }
 
+// Programmatic dependent launch: let the next kernel of the stream start; wait
+// until the kernel ahead (if this one was launched after it that way) has
+// finished and its writes are visible.
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Read-only global loads through the non-coherent path.
 template <typename T>
 __device__ __forceinline__ T ldg(const T *p)
 {
     return __ldg(p);
+}
+
+// Gathers of node fields and element rows: through L2 only (a block reads a
+// sector of them once; what is left of the L1 beside the shared memory holds
+// fewer lines than a block has in flight).  Diffusion, porder 7 on 32^3 hexes
+// 0.791 against 0.817 ms through L1, porder 6 on 40^3 1.005 / 1.033, porder 4 on
+// 64^3 0.951 / 0.961; convection, porder 7 0.781 / 0.795, porder 4 0.941 / 0.936.
+template <typename T>
+__device__ __forceinline__ T ldg_once(const T *p)
+{
+    return __ldcg(p);
 }
 
 // Per-porder launch geometry of the line-parallel element kernels.

@@ -39,20 +39,27 @@
 namespace msod {
 namespace {
 
+// 1-D derivative matrices of the current call, per porder (large meshes: copied
+// from the per-call table area before the launch).
 __constant__ float c_Df[MSOD_MAX_PORDER + 1][kTableDMax];
-__constant__ double c_Dd[MSOD_MAX_PORDER + 1][kTableDMax];
-template <typename real>
-__device__ __forceinline__ real cD(int P, int i);
-template <>
-__device__ __forceinline__ float cD<float>(int P, int i)
-{
-    return c_Df[P][i];
-}
-template <>
-__device__ __forceinline__ double cD<double>(int P, int i)
-{
-    return c_Dd[P][i];
-}
+
+// The matrices' rows: shared-memory tables of the block, or (CONSTD) operands
+// from the constant bank.
+template <class G, bool CONSTD>
+struct DiffuRows {
+    GroupRows<G, false> tab;
+    __device__ __forceinline__ explicit DiffuRows(const GroupTables<G, false> &t) : tab(t) {}
+    __device__ __forceinline__ void row(typename G::real (&v)[G::Q], int dir, int r) const { tab.row(v, dir, r); }
+};
+template <class G>
+struct DiffuRows<G, true> {
+    __device__ __forceinline__ explicit DiffuRows(const GroupTables<G, false> &) {}
+    __device__ __forceinline__ void row(typename G::real (&v)[G::Q], int dir, int r) const
+    {
+#pragma unroll
+        for (int c = 0; c < G::Q; ++c) v[c] = c_Df[G::P][(dir * G::Q + r) * G::Q + c];
+    }
+};
 
 // Viscosity source of the diffusion kernel: the mu_e array, or one value per
 // element (mu_e(e, a) = rho(a) nu_elem(e)).
@@ -60,15 +67,17 @@ enum { VISC_MU_E = 0, VISC_NU_ELEM = 1 };
 
 // Elements per block and blocks per SM that the register budget allows for.
 // Whole warps of lines (5 x 25 lines at porder 4: 125 of 128 threads) count
-// most; the FP64 kernels, bound by FP64 issue, which a warp pays for its idle
-// lanes too, take the same groups.  Measured in FP32 (ms, 64^3 hexes at porder
-// 4): 5 elements at four blocks 1.141, at three 1.152, 8 elements at two 1.302,
-// 9 at two 1.284, 4 at four 1.236.  Porder 5 (51^3): 3 elements at three blocks
-// 1.162, at four 1.409 (spills), 4 at two 1.250, 7 at one 1.546.  Porder 6
-// (40^3): 3 at one 1.229, 2 at two 1.266, 4 at one 1.394.  Porder 7 (32^3): 2
-// at two 0.991, 1 at three 1.142, 3 at one 1.043.  Porder 8 (26^3): 1 0.922, 2
-// 1.007, 3 0.950.  Porder 2 (100^3): 16 at four 0.707, at the compiler's choice
-// 0.738; porder 3 (80^3): 8 at four 0.922, at the compiler's choice 0.937.
+// most, then the L1 that the blocks' shared memory leaves for the gathers'
+// lines in flight (porder 5: three blocks of 65.6 KB, within a 196 KB carveout,
+// 1.00 ms on 51^3; of 67.7 KB, beyond it, 1.37).  The FP64 kernels, bound by
+// FP64 issue, which a warp pays for its idle lanes too, take the same groups.
+// FP32, ms: porder 4 (64^3) 5 elements at three blocks 1.030, at four (128
+// registers, spills) 1.077; before the divisions left the point work, 8
+// elements at two blocks took 1.302, 9 1.284, 4 at four 1.236, where 5 took
+// 1.152.  Porder 5 (51^3) 3 elements at three 0.996, 4 at two 1.053; 6 (40^3) 3
+// 1.094, 2 at two 1.156; 7 (32^3) 2 at two 0.853; 8 (26^3) 1 0.717; 3 (80^3) 8 at
+// the compiler's choice 0.779, at four 0.795; 2 (100^3) 16 at four 0.619, at the
+// compiler's choice 0.717.
 template <typename real, int P>
 constexpr int diffu_ne()
 {
@@ -78,11 +87,25 @@ constexpr int diffu_ne()
 template <typename real, int P>
 constexpr int diffu_minb()
 {
-    constexpr int nb[9] = {0, 1, 4, 4, 4, 3, 1, 2, 1};
+    constexpr int nb[9] = {0, 1, 4, 1, 3, 3, 1, 2, 1};
     return sizeof(real) == 4 ? nb[P] : 1;
 }
 template <typename real, int P>
 using DiffuGeom = GroupGeom<real, P, diffu_ne<real, P>()>;
+
+// Element points from which the FP32 kernel takes its matrices from the constant
+// bank.  That saves it registers and shared-memory loads, and at porders 5 and 6
+// the L1 that the tables' shared memory costs (ms, bank / shared memory: porder
+// 5 51^3 0.996 / 1.327, 6 40^3 1.094 / 1.405, 4 64^3 1.030 / 1.046, 3 80^3 0.779 /
+// 0.854, 2 100^3 0.619 / 0.680, 1 128^3 0.392 / 0.425, 7 32^3 0.853 / 0.882, 8 26^3
+// 0.717 / 0.754), but costs the call the table kernel and a copy to the bank,
+// ~6 us: the lines below are where the two meet.  FP64 stays with shared memory
+// (porder 4 20^3 0.650 against 0.798).
+template <int P>
+constexpr long long diffu_const_points()
+{
+    return P == 5 || P == 6 ? 500000 : (P == 4 ? 12000000 : 3000000);
+}
 
 // Shared memory of a block.  X1 and X3 hold the xi and eta derivatives of
 // (rho, T, u1, u2), then the fluxes (and divergences) of grad rho, tauU, grad T
@@ -97,12 +120,14 @@ struct DiffuShared {
     static constexpr size_t kU = k3 + G::NREC * sizeof(Four<real>);
     static constexpr size_t kE1 = kU + G::NREC * sizeof(real);
     static constexpr size_t kE3 = kE1 + G::NREC * sizeof(real);
-    static constexpr size_t kBytes = kE3 + G::NREC * sizeof(real);
+    static constexpr size_t kTab = (kE3 + G::NREC * sizeof(real) + 15) / 16 * 16;
+    static constexpr size_t bytes(bool constd) { return kTab + (constd ? 0 : GroupTables<G, false>::kBytes); }
     unsigned char *base;
     __device__ __forceinline__ unsigned long long *bar() const
     {
         return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
     }
+    __device__ __forceinline__ GroupTables<G, false> tab() const { return GroupTables<G, false>{base + kTab}; }
     __device__ __forceinline__ Four<real> *X1() const { return reinterpret_cast<Four<real> *>(base + k1); }
     __device__ __forceinline__ Four<real> *X2() const { return reinterpret_cast<Four<real> *>(base + k2); }
     __device__ __forceinline__ Four<real> *X3() const { return reinterpret_cast<Four<real> *>(base + k3); }
@@ -112,12 +137,12 @@ struct DiffuShared {
 };
 
 // Derivatives of the five fields along the thread's line in direction DIR.
-template <class G, int DIR>
-__device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuShared<G> &sm)
+template <class G, int DIR, bool CONSTD>
+__device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuShared<G> &sm, const DiffuRows<G, CONSTD> &tab)
 {
     using real = typename G::real;
     using R2 = Two<real>;
-    constexpr int Q = G::Q, P = G::P;
+    constexpr int Q = G::Q;
     const int base = t.rec0(DIR);
     Four<real> f[Q];
     real u3[Q];
@@ -126,6 +151,9 @@ __device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuS
         f[c] = sm.X2()[base + c * G::template step<DIR>()];
         u3[c] = sm.U3()[base + c * G::template step<DIR>()];
     }
+    real D[Q][Q];  // all rows before the first store: no load waits behind one
+#pragma unroll
+    for (int r = 0; r < Q; ++r) tab.row(D[r], DIR, r);
 #pragma unroll
     for (int r = 0; r < Q; ++r) {
         Four<real> g;
@@ -133,10 +161,9 @@ __device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuS
         real g3 = (real)0;
 #pragma unroll
         for (int c = 0; c < Q; ++c) {
-            const real D = cD<real>(P, (DIR * Q + r) * Q + c);
-            g.a = fma2(two(D, D), f[c].a, g.a);
-            g.b = fma2(two(D, D), f[c].b, g.b);
-            g3 = fma(D, u3[c], g3);
+            g.a = fma2(two(D[r][c], D[r][c]), f[c].a, g.a);
+            g.b = fma2(two(D[r][c], D[r][c]), f[c].b, g.b);
+            g3 = fma(D[r][c], u3[c], g3);
         }
         const int o = base + r * G::template step<DIR>();
         (DIR == 0 ? sm.X1() : sm.X3())[o] = g;
@@ -145,54 +172,50 @@ __device__ __forceinline__ void diffu_grad(const GroupThread<G> &t, const DiffuS
 }
 
 // Weak divergence of the thread's line in direction DIR, in place.
-template <class G, int DIR>
-__device__ __forceinline__ void diffu_div(const GroupThread<G> &t, const DiffuShared<G> &sm)
+template <class G, int DIR, bool CONSTD>
+__device__ __forceinline__ void diffu_div(const GroupThread<G> &t, const DiffuShared<G> &sm, const DiffuRows<G, CONSTD> &tab)
 {
     using real = typename G::real;
     using R2 = Two<real>;
-    constexpr int Q = G::Q, P = G::P;
+    constexpr int Q = G::Q;
     const int base = t.rec0(DIR);
     Four<real> *X = DIR == 0 ? sm.X1() : sm.X3();
-    {
-        Four<real> f[Q];
-#pragma unroll
-        for (int c = 0; c < Q; ++c) f[c] = X[base + c * G::template step<DIR>()];
-#pragma unroll
-        for (int r = 0; r < Q; ++r) {
-            Four<real> s;
-            s.a = s.b = two((real)0, (real)0);
-#pragma unroll
-            for (int c = 0; c < Q; ++c) {
-                const real D = cD<real>(P, (DIR * Q + c) * Q + r);
-                s.a = fma2(two(D, D), f[c].a, s.a);
-                s.b = fma2(two(D, D), f[c].b, s.b);
-            }
-            X[base + r * G::template step<DIR>()] = s;
-        }
-    }
-    R2 f[Q];
+    Four<real> f[Q];
+    R2 f2[Q];
 #pragma unroll
     for (int c = 0; c < Q; ++c) {
-        const Four<real> *x = sm.X2() + base + c * G::template step<DIR>();
-        f[c] = DIR == 0 ? x->a : x->b;
+        const int o = base + c * G::template step<DIR>();
+        const Four<real> *x2 = sm.X2() + o;
+        f[c] = X[o];
+        f2[c] = DIR == 0 ? x2->a : x2->b;
     }
+    real D[Q][Q];
+#pragma unroll
+    for (int c = 0; c < Q; ++c) tab.row(D[c], DIR, c);
 #pragma unroll
     for (int r = 0; r < Q; ++r) {
-        R2 s = two((real)0, (real)0);
+        Four<real> s;
+        R2 s2 = two((real)0, (real)0);
+        s.a = s.b = s2;
 #pragma unroll
         for (int c = 0; c < Q; ++c) {
-            const real D = cD<real>(P, (DIR * Q + c) * Q + r);
-            s = fma2(two(D, D), f[c], s);
+            const R2 Dc = two(D[c][r], D[c][r]);
+            s.a = fma2(Dc, f[c].a, s.a);
+            s.b = fma2(Dc, f[c].b, s.b);
+            s2 = fma2(Dc, f2[c], s2);
         }
-        Four<real> *x = sm.X2() + base + r * G::template step<DIR>();
-        (DIR == 0 ? x->a : x->b) = s;
+        const int o = base + r * G::template step<DIR>();
+        Four<real> *x2 = sm.X2() + o;
+        X[o] = s;
+        (DIR == 0 ? x2->a : x2->b) = s2;
     }
 }
 
-template <class G, int VISC, int MINB>
+template <class G, int VISC, int MINB, bool CONSTD>
 __global__ void __launch_bounds__(G::NT, MINB)
     diffu_kernel(int nelem, int npoin, const int *__restrict__ connec, const typename G::real *__restrict__ He,
-                 const typename G::real *__restrict__ gpvol, const TableScratch *__restrict__ tabs,
+                 const typename G::real *__restrict__ gpvol, const int *__restrict__ inv,
+                 const typename G::real *__restrict__ dlxigp_ip, const TableScratch *__restrict__ tabs,
                  typename G::real Cp, typename G::real Pr, const typename G::real *__restrict__ rho,
                  const typename G::real *__restrict__ u, const typename G::real *__restrict__ Tem,
                  const typename G::real *__restrict__ mu_fluid, const typename G::real *__restrict__ mu_e,
@@ -202,7 +225,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
 {
     using real = typename G::real;
     using R2 = Two<real>;
-    constexpr int Q = G::Q, P = G::P, N = G::N;
+    constexpr int Q = G::Q;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const DiffuShared<G> sm{smem_raw};
     const int tid = threadIdx.x, e0 = blockIdx.x * G::NE;
@@ -217,22 +240,23 @@ __global__ void __launch_bounds__(G::NT, MINB)
     R2 rT[Q], u12[Q];
     real u3[Q], muf[Q], ms[Q], me[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) pt[k] = ldg(&tabs->perm[t.template lat<2>(k)]);
+    for (int k = 0; k < Q; ++k) pt[k] = GroupTables<G, false>::node(inv, t.template lat<2>(k));
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
-        const int v = in ? ldg(connec + (size_t)pt[k] * nelem + e) - 1 : -1;
+        const int v = in ? ldg_once(connec + (size_t)pt[k] * nelem + e) - 1 : -1;
         id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
     }
+    if (!CONSTD) sm.tab().build(inv, dlxigp_ip, tid);
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const bool ok = id[k] >= 0;
         const size_t p = ok ? (size_t)id[k] : 0, i = in ? (size_t)pt[k] * nelem + e : 0;
-        rT[k] = two(ok ? ldg(rho + p) : (real)0, ok ? ldg(Tem + p) : (real)0);
-        u12[k] = two(ok ? ldg(u + p) : (real)0, ok ? ldg(u + np + p) : (real)0);
-        u3[k] = ok ? ldg(u + 2 * np + p) : (real)0;
-        muf[k] = ok ? ldg(mu_fluid + p) : (real)0;
-        ms[k] = in ? ldg(mu_sgs + i) : (real)0;
-        me[k] = (VISC == VISC_MU_E && in) ? ldg(mu_e + i) : (real)0;
+        rT[k] = two(ok ? ldg_once(rho + p) : (real)0, ok ? ldg_once(Tem + p) : (real)0);
+        u12[k] = two(ok ? ldg_once(u + p) : (real)0, ok ? ldg_once(u + np + p) : (real)0);
+        u3[k] = ok ? ldg_once(u + 2 * np + p) : (real)0;
+        muf[k] = ok ? ldg_once(mu_fluid + p) : (real)0;
+        ms[k] = in ? ldg_once(mu_sgs + i) : (real)0;
+        me[k] = (VISC == VISC_MU_E && in) ? ldg_once(mu_e + i) : (real)0;
     }
     if (VISC == VISC_NU_ELEM) {
         const real nu = in ? ldg(nu_elem + e) : (real)0;
@@ -249,9 +273,10 @@ __global__ void __launch_bounds__(G::NT, MINB)
             sm.U3()[base + k * G::template step<2>()] = u3[k];
         }
     __syncthreads();
+    const DiffuRows<G, CONSTD> tab(sm.tab());
     if (t.active) {
-        diffu_grad<G, 0>(t, sm);
-        diffu_grad<G, 1>(t, sm);
+        diffu_grad<G, 0, CONSTD>(t, sm, tab);
+        diffu_grad<G, 1, CONSTD>(t, sm, tab);
     }
     // Bounded wait for the bulk copies; a wait that ran out is reported and
     // nothing is assembled.
@@ -268,10 +293,14 @@ __global__ void __launch_bounds__(G::NT, MINB)
 #pragma unroll
     for (int r = 0; r < Q; ++r) acc[r][0] = acc[r][1] = acc[r][2] = two((real)0, (real)0);
     if (t.active) {
+        real Dn[Q];
+        tab.row(Dn, 2, 0);
 #pragma unroll
         for (int c = 0; c < Q; ++c) {
             const int o = base + c * G::template step<2>();
-            real H[9];
+            real Dr[Q], H[9];
+#pragma unroll
+            for (int j = 0; j < Q; ++j) Dr[j] = Dn[j];
             const real *hp = gm.he(t.el, pt[c]);
 #pragma unroll
             for (int j = 0; j < 9; ++j) H[j] = hp[j];
@@ -279,9 +308,10 @@ __global__ void __launch_bounds__(G::NT, MINB)
             const Four<real> gx = sm.X1()[o], ge = sm.X3()[o];
             R2 za = two((real)0, (real)0), zb = za;
             real z3 = (real)0;
+            if (c + 1 < Q) tab.row(Dn, 2, c + 1);  // before this point's stores
 #pragma unroll
             for (int j = 0; j < Q; ++j) {
-                const real D = cD<real>(P, (2 * Q + c) * Q + j);
+                const real D = Dr[j];
                 za = fma2(two(D, D), rT[j], za);
                 zb = fma2(two(D, D), u12[j], zb);
                 z3 = fma(D, u3[j], z3);
@@ -331,7 +361,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
             sm.X2()[o] = s;
 #pragma unroll
             for (int rr = 0; rr < Q; ++rr) {
-                const real D = cD<real>(P, (2 * Q + c) * Q + rr);
+                const real D = Dr[rr];
 #pragma unroll
                 for (int x = 0; x < 3; ++x) acc[rr][x] = fma2(two(D, D), F[2][x], acc[rr][x]);
             }
@@ -341,9 +371,10 @@ __global__ void __launch_bounds__(G::NT, MINB)
     }
     __syncthreads();
     if (t.active) {
-        diffu_div<G, 0>(t, sm);
-        diffu_div<G, 1>(t, sm);
+        diffu_div<G, 0, CONSTD>(t, sm, tab);
+        diffu_div<G, 1, CONSTD>(t, sm, tab);
     }
+    grid_dependency_wait();  // the residuals are zeroed
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
@@ -360,29 +391,39 @@ __global__ void __launch_bounds__(G::NT, MINB)
     }
 }
 
-template <typename real, int P, int VISC>
-cudaError_t launch_diffu_pn(const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st)
+template <typename real, int P, int VISC, bool CONSTD>
+cudaError_t launch_diffu_pc(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
 {
     using G = DiffuGeom<real, P>;
-    constexpr size_t smem = DiffuShared<G>::kBytes;
+    constexpr size_t smem = DiffuShared<G>::bytes(CONSTD);
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    auto kern = diffu_kernel<G, VISC, diffu_minb<real, P>()>;
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kern = diffu_kernel<G, VISC, diffu_minb<real, P>(), CONSTD>;
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
-    constexpr size_t nb = sizeof(real) * 3 * G::Q * G::Q, off = sizeof(real) * kTableDMax * P;
-    if (sizeof(real) == 4)
-        err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, nb, off, cudaMemcpyDeviceToDevice, st);
-    else
-        err = cudaMemcpyToSymbolAsync(c_Dd, tabs->Dd, nb, off, cudaMemcpyDeviceToDevice, st);
-    if (err != cudaSuccess) return err;
+    if constexpr (CONSTD) {
+        err = launch_table_prep<real>(P, a, tabs, st);
+        if (err == cudaSuccess)
+            err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, sizeof(float) * 3 * G::Q * G::Q,
+                                          sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
+        if (err != cudaSuccess) return err;
+    }
     const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
-    kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem,
-                                    a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem, a.Rmass, a.Rmom, a.Rener);
-    return cudaGetLastError();
+    return launch_after(kern, grid, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK,
+                        a.dlxigp_ip, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
+                        a.Rmass, a.Rmom, a.Rener);
+}
+template <typename real, int P, int VISC>
+cudaError_t launch_diffu_pn(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
+{
+    if constexpr (sizeof(real) == 4)
+        if ((long long)a.nelem * DiffuGeom<real, P>::N >= diffu_const_points<P>())
+            return launch_diffu_pc<real, P, VISC, true>(a, tabs, st);
+    return launch_diffu_pc<real, P, VISC, false>(a, tabs, st);
 }
 
 template <typename real, int P>
-cudaError_t launch_diffu_p(const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_diffu_p(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
 {
     if (a.nu_elem) return launch_diffu_pn<real, P, VISC_NU_ELEM>(a, tabs, st);
     return launch_diffu_pn<real, P, VISC_MU_E>(a, tabs, st);
@@ -391,7 +432,7 @@ cudaError_t launch_diffu_p(const DiffuArgs<real> &a, const TableScratch *tabs, c
 }  // namespace
 
 template <typename real>
-cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
 {
     switch (porder) {
     case 1: return launch_diffu_p<real, 1>(a, tabs, st);
@@ -406,7 +447,7 @@ cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, const Table
     }
 }
 
-template cudaError_t launch_diffu_plain<float>(int, const DiffuArgs<float> &, const TableScratch *, cudaStream_t);
-template cudaError_t launch_diffu_plain<double>(int, const DiffuArgs<double> &, const TableScratch *, cudaStream_t);
+template cudaError_t launch_diffu_plain<float>(int, const DiffuArgs<float> &, TableScratch *, cudaStream_t);
+template cudaError_t launch_diffu_plain<double>(int, const DiffuArgs<double> &, TableScratch *, cudaStream_t);
 
 }  // namespace msod

@@ -119,12 +119,11 @@ struct GroupGeom {
     static constexpr int LT = ((NE * L + 31) / 32) * 32;  // threads of one segment
     static constexpr int NT = S * LT;
     // Pitch of an element's He and gpvol in shared memory.  Where an element's
-    // span is a multiple of 16 bytes (odd porders) it is copied by itself, to a
-    // pitch of 16 bytes more than a multiple of all banks, so that the elements
-    // of a warp do not fall on one bank (64 x 9 and 512 x 9 words are multiples
-    // of 32); the other spans have odd lengths and are copied as one.
+    // He is a multiple of all banks (porders 3 and 7: 64 x 9 and 512 x 9 words)
+    // it is copied by itself, to a pitch of 16 bytes more, so that the elements
+    // of a warp do not fall on one bank; other groups are copied as one span.
     static constexpr bool STAGED = sizeof(real) == 4;  // FP64: read in place (bound by FP64 issue, short of shared memory)
-    static constexpr bool SPLIT = STAGED && N >= 64 && (N * sizeof(real)) % 16 == 0;
+    static constexpr bool SPLIT = STAGED && N >= 64 && (9 * N) % 32 == 0;
     static constexpr int BANKS = 128 / (int)sizeof(real), OFF = 16 / (int)sizeof(real);
     static constexpr int pitch(int n) { return SPLIT ? n + (BANKS + OFF - n % BANKS) % BANKS : n; }
     static constexpr int HEP = pitch(9 * N), GPP = pitch(N);
@@ -234,6 +233,120 @@ struct GroupMetric {
         }
         He = reinterpret_cast<real *>(hs + hsh);
         gp = reinterpret_cast<const real *>(gs + gsh);
+    }
+};
+
+// The element tables of a call in shared memory, built by each block from the
+// caller's arrays while its first loads are in flight: gmsh node of a lattice
+// point, the directions' 1-D derivative matrices and their transposes (rows
+// padded for vector loads), and their row sums.  dlxigp_ip(g, d, c) depends on g
+// through its 1-D index in direction d only (elem_hex.f90:43-44).  Indices are
+// clamped, so malformed tables give wrong numbers (reported by
+// msod_check_element_tables), never accesses out of bounds.  A block spends two
+// dependent loads of a few lanes on it, hidden behind the gather; the table
+// kernel and the copy to the constant bank that this replaces were two
+// launches per call (porder-4 convection on 16^3 hexes 43 -> 20 us with the
+// zeroing in one launch; on 64^3 0.950 ms with the coefficients from shared
+// memory, 0.944 from the constant bank).
+// FULL: transposes, row sums and the node permutation too (the diffusion reads
+// each matrix whole and needs none of them).
+template <class G, bool FULL>
+struct GroupTables {
+    using real = typename G::real;
+    static constexpr int Q = G::Q, N = G::N;
+    static constexpr int ROW = (Q + 3) / 4 * 4;  // pitch of a row
+    static constexpr size_t kD = (size_t)(FULL ? 6 : 3) * Q * ROW * sizeof(real);
+    static constexpr size_t kBytes = kD + (FULL ? (size_t)(3 * Q) * sizeof(real) + (size_t)N * sizeof(int) : 0);
+    unsigned char *base;  // 16-byte aligned
+    __device__ __forceinline__ real *D(int dir, int r) const { return reinterpret_cast<real *>(base) + (dir * Q + r) * ROW; }
+    __device__ __forceinline__ real *Dt(int dir, int c) const { return D(3 + dir, c); }
+    __device__ __forceinline__ real *sums() const { return reinterpret_cast<real *>(base + kD); }  // [dir Q + r]
+    __device__ __forceinline__ int *perm() const { return reinterpret_cast<int *>(sums() + 3 * Q); }
+    static __device__ __forceinline__ int node(const int *inv, int l) { return min(max(ldg(inv + l) - 1, 0), N - 1); }
+    // All threads call it; complete after the next barrier.
+    __device__ __forceinline__ void build(const int *__restrict__ inv, const real *__restrict__ dlx, int tid) const
+    {
+        if (FULL)
+            for (int i = tid; i < N; i += G::NT) perm()[i] = node(inv, i);
+        const int i = tid - (G::NT - 32);  // the last warp: one row per lane
+        if (i >= 0 && i < 3 * Q) {
+            const int d = i / Q, r = i - d * Q;
+            const int a = node(inv, d == 0 ? r : (d == 1 ? r * Q : r * Q * Q));
+            real v[Q];
+#pragma unroll
+            for (int c = 0; c < Q; ++c) v[c] = ldg(dlx + (size_t)(c * 3 + d) * N + a);
+            double sum = 0.0;
+#pragma unroll
+            for (int c = 0; c < Q; ++c) {
+                D(d, r)[c] = v[c];
+                if (FULL) {
+                    Dt(d, c)[r] = v[c];
+                    sum += (double)v[c];
+                }
+            }
+            if (FULL) sums()[i] = (real)sum;
+        }
+    }
+};
+
+// Loads of shared memory that no thread writes any more: plain functions of the
+// address to the compiler, which may move them across the stores of the sums
+// and fluxes (it cannot tell them apart from other shared memory) and so hide
+// their latency.  The address comes from after_barrier, which keeps them below
+// the barrier that completed the data.
+__device__ __forceinline__ unsigned after_barrier(const void *p)
+{
+    unsigned a;
+    asm volatile("mov.u32 %0, %1;" : "=r"(a) : "r"(smem_u32(p)) : "memory");
+    return a;
+}
+__device__ __forceinline__ void lds(int &v, unsigned a) { asm("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(float &v, unsigned a) { asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(double &v, unsigned a) { asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(Four<float> &v, unsigned a)
+{
+    asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.a.x), "=f"(v.a.y), "=f"(v.b.x), "=f"(v.b.y) : "r"(a));
+}
+__device__ __forceinline__ void lds(Four<double> &v, unsigned a)
+{
+    asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.a.x), "=d"(v.a.y) : "r"(a));
+    asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.b.x), "=d"(v.b.y) : "r"(a + 16));
+}
+
+// The tables as the passes read them (after the barrier that follows build).
+template <class G, bool FULL>
+struct GroupRows {
+    using real = typename G::real;
+    using T = GroupTables<G, FULL>;
+    unsigned base;
+    __device__ __forceinline__ explicit GroupRows(const T &t) : base(after_barrier(t.base)) {}
+    __device__ __forceinline__ void load(real (&v)[G::Q], int row) const
+    {
+        constexpr int Q = G::Q;
+#pragma unroll
+        for (int c = 0; c < Q; c += 4) {
+            Four<real> f;
+            lds(f, base + (unsigned)((row * T::ROW + c) * sizeof(real)));
+            v[c] = f.a.x;
+            if (c + 1 < Q) v[c + 1 < Q ? c + 1 : 0] = f.a.y;
+            if (c + 2 < Q) v[c + 2 < Q ? c + 2 : 0] = f.b.x;
+            if (c + 3 < Q) v[c + 3 < Q ? c + 3 : 0] = f.b.y;
+        }
+    }
+    // Row r, column c of direction dir's matrix; its row sums; lattice -> gmsh node.
+    __device__ __forceinline__ void row(real (&v)[G::Q], int dir, int r) const { load(v, dir * G::Q + r); }
+    __device__ __forceinline__ void col(real (&v)[G::Q], int dir, int c) const { load(v, (3 + dir) * G::Q + c); }
+    __device__ __forceinline__ real sum(int dir, int r) const
+    {
+        real v;
+        lds(v, base + (unsigned)(T::kD + (dir * G::Q + r) * sizeof(real)));
+        return v;
+    }
+    __device__ __forceinline__ int node(int l) const
+    {
+        int v;
+        lds(v, base + (unsigned)(T::kD + 3 * G::Q * sizeof(real) + l * sizeof(int)));
+        return v;
     }
 };
 

@@ -4,6 +4,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "msod.h"
 
 namespace msod {
@@ -13,13 +15,10 @@ namespace msod {
 // FP64 copies), lattice -> gmsh node (perm) and gmsh node -> padded lattice
 // offset (lat).
 constexpr int kTableDMax = 3 * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
-// D[d][r][c] at [(d*Q + r)*Q + c], followed at 3*Q*Q by its row sums [d*Q + r].
-constexpr int kTableDSMax = kTableDMax + 3 * (MSOD_MAX_PORDER + 1);
 constexpr int kTableNMax = (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
 struct TableScratch {
-    float Df[kTableDSMax];
-    int same_dirs;  // 1 when the three directions' matrices are equal
-    double Dd[kTableDSMax];
+    float Df[kTableDMax];
+    double Dd[kTableDMax];
     int perm[kTableNMax];
     int lat[kTableNMax];
     // Set (sticky, zero at allocation) by a kernel whose bounded wait for a
@@ -75,15 +74,66 @@ struct DiffuArgs : ElementArgs<real> {
     real *Rmass, *Rmom, *Rener;
 };
 
+// Zeroes up to six residual arrays (one launch).  The kernels below that follow
+// it on the stream with launch_after start while it still runs and wait for it
+// before their first reduction.
+struct ZeroSpans {
+    void *p[6];
+    size_t bytes[6];
+    int n = 0;
+    void add(void *ptr, size_t b)
+    {
+        p[n] = ptr;
+        bytes[n++] = b;
+    }
+};
+cudaError_t launch_zero(const ZeroSpans &z, cudaStream_t st);
+
+// Allows kern `smem` bytes of dynamic shared memory on the current device, once
+// per device and kernel (done: one bit per device, owned by the kernel's launcher).
+template <typename Kernel>
+inline cudaError_t allow_smem(std::atomic<unsigned long long> &done, Kernel kern, size_t smem)
+{
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return err;
+}
+
+// Launches kern so that its blocks may start before the kernel ahead of it on
+// the stream has finished (programmatic dependent launch); kern calls
+// grid_dependency_wait() before it touches what that kernel writes.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                                A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Tables of one call (one block, stream-ordered before the kernels).
 template <typename real>
 cudaError_t launch_table_prep(int porder, const ElementArgs<real> &a, TableScratch *scratch, cudaStream_t st);
 
-// Plain kernels (outputs must be zeroed by the caller; tables prepared).
+// Plain kernels (outputs zeroed by launch_zero just before, or earlier on the
+// stream; tabs: where a bounded wait that ran out is recorded).
 template <typename real>
 cudaError_t launch_convec_plain(int porder, const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
 template <typename real>
-cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
+cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st);
 // Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by the
 // caller; tables prepared).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
 struct MixedConvecArgs {

@@ -1,6 +1,7 @@
-// msod_tables.cu -- per-call element tables for the line-parallel kernels.
+// msod_tables.cu -- per-call element tables of the viscosity and tensor-core
+// kernels, and the zeroing of the residuals.
 //
-// Every kernel call first runs table_prep_kernel, one block that reads the
+// Those kernels' calls first run table_prep_kernel, one block that reads the
 // caller's dlxigp_ip / invAtoIJK / gmshAtoI/J/K (device arrays in the
 // reference's layouts) and writes, into a small library-owned device area:
 //   perm[l]  lattice point l = (K*Q+J)*Q+I (SOD 1-D indices) -> gmsh node a
@@ -44,16 +45,34 @@ __global__ void table_prep_kernel(const int *__restrict__ invAtoIJK, const int *
         const int l = d == 0 ? r : (d == 1 ? r * Q : r * Q * Q);
         D[i] = dlxigp_ip[(size_t)(c * 3 + d) * N + sperm[l]];
     }
-    __syncthreads();  // D complete
-    for (int i = threadIdx.x; i < 3 * Q; i += blockDim.x) {
-        double sum = 0.0;
-        for (int c = 0; c < Q; ++c) sum += (double)D[i * Q + c];
-        D[3 * Q * Q + i] = (real)sum;
-    }
-    if (threadIdx.x == 0) {
-        bool same = true;
-        for (int i = 0; i < Q * Q; ++i) same = same && D[Q * Q + i] == D[i] && D[2 * Q * Q + i] == D[i];
-        out->same_dirs = same ? 1 : 0;
+}
+
+// Each block zeroes one 16 KB piece of one array (four 16-byte stores a
+// thread); the ends of an array that are not 16-byte aligned go to its first
+// block.
+constexpr size_t kZeroPiece = 16384;
+struct ZeroPlan {
+    ZeroSpans z;
+    unsigned first[7];  // first block of each array
+};
+__global__ void __launch_bounds__(256) zero_kernel(ZeroPlan pl)
+{
+    grid_dependents_launch();  // the residual kernel may start (it waits before its first reduction)
+    int k = 0;
+    while (k + 1 < pl.z.n && blockIdx.x >= pl.first[k + 1]) ++k;
+    const unsigned piece = blockIdx.x - pl.first[k];
+    const size_t a = reinterpret_cast<size_t>(pl.z.p[k]), e = a + pl.z.bytes[k];
+    size_t a16 = (a + 15) & ~(size_t)15, e16 = e & ~(size_t)15;
+    if (a16 > e16) a16 = e16 = e;  // no aligned 16 bytes: words only
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const size_t i0 = a16 + piece * kZeroPiece + 16 * threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (i0 + 4096 * j < e16) *reinterpret_cast<float4 *>(i0 + 4096 * j) = zero;
+    if (piece == 0 && threadIdx.x < 8) {
+        const size_t h = a + 4 * threadIdx.x, t = e16 + 4 * threadIdx.x;
+        if (h < a16) *reinterpret_cast<float *>(h) = 0.0f;
+        if (t < e) *reinterpret_cast<float *>(t) = 0.0f;
     }
 }
 
@@ -65,6 +84,19 @@ cudaError_t prep_p(const ElementArgs<real> &a, TableScratch *scratch, cudaStream
 }
 
 }  // namespace
+
+cudaError_t launch_zero(const ZeroSpans &z, cudaStream_t st)
+{
+    ZeroPlan pl;
+    pl.z = z;
+    unsigned n = 0;
+    for (int k = 0; k < z.n; ++k) {
+        pl.first[k] = n;
+        n += (unsigned)((z.bytes[k] + kZeroPiece) / kZeroPiece);
+    }
+    zero_kernel<<<n, 256, 0, st>>>(pl);
+    return cudaGetLastError();
+}
 
 template <typename real>
 cudaError_t launch_table_prep(int porder, const ElementArgs<real> &a, TableScratch *scratch, cudaStream_t st)

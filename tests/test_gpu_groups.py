@@ -66,3 +66,41 @@ def test_group_edges(cuda, P, dims, shift, odd):
     ref = [O.full_diffusion_ijk(*a, g, 1004.5, 0.71, f["rho"], f["u"], f["Tem"], f["mu_fluid"], *mu, dt, nthreads=NTH)
            for g, dt in ((geom, np.float32), (g64, np.float64))]
     _compare(out, ref[0], TOL32, "diffu group edges P=%d" % P, ref[1])
+
+
+@pytest.mark.parametrize("P", range(1, 9))
+def test_large_meshes_as_small_ones(cuda, P):
+    """Large meshes take the diffusion's matrices from the constant bank (the line lies between half a
+    million and twelve million element points): copies of a small mesh, whose own call reads them
+    from shared memory, give the small mesh's residuals on every copy.  The operations are the same;
+    1e-6 leaves room for the order of the nodes' sums."""
+    import torch
+
+    t = fem.element_tables(P, np.float32)
+    connec, coord, ne, npn = fem.structured_mesh(P, 3, 2, 2, t, 0.1, P)
+    He, gp = O.elem_jacobian(P, ne, npn, connec, coord, t["dNgp"], t["wgp"], np.float32)
+    n = (P + 1) ** 3
+    rng = np.random.default_rng(P)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda)
+    f = {k: up((1.0 + 0.3 * rng.random(npn)).astype(np.float32)) for k in ("rho", "Tem", "mu_fluid")}
+    f["u"] = up(rng.standard_normal(3 * npn).astype(np.float32))
+    mu = [up(rng.random(ne * n).astype(np.float32)) for _ in range(2)]
+    con, He, gp = up(connec), up(He), up(gp)
+    tab = [up(t[k]) for k in ("dlxigp_ip", "invAtoIJK", "AtoI", "AtoJ", "AtoK")]
+
+    def run(copies):
+        c = con.view(n, 1, ne) + (torch.arange(copies, device=cuda, dtype=torch.int32) * npn).view(1, -1, 1)
+        rep = lambda x, lead: x.view(lead, 1, -1).expand(lead, copies, -1).reshape(-1).contiguous()
+        m = npn * copies
+        out = [torch.empty(k * m, device=cuda) for k in (1, 3, 1)]
+        kernels.full_diffusion_ijk(ne * copies, m, c.reshape(-1).contiguous(), None, None, rep(He, 1), rep(gp, 1), tab[0],
+                                   None, *tab[1:], 1004.5, 0.71, rep(f["rho"], 1), rep(f["u"], 3), rep(f["Tem"], 1),
+                                   rep(f["mu_fluid"], 1), *[rep(x, n) for x in mu], *out)
+        return [o.view(k, copies, npn) for o, k in zip(out, (1, 3, 1))]
+
+    small = run(1)
+    limit = 500000 if P in (5, 6) else (12000000 if P == 4 else 3000000)
+    large = run(limit // (ne * n) + 2)
+    for a, b in zip(large, small):
+        err = torch.linalg.vector_norm((a - b).double()) / torch.linalg.vector_norm(b.double().expand_as(a))
+        assert float(err) <= 1e-6, (P, float(err))
