@@ -137,4 +137,23 @@ def check(rc):
 
 
 def call(name, *args):
-    return check(getattr(lib(), name)(*args))
+    return check(getattr(_lib or lib(), name)(*args))
+
+
+_raw_stream = None
+
+
+def current_stream():
+    """Handle of torch's current CUDA stream on the current device (as current_stream().cuda_stream
+    gives it, without the Stream object: 0.3 against 3 us, a seventh of a small call)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+
+        c = torch._C
+        if hasattr(c, "_cuda_getCurrentRawStream") and hasattr(c, "_cuda_getDevice"):
+            torch.cuda.current_stream()  # initialises CUDA
+            _raw_stream = lambda: c._cuda_getCurrentRawStream(c._cuda_getDevice())  # noqa: E731
+        else:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _raw_stream()

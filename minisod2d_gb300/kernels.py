@@ -10,16 +10,20 @@ path: a tensor on another device is an error.
 from . import capi
 
 
+_PORDER = {(p + 1) ** 3: p for p in range(1, 9)}
+_Tensor = None
+
+
 def _stream(stream):
     if stream is not None:
         return stream
-    import torch
-
-    return torch.cuda.current_stream().cuda_stream
+    return capi.current_stream()
 
 
 def _porder_from(gmshAtoI):
     n = int(gmshAtoI.numel())
+    if n in _PORDER:
+        return _PORDER[n]
     q = int(round(n ** (1.0 / 3.0)))
     if q ** 3 != n or q < 2:
         raise ValueError("gmshAtoI has %d entries, not (porder+1)^3" % n)
@@ -27,11 +31,19 @@ def _porder_from(gmshAtoI):
 
 
 def _ptr(t, name, dtype, numel=None):
-    import torch
-
+    # A call checks some twenty arrays, and on small meshes the host's time per call exceeds the
+    # kernel's: the valid array goes through one expression, the errors are told apart below it.
+    global _Tensor
     if t is None:
         return None
-    if not isinstance(t, torch.Tensor):
+    if _Tensor is None:
+        import torch
+
+        _Tensor = torch.Tensor
+    if (isinstance(t, _Tensor) and t.is_cuda and t.dtype is dtype and t.is_contiguous()
+            and (numel is None or t.numel() == numel)):
+        return t.data_ptr()
+    if not isinstance(t, _Tensor):
         raise TypeError("%s must be a torch tensor" % name)
     if not t.is_cuda:
         raise ValueError("%s must be a CUDA tensor (the library has no CPU path)" % name)
@@ -39,9 +51,7 @@ def _ptr(t, name, dtype, numel=None):
         raise TypeError("%s must be %s, got %s" % (name, dtype, t.dtype))
     if not t.is_contiguous():
         raise ValueError("%s must be contiguous" % name)
-    if numel is not None and t.numel() != numel:
-        raise ValueError("%s has %d elements, expected %d" % (name, t.numel(), numel))
-    return t.data_ptr()
+    raise ValueError("%s has %d elements, expected %d" % (name, t.numel(), numel))
 
 
 def _geometry(nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK, real):

@@ -44,11 +44,7 @@ def _p(t):
 
 
 def _stream(stream):
-    if stream is not None:
-        return stream
-    import torch
-
-    return torch.cuda.current_stream().cuda_stream
+    return stream if stream is not None else capi.current_stream()
 
 
 def _geo(dev):
