@@ -184,6 +184,7 @@ struct GroupMetric {
     real *He;
     const real *gp;
     int last;  // the group's last element
+    __device__ __forceinline__ GroupMetric() : He(nullptr), gp(nullptr), last(0) {}
     __device__ __forceinline__ real *he(int el, int a) const
     {
         return He + (G::STAGED ? el : min(el, last)) * G::HEP + a * 9;

@@ -226,7 +226,6 @@ struct ViscArgs {
     // of flagged elements written by launch_mlp_predict), write nu only.
     const int *list, *count;
     float *mu_e, *nu, *numax;
-    const TableScratch *tabs;  // the call's element tables (table_prep_kernel)
 };
 
 struct FeatureArgs {

@@ -99,13 +99,6 @@ int prep_tables(int porder, int nelem, int npoin, const int *connec, const float
     return cuda_rc(launch_table_prep<float>(porder, ea, tabs, st), "table preparation launch");
 }
 
-// The tables prepared by the last prep_tables call of this porder on this device.
-const TableScratch *prepared_tables(int porder)
-{
-    return static_cast<TableScratch *>(scratch(SLOT_TABLES, sizeof(TableScratch) * (MSOD_MAX_PORDER + 1))) +
-           porder;
-}
-
 uint32_t crc32(const unsigned char *p, size_t n)
 {
     uint32_t c = 0xFFFFFFFFu;
@@ -151,16 +144,11 @@ int msod_entropy_viscosity(int porder, int nelem, int npoin, const int *connec, 
     EntropyStats *stats = nullptr;
     rc = run_stats(npoin, rho, pr, 0.0f, gamma, &stats, st);
     if (rc) return rc;
-    TableScratch *tabs = nullptr;
-    rc = prep_tables(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
-                     &tabs, st);
-    if (rc) return rc;
     ViscArgs a{};
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlxigp_ip;
     a.invAtoIJK = invAtoIJK; a.AtoI = gmshAtoI; a.AtoJ = gmshAtoJ; a.AtoK = gmshAtoK;
     a.rho = rho; a.u = u; a.p_or_T = pr; a.Rgas = 0.0f; a.gamma = gamma; a.ce = ce; a.cmax = cmax;
     a.normalise = normalise; a.stats = stats; a.list = nullptr; a.count = nullptr; a.mu_e = mu_e; a.nu = nu_elem; a.numax = numax_elem;
-    a.tabs = tabs;
     return cuda_rc(launch_entropy_visc(porder, a, st), "entropy viscosity launch");
 }
 
@@ -439,7 +427,6 @@ static int learned_nu(const msod_mlp *m, int porder, int nelem, int npoin, const
     a.invAtoIJK = invAtoIJK; a.AtoI = gmshAtoI; a.AtoJ = gmshAtoJ; a.AtoK = gmshAtoK;
     a.rho = rho; a.u = u; a.p_or_T = p_or_T; a.Rgas = Rgas; a.gamma = gamma; a.ce = ce; a.cmax = cmax;
     a.normalise = 1; a.stats = stats; a.list = list; a.count = count; a.mu_e = nullptr; a.nu = nu; a.numax = nullptr;
-    a.tabs = prepared_tables(porder);  // prepared by the feature call above
     return cuda_rc(launch_entropy_visc(porder, a, st), "fallback estimator launch");
 }
 

@@ -19,19 +19,9 @@
 //                nu_E   = ce h^2 max_e |R| / n_eta,
 //                nu     = min(nu_max, nu_E)
 //   output       mu_e(e, a) = rho(a) nu(e)   in the reference's mu_e layout.
-// The derivatives are one convection-type pass: the same line-parallel sum
-// factorisation as the convection kernel, over eta, eta u and u.
 #include <cuda_runtime.h>
 
-#include "msod_device.cuh"
-#include "msod_kernels.h"
-
-// L2 prefetch of a group's He and gpvol spans at its start (0 = none; not in
-// the list mode, whose groups are scattered elements).  64^3 porder-4 hexes:
-// 0.924 ms against 0.964 ms; porder 5 on 51^3: 0.905 against 0.958 ms.
-#ifndef VISC_PREFETCH
-#define VISC_PREFETCH 1
-#endif
+#include "msod_group.cuh"
 
 namespace msod {
 
@@ -111,298 +101,280 @@ __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, c
 }
 
 // ---------------------------------------------------------------------------
-// Plain estimator: one group of NE elements per block, one thread per line.
+// Plain estimator: one group of NE elements per block, one thread per line
+// (msod_group.cuh).
+//
+//   * each thread gathers its zeta line, forms eta and |u| + c once per point and
+//     stores the records (u, eta); each of the three passes loads a line's
+//     records, forms eta u and applies the derivative matrix to (u, eta, eta u);
+//   * the xi and eta passes add their shares in shared memory; maxima per element
+//     by integer atomics on the floats' bits, the volume as a sum of line sums in
+//     a fixed order;
+//   * He and gpvol come by bulk copy.  In list mode (the per-element fallback)
+//     the group's elements are scattered, and both are read in place.
+// Bound by the gathers' latency and the L1 / shared-memory pipe.  Estimator with
+// its statistics, before / now: porder 4 64^3 0.923 / 0.594 ms, 5 51^3 0.901 /
+// 0.611, 7 32^3 0.772 / 0.412, 2 100^3 0.707 / 0.383, 1 128^3 0.533 / 0.241.
+// The line arithmetic is operation for operation the one that the shipped
+// networks were trained against: on smooth shock fields R is near its rounding
+// floor, and the product-rule defect formed from differences of nodal values
+// (as the convection forms its terms, no faster here) moves the fallback's
+// viscosity by 3e-4.
 // ---------------------------------------------------------------------------
-// 1-D derivative matrices of the current call, per porder (copied from the
-// call's table area before the launch): constant-bank operands of the line
-// passes when one thread owns a line.
-__constant__ float c_VD[MSOD_MAX_PORDER + 1][kTableDMax];
+// Elements per block (ms, estimator with the statistics, with that other line
+// arithmetic, which takes as long): porder 4 (64^3) 8 0.597,
+// 4 0.640, 5 0.647, 10 0.756; 5 (51^3) 4 0.605, 7 0.629, 8 0.672, 3 0.696; 6 (40^3) 3
+// 0.549, 4 0.553, 2 0.616; 7 (32^3) 3 0.438, 2 0.476, 4 0.561; 3 (80^3) 8 0.491, 4
+// 0.609; 2 (100^3) 16 0.356, 14 0.373; 1 (128^3) 32 0.251, 16 0.264.
+template <int P, bool LIST>
+struct ViscGroup {
+    static constexpr int ne[8] = {0, 32, 16, 8, 8, 4, 3, 3};
+    using G = GroupGeom<float, P, ne[P]>;
+};
 
-enum { V_RHO = 0, V_P, V_U0, V_U1, V_U2, NVF };
-constexpr int V_ETA = V_P;  // after the per-point preparation the pressure plane holds eta
+template <class G, bool LIST>
+struct ViscShared {
+    static constexpr size_t kHe = LIST ? 0 : G::HEB + G::GPB + 16;
+    static constexpr size_t kR = kHe + G::NREC * sizeof(Four<float>);
+    static constexpr size_t kV = kR + G::NREC * sizeof(float);
+    static constexpr size_t kEl = kV + (size_t)G::NE * G::L * sizeof(float);  // per element: max speed, max |R|, nu
+    static constexpr size_t kTab = (kEl + 3 * (size_t)G::NE * sizeof(float) + 15) / 16 * 16;
+    static constexpr size_t kBytes = kTab + GroupTables<G, false>::kBytes;
+    unsigned char *base;
+    __device__ __forceinline__ unsigned long long *bar() const
+    {
+        return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
+    }
+    __device__ __forceinline__ Four<float> *W() const { return reinterpret_cast<Four<float> *>(base + kHe); }  // u, eta
+    __device__ __forceinline__ float *R() const { return reinterpret_cast<float *>(base + kR); }
+    __device__ __forceinline__ float *vol() const { return reinterpret_cast<float *>(base + kV); }  // line sums
+    __device__ __forceinline__ int *speed() const { return reinterpret_cast<int *>(base + kEl); }
+    __device__ __forceinline__ unsigned *res() const { return reinterpret_cast<unsigned *>(speed() + G::NE); }
+    __device__ __forceinline__ float *nu() const { return reinterpret_cast<float *>(res() + G::NE); }
+    __device__ __forceinline__ GroupTables<G, false> tab() const { return GroupTables<G, false>{base + kTab}; }
+};
 
-template <class G, int DIR>
-__device__ __forceinline__ void residual_pass(const LineThread<G> &lt, const float *__restrict__ sF,
-                                              float *__restrict__ sR, const int *__restrict__ sPerm,
-                                              const float *__restrict__ sD, const float *__restrict__ He, int e,
-                                              float gamma)
+// Direction DIR's share of R at the line's points.
+template <class G, int DIR, class HeAt>
+__device__ __forceinline__ void visc_line(const Four<float> (&w)[G::Q], const GroupThread<G> &t,
+                                          const GroupRows<G, false> &tab, const HeAt &he,
+                                          const int (&pt)[G::Q], float (&R)[G::Q])
 {
-    constexpr int Q = G::Q, QP = G::QP, R = G::R, NPL = G::NPL;
-    constexpr int OST = DIR == 0 ? 1 : (DIR == 1 ? QP : Q * QP);
-    const int base = lt.el * G::ES + line_off<DIR, Q, QP>(lt.la, lt.lb, 0);
-    float eta[Q], u_[3][Q], eu[3][Q];
+    constexpr int Q = G::Q;
+    float2 e12[Q];  // eta u_1, eta u_2
+    float e3[Q];
 #pragma unroll
     for (int c = 0; c < Q; ++c) {
-        const int o = base + c * OST;
-        eta[c] = sF[V_ETA * NPL + o];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            u_[i][c] = sF[(V_U0 + i) * NPL + o];
-            eu[i][c] = eta[c] * u_[i][c];
-        }
+        e12[c] = mul2(w[c].a, two(w[c].b.y, w[c].b.y));
+        e3[c] = w[c].b.y * w[c].b.x;
     }
 #pragma unroll
-    for (int rr = 0; rr < R; ++rr) {
-        if (!lt.owns(rr)) continue;
-        const int r = lt.r0 + rr;
-        const int a = sPerm[line_lat<DIR, Q>(lt.la, lt.lb, r)];
-        const float *hp = He + ((size_t)e * G::N + a) * 9 + DIR * 3;
-        const float h0 = ldg(hp), h1 = ldg(hp + 1), h2 = ldg(hp + 2);
-        const float hh[3] = {h0, h1, h2};
-        float deta = 0.0f, ddiv = 0.0f, dveta = 0.0f;  // D.eta, sum_i h_i D.(eta u_i), sum_i h_i D.u_i
-        float dv[3] = {0.0f, 0.0f, 0.0f}, deu[3] = {0.0f, 0.0f, 0.0f};
+    for (int r = 0; r < Q; ++r) {
+        const float *hp = he(pt[r]) + DIR * 3;
+        const float h0 = hp[0], h1 = hp[1], h2 = hp[2];
+        float D[Q], de3 = 0.0f;
+        float2 du = two(0.0f, 0.0f), dw = du, de = du;  // D.(u_1, u_2), D.(u_3, eta), D.(eta u_1, eta u_2)
+        tab.row(D, DIR, r);
 #pragma unroll
         for (int c = 0; c < Q; ++c) {
-            const float d = G::S == 1 ? c_VD[G::P][(DIR * Q + rr) * Q + c] : sD[(DIR * Q + r) * Q + c];
-            deta = fmaf(d, eta[c], deta);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                deu[i] = fmaf(d, eu[i][c], deu[i]);
-                dv[i] = fmaf(d, u_[i][c], dv[i]);
-            }
+            const float2 DD = two(D[c], D[c]);
+            du = fma2(DD, w[c].a, du);
+            dw = fma2(DD, w[c].b, dw);
+            de = fma2(DD, e12[c], de);
+            de3 = fmaf(D[c], e3[c], de3);
         }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) ddiv = fmaf(hh[i], deu[i], ddiv);
-        float own_eta = eta[0], own_u[3] = {u_[0][0], u_[1][0], u_[2][0]};
-#pragma unroll
-        for (int c = 1; c < Q; ++c)
-            if (c == r) {
-                own_eta = eta[c];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) own_u[i] = u_[i][c];
-            }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) dveta = fmaf(hh[i], dv[i], dveta);
-        const float su = own_u[0] * h0 + own_u[1] * h1 + own_u[2] * h2;
-        const float contrib = ddiv - own_eta * dveta - su * deta;
-        const int o = base + r * OST;
-        sR[o] = DIR == 0 ? contrib : sR[o] + contrib;
+        const float div_eu = fmaf(h2, de3, fmaf(h1, de.y, h0 * de.x)), div_u = fmaf(h2, dw.x, fmaf(h1, du.y, h0 * du.x));
+        const float U = w[r].a.x * h0 + w[r].a.y * h1 + w[r].b.x * h2;
+        R[r] = div_eu - w[r].b.y * div_u - U * dw.y;
     }
 }
+template <class G, int DIR>
+__device__ __forceinline__ void visc_load(Four<float> (&w)[G::Q], const GroupThread<G> &t, const Four<float> *W)
+{
+    const int base = t.rec0(DIR);
+#pragma unroll
+    for (int s = 0; s < G::Q; ++s) w[s] = W[base + s * G::template step<DIR>()];
+}
 
-// Elements per block at porders 4 and 5 (0: the line-geometry default, five
-// and seven) and minimum resident blocks per SM (0: the block-size bound).
-// Measured (plain estimator, CUDA events): porder 4 on 48^3 hexes 0.398 ms at
-// three elements per 96-thread block against 0.413 ms at five (ten: 0.412 ms);
-// porder 5 on 96^3 hexes 5.78 ms at seven against 5.91 / 6.19 ms at five /
-// three; a minimum of two blocks per SM (more registers) 0.578 / 7.65 ms.
-#ifndef VISC_NE4
-#define VISC_NE4 3
-#endif
-#ifndef VISC_NE5
-#define VISC_NE5 0
-#endif
-#ifndef VISC_MINB
-#define VISC_MINB 0
-#endif
-
-template <class G>
-__global__ void __launch_bounds__(G::NT, VISC_MINB)
+template <class G, bool LIST>
+__global__ void __launch_bounds__(G::NT)
     entropy_visc_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
-                        const float *__restrict__ gpvol, const float *__restrict__ rho, const float *__restrict__ u,
-                        const float *__restrict__ p_or_T, float Rgas, float gamma, float ce, float cmax,
-                        int normalise, const EntropyStats *__restrict__ st, const int *__restrict__ list,
-                        const int *__restrict__ count, float *__restrict__ mu_e, float *__restrict__ nu_out,
-                        float *__restrict__ numax_out, const TableScratch *__restrict__ tabs)
+                        const float *__restrict__ gpvol, const int *__restrict__ inv,
+                        const float *__restrict__ dlxigp_ip, const float *__restrict__ rho,
+                        const float *__restrict__ u, const float *__restrict__ p_or_T, float Rgas, float gamma,
+                        float ce, float cmax, int normalise, const EntropyStats *__restrict__ st,
+                        const int *__restrict__ list, const int *__restrict__ count, float *__restrict__ mu_e,
+                        float *__restrict__ nu_out, float *__restrict__ numax_out)
 {
-    constexpr int Q = G::Q, N = G::N, QP = G::QP, ES = G::ES, NE = G::NE, NT = G::NT, NPL = G::NPL;
+    constexpr int Q = G::Q, N = G::N, NE = G::NE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *sF = reinterpret_cast<float *>(smem_raw);  // [NVF][NPL]
-    float *sR = sF + NVF * NPL;                        // [NPL]
-    float *sD = sR + NPL;                              // [3][Q][Q]
-    int *sNode = reinterpret_cast<int *>(sD + 3 * Q * Q);
-    int *sPerm = sNode + NPL;
-    int *sLat = sPerm + N;
-    __shared__ int s_kS[NE], s_eid[NE];
-    __shared__ float s_vol[NE], s_nu[NE];
-
+    const ViscShared<G, LIST> sm{smem_raw};
     const int tid = threadIdx.x;
-    // The block's elements: e0 .. e0+NE-1 (one group per block), or in list
-    // mode (the per-element fallback) the entries e0 .. of the compacted list,
-    // the blocks striding over the list's groups; -1 beyond the end.
-    const int nwork = list ? ldg(count) : nelem;
+    const GroupThread<G> t(tid);
+    // The block's elements: e0 .. e0+NE-1 (one group per block), or in list mode
+    // the entries e0 .. of the compacted list, the blocks striding over the
+    // list's groups; -1 beyond the end.
+    const int nwork = LIST ? ldg(count) : nelem;
+    bool first = true;
     for (int gb = blockIdx.x; gb * NE < nwork; gb += gridDim.x) {
-    const int e0 = gb * NE;
-    if (VISC_PREFETCH != 0 && !list && tid == 0) {
-        // The group's He and gpvol spans into L2 while its node fields are gathered.
-        const int e1 = min(e0 + NE, nelem);
-        prefetch_span_l2(He + (size_t)e0 * N * 9, (size_t)(e1 - e0) * N * 9 * sizeof(float));
-        prefetch_span_l2(gpvol + (size_t)e0 * N, (size_t)(e1 - e0) * N * sizeof(float));
-    }
-    __syncthreads();  // the previous group's shared-memory reads are complete
-    if (tid < NE) s_eid[tid] = e0 + tid < nwork ? (list ? ldg(list + e0 + tid) : e0 + tid) : -1;
-    __syncthreads();
-    // Node ids of the group (connec is element-fastest) into registers while
-    // the call's tables are copied into shared memory.
-    constexpr int IPT = (NE * N + NT - 1) / NT;
-    int ids[IPT];
+        const int e0 = gb * NE;
+        const GroupMetric<G> gm = [&]() {
+            if constexpr (LIST)
+                return GroupMetric<G>();
+            else
+                return GroupMetric<G>(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);
+        }();
+        auto element = [&](int el) { return e0 + el < nwork ? (LIST ? ldg(list + e0 + el) : e0 + el) : -1; };
+        const int e = t.active ? element(t.el) : -1;
+        auto he = [&](int a) -> const float * {
+            if constexpr (LIST)
+                return He + ((size_t)(e < 0 ? 0 : e) * N + a) * 9;
+            else
+                return gm.he(t.el, a);
+        };
+        int pt[Q], id[Q];
 #pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = tid + k * NT;
-        const int el = i % NE, a = i / NE, e = s_eid[el];
-        ids[k] = (i < NE * N && e >= 0) ? ldg(connec + (size_t)a * nelem + e) - 1 : -1;
-    }
-    for (int i = tid; i < N; i += NT) {
-        sPerm[i] = tabs->perm[i];
-        sLat[i] = tabs->lat[i];
-    }
-    if (G::S > 1)
-        for (int i = tid; i < 3 * Q * Q; i += NT) sD[i] = tabs->Df[i];
-    if (tid < NE) {
-        s_kS[tid] = 0;
-        s_vol[tid] = 0.0f;
-    }
-    __syncthreads();
+        for (int k = 0; k < Q; ++k) pt[k] = GroupTables<G, false>::node(inv, t.template lat<2>(k));
 #pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int i = tid + k * NT;
-        if (i < NE * N) {
-            const int v = ids[k];
-            sNode[(i % NE) * ES + sLat[i / NE]] = (v >= 0 && v < npoin) ? v : -1;
+        for (int k = 0; k < Q; ++k) {
+            const int v = e >= 0 ? ldg_once(connec + (size_t)pt[k] * nelem + e) - 1 : -1;
+            id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
         }
-    }
-    __syncthreads();
-    const size_t np = (size_t)npoin;
-    for (int i = tid; i < NE * N; i += NT) {
-        const int el = i / N, l = i - el * N;
-        const int o = el * ES + (l / (Q * Q) * Q + (l / Q) % Q) * QP + l % Q;
-        const int p = sNode[o];
-        float v[NVF] = {1.0f, 1.0f, 0.0f, 0.0f, 0.0f};
-        if (p >= 0) {
-            v[V_RHO] = ldg(rho + p);
-            v[V_P] = Rgas > 0.0f ? v[V_RHO] * Rgas * ldg(p_or_T + p) : ldg(p_or_T + p);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) v[V_U0 + c] = ldg(u + c * np + p);
+        if (first) sm.tab().build(inv, dlxigp_ip, tid);
+        if (tid < NE) {
+            sm.speed()[tid] = 0;
+            sm.res()[tid] = 0u;
         }
-        // Per point once: the entropy (replacing the pressure), the element
-        // maxima of |u| + c and the element volume.
-        const float spd = sqrtf(v[V_U0] * v[V_U0] + v[V_U1] * v[V_U1] + v[V_U2] * v[V_U2]) +
-                          sqrtf(gamma * v[V_P] / v[V_RHO]);
-        v[V_ETA] = v[V_RHO] / (gamma - 1.0f) * (logf(v[V_P]) - gamma * logf(v[V_RHO]));
+        Four<float> w[Q];
+        float rh[Q], spd = 0.0f, vol = 0.0f;
+        {
+            const size_t np = (size_t)npoin;
+            float f[Q][5];
 #pragma unroll
-        for (int c = 0; c < NVF; ++c) sF[c * NPL + o] = v[c];
-        sR[o] = spd;  // the residual plane is free until the first pass
-    }
-    __syncthreads();
-    // One warp per element: max |u| + c and the volume (warp reductions, no
-    // shared-memory atomics on one address per element).
-    {
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int el = warp; el < NE; el += NT / 32) {
-            const int ee = s_eid[el];
-            unsigned mx = 0u;
-            float vol = 0.0f;
-            if (ee >= 0)
-                for (int l = lane; l < N; l += 32) {
-                    const int o = el * ES + (l / (Q * Q) * Q + (l / Q) % Q) * QP + l % Q;
-                    mx = max(mx, __float_as_uint(sR[o]));  // non-negative floats order like their bits
-                    vol += ldg(gpvol + (size_t)ee * N + sPerm[l]);
-                }
-            mx = __reduce_max_sync(0xffffffffu, mx);
+            for (int k = 0; k < Q; ++k) {
+                const bool ok = id[k] >= 0;
+                const size_t p = ok ? (size_t)id[k] : 0;
+                f[k][0] = ok ? ldg_once(rho + p) : 1.0f;
+                f[k][1] = ok ? ldg_once(p_or_T + p) : 1.0f;
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, off);
-            if (lane == 0) {
-                s_kS[el] = (int)mx;
-                s_vol[el] = vol;
+                for (int c = 0; c < 3; ++c) f[k][2 + c] = ok ? ldg_once(u + c * np + p) : 0.0f;
             }
-        }
-    }
-    __syncthreads();
-    const LineThread<G> lt(tid);
-    const int e = s_eid[lt.el];
-    const bool live = lt.active && e >= 0;
-    if (live) residual_pass<G, 0>(lt, sF, sR, sPerm, sD, He, e, gamma);
-    __syncthreads();
-    if (live) residual_pass<G, 1>(lt, sF, sR, sPerm, sD, He, e, gamma);
-    __syncthreads();
-    if (live) residual_pass<G, 2>(lt, sF, sR, sPerm, sD, He, e, gamma);
-    __syncthreads();
-    float neta = 1.0f;
-    if (normalise) {
-        const double mean = st->sum / (double)npoin;
-        const double lo = (double)key2f(st->kmin), hi = (double)key2f(st->kmax);
-        neta = (float)fmax(hi - mean, mean - lo);
-        if (!(neta > 0.0f)) neta = 1.0f;
-    }
-    // Element maxima of |R| and the element viscosity (one warp per element).
-    {
-        const int lane = tid & 31, warp = tid >> 5;
-        for (int el = warp; el < NE; el += NT / 32) {
-            const int ee = s_eid[el];
-            unsigned mx = 0u;
-            if (ee >= 0)
-                for (int l = lane; l < N; l += 32) {
-                    const int o = el * ES + (l / (Q * Q) * Q + (l / Q) % Q) * QP + l % Q;
-                    mx = max(mx, __float_as_uint(fabsf(sR[o])));
-                }
-            mx = __reduce_max_sync(0xffffffffu, mx);
-            if (lane == 0) {
-                const float h = cbrtf(s_vol[el]) / (float)(Q - 1);
-                const float numax = cmax * h * __int_as_float(s_kS[el]);
-                const float nuE = ce * h * h * __uint_as_float(mx) / neta;
-                const float nu = fminf(numax, nuE);
-                s_nu[el] = nu;
-                if (ee >= 0) {
-                    if (nu_out) nu_out[ee] = nu;
-                    if (numax_out && !list) numax_out[ee] = numax;
-                }
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                const float r = f[k][0], p = (Rgas > 0.0f && id[k] >= 0) ? r * Rgas * f[k][1] : f[k][1];
+                const float s = sqrtf(f[k][2] * f[k][2] + f[k][3] * f[k][3] + f[k][4] * f[k][4]) + sqrtf(gamma * p / r);
+                spd = __uint_as_float(max(__float_as_uint(spd), __float_as_uint(s)));  // as their bits: NaN counts
+                rh[k] = r;
+                w[k].a = two(f[k][2], f[k][3]);
+                w[k].b = two(f[k][4], r / (gamma - 1.0f) * (logf(p) - gamma * logf(r)));
             }
+            const int base = t.rec0(2);
+            if (t.active)
+#pragma unroll
+                for (int k = 0; k < Q; ++k) sm.W()[base + k * G::template step<2>()] = w[k];
         }
-    }
-    if (list) continue;
-    if (mu_e) {
         __syncthreads();
-        for (int i = tid; i < NE * N; i += NT) {
-            const int el = i % NE, a = i / NE, ee = s_eid[el];
-            if (ee < 0) continue;
-            mu_e[(size_t)a * nelem + ee] = sF[V_RHO * NPL + el * ES + sLat[a]] * s_nu[el];
+        first = false;
+        const GroupRows<G, false> tab(sm.tab());
+        // A bounded wait that ran out leaves the group's viscosity NaN.
+        const bool ok = LIST || gm.wait(sm.bar());
+        float R[Q];
+        int lp[Q];
+        if (t.active) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                if constexpr (LIST)
+                    vol += e >= 0 ? ldg(gpvol + (size_t)e * N + pt[k]) : 0.0f;
+                else
+                    vol += *gm.vol(t.el, pt[k]);
+            }
+            sm.vol()[(t.q1 * Q + t.q0) * NE + t.el] = ok ? vol : __int_as_float(0x7fffffff);
+            if (e >= 0) atomicMax(reinterpret_cast<unsigned *>(sm.speed()) + t.el, __float_as_uint(spd));
+            visc_line<G, 2>(w, t, tab, he, pt, R);
+            const int base = t.rec0(2);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) sm.R()[base + k * G::template step<2>()] = R[k];
         }
-    }
-    break;  // one group per block outside list mode
+        __syncthreads();
+        if (t.active) {
+            visc_load<G, 0>(w, t, sm.W());
+#pragma unroll
+            for (int k = 0; k < Q; ++k) lp[k] = GroupTables<G, false>::node(inv, t.template lat<0>(k));
+            visc_line<G, 0>(w, t, tab, he, lp, R);
+            const int base = t.rec0(0);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) sm.R()[base + k] += R[k];
+        }
+        __syncthreads();
+        if (t.active) {
+            visc_load<G, 1>(w, t, sm.W());
+#pragma unroll
+            for (int k = 0; k < Q; ++k) lp[k] = GroupTables<G, false>::node(inv, t.template lat<1>(k));
+            visc_line<G, 1>(w, t, tab, he, lp, R);
+            const int base = t.rec0(1);
+            unsigned mx = 0u;
+#pragma unroll
+            for (int k = 0; k < Q; ++k)
+                mx = max(mx, __float_as_uint(fabsf(sm.R()[base + k * G::template step<1>()] + R[k])));
+            if (e >= 0) atomicMax(sm.res() + t.el, mx);
+        }
+        __syncthreads();
+        if (tid < NE) {
+            const int ee = element(tid);
+            float neta = 1.0f;
+            if (normalise) {
+                const double mean = st->sum / (double)npoin;
+                const double lo = (double)key2f(st->kmin), hi = (double)key2f(st->kmax);
+                neta = (float)fmax(hi - mean, mean - lo);
+                if (!(neta > 0.0f)) neta = 1.0f;
+            }
+            float v = 0.0f;
+            for (int l = 0; l < G::L; ++l) v += sm.vol()[l * NE + tid];
+            const float h = cbrtf(v) / (float)(Q - 1);
+            const float numax = cmax * h * __int_as_float(sm.speed()[tid]);
+            const float nuE = ce * h * h * __uint_as_float(sm.res()[tid]) / neta;
+            const float nu = fminf(numax, nuE);
+            sm.nu()[tid] = nu;
+            if (ee >= 0) {
+                if (nu_out) nu_out[ee] = nu;
+                if (numax_out && !LIST) numax_out[ee] = numax;
+            }
+        }
+        __syncthreads();
+        if constexpr (LIST) continue;
+        if (mu_e && e >= 0) {
+            const float nu = sm.nu()[t.el];
+#pragma unroll
+            for (int k = 0; k < Q; ++k) mu_e[(size_t)pt[k] * nelem + e] = rh[k] * nu;
+        }
+        break;  // one group per block outside list mode
     }
 }
 
-template <int P>
-using ViscGeom = LineGeom<float, P, (P == 4 && VISC_NE4 > 0) ? VISC_NE4 : ((P == 5 && VISC_NE5 > 0) ? VISC_NE5 : 64)>;
-
-// Preferred shared-memory carveout of the porder-5 estimator, percent of the
-// maximum (-1: none). Its 51.5 KB blocks fill a 228 KB carveout four to an SM
-// and leave ~28 KB of L1; at 58 % (132 KB: two blocks, ~124 KB of L1) it runs
-// 1.80 ms instead of 2.36 ms on 64^3 hexes (72 %, three blocks: 1.86 ms).
-// Porder 4 measures the same with or without (0.89 ms).
-#ifndef VISC_CARVE5
-#define VISC_CARVE5 58
-#endif
-
-template <int P>
-cudaError_t visc_p(const ViscArgs &a, cudaStream_t st)
+template <int P, bool LIST>
+cudaError_t visc_pl(const ViscArgs &a, cudaStream_t st)
 {
-    using G = ViscGeom<P>;
-    constexpr size_t smem = (size_t)(NVF + 1) * G::NPL * sizeof(float) + 3 * G::Q * G::Q * sizeof(float) +
-                            (size_t)(G::NPL + 2 * G::N) * sizeof(int);
+    using G = typename ViscGroup<P, LIST>::G;
+    constexpr size_t smem = ViscShared<G, LIST>::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    auto kern = entropy_visc_kernel<G>;
-    if (!a.tabs) return cudaErrorInvalidValue;
-    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto kern = entropy_visc_kernel<G, LIST>;
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
-    if (P == 5 && VISC_CARVE5 >= 0) {
-        err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, VISC_CARVE5);
-        if (err != cudaSuccess) return err;
-    }
-    if (G::S == 1) {
-        err = cudaMemcpyToSymbolAsync(c_VD, a.tabs->Df, sizeof(float) * 3 * G::Q * G::Q, sizeof(float) * kTableDMax * P,
-                                      cudaMemcpyDeviceToDevice, st);
-        if (err != cudaSuccess) return err;
-    }
     // List mode: resident blocks stride over the list (its length is known on
     // the device only); otherwise one group per block.
     const int ngroups = (a.nelem + G::NE - 1) / G::NE;
-    const unsigned grid = (unsigned)(a.list ? persistent_grid(kern, G::NT, smem, ngroups) : ngroups);
+    const unsigned grid = (unsigned)(LIST ? persistent_grid(kern, G::NT, smem, ngroups) : ngroups);
     if (grid == 0) return cudaErrorInvalidConfiguration;
-    kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.rho, a.u, a.p_or_T, a.Rgas, a.gamma,
-                                    a.ce, a.cmax, a.normalise,
-                                    a.stats, a.list, a.count, a.mu_e, a.nu, a.numax, a.tabs);
+    kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK, a.dlxigp_ip, a.rho, a.u,
+                                    a.p_or_T, a.Rgas, a.gamma, a.ce, a.cmax, a.normalise, a.stats, a.list, a.count,
+                                    a.mu_e, a.nu, a.numax);
     return cudaGetLastError();
+}
+template <int P>
+cudaError_t visc_p(const ViscArgs &a, cudaStream_t st)
+{
+    return a.list ? visc_pl<P, true>(a, st) : visc_pl<P, false>(a, st);
 }
 
 }  // namespace
