@@ -19,9 +19,10 @@
 // D = D_hi + D_lo.  Products, shifts and scalings use explicit roundings, so
 // a field that is constant over the element splits into exact zeros.
 //
-// Contraction.  Per (field, direction, 16 lines) two accumulating
+// Contraction.  Per (two fields, direction, tile of 8 lines) two accumulating
 // mma.sync.m16n8k16:
-//   A (16x16) = [f_hi | f_lo]          rows: line, cols: input point (hi | lo)
+//   A (16x16) = [f_hi | f_lo]          rows: line of the first / second field,
+//                                      cols: input point (hi | lo)
 //   B1 (16x8) = [D_hi^T ; D_hi^T]      rows: input point (hi | lo), cols: output point
 //   B2 (16x8) = [D_lo^T ; 0]
 // C = f_hi D_hi^T + f_lo D_hi^T + f_hi D_lo^T (the dropped f_lo D_lo^T is
@@ -38,7 +39,13 @@
 // that direction and the point's own nodal values, to seven per-point
 // accumulators in shared memory; the last pass assembles the energy residual
 // in FP64 and scatter-adds all residuals with red.global.add.f64.
-// porder 1..7; persistent blocks of four warps, one element at a time.
+// porder 1..7; persistent blocks of one warp per tile (Q warps), one element at
+// a time.  The kernel waits on its phases' loads, so residency pays: two fields
+// of one tile per contraction instead of one field of two tiles halves a
+// thread's state (two points instead of four) and leaves no warp without a tile.
+// FP16, two tiles per warp in blocks of four warps / now: porder 7 24^3 0.907 /
+// 0.815 ms, 6 32^3 1.842 / 1.424, 5 40^3 2.354 / 2.052, 4 48^3 4.918 / 2.692, 3
+// 48^3 2.647 / 1.867, 2 64^3 5.990 / 3.180, 1 64^3 5.532 / 2.139.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -51,8 +58,6 @@ namespace msod {
 namespace {
 
 constexpr int kNF = 31;       // differentiated products
-constexpr int kThreads = 128;
-
 enum { B_RHO = 0, B_P, B_E, B_U0, B_U1, B_U2, B_Q0, B_Q1, B_Q2, NBASE };
 enum { A_M = 0, A_MOM0, A_MOM1, A_MOM2, A_E, A_DIVU, A_DIVQ, NACC };
 
@@ -97,18 +102,16 @@ __device__ __forceinline__ float field(int f, const Nodal &n)
     return __fmul_rn(n.H, n.u[f - 28]);
 }
 
-// Lattice point of slot s (s = 0, 1: line g of tile o1; 2, 3: line g of tile
-// o2; output point 2t + (s & 1) along direction d); -1 when padded.
+// Lattice point of slot s (output point 2t + s along direction d of line g of
+// tile o); -1 when padded.
 template <int Q>
-__device__ __forceinline__ int pass_point(int d, int s, int g, int tq, int o1, int o2, bool has1, bool has2)
+__device__ __forceinline__ int pass_point(int d, int s, int g, int tq, int o)
 {
-    const int o = s < 2 ? o1 : o2;
-    const int pt = 2 * tq + (s & 1);
+    const int pt = 2 * tq + s;
     const int I = d == 0 ? pt : g;
     const int J = d == 0 ? g : (d == 1 ? pt : o);
     const int K = d == 2 ? pt : o;
-    const bool live = (s < 2 ? has1 : has2) && g < Q && pt < Q;
-    return live ? (K * Q + J) * Q + I : -1;
+    return g < Q && pt < Q ? (K * Q + J) * Q + I : -1;
 }
 
 // Per-point coefficients of one direction pass.
@@ -158,17 +161,20 @@ __device__ __forceinline__ void apply_field(int f, float dv, const PointCoef &c,
 template <int P, bool BF16>
 struct MixedGeom {
     static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2;
+    static constexpr int NT = 32 * Q;        // one warp per tile (k-plane or j-plane) of lines
     static constexpr int NTASK = Q * Q * W;  // task: points (2w, 2w+1) of one i-row
-    static constexpr int TPT = (NTASK + kThreads - 1) / kThreads;
+    static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
     static constexpr size_t half_bytes = (size_t)2 * kNF * PB + plane_guard_bytes<Q>();
     static constexpr size_t smem = half_bytes + (size_t)(NBASE + NACC) * N * sizeof(float) +
                                    (size_t)2 * N * sizeof(int) + 2 * 32 * sizeof(float);
+    // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
+    static constexpr int MINB = mixed_blocks(smem, NT, kMixedRegs);
 };
 
 template <int P, bool BF16>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
     convec_mixed_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
                         const float *__restrict__ gpvol, const TableScratch *__restrict__ tabs,
                         const float *__restrict__ u, const float *__restrict__ q, const float *__restrict__ rho,
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(kThreads)
                         double *__restrict__ Rmom, double *__restrict__ Rener)
 {
     using G = MixedGeom<P, BF16>;
-    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, TPT = G::TPT;
+    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *sHalf = smem_raw;                                  // [2*kNF][G::PB]: hi, lo of each field
     float *sBase = reinterpret_cast<float *>(sHalf + G::half_bytes);  // [NBASE][N], lattice (K*Q+J)*Q+I
@@ -190,10 +196,10 @@ __global__ void __launch_bounds__(kThreads)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Once per block: tables, the zero padding of the half planes (rows and
     // points beyond Q are never written), the B fragments.
-    for (int i = tid; i < N; i += kThreads) sPerm[i] = tabs->perm[i];
+    for (int i = tid; i < N; i += NT) sPerm[i] = tabs->perm[i];
     if (Q < 8) {
         uint4 *z = reinterpret_cast<uint4 *>(sHalf);
-        for (int i = tid; i < (int)(G::half_bytes / 16); i += kThreads) z[i] = make_uint4(0, 0, 0, 0);
+        for (int i = tid; i < (int)(G::half_bytes / 16); i += NT) z[i] = make_uint4(0, 0, 0, 0);
     }
     // B fragments per direction: col lane/4 (output point), rows 2t, 2t+1 (input point).
     unsigned Bh[3], Bl[3];
@@ -207,13 +213,9 @@ __global__ void __launch_bounds__(kThreads)
     const size_t np = (size_t)npoin;
 #pragma unroll 1
     for (int e = blockIdx.x; e < nelem; e += gridDim.x) {
-    if (MIXED_PREFETCH != 0 && tid == 0) {  // He and gpvol spans into L2, an element ahead
-        if (e == (int)blockIdx.x) prefetch_element_l2(He, gpvol, e, N);
-        if (e + (int)gridDim.x < nelem) prefetch_element_l2(He, gpvol, e + gridDim.x, N);
-    }
     __syncthreads();  // the previous element's passes are done with every shared array
     if (tid < 32) sMax[tid] = 0u;
-    for (int l = tid; l < N; l += kThreads) {
+    for (int l = tid; l < N; l += NT) {
         const int a = sPerm[l];
         const int v = ldg(connec + (size_t)a * nelem + e) - 1;
         const bool ok = (unsigned)v < (unsigned)npoin;
@@ -235,48 +237,34 @@ __global__ void __launch_bounds__(kThreads)
 
     // He columns of the first direction pass, in flight during the split.
     const int g = lane >> 2, tq = lane & 3;
-    const int o1 = warp, o2 = warp + 4 < Q ? warp + 4 : warp;
-    const bool has1 = o1 < Q, has2 = warp + 4 < Q;
-    float hcur[4][3];
+    float hcur[2][3];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int l = pass_point<Q>(0, s, g, tq, o1, o2, has1, has2);
+    for (int s = 0; s < 2; ++s) {
+        const int l = pass_point<Q>(0, s, g, tq, warp);
         const float *hp = He + ((size_t)e * N + sPerm[l < 0 ? 0 : l]) * 9;
 #pragma unroll
         for (int c = 0; c < 3; ++c) hcur[s][c] = ldg(hp + c);
     }
 
-    // Shifted products of the thread's tasks (two points each) in registers,
-    // their per-field maxima over the element (non-negative floats order like
-    // their bit patterns), then the split into the half planes.
-    const Nodal nref = nodal_from(sBase, N, 0);
-    float v[TPT][kNF][2];
+    // Shifted products of the thread's task (two points) in registers, their
+    // per-field maxima over the element (non-negative floats order like their
+    // bit patterns), then the split into the half planes.
+    const bool valid = tid < NTASK;
+    const int row = valid ? tid / W : 0, w = valid ? tid - row * W : 0;
+    const bool two = valid && 2 * w + 1 < Q;
+    float v[kNF][2];
     {
-        float mx[kNF];
-#pragma unroll
-        for (int f = 0; f < kNF; ++f) mx[f] = 0.0f;
-#pragma unroll
-        for (int tk = 0; tk < TPT; ++tk) {
-            const int t = tid + tk * kThreads;
-            const bool valid = t < NTASK;
-            const int row = valid ? t / W : 0, w = valid ? t - row * W : 0;
-            const int l0 = row * Q + 2 * w;
-            const bool two = valid && 2 * w + 1 < Q;
-            const Nodal n0 = nodal_from(sBase, N, l0);
-            const Nodal n1 = nodal_from(sBase, N, two ? l0 + 1 : l0);
-#pragma unroll
-            for (int f = 0; f < kNF; ++f) {
-                const float fr = field(f, nref);
-                const float a = valid ? __fsub_rn(field(f, n0), fr) : 0.0f;
-                const float b = two ? __fsub_rn(field(f, n1), fr) : 0.0f;
-                v[tk][f][0] = a;
-                v[tk][f][1] = b;
-                mx[f] = fmaxf(mx[f], fmaxf(fabsf(a), fabsf(b)));
-            }
-        }
+        const Nodal nref = nodal_from(sBase, N, 0);
+        const int l0 = row * Q + 2 * w;
+        const Nodal n0 = nodal_from(sBase, N, l0);
+        const Nodal n1 = nodal_from(sBase, N, two ? l0 + 1 : l0);
 #pragma unroll
         for (int f = 0; f < kNF; ++f) {
-            const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx[f]));
+            const float fr = field(f, nref);
+            v[f][0] = valid ? __fsub_rn(field(f, n0), fr) : 0.0f;
+            v[f][1] = two ? __fsub_rn(field(f, n1), fr) : 0.0f;
+            const float mx = fmaxf(0.0f, fmaxf(fabsf(v[f][0]), fabsf(v[f][1])));
+            const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
             if (lane == 0) atomicMax(&sMax[f], mb);
         }
     }
@@ -289,45 +277,38 @@ __global__ void __launch_bounds__(kThreads)
         sInv[tid] = __int_as_float((127 + ex - (G::BITS - 1)) << 23);
     }
     __syncthreads();
-#pragma unroll
-    for (int tk = 0; tk < TPT; ++tk) {
-        const int t = tid + tk * kThreads;
-        if (t >= NTASK) break;
-        const int row = t / W, w = t - row * W;
+    if (valid) {
         const int rk = row / Q, rj = row - rk * Q;
         const int off = row_pos(rk, rj) * kRowB + 4 * w;
 #pragma unroll
         for (int f = 0; f < kNF; ++f) {
             const float s = sScale[f];
-            const float a = __fmul_rn(v[tk][f][0], s), b = __fmul_rn(v[tk][f][1], s);
-            const float M = 12582912.0f;  // 1.5 * 2^23: adding and subtracting it rounds to an integer
-            const float ha = __fsub_rn(__fadd_rn(a, M), M), hb = __fsub_rn(__fadd_rn(b, M), M);
-            *reinterpret_cast<unsigned *>(sHalf + (2 * f) * G::PB + off) = pack2<BF16>(ha, hb);
-            *reinterpret_cast<unsigned *>(sHalf + (2 * f + 1) * G::PB + off) =
-                pack2<BF16>(__fsub_rn(a, ha), __fsub_rn(b, hb));
+            unsigned hi, lo;
+            split_scaled<BF16>(__fmul_rn(v[f][0], s), __fmul_rn(v[f][1], s), hi, lo);
+            *reinterpret_cast<unsigned *>(sHalf + (2 * f) * G::PB + off) = hi;
+            *reinterpret_cast<unsigned *>(sHalf + (2 * f + 1) * G::PB + off) = lo;
         }
     }
     __syncthreads();
 
-    // Warp w takes the 16 lines of tiles o1 = w and o2 = w + 4 (k-planes for
-    // xi / eta lines, j-planes for zeta lines); ldmatrix matrix m of the A
-    // operand is (hi o1, hi o2, lo o1, lo o2), row r8.
+    // Warp w takes tile w (a k-plane for xi / eta lines, a j-plane for zeta
+    // lines) of two fields f, f+1 at a time; ldmatrix matrix m of the A operand is
+    // (hi f, hi f+1, lo f, lo f+1), row r8.  The last field stands alone: its rows
+    // twice, the second result unused.
     const int m = lane >> 3, r8 = lane & 7;
-    const int om = (m & 1) ? o2 : o1;
-    const int plane_off = (m >> 1) * G::PB;
+    const int alone = (m & 1) * 2 * G::PB, plane_off = alone + (m >> 1) * G::PB;
 #pragma unroll 1
     for (int d = 0; d < 3; ++d) {
         const unsigned bh = d == 0 ? Bh[0] : (d == 1 ? Bh[1] : Bh[2]);
         const unsigned bl = d == 0 ? Bl[0] : (d == 1 ? Bl[1] : Bl[2]);
-        // The thread's points: s = 0, 1 line g of tile o1, s = 2, 3 line g of
-        // tile o2; output points 2t and 2t+1 along the direction.
-        int lat[4];
-        bool live[4];
-        PointCoef cf[4];
-        float acc[4][NACC], gp[4];
+        // The thread's points: output points 2t and 2t+1 of line g of the tile.
+        int lat[2];
+        bool live[2];
+        PointCoef cf[2];
+        float acc[2][NACC], gp[2];
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const int lp = pass_point<Q>(d, s, g, tq, o1, o2, has1, has2);
+        for (int s = 0; s < 2; ++s) {
+            const int lp = pass_point<Q>(d, s, g, tq, warp);
             live[s] = lp >= 0;
             const int l = live[s] ? lp : 0;
             lat[s] = l;
@@ -347,9 +328,9 @@ __global__ void __launch_bounds__(kThreads)
         // Loads in flight during the contractions: the next pass's He columns,
         // or gpvol for the last pass's scatter.
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
+        for (int s = 0; s < 2; ++s) {
             if (d < 2) {
-                const int l = pass_point<Q>(d + 1, s, g, tq, o1, o2, has1, has2);
+                const int l = pass_point<Q>(d + 1, s, g, tq, warp);
                 const float *hp = He + ((size_t)e * N + sPerm[l < 0 ? 0 : l]) * 9 + (d + 1) * 3;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) hcur[s][c] = ldg(hp + c);
@@ -359,31 +340,36 @@ __global__ void __launch_bounds__(kThreads)
             }
         }
         const unsigned char *rowp =
-            sHalf + plane_off + (d == 2 ? row_pos(r8, om) : row_pos(om, r8)) * kRowB;
+            sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
 #pragma unroll
-        for (int f = 0; f < kNF; ++f) {
+        for (int f = 0; f < kNF; f += 2) {
+            const unsigned char *src = rowp + 2 * f * G::PB - (f + 1 < kNF ? 0 : alone);
             unsigned a[4];
             if (d == 0)
-                ldsm_x4(a, rowp + 2 * f * G::PB);
+                ldsm_x4(a, src);
             else
-                ldsm_x4_t(a, rowp + 2 * f * G::PB);
+                ldsm_x4_t(a, src);
             float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             mma_acc<BF16>(c, a, bh, bh);
             mma_acc<BF16>(c, a, bl, 0u);
-            const float inv = sInv[f];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) apply_field(f, c[s] * inv, cf[s], acc[s]);
+            for (int k = 0; k < 2; ++k) {
+                if (f + k >= kNF) break;
+                const float inv = sInv[f + k];
+#pragma unroll
+                for (int s = 0; s < 2; ++s) apply_field(f + k, c[2 * k + s] * inv, cf[s], acc[s]);
+            }
         }
         if (d < 2) {
 #pragma unroll
-            for (int s = 0; s < 4; ++s)
+            for (int s = 0; s < 2; ++s)
                 if (live[s])
 #pragma unroll
                     for (int k = 0; k < NACC; ++k) sAcc[k * N + lat[s]] = acc[s][k];
             __syncthreads();
         } else {
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
+            for (int s = 0; s < 2; ++s) {
                 if (!live[s]) continue;
                 const int node = sNode[lat[s]];
                 if (node < 0) continue;
@@ -414,9 +400,9 @@ cudaError_t launch_mixed_pb(const MixedConvecArgs &a, const TableScratch *tabs, 
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
     if (err != cudaSuccess) return err;
     if (a.nelem == 0) return cudaSuccess;
-    const int grid = persistent_grid(kern, kThreads, G::smem, a.nelem);
+    const int grid = persistent_grid(kern, G::NT, G::smem, a.nelem);
     if (grid < 1) return cudaErrorInvalidConfiguration;
-    kern<<<grid, kThreads, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.u, a.q, a.rho,
+    kern<<<grid, G::NT, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.u, a.q, a.rho,
                                              a.pr, a.E, a.Rmass, a.Rmom, a.Rener);
     return cudaGetLastError();
 }

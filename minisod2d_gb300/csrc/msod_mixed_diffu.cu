@@ -5,12 +5,12 @@
 // cores as FP16 (or BF16) hi + lo split products (FP32 accumulation) and the
 // energy-flux assembly and the nodal scatter-add in FP64 (FP64 outputs).
 //
-// Per element (one block of four warps, persistent over elements):
+// Per element (one block of one warp per tile, persistent over elements):
 //   1. gather rho, T, u, mu_fluid, mu_e, mu_sgs into a lattice in shared memory;
 //   2. gradient stage: rho, T, u_1..3 are shifted by their value at lattice
 //      node (0,0,0) (the derivative annihilates constants), scaled by a power
 //      of two per element and field, split into hi + lo half planes; per
-//      direction, two accumulating mma.sync.m16n8k16 per field and 16 lines
+//      direction, two accumulating mma.sync.m16n8k16 per two fields and 8 lines
 //      (A = [f_hi | f_lo], B = [D_hi^T ; D_hi^T] then [D_lo^T ; 0]) give the
 //      15 iso-parametric derivatives per point;
 //   3. point pass: physical gradients, stress tau, tau.u and the contravariant
@@ -27,7 +27,10 @@
 //   5. Rmass += nu_e sum(grad rho), Rmom_m += sum(tau_m), and in FP64
 //      Rener += sum(tau.u) + kappa_e sum(grad T); red.global.add.f64.
 // Shared-memory half planes use the swizzled layout of msod_mma.cuh.
-// porder 1..7.
+// porder 1..7.  One tile per warp, as in msod_mixed.cu: two tiles per warp in
+// blocks of four warps / now, FP16: porder 7 24^3 0.851 / 0.706 ms, 6 32^3 1.555 /
+// 1.444, 5 40^3 1.996 / 1.776, 4 48^3 2.164 / 2.114, 3 48^3 1.620 / 1.530, 2 64^3
+// 3.508 / 2.434, 1 64^3 3.377 / 1.718.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -39,7 +42,6 @@
 namespace msod {
 namespace {
 
-constexpr int kThreads = 128;
 constexpr int kNG = 5;   // differentiated node fields: rho, T, u_1..3
 constexpr int kNX = 6;   // flux vectors: grad rho, tau.u, grad T, tau rows 1..3
 constexpr int kNFX = 3 * kNX;
@@ -50,30 +52,31 @@ enum { X_GRHO = 0, X_TAUU, X_GT, X_TAU0, X_TAU1, X_TAU2 };
 template <int P, bool BF16>
 struct MixedDiffuGeom {
     static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2;
+    static constexpr int NT = 32 * Q;        // one warp per tile (k-plane or j-plane) of lines
     static constexpr int NTASK = Q * Q * W;  // task: points (2w, 2w+1) of one i-row
-    static constexpr int TPT = (NTASK + kThreads - 1) / kThreads;
+    static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
     static constexpr size_t half_bytes = (size_t)2 * kNFX * PB + plane_guard_bytes<Q>();
     static constexpr size_t smem = half_bytes + (size_t)(NSB + 3 * kNG + 2) * N * sizeof(float) +
                                    (size_t)2 * N * sizeof(int) + 3 * 32 * sizeof(float);
+    // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
+    static constexpr int MINB = mixed_blocks(smem, NT, kMixedRegs);
 };
 
 // Lattice point of slot s of a pass (see msod_mixed.cu); -1 when padded.
 template <int Q>
-__device__ __forceinline__ int dpass_point(int d, int s, int g, int tq, int o1, int o2, bool has1, bool has2)
+__device__ __forceinline__ int dpass_point(int d, int s, int g, int tq, int o)
 {
-    const int o = s < 2 ? o1 : o2;
-    const int pt = 2 * tq + (s & 1);
+    const int pt = 2 * tq + s;
     const int I = d == 0 ? pt : g;
     const int J = d == 0 ? g : (d == 1 ? pt : o);
     const int K = d == 2 ? pt : o;
-    const bool live = (s < 2 ? has1 : has2) && g < Q && pt < Q;
-    return live ? (K * Q + J) * Q + I : -1;
+    return g < Q && pt < Q ? (K * Q + J) * Q + I : -1;
 }
 
 template <int P, bool BF16, bool NUE>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
     diffu_mixed_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
                        const float *__restrict__ gpvol, const TableScratch *__restrict__ tabs, float Cp, float Pr,
                        const float *__restrict__ rho, const float *__restrict__ u, const float *__restrict__ Tem,
@@ -82,7 +85,7 @@ __global__ void __launch_bounds__(kThreads)
                        double *__restrict__ Rmass, double *__restrict__ Rmom, double *__restrict__ Rener)
 {
     using G = MixedDiffuGeom<P, BF16>;
-    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, TPT = G::TPT;
+    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *sHalf = smem_raw;                                  // [2*kNFX][G::PB]
     float *sB = reinterpret_cast<float *>(sHalf + G::half_bytes);     // [NSB][N] lattice (K*Q+J)*Q+I
@@ -97,10 +100,10 @@ __global__ void __launch_bounds__(kThreads)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    for (int i = tid; i < N; i += kThreads) sPerm[i] = tabs->perm[i];
+    for (int i = tid; i < N; i += NT) sPerm[i] = tabs->perm[i];
     if (Q < 8) {  // rows and points beyond Q are never written and stay zero
         uint4 *z = reinterpret_cast<uint4 *>(sHalf);
-        for (int i = tid; i < (int)(G::half_bytes / 16); i += kThreads) z[i] = make_uint4(0, 0, 0, 0);
+        for (int i = tid; i < (int)(G::half_bytes / 16); i += NT) z[i] = make_uint4(0, 0, 0, 0);
     }
     // B fragments per direction.  Gradient: B[k][n] = D[n][k]; divergence:
     // B[k][n] = D[k][n] (k input point, n output point); hi and lo halves.
@@ -126,24 +129,25 @@ __global__ void __launch_bounds__(kThreads)
                 for (int c = 0; c < Q; ++c) cs += (double)tabs->Df[(d * Q + c) * Q + a];
             colsum[d][h] = (float)cs;
         }
-    const int o1 = warp, o2 = warp + 4 < Q ? warp + 4 : warp;
-    const bool has1 = o1 < Q, has2 = warp + 4 < Q;
+    // ldmatrix matrix m of the A operand is (hi f, hi f+1, lo f, lo f+1), row r8
+    // of tile w = warp; a field that stands alone is loaded twice.
     const int m = lane >> 3, r8 = lane & 7;
-    const int om = (m & 1) ? o2 : o1;
-    const int plane_off = (m >> 1) * G::PB;
+    const int alone = (m & 1) * 2 * G::PB, plane_off = alone + (m >> 1) * G::PB;
+    // The thread's task of the split and the point pass: points (2w, 2w+1) of i-row `row`.
+    const bool valid = tid < NTASK;
+    const int row = valid ? tid / W : 0, w = valid ? tid - row * W : 0;
+    const int row_off = row_pos(row / Q, row % Q) * kRowB + 4 * w;
+    const int l0 = row * Q + 2 * w;
+    const bool two = valid && 2 * w + 1 < Q;
     const size_t np = (size_t)npoin;
     const float twoThirds = 2.0f / 3.0f;
 
 #pragma unroll 1
     for (int e = blockIdx.x; e < nelem; e += gridDim.x) {
-        if (MIXED_PREFETCH != 0 && tid == 0) {  // He and gpvol spans into L2, an element ahead
-            if (e == (int)blockIdx.x) prefetch_element_l2(He, gpvol, e, N);
-            if (e + (int)gridDim.x < nelem) prefetch_element_l2(He, gpvol, e + gridDim.x, N);
-        }
         __syncthreads();  // the previous element is done with every shared array
         if (tid < 32) sMax[tid] = 0u;
         const float nue = NUE ? ldg(nu_elem + e) : 0.0f;
-        for (int l = tid; l < N; l += kThreads) {
+        for (int l = tid; l < N; l += NT) {
             const int a = sPerm[l];
             const int v = ldg(connec + (size_t)a * nelem + e) - 1;
             const bool ok = (unsigned)v < (unsigned)npoin;
@@ -164,19 +168,13 @@ __global__ void __launch_bounds__(kThreads)
         }
         cp_async_commit();
         // He and gpvol of the point-pass points, in flight during the gradient stage.
-        float hv[TPT][2][9], gv[TPT][2];
+        float hv[2][9], gv[2];
 #pragma unroll
-        for (int tk = 0; tk < TPT; ++tk) {
-            const int t = tid + tk * kThreads;
-            const int row = t < NTASK ? t / W : 0, w = t < NTASK ? t - row * W : 0;
+        for (int h = 0; h < 2; ++h) {
+            const size_t base = (size_t)e * N + sPerm[(h ? two : valid) ? l0 + h : 0];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int l = (t < NTASK && 2 * w + h < Q) ? row * Q + 2 * w + h : 0;
-                const size_t base = (size_t)e * N + sPerm[l];
-#pragma unroll
-                for (int j = 0; j < 9; ++j) hv[tk][h][j] = ldg(He + base * 9 + j);
-                gv[tk][h] = ldg(gpvol + base);
-            }
+            for (int j = 0; j < 9; ++j) hv[h][j] = ldg(He + base * 9 + j);
+            gv[h] = ldg(gpvol + base);
         }
         cp_async_wait_all();
         __syncthreads();
@@ -186,47 +184,26 @@ __global__ void __launch_bounds__(kThreads)
             float ref[kNG];
 #pragma unroll
             for (int f = 0; f < kNG; ++f) ref[f] = sB[f * N];  // planes S_RHO..S_U2 are fields 0..4
-            float v[TPT][kNG][2], mx[kNG];
-#pragma unroll
-            for (int f = 0; f < kNG; ++f) mx[f] = 0.0f;
-#pragma unroll
-            for (int tk = 0; tk < TPT; ++tk) {
-                const int t = tid + tk * kThreads;
-                const bool valid = t < NTASK;
-                const int row = valid ? t / W : 0, w = valid ? t - row * W : 0;
-                const int l0 = row * Q + 2 * w;
-                const bool two = valid && 2 * w + 1 < Q;
-#pragma unroll
-                for (int f = 0; f < kNG; ++f) {
-                    const float a = valid ? __fsub_rn(sB[f * N + l0], ref[f]) : 0.0f;
-                    const float b = two ? __fsub_rn(sB[f * N + l0 + 1], ref[f]) : 0.0f;
-                    v[tk][f][0] = a;
-                    v[tk][f][1] = b;
-                    mx[f] = fmaxf(mx[f], fmaxf(fabsf(a), fabsf(b)));
-                }
-            }
+            float v[kNG][2];
 #pragma unroll
             for (int f = 0; f < kNG; ++f) {
-                const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx[f]));
+                v[f][0] = valid ? __fsub_rn(sB[f * N + l0], ref[f]) : 0.0f;
+                v[f][1] = two ? __fsub_rn(sB[f * N + l0 + 1], ref[f]) : 0.0f;
+                const float mx = fmaxf(0.0f, fmaxf(fabsf(v[f][0]), fabsf(v[f][1])));
+                const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
                 if (lane == 0) atomicMax(&sMax[f], mb);
             }
             __syncthreads();
             if (tid < kNG) scale_from_max(sMax[tid], G::BITS, sScale[tid], sInv[tid]);
             __syncthreads();
-#pragma unroll
-            for (int tk = 0; tk < TPT; ++tk) {
-                const int t = tid + tk * kThreads;
-                if (t >= NTASK) break;
-                const int row = t / W, w = t - row * W;
-                const int rk = row / Q, rj = row - rk * Q;
-                const int off = row_pos(rk, rj) * kRowB + 4 * w;
+            if (valid) {
 #pragma unroll
                 for (int f = 0; f < kNG; ++f) {
                     const float s = sScale[f];
                     unsigned hi, lo;
-                    split_scaled<BF16>(__fmul_rn(v[tk][f][0], s), __fmul_rn(v[tk][f][1], s), hi, lo);
-                    *reinterpret_cast<unsigned *>(sHalf + (2 * f) * G::PB + off) = hi;
-                    *reinterpret_cast<unsigned *>(sHalf + (2 * f + 1) * G::PB + off) = lo;
+                    split_scaled<BF16>(__fmul_rn(v[f][0], s), __fmul_rn(v[f][1], s), hi, lo);
+                    *reinterpret_cast<unsigned *>(sHalf + (2 * f) * G::PB + row_off) = hi;
+                    *reinterpret_cast<unsigned *>(sHalf + (2 * f + 1) * G::PB + row_off) = lo;
                 }
             }
         }
@@ -235,129 +212,109 @@ __global__ void __launch_bounds__(kThreads)
         for (int d = 0; d < 3; ++d) {
             const unsigned bh = d == 0 ? Bgh[0] : (d == 1 ? Bgh[1] : Bgh[2]);
             const unsigned bl = d == 0 ? Bgl[0] : (d == 1 ? Bgl[1] : Bgl[2]);
-            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, om) : row_pos(om, r8)) * kRowB;
-            int lat[4];
+            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
+            int lat[2];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) lat[s] = dpass_point<Q>(d, s, g, tq, o1, o2, has1, has2);
+            for (int s = 0; s < 2; ++s) lat[s] = dpass_point<Q>(d, s, g, tq, warp);
 #pragma unroll
-            for (int f = 0; f < kNG; ++f) {
+            for (int f = 0; f < kNG; f += 2) {
+                const unsigned char *src = rowp + 2 * f * G::PB - (f + 1 < kNG ? 0 : alone);
                 unsigned a[4];
                 if (d == 0)
-                    ldsm_x4(a, rowp + 2 * f * G::PB);
+                    ldsm_x4(a, src);
                 else
-                    ldsm_x4_t(a, rowp + 2 * f * G::PB);
+                    ldsm_x4_t(a, src);
                 float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 mma_acc<BF16>(c, a, bh, bh);
                 mma_acc<BF16>(c, a, bl, 0u);
-                const float inv = sInv[f];
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    if (lat[s] >= 0) sG[(d * kNG + f) * N + lat[s]] = c[s] * inv;
+                for (int k = 0; k < 2; ++k) {
+                    if (f + k >= kNG) break;
+                    const float inv = sInv[f + k];
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        if (lat[s] >= 0) sG[(d * kNG + f + k) * N + lat[s]] = c[2 * k + s] * inv;
+                }
             }
         }
         __syncthreads();
 
         // ---- point pass: stress, fluxes, nu_e, kappa_e; flux maxima ----
         {
-            float fl[TPT][2][kNFX];
-            float mx[kNFX];
+            float fl[2][kNFX];
 #pragma unroll
-            for (int x = 0; x < kNFX; ++x) mx[x] = 0.0f;
+            for (int h = 0; h < 2; ++h) {
+                const bool live = h ? two : valid;
+                const int l = live ? l0 + h : 0;
+                float gi[3][kNG];
 #pragma unroll
-            for (int tk = 0; tk < TPT; ++tk) {
-                const int t = tid + tk * kThreads;
-                const int row = t < NTASK ? t / W : 0, w = t < NTASK ? t - row * W : 0;
+                for (int d = 0; d < 3; ++d)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const bool live = t < NTASK && 2 * w + h < Q;
-                    const int l = live ? row * Q + 2 * w + h : 0;
-                    float gi[3][kNG];
+                    for (int f = 0; f < kNG; ++f) gi[d][f] = sG[(d * kNG + f) * N + l];
+                const float r = sB[S_RHO * N + l];
+                const float uu[3] = {sB[S_U0 * N + l], sB[S_U1 * N + l], sB[S_U2 * N + l]};
+                const float muf = sB[S_MUF * N + l], me = sB[S_MUE * N + l], ms = sB[S_MUS * N + l];
+                const float(&Hm)[9] = hv[h];  // Hm[j*3+i] = He(i, j)
+                float gR[3], gT[3], gU[3][3];
 #pragma unroll
-                    for (int d = 0; d < 3; ++d)
+                for (int i = 0; i < 3; ++i) {
+                    gR[i] = Hm[i] * gi[0][0] + Hm[3 + i] * gi[1][0] + Hm[6 + i] * gi[2][0];
+                    gT[i] = Hm[i] * gi[0][1] + Hm[3 + i] * gi[1][1] + Hm[6 + i] * gi[2][1];
 #pragma unroll
-                        for (int f = 0; f < kNG; ++f) gi[d][f] = sG[(d * kNG + f) * N + l];
-                    const float r = sB[S_RHO * N + l];
-                    const float uu[3] = {sB[S_U0 * N + l], sB[S_U1 * N + l], sB[S_U2 * N + l]};
-                    const float muf = sB[S_MUF * N + l], me = sB[S_MUE * N + l], ms = sB[S_MUS * N + l];
-                    const float(&Hm)[9] = hv[tk][h];  // Hm[j*3+i] = He(i, j)
-                    float gR[3], gT[3], gU[3][3];
+                    for (int j = 0; j < 3; ++j)
+                        gU[i][j] = Hm[j] * gi[0][2 + i] + Hm[3 + j] * gi[1][2 + i] + Hm[6 + j] * gi[2][2 + i];
+                }
+                const float mu_fgp = muf + r * ms;
+                const float mu_tot = mu_fgp + me;
+                const float divU = gU[0][0] + gU[1][1] + gU[2][2];
+                float tau[3][3], tauU[3];
 #pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        gR[i] = Hm[i] * gi[0][0] + Hm[3 + i] * gi[1][0] + Hm[6 + i] * gi[2][0];
-                        gT[i] = Hm[i] * gi[0][1] + Hm[3 + i] * gi[1][1] + Hm[6 + i] * gi[2][1];
+                for (int i = 0; i < 3; ++i)
 #pragma unroll
-                        for (int j = 0; j < 3; ++j)
-                            gU[i][j] = Hm[j] * gi[0][2 + i] + Hm[3 + j] * gi[1][2 + i] + Hm[6 + j] * gi[2][2 + i];
+                    for (int j = 0; j < 3; ++j) tau[i][j] = mu_tot * (gU[i][j] + gU[j][i]);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) tau[i][i] -= mu_fgp * twoThirds * divU;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) tauU[i] = tau[i][0] * uu[0] + tau[i][1] * uu[1] + tau[i][2] * uu[2];
+                const float *Xv[kNX] = {gR, tauU, gT, tau[0], tau[1], tau[2]};
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int x = 0; x < kNX; ++x) {
+                        const float val =
+                            live ? gv[h] * (Hm[d * 3] * Xv[x][0] + Hm[d * 3 + 1] * Xv[x][1] +
+                                                Hm[d * 3 + 2] * Xv[x][2])
+                                 : 0.0f;
+                        fl[h][d * kNX + x] = val;
                     }
-                    const float mu_fgp = muf + r * ms;
-                    const float mu_tot = mu_fgp + me;
-                    const float divU = gU[0][0] + gU[1][1] + gU[2][2];
-                    float tau[3][3], tauU[3];
-#pragma unroll
-                    for (int i = 0; i < 3; ++i)
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) tau[i][j] = mu_tot * (gU[i][j] + gU[j][i]);
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) tau[i][i] -= mu_fgp * twoThirds * divU;
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) tauU[i] = tau[i][0] * uu[0] + tau[i][1] * uu[1] + tau[i][2] * uu[2];
-                    const float *Xv[kNX] = {gR, tauU, gT, tau[0], tau[1], tau[2]};
-#pragma unroll
-                    for (int d = 0; d < 3; ++d)
-#pragma unroll
-                        for (int x = 0; x < kNX; ++x) {
-                            const float val =
-                                live ? gv[tk][h] * (Hm[d * 3] * Xv[x][0] + Hm[d * 3 + 1] * Xv[x][1] +
-                                                    Hm[d * 3 + 2] * Xv[x][2])
-                                     : 0.0f;
-                            fl[tk][h][d * kNX + x] = val;
-                        }
-                    if (live) {
-                        sNK[l] = me / r;
-                        sNK[N + l] = muf * Cp / Pr + me * Cp / Pr + Cp * r * ms / 0.9f;
-                    }
+                if (live) {
+                    sNK[l] = me / r;
+                    sNK[N + l] = muf * Cp / Pr + me * Cp / Pr + Cp * r * ms / 0.9f;
                 }
             }
             if (tid == 0)  // task 0, first point: lattice node (0,0,0)
 #pragma unroll
-                for (int x = 0; x < kNFX; ++x) sRef[x] = fl[0][0][x];
+                for (int x = 0; x < kNFX; ++x) sRef[x] = fl[0][x];
             __syncthreads();
 #pragma unroll
-            for (int tk = 0; tk < TPT; ++tk) {
-                const int t = tid + tk * kThreads;
-                const int w = t < NTASK ? t % W : 0;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const bool live = t < NTASK && 2 * w + h < Q;
-#pragma unroll
-                    for (int x = 0; x < kNFX; ++x) {
-                        fl[tk][h][x] = live ? __fsub_rn(fl[tk][h][x], sRef[x]) : 0.0f;
-                        mx[x] = fmaxf(mx[x], fabsf(fl[tk][h][x]));
-                    }
-                }
-            }
-#pragma unroll
             for (int x = 0; x < kNFX; ++x) {
-                const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx[x]));
+                fl[0][x] = valid ? __fsub_rn(fl[0][x], sRef[x]) : 0.0f;
+                fl[1][x] = two ? __fsub_rn(fl[1][x], sRef[x]) : 0.0f;
+                const float mx = fmaxf(0.0f, fmaxf(fabsf(fl[0][x]), fabsf(fl[1][x])));
+                const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
                 if (lane == 0) atomicMax(&sMax[kNG + x], mb);
             }
             __syncthreads();
             if (tid >= kNG && tid < kNG + kNFX) scale_from_max(sMax[tid], G::BITS, sScale[tid], sInv[tid]);
             __syncthreads();
-#pragma unroll
-            for (int tk = 0; tk < TPT; ++tk) {
-                const int t = tid + tk * kThreads;
-                if (t >= NTASK) break;
-                const int row = t / W, w = t - row * W;
-                const int rk = row / Q, rj = row - rk * Q;
-                const int off = row_pos(rk, rj) * kRowB + 4 * w;
+            if (valid) {
 #pragma unroll
                 for (int x = 0; x < kNFX; ++x) {
                     const float s = sScale[kNG + x];
                     unsigned hi, lo;
-                    split_scaled<BF16>(__fmul_rn(fl[tk][0][x], s), __fmul_rn(fl[tk][1][x], s), hi, lo);
-                    *reinterpret_cast<unsigned *>(sHalf + (2 * x) * G::PB + off) = hi;
-                    *reinterpret_cast<unsigned *>(sHalf + (2 * x + 1) * G::PB + off) = lo;
+                    split_scaled<BF16>(__fmul_rn(fl[0][x], s), __fmul_rn(fl[1][x], s), hi, lo);
+                    *reinterpret_cast<unsigned *>(sHalf + (2 * x) * G::PB + row_off) = hi;
+                    *reinterpret_cast<unsigned *>(sHalf + (2 * x + 1) * G::PB + row_off) = lo;
                 }
             }
         }
@@ -369,42 +326,47 @@ __global__ void __launch_bounds__(kThreads)
         for (int d = 0; d < 3; ++d) {
             const unsigned bh = d == 0 ? Bdh[0] : (d == 1 ? Bdh[1] : Bdh[2]);
             const unsigned bl = d == 0 ? Bdl[0] : (d == 1 ? Bdl[1] : Bdl[2]);
-            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, om) : row_pos(om, r8)) * kRowB;
-            int lat[4];
-            float acc[4][kNX];
+            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
+            int lat[2];
+            float acc[2][kNX];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                lat[s] = dpass_point<Q>(d, s, g, tq, o1, o2, has1, has2);
+            for (int s = 0; s < 2; ++s) {
+                lat[s] = dpass_point<Q>(d, s, g, tq, warp);
 #pragma unroll
                 for (int x = 0; x < kNX; ++x) acc[s][x] = (d == 0 || lat[s] < 0) ? 0.0f : sAcc[x * N + lat[s]];
             }
 #pragma unroll
-            for (int x = 0; x < kNX; ++x) {
-                const int fx = d * kNX + x;
+            for (int x = 0; x < kNX; x += 2) {
+                const unsigned char *src = rowp + 2 * (d * kNX + x) * G::PB;
                 unsigned a[4];
                 if (d == 0)
-                    ldsm_x4(a, rowp + 2 * fx * G::PB);
+                    ldsm_x4(a, src);
                 else
-                    ldsm_x4_t(a, rowp + 2 * fx * G::PB);
+                    ldsm_x4_t(a, src);
                 float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 mma_acc<BF16>(c, a, bh, bh);
                 mma_acc<BF16>(c, a, bl, 0u);
-                const float inv = sInv[kNG + fx], ref = sRef[fx];
                 const float cs0 = d == 0 ? colsum[0][0] : (d == 1 ? colsum[1][0] : colsum[2][0]);
                 const float cs1 = d == 0 ? colsum[0][1] : (d == 1 ? colsum[1][1] : colsum[2][1]);
 #pragma unroll
-                for (int s = 0; s < 4; ++s) acc[s][x] = fmaf(c[s], inv, fmaf(ref, (s & 1) ? cs1 : cs0, acc[s][x]));
+                for (int k = 0; k < 2; ++k) {
+                    const int fx = d * kNX + x + k;
+                    const float inv = sInv[kNG + fx], ref = sRef[fx];
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        acc[s][x + k] = fmaf(c[2 * k + s], inv, fmaf(ref, s ? cs1 : cs0, acc[s][x + k]));
+                }
             }
             if (d < 2) {
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
+                for (int s = 0; s < 2; ++s)
                     if (lat[s] >= 0)
 #pragma unroll
                         for (int x = 0; x < kNX; ++x) sAcc[x * N + lat[s]] = acc[s][x];
                 __syncthreads();
             } else {
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
+                for (int s = 0; s < 2; ++s) {
                     if (lat[s] < 0) continue;
                     const int node = sNode[lat[s]];
                     if (node < 0) continue;
@@ -428,9 +390,9 @@ cudaError_t launch_pbn(const MixedDiffuArgs &a, const TableScratch *tabs, cudaSt
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem);
     if (err != cudaSuccess) return err;
     if (a.nelem == 0) return cudaSuccess;
-    const int grid = persistent_grid(kern, kThreads, G::smem, a.nelem);
+    const int grid = persistent_grid(kern, G::NT, G::smem, a.nelem);
     if (grid < 1) return cudaErrorInvalidConfiguration;
-    kern<<<grid, kThreads, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u,
+    kern<<<grid, G::NT, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u,
                                           a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem, a.Rmass, a.Rmom, a.Rener);
     return cudaGetLastError();
 }

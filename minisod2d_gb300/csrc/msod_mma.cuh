@@ -9,21 +9,27 @@
 
 namespace msod {
 
-// L2 prefetch of each element's He and gpvol spans an element ahead in the
-// mixed-precision kernels (1; 0 = none).  Off: measured slower, FP16
-// convection / diffusion 6.16 / 4.36 ms against 4.82 / 4.14 ms on 51^3
-// porder-5 hexes, 2.05 / 2.09 against 2.05 / 2.05 ms on 32^3 porder 7 (the
-// plain kernels gain 1-3 % from the same prefetch).
-#ifndef MIXED_PREFETCH
-#define MIXED_PREFETCH 0
-#endif
+// Registers a thread keeps at least when blocks are added to an SM.  Measured
+// (ms, convection / diffusion FP16, porder 4 48^3): 112 2.830 / 2.483, 96 2.692 /
+// 2.114, 80 2.687 / 2.121; porder 5 40^3 diffusion 1.775, 1.776, 1.926; porder 2
+// 64^3 3.417 / 2.788, 3.180 / 2.434, 3.122 / 2.490; porders 6 and 7 are alike (two
+// blocks by shared memory).
+constexpr int kMixedRegs = 96;
+// Blocks of `threads` threads and `smem` bytes that an SM holds when every
+// thread has `regs` registers at least.
+constexpr int mixed_blocks(size_t smem, int threads, int regs)
+{
+    const int by_smem = (int)((size_t)228 * 1024 / (smem + 1024)), by_regs = 65536 / (threads * regs);
+    const int b = by_smem < by_regs ? by_smem : by_regs;
+    return b < 1 ? 1 : b;
+}
 
 constexpr int kRowB = 16;  // bytes per half-plane row: 8 halves along i
 
 // One field half of an element: 8 rows per k-plane of the element, 8 Q rows.
 // The transposed (zeta) reads of input points beyond Q, which meet zero
-// coefficients, and the discarded tiles of low orders reach up to row 63:
-// past the last plane they land in a zero guard of (64 - 8 Q) rows.
+// coefficients, reach up to row 63: past the last plane they land in a zero
+// guard of (64 - 8 Q) rows.
 // Measured against 8 x 8-row planes for every order (48^3 hexes): porder-5
 // convection 5.24 -> 4.04 ms and porder-4 diffusion 2.78 -> 2.27 ms (more
 // blocks per SM), the other kernels unchanged (0 selects the full planes).
