@@ -26,6 +26,14 @@ __device__ __forceinline__ void red_add(double *addr, double v)
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The statistics' norm, once the kernel that forms it has finished (it may be
+// the kernel ahead that this one overlaps).
+__device__ __forceinline__ float entropy_norm(const float *norm)
+{
+    grid_dependency_wait();
+    return *const_cast<const volatile float *>(norm);
+}
+
 // Read-only global loads through the non-coherent path.
 template <typename T>
 __device__ __forceinline__ T ldg(const T *p)

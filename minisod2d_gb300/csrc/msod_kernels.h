@@ -167,6 +167,8 @@ struct EntropyStats {
     double sum;  // sum of eta over the nodes
     int kmin;    // order-preserving int keys of min / max eta
     int kmax;
+    unsigned done;  // blocks that have added their share
+    float norm;     // || eta - mean(eta) ||_inf (1 if it vanishes)
 };
 
 constexpr int kMlpIn = 12, kMlpH = 32;
@@ -232,15 +234,18 @@ struct FeatureArgs {
     int nelem, npoin;
     const int *connec;
     const float *He, *gpvol;
-    const TableScratch *tabs;
+    const float *dlxigp_ip;
+    const int *invAtoIJK;
     const float *rho, *u, *p_or_T;
     float Rgas, gamma, cmax;
     const EntropyStats *stats;
     float *feat, *numax;
 };
 
+// count, if given, is set to zero ahead of the kernels that follow.  launch_features
+// and launch_entropy_visc without a list come right behind it on the stream.
 cudaError_t launch_entropy_stats(int npoin, const float *rho, const float *p_or_T, float Rgas, float gamma,
-                                 EntropyStats *st, cudaStream_t s);
+                                 EntropyStats *st, int *count, cudaStream_t s);
 cudaError_t launch_entropy_visc(int porder, const ViscArgs &a, cudaStream_t st);
 cudaError_t launch_features(int porder, const FeatureArgs &a, cudaStream_t st);
 // y = 10^-s, nu = y numax (if nu), flag = 1 outside the training range (if

@@ -59,7 +59,7 @@ void *scratch(int slot, size_t bytes)
     }
     return s.p;
 }
-enum { SLOT_STATS = 0, SLOT_TABLES, SLOT_FEAT, SLOT_NUMAX, SLOT_NU, SLOT_LIST, SLOT_COUNT };
+enum { SLOT_STATS = 0, SLOT_FEAT, SLOT_NUMAX, SLOT_NU, SLOT_LIST, SLOT_COUNT };
 
 int geometry_ok(int porder, int nelem, int npoin, const void *connec, const void *He, const void *gpvol,
                 const void *dlx, const void *inv, const void *ai, const void *aj, const void *ak)
@@ -75,28 +75,12 @@ int geometry_ok(int porder, int nelem, int npoin, const void *connec, const void
 }
 
 int run_stats(int npoin, const float *rho, const float *p_or_T, float Rgas, float gamma, EntropyStats **out,
-              cudaStream_t st)
+              int *count, cudaStream_t st)
 {
     auto *s = static_cast<EntropyStats *>(scratch(SLOT_STATS, sizeof(EntropyStats)));
     if (!s) return set_error(MSOD_ERR_CUDA, "could not allocate the entropy statistics");
     *out = s;
-    return cuda_rc(launch_entropy_stats(npoin, rho, p_or_T, Rgas, gamma, s, st), "entropy statistics launch");
-}
-
-// The call's element tables (perm, lat, derivative matrices) in the
-// library-owned table area, prepared on the call's stream.
-int prep_tables(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
-                const float *dlxigp_ip, const int *invAtoIJK, const int *AtoI, const int *AtoJ, const int *AtoK,
-                TableScratch **out, cudaStream_t st)
-{
-    auto *area = static_cast<TableScratch *>(scratch(SLOT_TABLES, sizeof(TableScratch) * (MSOD_MAX_PORDER + 1)));
-    if (!area) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
-    TableScratch *tabs = area + porder;  // one table area per porder
-    *out = tabs;
-    ElementArgs<float> ea{};
-    ea.nelem = nelem; ea.npoin = npoin; ea.connec = connec; ea.He = He; ea.gpvol = gpvol; ea.dlxigp_ip = dlxigp_ip;
-    ea.invAtoIJK = invAtoIJK; ea.AtoI = AtoI; ea.AtoJ = AtoJ; ea.AtoK = AtoK;
-    return cuda_rc(launch_table_prep<float>(porder, ea, tabs, st), "table preparation launch");
+    return cuda_rc(launch_entropy_stats(npoin, rho, p_or_T, Rgas, gamma, s, count, st), "entropy statistics launch");
 }
 
 uint32_t crc32(const unsigned char *p, size_t n)
@@ -142,7 +126,7 @@ int msod_entropy_viscosity(int porder, int nelem, int npoin, const int *connec, 
     if (!(gamma > 1.0f)) return set_error(MSOD_ERR_INVALID_ARG, "gamma must exceed 1");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     EntropyStats *stats = nullptr;
-    rc = run_stats(npoin, rho, pr, 0.0f, gamma, &stats, st);
+    rc = run_stats(npoin, rho, pr, 0.0f, gamma, &stats, nullptr, st);
     if (rc) return rc;
     ViscArgs a{};
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlxigp_ip;
@@ -152,11 +136,11 @@ int msod_entropy_viscosity(int porder, int nelem, int npoin, const int *connec, 
     return cuda_rc(launch_entropy_visc(porder, a, st), "entropy viscosity launch");
 }
 
-// Features (and, with norm, the out-of-range flags of a trained network).
+// Features; count, if given, is set to zero on the way (for the prediction's list).
 static int features_impl(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                          const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
                          const int *gmshAtoK, const float *rho, const float *u, const float *p_or_T, float Rgas,
-                         float gamma, float cmax, float *feat, float *numax_elem, void *stream);
+                         float gamma, float cmax, float *feat, float *numax_elem, int *count, void *stream);
 
 int msod_mlp_features(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                       const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
@@ -165,27 +149,24 @@ int msod_mlp_features(int porder, int nelem, int npoin, const int *connec, const
 {
     clear_error();
     return features_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
-                         rho, u, p_or_T, Rgas, gamma, cmax, feat, numax_elem, stream);
+                         rho, u, p_or_T, Rgas, gamma, cmax, feat, numax_elem, nullptr, stream);
 }
 
 static int features_impl(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                          const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
                          const int *gmshAtoK, const float *rho, const float *u, const float *p_or_T, float Rgas,
-                         float gamma, float cmax, float *feat, float *numax_elem, void *stream)
+                         float gamma, float cmax, float *feat, float *numax_elem, int *count, void *stream)
 {
     int rc = geometry_ok(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK);
     if (rc) return rc;
     if (!rho || !u || !p_or_T || !feat) return set_error(MSOD_ERR_INVALID_ARG, "NULL field or feature array");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     EntropyStats *stats = nullptr;
-    rc = run_stats(npoin, rho, p_or_T, Rgas, gamma, &stats, st);
-    if (rc) return rc;
-    TableScratch *tabs = nullptr;
-    rc = prep_tables(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
-                     &tabs, st);
+    rc = run_stats(npoin, rho, p_or_T, Rgas, gamma, &stats, count, st);
     if (rc) return rc;
     FeatureArgs fa{};
-    fa.nelem = nelem; fa.npoin = npoin; fa.connec = connec; fa.He = He; fa.gpvol = gpvol; fa.tabs = tabs;
+    fa.nelem = nelem; fa.npoin = npoin; fa.connec = connec; fa.He = He; fa.gpvol = gpvol;
+    fa.dlxigp_ip = dlxigp_ip; fa.invAtoIJK = invAtoIJK;
     fa.rho = rho; fa.u = u; fa.p_or_T = p_or_T; fa.Rgas = Rgas; fa.gamma = gamma; fa.cmax = cmax; fa.stats = stats;
     fa.feat = feat; fa.numax = numax_elem;
     return cuda_rc(launch_features(porder, fa, st), "feature launch");
@@ -416,7 +397,7 @@ static int learned_nu(const msod_mlp *m, int porder, int nelem, int npoin, const
     int *count = static_cast<int *>(scratch(SLOT_COUNT, sizeof(int)));
     if (!feat || !numax || !list || !count) return set_error(MSOD_ERR_CUDA, "could not allocate per-element scratch");
     int rc = features_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ,
-                           gmshAtoK, rho, u, p_or_T, Rgas, gamma, cmax, feat, numax, stream);
+                           gmshAtoK, rho, u, p_or_T, Rgas, gamma, cmax, feat, numax, count, stream);
     if (rc) return rc;
     rc = cuda_rc(launch_mlp_predict(nelem, feat, m->wh, m->norm, numax, nullptr, nu, flag, list, count, st),
                  "prediction launch");

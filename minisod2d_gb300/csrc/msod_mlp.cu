@@ -61,6 +61,12 @@ constexpr int feat_warps()
 // five and 0.313 ms at four (the block-size bound, 56-64 registers); porder 5
 // at five (48 registers) 2.69 ms on 96^3 hexes, against 2.87 ms at six and
 // 2.84 ms at four.
+// Bound by the gathers' latency and the L1 pipe (74 % busy at porder 4).  Features on
+// 48^3 porder-4 hexes 146 us with the norm's FP64 division in every warp and the
+// tables prepared by a kernel ahead, 132 us without either.  Measured slower: field
+// loads past L1 (ld.cg, learned viscosity 0.190 against 0.179 ms), and sums and
+// centre quantities through shared memory instead of shuffles (fewer
+// wavefronts, 136 us: the kilobyte is missing in L1).
 #ifndef FEAT_MINB
 #define FEAT_MINB -1
 #endif
@@ -73,10 +79,11 @@ constexpr int feat_minb()
 template <int P>
 __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
     features_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
-                    const float *__restrict__ gpvol, const TableScratch *__restrict__ tabs,
+                    const float *__restrict__ gpvol, const int *__restrict__ invAtoIJK,
+                    const float *__restrict__ dlxigp_ip,
                     const float *__restrict__ rho, const float *__restrict__ u, const float *__restrict__ p_or_T,
-                    float Rgas, float gamma, float cmax, const EntropyStats *__restrict__ st,
-                    float *__restrict__ feat, float *__restrict__ numax_out)
+                    float Rgas, float gamma, float cmax, const EntropyStats *st, float *__restrict__ feat,
+                    float *__restrict__ numax_out)
 {
     constexpr int Q = P + 1, N = Q * Q * Q, kFeatWarps = feat_warps<P>();
     constexpr int NPL = (N + 31) / 32;  // nodes per lane
@@ -84,12 +91,18 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
     // plane 0 first holds the element's node ids by gmsh node.
     __shared__ float sv[kFeatWarps][5][N];
     __shared__ int sPerm[N];         // lattice -> gmsh node
-    __shared__ float sD[3 * Q * Q];  // 1-D derivative matrices
+    __shared__ float sD[3 * Q];      // the centre node's row of the 1-D derivative matrices
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e0 = blockIdx.x * kFeatWarps, e = e0 + w;
-    const TableScratch *t = tabs;
-    for (int i = threadIdx.x; i < N; i += 32 * kFeatWarps) sPerm[i] = t->perm[i];
-    for (int i = threadIdx.x; i < 3 * Q * Q; i += 32 * kFeatWarps) sD[i] = t->Df[i];
+    // Centre node and the natural -> SOD 1-D index map (0 -> 0, P -> 1, k -> k+1).
+    const int mnat = P / 2;
+    const int ms = mnat == 0 ? 0 : (mnat == P ? 1 : mnat + 1);
+    auto gmsh = [&](int l) { return min(max(ldg(invAtoIJK + l) - 1, 0), N - 1); };
+    for (int i = threadIdx.x; i < N; i += 32 * kFeatWarps) sPerm[i] = gmsh(i);
+    for (int i = threadIdx.x; i < 3 * Q; i += 32 * kFeatWarps) {
+        const int d = i / Q, c = i - d * Q;
+        sD[i] = ldg(dlxigp_ip + (size_t)(c * 3 + d) * N + gmsh(d == 0 ? ms : (d == 1 ? ms * Q : ms * Q * Q)));
+    }
     // The block's node ids, element-fastest as connec stores them (the block's
     // elements share each 32-byte sector).
     for (int i = threadIdx.x; i < kFeatWarps * N; i += 32 * kFeatWarps) {
@@ -99,9 +112,6 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
     }
     __syncthreads();
     if (e >= nelem) return;
-    // Entropy normalisation (read early: its latency hides behind the gathers).
-    const double esum = st->sum;
-    const int ekmin = st->kmin, ekmax = st->kmax;
     float rmin = 3e38f, rmax = -3e38f, rsum = 0.f, pmin = 3e38f, pmax = -3e38f, psum = 0.f;
     float smin = 3e38f, smax = -3e38f, emin = 3e38f, emax = -3e38f, machmax = 0.f, usum = 0.f, csum = 0.f;
     float spdmax = 0.f, vol = 0.f;
@@ -173,9 +183,6 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
         vol += __shfl_xor_sync(~0u, vol, o);
     }
     __syncwarp();
-    // Centre node and the natural -> SOD 1-D index map (0 -> 0, P -> 1, k -> k+1).
-    const int mnat = P / 2;
-    const int ms = mnat == 0 ? 0 : (mnat == P ? 1 : mnat + 1);
     auto node = [&](int I, int J, int K) { return (K * Q + J) * Q + I; };  // lattice point (planes of sv)
     const int nat[3] = {0, ms, 1};  // SOD positions of natural 0, mid, P
     // Lanes 0-8: iso derivative gi[i][d] of u_i along d at the centre (lane 3i + d);
@@ -187,7 +194,7 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
         float sacc = 0.f;
         for (int c = 0; c < Q; ++c) {
             const int I = d == 0 ? c : ms, J = d == 1 ? c : ms, K = d == 2 ? c : ms;
-            sacc = fmaf(sD[(d * Q + ms) * Q + c], sv[w][2 + i][node(I, J, K)], sacc);
+            sacc = fmaf(sD[d * Q + c], sv[w][2 + i][node(I, J, K)], sacc);
         }
         gval = sacc;
     } else if (lane < 12) {
@@ -225,10 +232,7 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
     // Every lane holds the element's reductions; lane k < 12 forms feature k
     // (one division and at most one logarithm per lane) and the twelve lanes
     // store the element's features together.
-    const double mean = esum / (double)npoin;
-    const double lo = (double)key2f(ekmin), hi = (double)key2f(ekmax);
-    float neta = (float)fmax(hi - mean, mean - lo);
-    if (!(neta > 0.0f)) neta = 1.0f;
+    const float neta = entropy_norm(&st->norm);
     constexpr float invN = 1.0f / (float)N;
     const float rmean = rsum * invN, pmean = psum * invN, umean = usum * invN, cmean = csum * invN;
     const float h = cbrtf(vol) / (float)P;
@@ -267,10 +271,9 @@ cudaError_t features_p(const FeatureArgs &a, cudaStream_t st)
 {
     constexpr int kFeatWarps = feat_warps<P>();
     const unsigned grid = (unsigned)((a.nelem + kFeatWarps - 1) / kFeatWarps);
-    features_kernel<P><<<grid, 32 * kFeatWarps, 0, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.tabs, a.rho,
-                                                         a.u, a.p_or_T, a.Rgas, a.gamma, a.cmax, a.stats, a.feat,
-                                                         a.numax);
-    return cudaGetLastError();
+    return launch_after(features_kernel<P>, grid, 32 * kFeatWarps, 0, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol,
+                        a.invAtoIJK, a.dlxigp_ip, a.rho, a.u, a.p_or_T, a.Rgas, a.gamma, a.cmax, a.stats, a.feat,
+                        a.numax);
 }
 
 // ---------------------------------------------------------------------------
@@ -311,7 +314,7 @@ __global__ void mlp_predict_kernel(int nelem, const float *__restrict__ feat, co
                                    float *__restrict__ y, float *__restrict__ nu, int *__restrict__ flag,
                                    int *__restrict__ list, int *count)
 {
-    __shared__ float w[kMlpParams];
+    __shared__ __align__(16) float w[kMlpParams];
     __shared__ MlpNorm snm;
     for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) w[i] = __half2float(wh[i]);
     if (threadIdx.x == 0) snm = *nm;
@@ -491,10 +494,6 @@ cudaError_t launch_features(int porder, const FeatureArgs &a, cudaStream_t st)
 cudaError_t launch_mlp_predict(int nelem, const float *feat, const __half *wh, const MlpNorm *nm, const float *numax,
                                float *y, float *nu, int *flag, int *list, int *count, cudaStream_t st)
 {
-    if (list) {
-        const cudaError_t err = cudaMemsetAsync(count, 0, sizeof(int), st);
-        if (err != cudaSuccess) return err;
-    }
     mlp_predict_kernel<<<(nelem + 127) / 128, 128, 0, st>>>(nelem, feat, wh, nm, numax, y, nu, flag, list, count);
     return cudaGetLastError();
 }

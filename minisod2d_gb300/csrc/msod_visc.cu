@@ -30,17 +30,24 @@ namespace {
 // ---------------------------------------------------------------------------
 // Entropy statistics over the nodes: sum, min and max of eta.
 // ---------------------------------------------------------------------------
-__global__ void entropy_stats_init(EntropyStats *st)
+// Three kernels in a row, each started while the one ahead still runs: the
+// statistics load and form eta before they wait for the initial values, the
+// estimator and the features gather before they wait for the norm.
+__global__ void entropy_stats_init(EntropyStats *st, int *count)
 {
+    grid_dependents_launch();
     st->sum = 0.0;
     st->kmin = f2key(3.0e38f);
     st->kmax = f2key(-3.0e38f);
+    st->done = 0u;
+    if (count) *count = 0;
 }
 
 // p is given directly (pr) or as rho * Rgas * T (Tem with Rgas > 0).
 __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, const float *__restrict__ p_or_T,
                                      float Rgas, float gamma, EntropyStats *st)
 {
+    grid_dependents_launch();
     float s = 0.0f, mn = 3.0e38f, mx = -3.0e38f;
     auto add = [&](float r, float q) {
         const float p = Rgas > 0.0f ? r * Rgas * q : q;
@@ -93,9 +100,21 @@ __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, c
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         }
         if (lane == 0) {
+            grid_dependency_wait();  // the initial values
             atomicAdd(&st->sum, sd);
             atomicMin(&st->kmin, f2key(mn));
             atomicMax(&st->kmax, f2key(mx));
+            __threadfence();
+            // The last block forms the norm, once for the mesh: an FP64 division per
+            // element costs the features a third of their time on this GPU.
+            if (atomicAdd(&st->done, 1u) == gridDim.x - 1) {
+                __threadfence();
+                const volatile EntropyStats *v = st;
+                const double mean = v->sum / (double)npoin;
+                const double lo = (double)key2f(v->kmin), hi = (double)key2f(v->kmax);
+                const float norm = (float)fmax(hi - mean, mean - lo);
+                st->norm = norm > 0.0f ? norm : 1.0f;
+            }
         }
     }
 }
@@ -202,7 +221,7 @@ __global__ void __launch_bounds__(G::NT)
                         const float *__restrict__ gpvol, const int *__restrict__ inv,
                         const float *__restrict__ dlxigp_ip, const float *__restrict__ rho,
                         const float *__restrict__ u, const float *__restrict__ p_or_T, float Rgas, float gamma,
-                        float ce, float cmax, int normalise, const EntropyStats *__restrict__ st,
+                        float ce, float cmax, int normalise, const EntropyStats *st,
                         const int *__restrict__ list, const int *__restrict__ count, float *__restrict__ mu_e,
                         float *__restrict__ nu_out, float *__restrict__ numax_out)
 {
@@ -321,13 +340,7 @@ __global__ void __launch_bounds__(G::NT)
         __syncthreads();
         if (tid < NE) {
             const int ee = element(tid);
-            float neta = 1.0f;
-            if (normalise) {
-                const double mean = st->sum / (double)npoin;
-                const double lo = (double)key2f(st->kmin), hi = (double)key2f(st->kmax);
-                neta = (float)fmax(hi - mean, mean - lo);
-                if (!(neta > 0.0f)) neta = 1.0f;
-            }
+            const float neta = normalise ? entropy_norm(&st->norm) : 1.0f;
             float v = 0.0f;
             for (int l = 0; l < G::L; ++l) v += sm.vol()[l * NE + tid];
             const float h = cbrtf(v) / (float)(Q - 1);
@@ -366,6 +379,10 @@ cudaError_t visc_pl(const ViscArgs &a, cudaStream_t st)
     const int ngroups = (a.nelem + G::NE - 1) / G::NE;
     const unsigned grid = (unsigned)(LIST ? persistent_grid(kern, G::NT, smem, ngroups) : ngroups);
     if (grid == 0) return cudaErrorInvalidConfiguration;
+    if constexpr (!LIST)
+        return launch_after(kern, grid, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK,
+                            a.dlxigp_ip, a.rho, a.u, a.p_or_T, a.Rgas, a.gamma, a.ce, a.cmax, a.normalise, a.stats,
+                            a.list, a.count, a.mu_e, a.nu, a.numax);
     kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK, a.dlxigp_ip, a.rho, a.u,
                                     a.p_or_T, a.Rgas, a.gamma, a.ce, a.cmax, a.normalise, a.stats, a.list, a.count,
                                     a.mu_e, a.nu, a.numax);
@@ -380,17 +397,16 @@ cudaError_t visc_p(const ViscArgs &a, cudaStream_t st)
 }  // namespace
 
 cudaError_t launch_entropy_stats(int npoin, const float *rho, const float *p_or_T, float Rgas, float gamma,
-                                 EntropyStats *st, cudaStream_t s)
+                                 EntropyStats *st, int *count, cudaStream_t s)
 {
-    entropy_stats_init<<<1, 1, 0, s>>>(st);
+    entropy_stats_init<<<1, 1, 0, s>>>(st, count);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     int dev = 0, sms = 152;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int blocks = (npoin + 255) / 256;
     if (blocks > 8 * sms) blocks = 8 * sms;
-    entropy_stats_kernel<<<blocks, 256, 0, s>>>(npoin, rho, p_or_T, Rgas, gamma, st);
-    return cudaGetLastError();
+    return launch_after(entropy_stats_kernel, (unsigned)blocks, 256, 0, s, npoin, rho, p_or_T, Rgas, gamma, st);
 }
 
 cudaError_t launch_entropy_visc(int porder, const ViscArgs &a, cudaStream_t st)
