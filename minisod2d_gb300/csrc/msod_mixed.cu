@@ -43,9 +43,13 @@
 // a time.  The kernel waits on its phases' loads, so residency pays: two fields
 // of one tile per contraction instead of one field of two tiles halves a
 // thread's state (two points instead of four) and leaves no warp without a tile.
-// FP16, two tiles per warp in blocks of four warps / now: porder 7 24^3 0.907 /
-// 0.815 ms, 6 32^3 1.842 / 1.424, 5 40^3 2.354 / 2.052, 4 48^3 4.918 / 2.692, 3
-// 48^3 2.647 / 1.867, 2 64^3 5.990 / 3.180, 1 64^3 5.532 / 2.139.
+// A thread gathers the two points that it splits, with the node ids loaded an
+// element ahead, and the positions in shared memory (node_at) keep the passes'
+// nodal reads off each other's banks (a third of the L1 pipe's cycles before).
+// FP16, two tiles per warp in blocks of four warps / one tile per warp / now:
+// porder 7 24^3 0.907 / 0.815 / 0.677 ms, 6 32^3 1.842 / 1.424 / 1.343, 5 40^3
+// 2.354 / 2.052 / 1.925, 4 48^3 4.918 / 2.692 / 2.644, 3 48^3 2.647 / 1.867 / 1.821,
+// 2 64^3 5.990 / 3.180 / 3.347, 1 64^3 5.532 / 2.139 / 2.156.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -58,7 +62,7 @@ namespace msod {
 namespace {
 
 constexpr int kNF = 31;       // differentiated products
-enum { B_RHO = 0, B_P, B_E, B_U0, B_U1, B_U2, B_Q0, B_Q1, B_Q2, NBASE };
+enum { B_RHO = 0, B_H, B_U0, B_U1, B_U2, B_Q0, B_Q1, B_Q2, NBASE };
 enum { A_M = 0, A_MOM0, A_MOM1, A_MOM2, A_E, A_DIVU, A_DIVQ, NACC };
 
 // Field numbering: 0 rho, 1 p, 2-4 u_i, 5-7 q_i, 8-16 q_i u_j (i major),
@@ -68,19 +72,17 @@ struct Nodal {
     float r, p, u[3], q[3], H, rH;
 };
 
-__device__ __forceinline__ Nodal nodal_from(const float *sBase, int N, int l)
+// The point's nodal values as the passes use them (all but p).
+__device__ __forceinline__ Nodal nodal_from(const float *sBase, int np, int l)
 {
     Nodal n;
-    n.r = sBase[B_RHO * N + l];
-    n.p = sBase[B_P * N + l];
-    const float E = sBase[B_E * N + l];
+    n.r = sBase[B_RHO * np + l];
+    n.H = sBase[B_H * np + l];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        n.u[c] = sBase[(B_U0 + c) * N + l];
-        n.q[c] = sBase[(B_Q0 + c) * N + l];
+        n.u[c] = sBase[(B_U0 + c) * np + l];
+        n.q[c] = sBase[(B_Q0 + c) * np + l];
     }
-    const float k2 = __fmaf_rn(n.u[0], n.u[0], __fmaf_rn(n.u[1], n.u[1], __fmul_rn(n.u[2], n.u[2])));
-    n.H = __fmaf_rn(0.5f, k2, E);
     n.rH = __fmul_rn(n.r, n.H);
     return n;
 }
@@ -100,18 +102,6 @@ __device__ __forceinline__ float field(int f, const Nodal &n)
     if (f == 24) return n.rH;
     if (f < 28) return __fmul_rn(n.rH, n.u[f - 25]);
     return __fmul_rn(n.H, n.u[f - 28]);
-}
-
-// Lattice point of slot s (output point 2t + s along direction d of line g of
-// tile o); -1 when padded.
-template <int Q>
-__device__ __forceinline__ int pass_point(int d, int s, int g, int tq, int o)
-{
-    const int pt = 2 * tq + s;
-    const int I = d == 0 ? pt : g;
-    const int J = d == 0 ? g : (d == 1 ? pt : o);
-    const int K = d == 2 ? pt : o;
-    return g < Q && pt < Q ? (K * Q + J) * Q + I : -1;
 }
 
 // Per-point coefficients of one direction pass.
@@ -160,15 +150,15 @@ __device__ __forceinline__ void apply_field(int f, float dv, const PointCoef &c,
 
 template <int P, bool BF16>
 struct MixedGeom {
-    static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2;
+    static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2, NP = node_plane<Q>();
     static constexpr int NT = 32 * Q;        // one warp per tile (k-plane or j-plane) of lines
     static constexpr int NTASK = Q * Q * W;  // task: points (2w, 2w+1) of one i-row
     static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
     static constexpr size_t half_bytes = (size_t)2 * kNF * PB + plane_guard_bytes<Q>();
-    static constexpr size_t smem = half_bytes + (size_t)(NBASE + NACC) * N * sizeof(float) +
-                                   (size_t)2 * N * sizeof(int) + 2 * 32 * sizeof(float);
+    static constexpr size_t smem = half_bytes + (size_t)(NBASE + NACC) * NP * sizeof(float) +
+                                   (size_t)2 * NP * sizeof(int) + (2 * 32 + 4) * sizeof(float);
     // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
     static constexpr int MINB = mixed_blocks(smem, NT, kMixedRegs);
 };
@@ -182,21 +172,22 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
                         double *__restrict__ Rmom, double *__restrict__ Rener)
 {
     using G = MixedGeom<P, BF16>;
-    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT;
+    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT, NP = G::NP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *sHalf = smem_raw;                                  // [2*kNF][G::PB]: hi, lo of each field
-    float *sBase = reinterpret_cast<float *>(sHalf + G::half_bytes);  // [NBASE][N], lattice (K*Q+J)*Q+I
-    float *sAcc = sBase + NBASE * N;                                   // [NACC][N]
-    int *sNode = reinterpret_cast<int *>(sAcc + NACC * N);             // [N]
-    int *sPerm = sNode + N;                                            // lattice -> gmsh node
-    float *sScale = reinterpret_cast<float *>(sPerm + N);             // [32] s_f
+    float *sBase = reinterpret_cast<float *>(sHalf + G::half_bytes);  // [NBASE][NP], positions node_at
+    float *sAcc = sBase + NBASE * NP;                                  // [NACC][NP]
+    int *sNode = reinterpret_cast<int *>(sAcc + NACC * NP);            // [NP]
+    int *sPerm = sNode + NP;                                           // gmsh node
+    float *sScale = reinterpret_cast<float *>(sPerm + NP);            // [32] s_f
     float *sInv = sScale + 32;                                         // [32] 1 / s_f (max bits first)
+    float *sRefP = sInv + 32;                                          // p at lattice node (0,0,0)
     unsigned *sMax = reinterpret_cast<unsigned *>(sInv);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Once per block: tables, the zero padding of the half planes (rows and
     // points beyond Q are never written), the B fragments.
-    for (int i = tid; i < N; i += NT) sPerm[i] = tabs->perm[i];
+    for (int i = tid; i < N; i += NT) sPerm[node_at<Q>(i / (Q * Q), i / Q % Q, i % Q)] = tabs->perm[i];
     if (Q < 8) {
         uint4 *z = reinterpret_cast<uint4 *>(sHalf);
         for (int i = tid; i < (int)(G::half_bytes / 16); i += NT) z[i] = make_uint4(0, 0, 0, 0);
@@ -211,28 +202,58 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
         split_pair<BF16>(d0, d1, Bh[d], Bl[d]);
     }
     const size_t np = (size_t)npoin;
+    // The thread's task: points (2w, 2w+1) of i-row (rk, rj), which it gathers and
+    // splits.  The node ids are loaded an element ahead.
+    const bool valid = tid < NTASK;
+    const int row = valid ? tid / W : 0, w = valid ? tid - row * W : 0;
+    const bool two = valid && 2 * w + 1 < Q;
+    const int rk = row / Q, rj = row - rk * Q;
+    const int l0 = node_at<Q>(rk, rj, 2 * w), l1 = l0 + 1;
+    const int off = row_pos(rk, rj) * kRowB + 4 * w;
+    const int *con0 = connec + (size_t)tabs->perm[row * Q + 2 * w] * nelem;
+    const int *con1 = connec + (size_t)tabs->perm[row * Q + 2 * w + (two ? 1 : 0)] * nelem;
+    int id0 = ldg_once(con0 + blockIdx.x), id1 = ldg_once(con1 + blockIdx.x);  // the grid has nelem blocks at most
 #pragma unroll 1
     for (int e = blockIdx.x; e < nelem; e += gridDim.x) {
-    __syncthreads();  // the previous element's passes are done with every shared array
-    if (tid < 32) sMax[tid] = 0u;
-    for (int l = tid; l < N; l += NT) {
-        const int a = sPerm[l];
-        const int v = ldg(connec + (size_t)a * nelem + e) - 1;
-        const bool ok = (unsigned)v < (unsigned)npoin;
-        const int p = ok ? v : 0;
-        sNode[l] = ok ? v : -1;
-        // asynchronous copies (a missing node reads as zeros)
-        cp_async_elem(sBase + B_RHO * N + l, rho + p, ok);
-        cp_async_elem(sBase + B_P * N + l, pr + p, ok);
-        cp_async_elem(sBase + B_E * N + l, E + p, ok);
+    Nodal n0, n1;
+    {
+        auto gather = [&](int v, Nodal &n, bool own) {
+            const bool ok = own && (unsigned)v < (unsigned)npoin;  // a missing node reads as zeros
+            const size_t p = ok ? v : 0;
+            n.r = ok ? ldg_once(rho + p) : 0.0f;
+            n.p = ok ? ldg_once(pr + p) : 0.0f;
+            n.H = ok ? ldg_once(E + p) : 0.0f;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            cp_async_elem(sBase + (B_U0 + c) * N + l, u + c * np + p, ok);
-            cp_async_elem(sBase + (B_Q0 + c) * N + l, q + c * np + p, ok);
-        }
+            for (int c = 0; c < 3; ++c) {
+                n.u[c] = ok ? ldg_once(u + c * np + p) : 0.0f;
+                n.q[c] = ok ? ldg_once(q + c * np + p) : 0.0f;
+            }
+            return ok ? v : -1;
+        };
+        auto store = [&](int pos, int node, Nodal &n, bool own) {
+            const float k2 = __fmaf_rn(n.u[0], n.u[0], __fmaf_rn(n.u[1], n.u[1], __fmul_rn(n.u[2], n.u[2])));
+            n.H = __fmaf_rn(0.5f, k2, n.H);
+            n.rH = __fmul_rn(n.r, n.H);
+            if (!own) return;
+            sNode[pos] = node;
+            sBase[B_RHO * NP + pos] = n.r;
+            sBase[B_H * NP + pos] = n.H;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sBase[(B_U0 + c) * NP + pos] = n.u[c];
+                sBase[(B_Q0 + c) * NP + pos] = n.q[c];
+            }
+        };
+        const int v0 = gather(id0 - 1, n0, valid), v1 = gather(id1 - 1, n1, two);
+        const int en = e + (int)gridDim.x < nelem ? e + (int)gridDim.x : e;
+        id0 = ldg_once(con0 + en);
+        id1 = ldg_once(con1 + en);
+        __syncthreads();  // the previous element's passes are done with every shared array
+        if (tid < 32) sMax[tid] = 0u;
+        store(l0, v0, n0, valid);
+        store(l1, v1, n1, two);
+        if (tid == 0) *sRefP = n0.p;
     }
-    cp_async_commit();
-    cp_async_wait_all();
     __syncthreads();
 
     // He columns of the first direction pass, in flight during the split.
@@ -249,15 +270,10 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
     // Shifted products of the thread's task (two points) in registers, their
     // per-field maxima over the element (non-negative floats order like their
     // bit patterns), then the split into the half planes.
-    const bool valid = tid < NTASK;
-    const int row = valid ? tid / W : 0, w = valid ? tid - row * W : 0;
-    const bool two = valid && 2 * w + 1 < Q;
     float v[kNF][2];
     {
-        const Nodal nref = nodal_from(sBase, N, 0);
-        const int l0 = row * Q + 2 * w;
-        const Nodal n0 = nodal_from(sBase, N, l0);
-        const Nodal n1 = nodal_from(sBase, N, two ? l0 + 1 : l0);
+        Nodal nref = nodal_from(sBase, NP, 0);
+        nref.p = *sRefP;
 #pragma unroll
         for (int f = 0; f < kNF; ++f) {
             const float fr = field(f, nref);
@@ -278,11 +294,11 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
     }
     __syncthreads();
     if (valid) {
-        const int rk = row / Q, rj = row - rk * Q;
-        const int off = row_pos(rk, rj) * kRowB + 4 * w;
+        float4 sc;
 #pragma unroll
         for (int f = 0; f < kNF; ++f) {
-            const float s = sScale[f];
+            if (f % 4 == 0) sc = *reinterpret_cast<const float4 *>(sScale + f);
+            const float s = f % 4 == 0 ? sc.x : (f % 4 == 1 ? sc.y : (f % 4 == 2 ? sc.z : sc.w));
             unsigned hi, lo;
             split_scaled<BF16>(__fmul_rn(v[f][0], s), __fmul_rn(v[f][1], s), hi, lo);
             *reinterpret_cast<unsigned *>(sHalf + (2 * f) * G::PB + off) = hi;
@@ -312,7 +328,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
             live[s] = lp >= 0;
             const int l = live[s] ? lp : 0;
             lat[s] = l;
-            const Nodal n = nodal_from(sBase, N, l);
+            const Nodal n = nodal_from(sBase, NP, l);
             cf[s].rho = n.r;
             cf[s].H = n.H;
 #pragma unroll
@@ -323,7 +339,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
             cf[s].cu = n.u[0] * cf[s].h[0] + n.u[1] * cf[s].h[1] + n.u[2] * cf[s].h[2];
             cf[s].cq = n.q[0] * cf[s].h[0] + n.q[1] * cf[s].h[1] + n.q[2] * cf[s].h[2];
 #pragma unroll
-            for (int k = 0; k < NACC; ++k) acc[s][k] = (d == 0 || !live[s]) ? 0.0f : sAcc[k * N + l];
+            for (int k = 0; k < NACC; ++k) acc[s][k] = (d == 0 || !live[s]) ? 0.0f : sAcc[k * NP + l];
         }
         // Loads in flight during the contractions: the next pass's He columns,
         // or gpvol for the last pass's scatter.
@@ -352,10 +368,11 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
             float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             mma_acc<BF16>(c, a, bh, bh);
             mma_acc<BF16>(c, a, bl, 0u);
+            const float2 inv2 = *reinterpret_cast<const float2 *>(sInv + f);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 if (f + k >= kNF) break;
-                const float inv = sInv[f + k];
+                const float inv = k ? inv2.y : inv2.x;
 #pragma unroll
                 for (int s = 0; s < 2; ++s) apply_field(f + k, c[2 * k + s] * inv, cf[s], acc[s]);
             }
@@ -365,7 +382,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
             for (int s = 0; s < 2; ++s)
                 if (live[s])
 #pragma unroll
-                    for (int k = 0; k < NACC; ++k) sAcc[k * N + lat[s]] = acc[s][k];
+                    for (int k = 0; k < NACC; ++k) sAcc[k * NP + lat[s]] = acc[s][k];
             __syncthreads();
         } else {
 #pragma unroll
@@ -373,7 +390,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
                 if (!live[s]) continue;
                 const int node = sNode[lat[s]];
                 if (node < 0) continue;
-                const Nodal n = nodal_from(sBase, N, lat[s]);
+                const Nodal n = nodal_from(sBase, NP, lat[s]);
                 const float divU = acc[s][A_DIVU], divQ = acc[s][A_DIVQ];
                 const float rm = acc[s][A_M] + 0.5f * (divQ + n.r * divU);
                 red_add(Rmass + node, f2d(gp[s] * rm));

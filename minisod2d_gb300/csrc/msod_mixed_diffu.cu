@@ -6,7 +6,7 @@
 // energy-flux assembly and the nodal scatter-add in FP64 (FP64 outputs).
 //
 // Per element (one block of one warp per tile, persistent over elements):
-//   1. gather rho, T, u, mu_fluid, mu_e, mu_sgs into a lattice in shared memory;
+//   1. gather rho, T, u, mu_fluid, mu_e, mu_sgs, He, gpvol of the thread's two points;
 //   2. gradient stage: rho, T, u_1..3 are shifted by their value at lattice
 //      node (0,0,0) (the derivative annihilates constants), scaled by a power
 //      of two per element and field, split into hi + lo half planes; per
@@ -27,10 +27,12 @@
 //   5. Rmass += nu_e sum(grad rho), Rmom_m += sum(tau_m), and in FP64
 //      Rener += sum(tau.u) + kappa_e sum(grad T); red.global.add.f64.
 // Shared-memory half planes use the swizzled layout of msod_mma.cuh.
-// porder 1..7.  One tile per warp, as in msod_mixed.cu: two tiles per warp in
-// blocks of four warps / now, FP16: porder 7 24^3 0.851 / 0.706 ms, 6 32^3 1.555 /
-// 1.444, 5 40^3 1.996 / 1.776, 4 48^3 2.164 / 2.114, 3 48^3 1.620 / 1.530, 2 64^3
-// 3.508 / 2.434, 1 64^3 3.377 / 1.718.
+// porder 1..7.  One tile per warp, as in msod_mixed.cu; a thread's two points stay in
+// its registers from the gather to the point pass.  Two tiles per warp in blocks of
+// four warps / one tile per warp / now, FP16: porder 7 24^3 0.851 / 0.706 / 0.635 ms,
+// 6 32^3 1.555 / 1.444 / 1.311, 5 40^3 1.996 / 1.776 / 1.742, 4 48^3 2.164 / 2.114 /
+// 2.182, 3 48^3 1.620 / 1.530 / 1.533, 2 64^3 3.508 / 2.434 / 2.736, 1 64^3 3.377 /
+// 1.718 / 1.741.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -46,34 +48,23 @@ constexpr int kNG = 5;   // differentiated node fields: rho, T, u_1..3
 constexpr int kNX = 6;   // flux vectors: grad rho, tau.u, grad T, tau rows 1..3
 constexpr int kNFX = 3 * kNX;
 
-enum { S_RHO = 0, S_T, S_U0, S_U1, S_U2, S_MUF, S_MUE, S_MUS, NSB };  // gathered planes
+constexpr int kFx0 = 8;  // scale of the first flux, behind the node fields'
 enum { X_GRHO = 0, X_TAUU, X_GT, X_TAU0, X_TAU1, X_TAU2 };
 
 template <int P, bool BF16>
 struct MixedDiffuGeom {
-    static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2;
+    static constexpr int Q = P + 1, N = Q * Q * Q, W = (Q + 1) / 2, NP = node_plane<Q>();
     static constexpr int NT = 32 * Q;        // one warp per tile (k-plane or j-plane) of lines
     static constexpr int NTASK = Q * Q * W;  // task: points (2w, 2w+1) of one i-row
     static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
     static constexpr size_t half_bytes = (size_t)2 * kNFX * PB + plane_guard_bytes<Q>();
-    static constexpr size_t smem = half_bytes + (size_t)(NSB + 3 * kNG + 2) * N * sizeof(float) +
-                                   (size_t)2 * N * sizeof(int) + 3 * 32 * sizeof(float);
+    static constexpr size_t smem = half_bytes + (size_t)(3 * kNG + 2) * NP * sizeof(float) +
+                                   (size_t)2 * NP * sizeof(int) + (3 * 32 + 8) * sizeof(float);
     // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
     static constexpr int MINB = mixed_blocks(smem, NT, kMixedRegs);
 };
-
-// Lattice point of slot s of a pass (see msod_mixed.cu); -1 when padded.
-template <int Q>
-__device__ __forceinline__ int dpass_point(int d, int s, int g, int tq, int o)
-{
-    const int pt = 2 * tq + s;
-    const int I = d == 0 ? pt : g;
-    const int J = d == 0 ? g : (d == 1 ? pt : o);
-    const int K = d == 2 ? pt : o;
-    return g < Q && pt < Q ? (K * Q + J) * Q + I : -1;
-}
 
 template <int P, bool BF16, bool NUE>
 __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
@@ -85,22 +76,22 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                        double *__restrict__ Rmass, double *__restrict__ Rmom, double *__restrict__ Rener)
 {
     using G = MixedDiffuGeom<P, BF16>;
-    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT;
+    constexpr int Q = G::Q, N = G::N, W = G::W, NTASK = G::NTASK, NT = G::NT, NP = G::NP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char *sHalf = smem_raw;                                  // [2*kNFX][G::PB]
-    float *sB = reinterpret_cast<float *>(sHalf + G::half_bytes);     // [NSB][N] lattice (K*Q+J)*Q+I
-    float *sG = sB + NSB * N;                                          // [15][N] iso-derivatives; then [6][N] sums
-    float *sNK = sG + 3 * kNG * N;                                     // [2][N] nu_e, kappa_e
-    int *sNode = reinterpret_cast<int *>(sNK + 2 * N);                 // [N]
-    int *sPerm = sNode + N;                                            // lattice -> gmsh node
-    float *sScale = reinterpret_cast<float *>(sPerm + N);             // [32]: 0..4 gradient fields, 5..22 fluxes
+    float *sG = reinterpret_cast<float *>(sHalf + G::half_bytes);     // [15][NP] iso-derivatives; then [6][NP] sums
+    float *sNK = sG + 3 * kNG * NP;                                    // [2][NP] nu_e, kappa_e
+    int *sNode = reinterpret_cast<int *>(sNK + 2 * NP);                // [NP], positions node_at
+    int *sPerm = sNode + NP;                                           // gmsh node
+    float *sScale = reinterpret_cast<float *>(sPerm + NP);            // [32]: 0..4 node fields, kFx0.. fluxes
     float *sInv = sScale + 32;
     unsigned *sMax = reinterpret_cast<unsigned *>(sInv);
     float *sRef = sInv + 32;  // [kNFX] flux values at lattice node (0,0,0)
+    float *sRefG = sRef + 32;  // [kNG] node fields there
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    for (int i = tid; i < N; i += NT) sPerm[i] = tabs->perm[i];
+    for (int i = tid; i < N; i += NT) sPerm[node_at<Q>(i / (Q * Q), i / Q % Q, i % Q)] = tabs->perm[i];
     if (Q < 8) {  // rows and points beyond Q are never written and stay zero
         uint4 *z = reinterpret_cast<uint4 *>(sHalf);
         for (int i = tid; i < (int)(G::half_bytes / 16); i += NT) z[i] = make_uint4(0, 0, 0, 0);
@@ -137,58 +128,60 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
     const bool valid = tid < NTASK;
     const int row = valid ? tid / W : 0, w = valid ? tid - row * W : 0;
     const int row_off = row_pos(row / Q, row % Q) * kRowB + 4 * w;
-    const int l0 = row * Q + 2 * w;
     const bool two = valid && 2 * w + 1 < Q;
+    const int l0 = node_at<Q>(row / Q, row % Q, 2 * w);
+    const int a0 = tabs->perm[row * Q + 2 * w], a1 = tabs->perm[row * Q + 2 * w + (two ? 1 : 0)];
+    // Node ids, loaded an element ahead (the grid has nelem blocks at most).
+    int id[2] = {ldg_once(connec + (size_t)a0 * nelem + blockIdx.x), ldg_once(connec + (size_t)a1 * nelem + blockIdx.x)};
     const size_t np = (size_t)npoin;
     const float twoThirds = 2.0f / 3.0f;
 
 #pragma unroll 1
     for (int e = blockIdx.x; e < nelem; e += gridDim.x) {
-        __syncthreads();  // the previous element is done with every shared array
-        if (tid < 32) sMax[tid] = 0u;
         const float nue = NUE ? ldg(nu_elem + e) : 0.0f;
-        for (int l = tid; l < N; l += NT) {
-            const int a = sPerm[l];
-            const int v = ldg(connec + (size_t)a * nelem + e) - 1;
-            const bool ok = (unsigned)v < (unsigned)npoin;
-            const int p = ok ? v : 0;
-            sNode[l] = ok ? v : -1;
-            const float r = ok ? ldg(rho + p) : 1.0f;  // 1 at a missing node keeps nu_e = mu_e / rho finite
-            sB[S_RHO * N + l] = r;
-            // the other fields by asynchronous copies (a missing node reads as zeros)
-            cp_async_elem(sB + S_T * N + l, Tem + p, ok);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) cp_async_elem(sB + (S_U0 + c) * N + l, u + c * np + p, ok);
-            cp_async_elem(sB + S_MUF * N + l, mu_fluid + p, ok);
-            if (NUE)
-                sB[S_MUE * N + l] = r * nue;
-            else
-                cp_async_elem(sB + S_MUE * N + l, mu_e + (size_t)a * nelem + e, true);
-            cp_async_elem(sB + S_MUS * N + l, mu_sgs + (size_t)a * nelem + e, true);
-        }
-        cp_async_commit();
-        // He and gpvol of the point-pass points, in flight during the gradient stage.
-        float hv[2][9], gv[2];
+        // The thread's two points: node fields, viscosities, He and gpvol, kept in registers.
+        float fld[2][kNG], muf[2], mue[2], mus[2], hv[2][9], gv[2];
+        int node[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const size_t base = (size_t)e * N + sPerm[(h ? two : valid) ? l0 + h : 0];
+            const int a = h ? a1 : a0, v = id[h] - 1;
+            const bool ok = (h ? two : valid) && (unsigned)v < (unsigned)npoin;
+            const size_t p = ok ? v : 0;
+            node[h] = ok ? v : -1;
+            fld[h][0] = ok ? ldg_once(rho + p) : 1.0f;  // 1 at a missing node keeps nu_e = mu_e / rho finite
+            fld[h][1] = ok ? ldg_once(Tem + p) : 0.0f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) fld[h][2 + c] = ok ? ldg_once(u + c * np + p) : 0.0f;
+            muf[h] = ok ? ldg_once(mu_fluid + p) : 0.0f;
+            mue[h] = NUE ? nue : ldg(mu_e + (size_t)a * nelem + e);
+            mus[h] = ldg(mu_sgs + (size_t)a * nelem + e);
+            const size_t base = (size_t)e * N + a;
 #pragma unroll
             for (int j = 0; j < 9; ++j) hv[h][j] = ldg(He + base * 9 + j);
             gv[h] = ldg(gpvol + base);
         }
-        cp_async_wait_all();
+        {
+            const int en = e + (int)gridDim.x < nelem ? e + (int)gridDim.x : e;
+            id[0] = ldg_once(connec + (size_t)a0 * nelem + en);
+            id[1] = ldg_once(connec + (size_t)a1 * nelem + en);
+        }
+        __syncthreads();  // the previous element is done with every shared array
+        if (tid < 32) sMax[tid] = 0u;
+        if (valid) sNode[l0] = node[0];
+        if (two) sNode[l0 + 1] = node[1];
+        if (tid == 0)  // task 0, first point: lattice node (0,0,0)
+#pragma unroll
+            for (int f = 0; f < kNG; ++f) sRefG[f] = fld[0][f];
         __syncthreads();
 
         // ---- gradient stage: split rho, T, u_1..3 (shifted by node (0,0,0)) ----
         {
-            float ref[kNG];
-#pragma unroll
-            for (int f = 0; f < kNG; ++f) ref[f] = sB[f * N];  // planes S_RHO..S_U2 are fields 0..4
             float v[kNG][2];
 #pragma unroll
             for (int f = 0; f < kNG; ++f) {
-                v[f][0] = valid ? __fsub_rn(sB[f * N + l0], ref[f]) : 0.0f;
-                v[f][1] = two ? __fsub_rn(sB[f * N + l0 + 1], ref[f]) : 0.0f;
+                const float ref = sRefG[f];
+                v[f][0] = valid ? __fsub_rn(fld[0][f], ref) : 0.0f;
+                v[f][1] = two ? __fsub_rn(fld[1][f], ref) : 0.0f;
                 const float mx = fmaxf(0.0f, fmaxf(fabsf(v[f][0]), fabsf(v[f][1])));
                 const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
                 if (lane == 0) atomicMax(&sMax[f], mb);
@@ -215,7 +208,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
             const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
             int lat[2];
 #pragma unroll
-            for (int s = 0; s < 2; ++s) lat[s] = dpass_point<Q>(d, s, g, tq, warp);
+            for (int s = 0; s < 2; ++s) lat[s] = pass_point<Q>(d, s, g, tq, warp);
 #pragma unroll
             for (int f = 0; f < kNG; f += 2) {
                 const unsigned char *src = rowp + 2 * f * G::PB - (f + 1 < kNG ? 0 : alone);
@@ -233,7 +226,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                     const float inv = sInv[f + k];
 #pragma unroll
                     for (int s = 0; s < 2; ++s)
-                        if (lat[s] >= 0) sG[(d * kNG + f + k) * N + lat[s]] = c[2 * k + s] * inv;
+                        if (lat[s] >= 0) sG[(d * kNG + f + k) * NP + lat[s]] = c[2 * k + s] * inv;
                 }
             }
         }
@@ -250,10 +243,9 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
 #pragma unroll
-                    for (int f = 0; f < kNG; ++f) gi[d][f] = sG[(d * kNG + f) * N + l];
-                const float r = sB[S_RHO * N + l];
-                const float uu[3] = {sB[S_U0 * N + l], sB[S_U1 * N + l], sB[S_U2 * N + l]};
-                const float muf = sB[S_MUF * N + l], me = sB[S_MUE * N + l], ms = sB[S_MUS * N + l];
+                    for (int f = 0; f < kNG; ++f) gi[d][f] = sG[(d * kNG + f) * NP + l];
+                const float r = fld[h][0], me = NUE ? r * mue[h] : mue[h], ms = mus[h];
+                const float(&uu)[5] = fld[h];  // u at 2..4
                 const float(&Hm)[9] = hv[h];  // Hm[j*3+i] = He(i, j)
                 float gR[3], gT[3], gU[3][3];
 #pragma unroll
@@ -264,7 +256,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                     for (int j = 0; j < 3; ++j)
                         gU[i][j] = Hm[j] * gi[0][2 + i] + Hm[3 + j] * gi[1][2 + i] + Hm[6 + j] * gi[2][2 + i];
                 }
-                const float mu_fgp = muf + r * ms;
+                const float mu_fgp = muf[h] + r * ms;
                 const float mu_tot = mu_fgp + me;
                 const float divU = gU[0][0] + gU[1][1] + gU[2][2];
                 float tau[3][3], tauU[3];
@@ -275,7 +267,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 #pragma unroll
                 for (int i = 0; i < 3; ++i) tau[i][i] -= mu_fgp * twoThirds * divU;
 #pragma unroll
-                for (int i = 0; i < 3; ++i) tauU[i] = tau[i][0] * uu[0] + tau[i][1] * uu[1] + tau[i][2] * uu[2];
+                for (int i = 0; i < 3; ++i) tauU[i] = tau[i][0] * uu[2] + tau[i][1] * uu[3] + tau[i][2] * uu[4];
                 const float *Xv[kNX] = {gR, tauU, gT, tau[0], tau[1], tau[2]};
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
@@ -289,7 +281,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                     }
                 if (live) {
                     sNK[l] = me / r;
-                    sNK[N + l] = muf * Cp / Pr + me * Cp / Pr + Cp * r * ms / 0.9f;
+                    sNK[NP + l] = muf[h] * Cp / Pr + me * Cp / Pr + Cp * r * ms / 0.9f;
                 }
             }
             if (tid == 0)  // task 0, first point: lattice node (0,0,0)
@@ -302,15 +294,15 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                 fl[1][x] = two ? __fsub_rn(fl[1][x], sRef[x]) : 0.0f;
                 const float mx = fmaxf(0.0f, fmaxf(fabsf(fl[0][x]), fabsf(fl[1][x])));
                 const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-                if (lane == 0) atomicMax(&sMax[kNG + x], mb);
+                if (lane == 0) atomicMax(&sMax[kFx0 + x], mb);
             }
             __syncthreads();
-            if (tid >= kNG && tid < kNG + kNFX) scale_from_max(sMax[tid], G::BITS, sScale[tid], sInv[tid]);
+            if (tid >= kFx0 && tid < kFx0 + kNFX) scale_from_max(sMax[tid], G::BITS, sScale[tid], sInv[tid]);
             __syncthreads();
             if (valid) {
 #pragma unroll
                 for (int x = 0; x < kNFX; ++x) {
-                    const float s = sScale[kNG + x];
+                    const float s = sScale[kFx0 + x];
                     unsigned hi, lo;
                     split_scaled<BF16>(__fmul_rn(fl[0][x], s), __fmul_rn(fl[1][x], s), hi, lo);
                     *reinterpret_cast<unsigned *>(sHalf + (2 * x) * G::PB + row_off) = hi;
@@ -331,9 +323,9 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
             float acc[2][kNX];
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-                lat[s] = dpass_point<Q>(d, s, g, tq, warp);
+                lat[s] = pass_point<Q>(d, s, g, tq, warp);
 #pragma unroll
-                for (int x = 0; x < kNX; ++x) acc[s][x] = (d == 0 || lat[s] < 0) ? 0.0f : sAcc[x * N + lat[s]];
+                for (int x = 0; x < kNX; ++x) acc[s][x] = (d == 0 || lat[s] < 0) ? 0.0f : sAcc[x * NP + lat[s]];
             }
 #pragma unroll
             for (int x = 0; x < kNX; x += 2) {
@@ -348,10 +340,11 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                 mma_acc<BF16>(c, a, bl, 0u);
                 const float cs0 = d == 0 ? colsum[0][0] : (d == 1 ? colsum[1][0] : colsum[2][0]);
                 const float cs1 = d == 0 ? colsum[0][1] : (d == 1 ? colsum[1][1] : colsum[2][1]);
+                const float2 inv2 = *reinterpret_cast<const float2 *>(sInv + kFx0 + d * kNX + x);
+                const float2 ref2 = *reinterpret_cast<const float2 *>(sRef + d * kNX + x);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    const int fx = d * kNX + x + k;
-                    const float inv = sInv[kNG + fx], ref = sRef[fx];
+                    const float inv = k ? inv2.y : inv2.x, ref = k ? ref2.y : ref2.x;
 #pragma unroll
                     for (int s = 0; s < 2; ++s)
                         acc[s][x + k] = fmaf(c[2 * k + s], inv, fmaf(ref, s ? cs1 : cs0, acc[s][x + k]));
@@ -362,7 +355,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
                 for (int s = 0; s < 2; ++s)
                     if (lat[s] >= 0)
 #pragma unroll
-                        for (int x = 0; x < kNX; ++x) sAcc[x * N + lat[s]] = acc[s][x];
+                        for (int x = 0; x < kNX; ++x) sAcc[x * NP + lat[s]] = acc[s][x];
                 __syncthreads();
             } else {
 #pragma unroll
@@ -374,7 +367,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 #pragma unroll
                     for (int i = 0; i < 3; ++i) red_add(Rmom + (size_t)i * npoin + node, f2d(acc[s][X_TAU0 + i]));
                     // energy-flux assembly in FP64
-                    red_add(Rener + node, fma(f2d(sNK[N + lat[s]]), f2d(acc[s][X_GT]), f2d(acc[s][X_TAUU])));
+                    red_add(Rener + node, fma(f2d(sNK[NP + lat[s]]), f2d(acc[s][X_GT]), f2d(acc[s][X_TAUU])));
                 }
             }
         }

@@ -16,11 +16,12 @@ namespace msod {
 // blocks by shared memory).
 constexpr int kMixedRegs = 96;
 // Blocks of `threads` threads and `smem` bytes that an SM holds when every
-// thread has `regs` registers at least.
+// thread has `regs` registers at least (each of the four schedulers has 512 for
+// each lane of its warps).
 constexpr int mixed_blocks(size_t smem, int threads, int regs)
 {
-    const int by_smem = (int)((size_t)228 * 1024 / (smem + 1024)), by_regs = 65536 / (threads * regs);
-    const int b = by_smem < by_regs ? by_smem : by_regs;
+    int b = (int)((size_t)228 * 1024 / (smem + 1024));
+    while (b > 1 && 512 / ((b * threads / 32 + 3) / 4) < regs) --b;
     return b < 1 ? 1 : b;
 }
 
@@ -45,6 +46,40 @@ template <int Q>
 constexpr int plane_guard_bytes()
 {
     return (MIXED_TRIM_PLANES ? 64 - 8 * Q : 0) * kRowB;
+}
+
+// Shared-memory position of lattice point (K, J, I) in a plane of node_plane<Q>()
+// words, I contiguous.  The passes read two points of each of up to eight lines
+// per thread quad (lines along I for xi, else along J or K): k-planes a few words
+// further apart, and for Q = 8 an exclusive-or of the rows, keep those reads on
+// distinct banks.
+template <int Q>
+constexpr int node_pitch()
+{
+    return Q == 4 ? 20 : (Q == 5 ? 28 : (Q == 7 ? 52 : Q * Q));
+}
+template <int Q>
+constexpr int node_plane()
+{
+    return (Q * node_pitch<Q>() + 3) / 4 * 4;
+}
+template <int Q>
+__device__ __forceinline__ int node_at(int K, int J, int I)
+{
+    if (Q == 8) return K * 64 + (((J >> 1 | (J & 1) << 2) ^ (K >> 1)) << 3) + I;
+    return K * node_pitch<Q>() + J * Q + I;
+}
+
+// Position of slot s of a pass (output point 2t + s along direction d of line g
+// of tile o); -1 when padded.
+template <int Q>
+__device__ __forceinline__ int pass_point(int d, int s, int g, int tq, int o)
+{
+    const int pt = 2 * tq + s;
+    const int I = d == 0 ? pt : g;
+    const int J = d == 0 ? g : (d == 1 ? pt : o);
+    const int K = d == 2 ? pt : o;
+    return g < Q && pt < Q ? node_at<Q>(K, J, I) : -1;
 }
 
 // Row (k, j) of a half plane sits at position 8k + (j xor k): the eight rows
