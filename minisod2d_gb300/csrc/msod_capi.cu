@@ -216,12 +216,13 @@ static int diffu_impl(int porder, int nelem, int npoin, const int *connec, const
     return rc;
 }
 
+// Both residuals behind one zeroing launch; joint: in one set of arrays (c and d the same).
 static int both_impl(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                       const float *dlx, const int *inv, const int *ai, const int *aj, const int *ak, float Cp,
                       float Pr, const float *u, const float *q, const float *rho, const float *pr, const float *E,
                       const float *Tem, const float *mu_fluid, const float *mu_e, const float *mu_sgs,
                       float *Rmass_c, float *Rmom_c, float *Rener_c, float *Rmass_d, float *Rmom_d,
-                      float *Rener_d, void *stream)
+                      float *Rener_d, bool joint, void *stream)
 {
     clear_error();
     int rc = check_geometry(porder, nelem, npoin, connec, He, gpvol, dlx, inv, ai, aj, ak);
@@ -232,7 +233,7 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     for (int i = 0; i < 6; ++i) {
         if (!outs[i]) return set_error(MSOD_ERR_INVALID_ARG, "NULL residual array");
         for (int j = 0; j < i; ++j)
-            if (outs[i] == outs[j]) return set_error(MSOD_ERR_INVALID_ARG, "the six residual arrays must be distinct");
+            if (!(joint && i == j + 3) && outs[i] == outs[j]) return set_error(MSOD_ERR_INVALID_ARG, "the six residual arrays must be distinct");
     }
     if (!(Pr != 0.0f)) return set_error(MSOD_ERR_INVALID_ARG, "Pr must be non-zero");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -244,7 +245,7 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
     ZeroSpans z;
     add_outputs(z, Rmass_c, Rmom_c, Rener_c, npoin);
-    add_outputs(z, Rmass_d, Rmom_d, Rener_d, npoin);
+    if (!joint) add_outputs(z, Rmass_d, Rmom_d, Rener_d, npoin);
     rc = cuda_status(launch_zero(z, st), "residual zeroing launch");
     if (rc) return rc;
     ConvecArgs<float> c;
@@ -259,6 +260,17 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     if (!rc) rc = cuda_status(launch_diffu_plain<float>(porder, d, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection + diffusion kernel");
     return rc;
+}
+
+int residual_sum(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
+                 const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
+                 const int *gmshAtoK, float Cp, float Pr, const float *u, const float *q, const float *rho,
+                 const float *pr, const float *E, const float *Tem, const float *mu_fluid, const float *mu_e,
+                 const float *mu_sgs, float *Rmass, float *Rmom, float *Rener, void *stream)
+{
+    return both_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK, Cp,
+                     Pr, u, q, rho, pr, E, Tem, mu_fluid, mu_e, mu_sgs, Rmass, Rmom, Rener, Rmass, Rmom, Rener, true,
+                     stream);
 }
 
 }  // namespace msod
@@ -401,7 +413,7 @@ int msod_convec_diffusion_ijk(int porder, int nelem, int npoin, const int *conne
     (void)Ngp; (void)dNgp; (void)xgp;
     return both_impl(porder, nelem, npoin, connec, He, gpvol, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK,
                       Cp, Pr, u, q, rho, pr, E, Tem, mu_fluid, mu_e, mu_sgs, Rmass_c, Rmom_c, Rener_c, Rmass_d,
-                      Rmom_d, Rener_d, stream);
+                      Rmom_d, Rener_d, false, stream);
 }
 
 int msod_diffusion_ijk_nu(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,

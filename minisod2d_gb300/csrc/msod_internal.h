@@ -21,6 +21,13 @@ bool checked_mode();
 bool mode_is_default_convec();
 bool mode_is_default_diffusion();
 void mode_release();
+// Convection + diffusion residual in one set of arrays (the default form of both
+// calls; msod_convec_diffusion_ijk's arguments and checks otherwise).
+int residual_sum(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
+                 const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
+                 const int *gmshAtoK, float Cp, float Pr, const float *u, const float *q, const float *rho,
+                 const float *pr, const float *E, const float *Tem, const float *mu_fluid, const float *mu_e,
+                 const float *mu_sgs, float *Rmass, float *Rmom, float *Rener, void *stream);
 int mode_convec(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
                 const float *dlxigp_ip, const int *invAtoIJK, const int *gmshAtoI, const int *gmshAtoJ,
                 const int *gmshAtoK, const float *u, const float *q, const float *rho, const float *pr,
