@@ -460,18 +460,13 @@ int msod_convec_ijk_mixed(int precision, int porder, int nelem, int npoin, const
         rc = run_check(porder, nelem, npoin, connec, dlxigp_ip, invAtoIJK, gmshAtoI, gmshAtoJ, gmshAtoK, st);
         if (rc) return rc;
     }
-    TableScratch *tabs = device_tables(porder);
-    if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
     rc = zero_outputs(Rmass, Rmom, Rener, npoin, st);
     if (rc) return rc;
-    ElementArgs<float> ea;
-    ea.nelem = nelem; ea.npoin = npoin; ea.connec = connec; ea.He = He; ea.gpvol = gpvol; ea.dlxigp_ip = dlxigp_ip;
-    ea.invAtoIJK = invAtoIJK; ea.AtoI = gmshAtoI; ea.AtoJ = gmshAtoJ; ea.AtoK = gmshAtoK;
     MixedConvecArgs a;
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol;
+    a.dlxigp_ip = dlxigp_ip; a.invAtoIJK = invAtoIJK;
     a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E; a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
-    rc = cuda_status(launch_table_prep<float>(porder, ea, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_convec_mixed(porder, prec, a, tabs, st), "mixed convection launch");
+    rc = cuda_status(launch_convec_mixed(porder, prec, a, st), "mixed convection launch");
     if (!rc && checked_mode()) rc = cuda_status(cudaStreamSynchronize(st), "mixed convection kernel");
     return rc;
 }
@@ -496,19 +491,14 @@ static int diffu_mixed_impl(int precision, int porder, int nelem, int npoin, con
         rc = run_check(porder, nelem, npoin, connec, dlx, inv, ai, aj, ak, st);
         if (rc) return rc;
     }
-    TableScratch *tabs = device_tables(porder);
-    if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
     rc = zero_outputs(Rmass, Rmom, Rener, npoin, st);
     if (rc) return rc;
-    ElementArgs<float> ea;
-    ea.nelem = nelem; ea.npoin = npoin; ea.connec = connec; ea.He = He; ea.gpvol = gpvol; ea.dlxigp_ip = dlx;
-    ea.invAtoIJK = inv; ea.AtoI = ai; ea.AtoJ = aj; ea.AtoK = ak;
     MixedDiffuArgs a;
-    a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.Cp = Cp; a.Pr = Pr;
+    a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol;
+    a.dlxigp_ip = dlx; a.invAtoIJK = inv; a.Cp = Cp; a.Pr = Pr;
     a.rho = rho; a.u = u; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mu_e = mu_e; a.mu_sgs = mu_sgs; a.nu_elem = nu_elem;
     a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
-    rc = cuda_status(launch_table_prep<float>(porder, ea, tabs, st), "table preparation launch");
-    if (!rc) rc = cuda_status(launch_diffu_mixed(porder, precision, a, tabs, st), "mixed diffusion launch");
+    rc = cuda_status(launch_diffu_mixed(porder, precision, a, st), "mixed diffusion launch");
     if (!rc && checked_mode()) rc = cuda_status(cudaStreamSynchronize(st), "mixed diffusion kernel");
     return rc;
 }

@@ -134,31 +134,23 @@ template <typename real>
 cudaError_t launch_convec_plain(int porder, const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
 template <typename real>
 cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st);
-// Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by the
-// caller; tables prepared).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
-struct MixedConvecArgs {
-    int nelem, npoin;
-    const int *connec;
-    const float *He, *gpvol;
+// Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by
+// launch_zero just before).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
+struct MixedConvecArgs : ElementArgs<float> {
     const float *u, *q, *rho, *pr, *E;
     double *Rmass, *Rmom, *Rener;
 };
-cudaError_t launch_convec_mixed(int porder, int precision, const MixedConvecArgs &a,
-                                const TableScratch *tabs, cudaStream_t st);
+cudaError_t launch_convec_mixed(int porder, int precision, const MixedConvecArgs &a, cudaStream_t st);
 
-// Mixed-precision diffusion: FP32 fields, FP64 residuals (zeroed by the
-// caller; tables prepared).  nu_elem set: mu_e(e, a) = rho(a) nu_elem[e] and
+// Mixed-precision diffusion: FP32 fields, FP64 residuals (zeroed by
+// launch_zero just before).  nu_elem set: mu_e(e, a) = rho(a) nu_elem[e] and
 // mu_e is not read.
-struct MixedDiffuArgs {
-    int nelem, npoin;
-    const int *connec;
-    const float *He, *gpvol;
+struct MixedDiffuArgs : ElementArgs<float> {
     float Cp, Pr;
     const float *rho, *u, *Tem, *mu_fluid, *mu_e, *mu_sgs, *nu_elem;
     double *Rmass, *Rmom, *Rener;
 };
-cudaError_t launch_diffu_mixed(int porder, int precision, const MixedDiffuArgs &a, const TableScratch *tabs,
-                               cudaStream_t st);
+cudaError_t launch_diffu_mixed(int porder, int precision, const MixedDiffuArgs &a, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Entropy viscosity and the learned estimator

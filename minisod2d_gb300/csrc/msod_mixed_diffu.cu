@@ -69,7 +69,8 @@ struct MixedDiffuGeom {
 template <int P, bool BF16, bool NUE>
 __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
     diffu_mixed_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
-                       const float *__restrict__ gpvol, const TableScratch *__restrict__ tabs, float Cp, float Pr,
+                       const float *__restrict__ gpvol, const int *__restrict__ inv,
+                       const float *__restrict__ dlxigp_ip, float Cp, float Pr,
                        const float *__restrict__ rho, const float *__restrict__ u, const float *__restrict__ Tem,
                        const float *__restrict__ mu_fluid, const float *__restrict__ mu_e,
                        const float *__restrict__ mu_sgs, const float *__restrict__ nu_elem,
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tq = lane & 3;
-    for (int i = tid; i < N; i += NT) sPerm[node_at<Q>(i / (Q * Q), i / Q % Q, i % Q)] = tabs->perm[i];
+    for (int i = tid; i < N; i += NT) sPerm[node_at<Q>(i / (Q * Q), i / Q % Q, i % Q)] = table_node<Q>(inv, i);
     if (Q < 8) {  // rows and points beyond Q are never written and stay zero
         uint4 *z = reinterpret_cast<uint4 *>(sHalf);
         for (int i = tid; i < (int)(G::half_bytes / 16); i += NT) z[i] = make_uint4(0, 0, 0, 0);
@@ -102,10 +103,10 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int c0 = 2 * tq, c1 = c0 + 1;
-        const float *D = tabs->Df + d * Q * Q;
-        split_pair<BF16>((g < Q && c0 < Q) ? D[g * Q + c0] : 0.0f, (g < Q && c1 < Q) ? D[g * Q + c1] : 0.0f,
+        auto D = [&](int r, int c) { return table_D<Q>(inv, dlxigp_ip, d, r, c); };
+        split_pair<BF16>((g < Q && c0 < Q) ? D(g, c0) : 0.0f, (g < Q && c1 < Q) ? D(g, c1) : 0.0f,
                          Bgh[d], Bgl[d]);
-        split_pair<BF16>((g < Q && c0 < Q) ? D[c0 * Q + g] : 0.0f, (g < Q && c1 < Q) ? D[c1 * Q + g] : 0.0f,
+        split_pair<BF16>((g < Q && c0 < Q) ? D(c0, g) : 0.0f, (g < Q && c1 < Q) ? D(c1, g) : 0.0f,
                          Bdh[d], Bdl[d]);
     }
     // Column sums of the divergence operator at the thread's output points 2t, 2t+1.
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
             const int a = 2 * tq + h;
             double cs = 0.0;
             if (a < Q)
-                for (int c = 0; c < Q; ++c) cs += (double)tabs->Df[(d * Q + c) * Q + a];
+                for (int c = 0; c < Q; ++c) cs += (double)table_D<Q>(inv, dlxigp_ip, d, c, a);
             colsum[d][h] = (float)cs;
         }
     // ldmatrix matrix m of the A operand is (hi f, hi f+1, lo f, lo f+1), row r8
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
     const int row_off = row_pos(row / Q, row % Q) * kRowB + 4 * w;
     const bool two = valid && 2 * w + 1 < Q;
     const int l0 = node_at<Q>(row / Q, row % Q, 2 * w);
-    const int a0 = tabs->perm[row * Q + 2 * w], a1 = tabs->perm[row * Q + 2 * w + (two ? 1 : 0)];
+    const int a0 = table_node<Q>(inv, row * Q + 2 * w), a1 = table_node<Q>(inv, row * Q + 2 * w + (two ? 1 : 0));
     // Node ids, loaded an element ahead (the grid has nelem blocks at most).
     int id[2] = {ldg_once(connec + (size_t)a0 * nelem + blockIdx.x), ldg_once(connec + (size_t)a1 * nelem + blockIdx.x)};
     const size_t np = (size_t)npoin;
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
 }
 
 template <int P, bool BF16, bool NUE>
-cudaError_t launch_pbn(const MixedDiffuArgs &a, const TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_pbn(const MixedDiffuArgs &a, cudaStream_t st)
 {
     using G = MixedDiffuGeom<P, BF16>;
     static_assert(G::smem <= 227 * 1024, "shared memory budget");
@@ -385,32 +386,34 @@ cudaError_t launch_pbn(const MixedDiffuArgs &a, const TableScratch *tabs, cudaSt
     if (a.nelem == 0) return cudaSuccess;
     const int grid = persistent_grid(kern, G::NT, G::smem, a.nelem);
     if (grid < 1) return cudaErrorInvalidConfiguration;
-    kern<<<grid, G::NT, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, tabs, a.Cp, a.Pr, a.rho, a.u,
-                                          a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem, a.Rmass, a.Rmom, a.Rener);
+    // Not launched over the zeroing kernel: blocks that start beside it are spread
+    // unevenly over the SMs for all of the kernel (porder-4 48^3 convection 2.83 against 2.68 ms).
+    kern<<<grid, G::NT, G::smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol,
+                        a.invAtoIJK, a.dlxigp_ip, a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs,
+                        a.nu_elem, a.Rmass, a.Rmom, a.Rener);
     return cudaGetLastError();
 }
 
 template <int P>
-cudaError_t launch_p(const MixedDiffuArgs &a, int precision, const TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_p(const MixedDiffuArgs &a, int precision, cudaStream_t st)
 {
     const bool bf = precision == MSOD_PREC_BF16, nue = a.nu_elem != nullptr;
-    if (bf) return nue ? launch_pbn<P, true, true>(a, tabs, st) : launch_pbn<P, true, false>(a, tabs, st);
-    return nue ? launch_pbn<P, false, true>(a, tabs, st) : launch_pbn<P, false, false>(a, tabs, st);
+    if (bf) return nue ? launch_pbn<P, true, true>(a, st) : launch_pbn<P, true, false>(a, st);
+    return nue ? launch_pbn<P, false, true>(a, st) : launch_pbn<P, false, false>(a, st);
 }
 
 }  // namespace
 
-cudaError_t launch_diffu_mixed(int porder, int precision, const MixedDiffuArgs &a, const TableScratch *tabs,
-                               cudaStream_t st)
+cudaError_t launch_diffu_mixed(int porder, int precision, const MixedDiffuArgs &a, cudaStream_t st)
 {
     switch (porder) {
-    case 1: return launch_p<1>(a, precision, tabs, st);
-    case 2: return launch_p<2>(a, precision, tabs, st);
-    case 3: return launch_p<3>(a, precision, tabs, st);
-    case 4: return launch_p<4>(a, precision, tabs, st);
-    case 5: return launch_p<5>(a, precision, tabs, st);
-    case 6: return launch_p<6>(a, precision, tabs, st);
-    case 7: return launch_p<7>(a, precision, tabs, st);
+    case 1: return launch_p<1>(a, precision, st);
+    case 2: return launch_p<2>(a, precision, st);
+    case 3: return launch_p<3>(a, precision, st);
+    case 4: return launch_p<4>(a, precision, st);
+    case 5: return launch_p<5>(a, precision, st);
+    case 6: return launch_p<6>(a, precision, st);
+    case 7: return launch_p<7>(a, precision, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -48,6 +48,21 @@ constexpr int plane_guard_bytes()
     return (MIXED_TRIM_PLANES ? 64 - 8 * Q : 0) * kRowB;
 }
 
+// gmsh node of lattice point l = (K Q + J) Q + I, and the 1-D derivative matrices
+// D(d, r, c) = dlxigp_ip(g, d, c) at a point g whose 1-D index in direction d is r,
+// read once per block (clamped: malformed tables give wrong numbers, never an
+// access out of bounds).
+template <int Q>
+__device__ __forceinline__ int table_node(const int *__restrict__ inv, int l)
+{
+    return min(max(__ldg(inv + l) - 1, 0), Q * Q * Q - 1);
+}
+template <int Q>
+__device__ __forceinline__ float table_D(const int *__restrict__ inv, const float *__restrict__ dlx, int d, int r, int c)
+{
+    return __ldg(dlx + (size_t)(c * 3 + d) * Q * Q * Q + table_node<Q>(inv, d == 0 ? r : (d == 1 ? r * Q : r * Q * Q)));
+}
+
 // Shared-memory position of lattice point (K, J, I) in a plane of node_plane<Q>()
 // words, I contiguous.  The passes read two points of each of up to eight lines
 // per thread quad (lines along I for xi, else along J or K): k-planes a few words

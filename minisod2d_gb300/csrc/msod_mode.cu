@@ -58,10 +58,30 @@ void *mode_buffer(int slot, size_t bytes)
     return g_buf[dev][slot];
 }
 
-__global__ void to_float_kernel(const double *__restrict__ src, float *__restrict__ dst, size_t n)
+// dst[k] = (float)src[k] for the three residual arrays in one launch; a block takes
+// kPiece numbers of one array, eight loads in flight per thread.  Bound by memory; a
+// pair of calls on 24^3 porder-7 hexes (two conversions of 24.1 M numbers) 1517 us with
+// grid-stride loops of one load in three launches, 1417 so and with the tensor-core
+// kernels reading the element tables themselves.
+constexpr int kPiece = 2048;
+struct ToFloat {
+    const double *src[3];
+    float *dst[3];
+    size_t n[3];
+    unsigned first[3];  // first block of each array
+};
+__global__ void __launch_bounds__(256) to_float_kernel(ToFloat t)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = (float)src[i];
+    const int k = blockIdx.x >= t.first[2] ? 2 : (blockIdx.x >= t.first[1] ? 1 : 0);
+    const size_t i0 = (size_t)(blockIdx.x - t.first[k]) * kPiece + threadIdx.x;
+    const double *__restrict__ src = t.src[k];
+    float *__restrict__ dst = t.dst[k];
+    double v[kPiece / 256];
+#pragma unroll
+    for (int j = 0; j < kPiece / 256; ++j) v[j] = i0 + 256 * j < t.n[k] ? __ldcs(src + i0 + 256 * j) : 0.0;
+#pragma unroll
+    for (int j = 0; j < kPiece / 256; ++j)
+        if (i0 + 256 * j < t.n[k]) dst[i0 + 256 * j] = (float)v[j];
 }
 
 __global__ void pressure_kernel(const float *__restrict__ rho, const float *__restrict__ Tem, float Rgas,
@@ -93,10 +113,14 @@ int r64_buffers(int npoin, R64 &r)
 
 int r64_to_float(const R64 &r, int npoin, float *Rmass, float *Rmom, float *Rener, cudaStream_t st)
 {
-    const int grid = 4 * 152, block = 256;
-    to_float_kernel<<<grid, block, 0, st>>>(r.mass, Rmass, (size_t)npoin);
-    to_float_kernel<<<grid, block, 0, st>>>(r.mom, Rmom, 3 * (size_t)npoin);
-    to_float_kernel<<<grid, block, 0, st>>>(r.ener, Rener, (size_t)npoin);
+    const size_t n = (size_t)npoin;
+    ToFloat t{{r.mass, r.mom, r.ener}, {Rmass, Rmom, Rener}, {n, 3 * n, n}, {}};
+    unsigned blocks = 0;
+    for (int k = 0; k < 3; ++k) {
+        t.first[k] = blocks;
+        blocks += (unsigned)((t.n[k] + kPiece - 1) / kPiece);
+    }
+    to_float_kernel<<<blocks, 256, 0, st>>>(t);
     return launch_status("residual conversion launch");
 }
 
