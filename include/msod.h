@@ -120,7 +120,7 @@ int msod_convec_ijk(int porder, int nelem, int npoin, const int *connec, const f
                     void *stream);
 
 /* full_convec_ijk_split (elem_convec.f90:433-836): same arguments and the same
- * residuals; served by the same fused single-pass kernel. */
+ * residuals; served by the same single-pass kernel. */
 int msod_convec_ijk_split(int porder, int nelem, int npoin, const int *connec, const float *Ngp,
                           const float *dNgp, const float *He, const float *gpvol,
                           const float *dlxigp_ip, const float *xgp, const int *invAtoIJK,

@@ -177,7 +177,7 @@ static int convec_impl(int porder, int nelem, int npoin, const int *connec, cons
     if (rc) return rc;
     ConvecArgs<real> a;
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlx;
-    a.invAtoIJK = inv; a.AtoI = ai; a.AtoJ = aj; a.AtoK = ak;
+    a.invAtoIJK = inv;
     a.u = u; a.q = q; a.rho = rho; a.pr = pr; a.E = E; a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
     rc = cuda_status(launch_convec_plain<real>(porder, a, tabs, st), "convection kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection kernel");
@@ -208,7 +208,7 @@ static int diffu_impl(int porder, int nelem, int npoin, const int *connec, const
     if (rc) return rc;
     DiffuArgs<real> a;
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlx;
-    a.invAtoIJK = inv; a.AtoI = ai; a.AtoJ = aj; a.AtoK = ak; a.Cp = Cp; a.Pr = Pr;
+    a.invAtoIJK = inv; a.Cp = Cp; a.Pr = Pr;
     a.rho = rho; a.u = u; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mu_e = mu_e; a.mu_sgs = mu_sgs; a.nu_elem = nu_elem;
     a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
     rc = cuda_status(launch_diffu_plain<real>(porder, a, tabs, st), "diffusion kernel launch");
@@ -250,7 +250,7 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     if (rc) return rc;
     ConvecArgs<float> c;
     c.nelem = nelem; c.npoin = npoin; c.connec = connec; c.He = He; c.gpvol = gpvol; c.dlxigp_ip = dlx;
-    c.invAtoIJK = inv; c.AtoI = ai; c.AtoJ = aj; c.AtoK = ak;
+    c.invAtoIJK = inv;
     c.u = u; c.q = q; c.rho = rho; c.pr = pr; c.E = E; c.Rmass = Rmass_c; c.Rmom = Rmom_c; c.Rener = Rener_c;
     DiffuArgs<float> d;
     static_cast<ElementArgs<float> &>(d) = c;

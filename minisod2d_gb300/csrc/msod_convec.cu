@@ -46,8 +46,8 @@
 //     and (rho, p) of its points to the shared-memory lattice;
 //   * three passes (zeta, xi, eta) evaluate the pairwise form along the lines of
 //     a direction, point after point of the line: the line's records sit in
-//     registers (the zeta pass has them from the gather), the derivative matrix
-//     is a constant-bank operand, and the five sums of a point (momentum,
+//     registers (the zeta pass has them from the gather), the derivative matrix's
+//     rows come from shared memory, and the five sums of a point (momentum,
 //     energy, mass) pass from one direction's thread to the next through
 //     shared memory;
 //   * the last pass applies gpvol and scatter-adds with red.global.add.

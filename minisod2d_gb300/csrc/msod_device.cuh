@@ -52,68 +52,6 @@ __device__ __forceinline__ T ldg_once(const T *p)
     return __ldcg(p);
 }
 
-// Per-porder launch geometry of the line-parallel element kernels.
-//   Q  = points per line, L = lines per direction, N = points per element.
-//   QP = padded row pitch in shared memory (odd, so that line loads along x
-//        hit distinct banks), ES = shared-memory words per element plane.
-//   S  = threads per line (each owns R consecutive points of the line; S_ > 0
-//        overrides the default),
-//   NE = elements per block (at most NECAP), NT = threads per block.
-template <typename real_t, int P_, int NECAP = 64, int S_ = 0>
-struct LineGeom {
-    using real = real_t;
-    static constexpr int P = P_;
-    static constexpr int Q = P + 1;
-    static constexpr int L = Q * Q;
-    static constexpr int N = Q * Q * Q;
-    static constexpr int QP = (Q % 2 == 0) ? Q + 1 : Q;
-    static constexpr int ES = Q * Q * QP;
-    static constexpr int S = S_ > 0 ? S_ : (sizeof(real) == 8 ? Q : (P <= 5 ? 1 : (P <= 7 ? 2 : 3)));
-    static constexpr int R = (Q + S - 1) / S;
-    static constexpr int TPE = L * S;  // threads per element
-    static constexpr int CAP = sizeof(real) == 8 ? (TPE <= 128 ? 128 : ((TPE + 31) / 32) * 32)
-                                                 : (TPE <= 32 ? 128 : 256);
-    static constexpr int NE0 = CAP / TPE > 0 ? CAP / TPE : 1;
-    static constexpr int NE = NE0 < NECAP ? NE0 : (NECAP > 0 ? NECAP : 1);
-    static constexpr int NT = ((NE * TPE + 31) / 32) * 32;
-    static constexpr int NPL = NE * ES;  // words per shared-memory plane
-};
-
-// Thread -> (element, line, segment) of the line-parallel passes.
-template <class G>
-struct LineThread {
-    int el, la, lb, r0;
-    bool active;
-    __device__ __forceinline__ LineThread(int tid)
-    {
-        active = tid < G::NE * G::TPE;
-        const int t = active ? tid : 0;
-        el = t / G::TPE;
-        const int rem = t - el * G::TPE;
-        const int line = G::S == 1 ? rem : rem / G::S;
-        const int seg = G::S == 1 ? 0 : rem - line * G::S;
-        la = line % G::Q;
-        lb = line / G::Q;
-        r0 = seg * G::R;
-    }
-    __device__ __forceinline__ bool owns(int rr) const { return (G::R * G::S == G::Q) || r0 + rr < G::Q; }
-    __device__ __forceinline__ int rc(int rr) const { return owns(rr) ? r0 + rr : 0; }
-};
-
-// Offset of point r of the line (la, lb) running in direction DIR, in the
-// padded lattice of one element, and its unpadded lattice index.
-template <int DIR, int Q, int QP>
-__host__ __device__ constexpr int line_off(int la, int lb, int r)
-{
-    return DIR == 0 ? (lb * Q + la) * QP + r : (DIR == 1 ? (lb * Q + r) * QP + la : (r * Q + lb) * QP + la);
-}
-
-template <int DIR, int Q>
-__device__ __forceinline__ int line_lat(int la, int lb, int r)
-{
-    return DIR == 0 ? (lb * Q + la) * Q + r : (DIR == 1 ? (lb * Q + r) * Q + la : (r * Q + lb) * Q + la);
-}
-
 // Order-preserving map of a float onto a signed int (for integer atomics).
 __device__ __forceinline__ int f2key(float f)
 {
@@ -121,19 +59,6 @@ __device__ __forceinline__ int f2key(float f)
     return i >= 0 ? i : i ^ 0x7FFFFFFF;
 }
 __device__ __forceinline__ float key2f(int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7FFFFFFF); }
-
-// Asynchronous 4/8-byte global->shared copies (cp.async); an invalid element is
-// zero-filled without reading global memory.
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T *dst_smem, const T *src, bool valid)
-{
-    const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst_smem);
-    const int nbytes = valid ? (int)sizeof(T) : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(saddr), "l"(src), "n"(sizeof(T)), "r"(nbytes)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // 1-D bulk copies (cp.async.bulk, the TMA engine's untiled form) completing on
@@ -154,9 +79,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, u
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
-// Orders this thread's earlier generic-proxy accesses of shared memory (and,
-// after a barrier, the block's) before later async-proxy writes (bulk copies).
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // dst (shared) <- src (global), `bytes` bytes; both addresses 16-byte aligned,
 // bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
@@ -188,12 +110,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
     return false;
 }
 
-// A contiguous global span [src, src + bytes) staged in shared memory at
-// dst_base + (src mod 16): the 16-byte-aligned interior by one bulk copy, the
-// unaligned head and tail (at most 12 bytes each; spans are 4-byte aligned) by
-// threads 0..5 with plain loads.  Returns the bulk bytes the caller's
-// mbar_arrive_expect_tx must announce.  Thread `issuer` issues the copy;
-// dst_base is 16-byte aligned and holds bytes + 32.
 // L2 prefetch of the 16-byte-aligned interior of [p, p + nbytes) by the bulk
 // copy unit (one thread; a hint with nothing to wait for; no byte outside the
 // span is touched).  No memory clobber: the prefetch writes nothing, and a
@@ -206,13 +122,12 @@ __device__ __forceinline__ void prefetch_span_l2(const void *p, size_t nbytes)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a16), "r"((unsigned)(e16 - a16)));
 }
 
-// He(3,3,ngaus,e) and gpvol(ngaus,e) of element e into L2 (one thread).
-__device__ __forceinline__ void prefetch_element_l2(const float *He, const float *gpvol, int e, int ngaus)
-{
-    prefetch_span_l2(He + (size_t)e * ngaus * 9, (size_t)ngaus * 9 * sizeof(float));
-    prefetch_span_l2(gpvol + (size_t)e * ngaus, (size_t)ngaus * sizeof(float));
-}
-
+// A contiguous global span [src, src + bytes) staged in shared memory at
+// dst_base + (src mod 16): the 16-byte-aligned interior by one bulk copy, the
+// unaligned head and tail (at most 12 bytes each; spans are 4-byte aligned) by
+// threads 0..5 with plain loads.  Returns the bulk bytes the caller's
+// mbar_arrive_expect_tx must announce.  Thread `issuer` issues the copy;
+// dst_base is 16-byte aligned and holds bytes + 32.
 struct SpanPlan {
     const char *src;
     unsigned bytes, head, bulk, tail, shift;

@@ -30,8 +30,8 @@
 //   4. the thread of the zeta line adds the three divergences of its points,
 //      forms the residuals and scatter-adds them with red.global.add.
 // The viscosities, nu_e, kappa_e and the node ids never leave the registers of
-// the zeta line's thread.  The 1-D derivative matrices are constant-bank
-// operands.
+// the zeta line's thread.  The 1-D derivative matrices come from shared memory or,
+// on large meshes, from the constant bank (diffu_const_points).
 #include <cuda_runtime.h>
 
 #include "msod_group.cuh"
@@ -402,7 +402,7 @@ cudaError_t launch_diffu_pc(const DiffuArgs<real> &a, TableScratch *tabs, cudaSt
     cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
     if constexpr (CONSTD) {
-        err = launch_table_prep<real>(P, a, tabs, st);
+        err = launch_table_prep(P, a, tabs, st);
         if (err == cudaSuccess)
             err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, sizeof(float) * 3 * G::Q * G::Q,
                                           sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);

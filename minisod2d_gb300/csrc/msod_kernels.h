@@ -10,17 +10,11 @@
 
 namespace msod {
 
-// Per-call element tables written by table_prep_kernel (msod_tables.cu) into a
-// library-owned device area: the 1-D derivative matrices D[d][r][c] (FP32 and
-// FP64 copies), lattice -> gmsh node (perm) and gmsh node -> padded lattice
-// offset (lat).
+// A porder's library-owned device area: the 1-D derivative matrices D[d][r][c] on
+// their way to the constant bank (written by table_prep_kernel, msod_tables.cu).
 constexpr int kTableDMax = 3 * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
-constexpr int kTableNMax = (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1) * (MSOD_MAX_PORDER + 1);
 struct TableScratch {
     float Df[kTableDMax];
-    double Dd[kTableDMax];
-    int perm[kTableNMax];
-    int lat[kTableNMax];
     // Set (sticky, zero at allocation) by a kernel whose bounded wait for a
     // bulk copy into shared memory ran out; the kernel then skipped its work.
     // Checked mode reads and clears it after each call.
@@ -33,29 +27,11 @@ __device__ __forceinline__ void report_wait_fault(const TableScratch *t)
     atomicOr(const_cast<int *>(&t->wait_fault), 1);
 }
 template <typename real>
-__host__ __device__ inline real *table_D(TableScratch *t);
-template <>
-__host__ __device__ inline float *table_D<float>(TableScratch *t)
-{
-    return t->Df;
-}
-template <>
-__host__ __device__ inline double *table_D<double>(TableScratch *t)
-{
-    return t->Dd;
-}
-template <typename real>
-__host__ __device__ inline const real *table_D(const TableScratch *t)
-{
-    return table_D<real>(const_cast<TableScratch *>(t));
-}
-
-template <typename real>
 struct ElementArgs {
     int nelem, npoin;
     const int *connec;
     const real *He, *gpvol, *dlxigp_ip;
-    const int *invAtoIJK, *AtoI, *AtoJ, *AtoK;
+    const int *invAtoIJK;
 };
 
 template <typename real>
@@ -124,9 +100,8 @@ inline cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned bloc
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
-// Tables of one call (one block, stream-ordered before the kernels).
-template <typename real>
-cudaError_t launch_table_prep(int porder, const ElementArgs<real> &a, TableScratch *scratch, cudaStream_t st);
+// D of one call (one block, stream-ordered before the kernel).
+cudaError_t launch_table_prep(int porder, const ElementArgs<float> &a, TableScratch *scratch, cudaStream_t st);
 
 // Plain kernels (outputs zeroed by launch_zero just before, or earlier on the
 // stream; tabs: where a bounded wait that ran out is recorded).
@@ -211,7 +186,7 @@ struct ViscArgs {
     int nelem, npoin;
     const int *connec;
     const float *He, *gpvol, *dlxigp_ip;
-    const int *invAtoIJK, *AtoI, *AtoJ, *AtoK;
+    const int *invAtoIJK;
     const float *rho, *u, *p_or_T;
     float Rgas, gamma, ce, cmax;
     int normalise;

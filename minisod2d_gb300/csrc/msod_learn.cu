@@ -130,7 +130,7 @@ int msod_entropy_viscosity(int porder, int nelem, int npoin, const int *connec, 
     if (rc) return rc;
     ViscArgs a{};
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlxigp_ip;
-    a.invAtoIJK = invAtoIJK; a.AtoI = gmshAtoI; a.AtoJ = gmshAtoJ; a.AtoK = gmshAtoK;
+    a.invAtoIJK = invAtoIJK;
     a.rho = rho; a.u = u; a.p_or_T = pr; a.Rgas = 0.0f; a.gamma = gamma; a.ce = ce; a.cmax = cmax;
     a.normalise = normalise; a.stats = stats; a.list = nullptr; a.count = nullptr; a.mu_e = mu_e; a.nu = nu_elem; a.numax = numax_elem;
     return cuda_rc(launch_entropy_visc(porder, a, st), "entropy viscosity launch");
@@ -405,7 +405,7 @@ static int learned_nu(const msod_mlp *m, int porder, int nelem, int npoin, const
     EntropyStats *stats = static_cast<EntropyStats *>(scratch(SLOT_STATS, sizeof(EntropyStats)));
     ViscArgs a{};
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlxigp_ip;
-    a.invAtoIJK = invAtoIJK; a.AtoI = gmshAtoI; a.AtoJ = gmshAtoJ; a.AtoK = gmshAtoK;
+    a.invAtoIJK = invAtoIJK;
     a.rho = rho; a.u = u; a.p_or_T = p_or_T; a.Rgas = Rgas; a.gamma = gamma; a.ce = ce; a.cmax = cmax;
     a.normalise = 1; a.stats = stats; a.list = list; a.count = count; a.mu_e = nullptr; a.nu = nu; a.numax = nullptr;
     return cuda_rc(launch_entropy_visc(porder, a, st), "fallback estimator launch");
