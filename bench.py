@@ -457,7 +457,8 @@ def run_ours(args, cfg, rank, local, world):
         "kernels": {"convec_ms": conv_ms, "diffu_ms": diff_ms, "convec_gbs": Bc / conv_ms / 1e6,
                     "diffu_gbs": Bd / diff_ms / 1e6,
                     "combined_frac": (Bc + Bd) / ((conv_ms + diff_ms) * 1e-3) / 1e9 / peak},
-        "gpu_launches": 4 * args.steps,  # per step: table preparation + kernel, for each of the two calls
+        # per step: zeroing + kernel of the convection; zeroing, table preparation and kernel of the diffusion
+        "gpu_launches": 5 * args.steps,
         "clocks": clocks,
         "e2e": e2e,
     }
@@ -701,7 +702,7 @@ def porder_sweep(reps=20, porders=range(1, 9), nodes_1d=256):
 
 def variant_fused(reps, host):
     """fused_64: the plain_64 step as the two drop-in calls and as one msod_convec_diffusion_ijk
-    call (one kernel at porder 4), with the agreement of the two forms' residuals."""
+    call (one zeroing, then both kernels), with the agreement of the two forms' residuals."""
     from minisod2d_gb300 import workload
 
     dev = workload.DeviceCase(host)

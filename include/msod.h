@@ -145,10 +145,9 @@ int msod_diffusion_ijk(int porder, int nelem, int npoin, const int *connec, cons
  * The fields are the convection's (u, q, rho, press = its pr, E) and the diffusion's
  * (rho, u shared; Tem, mu_fluid, mu_e, mu_sgs); the residuals go to Rmass_c,
  * Rmom_c, Rener_c (convection) and Rmass_d, Rmom_d, Rener_d (diffusion),
- * which must be six distinct arrays.  At porder 4 one kernel computes both
- * from one gather per element group; other porders run the two kernels on
- * one set of tables.  While msod_set_mode selects another
- * form, the call makes the two drop-in calls in turn. */
+ * which must be six distinct arrays.  One launch zeroes all six, then the two
+ * kernels run.  While msod_set_mode selects another form, the call makes the
+ * two drop-in calls in turn. */
 int msod_convec_diffusion_ijk(int porder, int nelem, int npoin, const int *connec,
                               const float *Ngp, const float *dNgp, const float *He,
                               const float *gpvol, const float *dlxigp_ip, const float *xgp,

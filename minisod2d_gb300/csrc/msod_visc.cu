@@ -144,11 +144,18 @@ __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, c
 // arithmetic, which takes as long): porder 4 (64^3) 8 0.597,
 // 4 0.640, 5 0.647, 10 0.756; 5 (51^3) 4 0.605, 7 0.629, 8 0.672, 3 0.696; 6 (40^3) 3
 // 0.549, 4 0.553, 2 0.616; 7 (32^3) 3 0.438, 2 0.476, 4 0.561; 3 (80^3) 8 0.491, 4
-// 0.609; 2 (100^3) 16 0.356, 14 0.373; 1 (128^3) 32 0.251, 16 0.264.
+// 0.609; 2 (100^3) 16 0.356, 14 0.373; 1 (128^3) 32 0.251, 16 0.264.  Without He in
+// shared memory the list's blocks are held by their registers, and few groups
+// share the SMs: porder 4, learned viscosity on 48^3 hexes (8 % of the elements in
+// the list) 218.9 us with 8 elements, 214.4 with 5, 212.2 with 5 in six blocks per
+// SM; their He spans prefetched into L2 216.2.  A bound on the registers gains
+// nothing without a list.
 template <int P, bool LIST>
 struct ViscGroup {
-    static constexpr int ne[8] = {0, 32, 16, 8, 8, 4, 3, 3};
-    using G = GroupGeom<float, P, ne[P]>;
+    static constexpr int ne[8] = {0, 32, 16, 8, 8, 4, 3, 3}, nl[8] = {0, 32, 16, 8, 5, 4, 3, 3};
+    using G = GroupGeom<float, P, LIST ? nl[P] : ne[P]>;
+    // Blocks per SM that the registers are held to (0: the compiler's choice).
+    static constexpr int MINB = LIST && P == 4 ? 6 : 0;
 };
 
 template <class G, bool LIST>
@@ -215,8 +222,8 @@ __device__ __forceinline__ void visc_load(Four<float> (&w)[G::Q], const GroupThr
     for (int s = 0; s < G::Q; ++s) w[s] = W[base + s * G::template step<DIR>()];
 }
 
-template <class G, bool LIST>
-__global__ void __launch_bounds__(G::NT)
+template <class G, bool LIST, int MINB>
+__global__ void __launch_bounds__(G::NT, MINB)
     entropy_visc_kernel(int nelem, int npoin, const int *__restrict__ connec, const float *__restrict__ He,
                         const float *__restrict__ gpvol, const int *__restrict__ inv,
                         const float *__restrict__ dlxigp_ip, const float *__restrict__ rho,
@@ -370,7 +377,7 @@ cudaError_t visc_pl(const ViscArgs &a, cudaStream_t st)
     using G = typename ViscGroup<P, LIST>::G;
     constexpr size_t smem = ViscShared<G, LIST>::kBytes;
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    auto kern = entropy_visc_kernel<G, LIST>;
+    auto kern = entropy_visc_kernel<G, LIST, ViscGroup<P, LIST>::MINB>;
     static std::atomic<unsigned long long> allowed{0};
     const cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
