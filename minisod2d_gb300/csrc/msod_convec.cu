@@ -124,12 +124,13 @@ struct ConvecShared {
     static constexpr size_t kV = kW + G::NREC * sizeof(Four<real>);
     static constexpr size_t kA = kV + G::NREC * sizeof(Four<real>);
     static constexpr bool kSlots = convec_slots<real, G::P>();
-    static constexpr size_t kZ = kA + G::NREC * (kSlots ? sizeof(Two<real>) : sizeof(Four<real>));
-    static constexpr size_t kM = kZ + G::NREC * sizeof(real);
-    static constexpr size_t kNode = kM + G::NREC * sizeof(real);
-    static constexpr size_t kTab = (kNode + (kSlots ? 0 : G::NREC * sizeof(int)) + 15) / 16 * 16;
+    static constexpr size_t kZ = kA + (kSlots ? G::NPR * sizeof(Two<real>) : G::NREC * sizeof(Four<real>));
+    static constexpr size_t kM = kZ + G::NSC * sizeof(real);
+    static constexpr size_t kNode = kM + G::NSC * sizeof(real);
+    static constexpr size_t kTab = (kNode + (kSlots ? 0 : G::NSC * sizeof(int)) + 15) / 16 * 16;
     static constexpr size_t kBytes = kTab + GroupTables<G, true>::kBytes;
     unsigned char *base;
+    int el;  // the thread's element
     __device__ __forceinline__ unsigned long long *bar() const
     {
         return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
@@ -137,9 +138,10 @@ struct ConvecShared {
     __device__ __forceinline__ Four<real> *W() const { return reinterpret_cast<Four<real> *>(base + kW); }  // u, H
     __device__ __forceinline__ Four<real> *V() const { return reinterpret_cast<Four<real> *>(base + kV); }  // q, p
     __device__ __forceinline__ Four<real> *A() const { return reinterpret_cast<Four<real> *>(base + kA); }  // 4 mom, 4 ener
-    __device__ __forceinline__ real *Z() const { return reinterpret_cast<real *>(base + kZ); }              // rho
-    __device__ __forceinline__ real *M() const { return reinterpret_cast<real *>(base + kM); }              // 2 mass
-    __device__ __forceinline__ int *node() const { return reinterpret_cast<int *>(base + kNode); }
+    __device__ __forceinline__ real *Z() const { return reinterpret_cast<real *>(base + kZ) + el * G::SK; }  // rho
+    __device__ __forceinline__ real *M() const { return reinterpret_cast<real *>(base + kM) + el * G::SK; }  // 2 mass
+    __device__ __forceinline__ int *node() const { return reinterpret_cast<int *>(base + kNode) + el * G::SK; }
+    __device__ __forceinline__ Two<real> *A2() const { return reinterpret_cast<Two<real> *>(base + kA) + el * G::HK; }
     // The sums of a point (record o, its He record at he) between the passes.
     // kSlots: the zeta column of a point's He record is read in the zeta pass
     // only, by the thread that owns the point's zeta line; from then on it holds
@@ -147,7 +149,7 @@ struct ConvecShared {
     __device__ __forceinline__ void put(int o, real *he, const Two<real> &a, const Two<real> &b, real m) const
     {
         if constexpr (kSlots) {
-            reinterpret_cast<Two<real> *>(base + kA)[o] = a;
+            A2()[o] = a;
             M()[o] = b.x;
             he[6] = b.y;
             he[7] = m;
@@ -162,7 +164,7 @@ struct ConvecShared {
     __device__ __forceinline__ void add(int o, const real *he, Two<real> &a, Two<real> &b, real &m) const
     {
         if constexpr (kSlots) {
-            a = add2(a, reinterpret_cast<const Two<real> *>(base + kA)[o]);
+            a = add2(a, A2()[o]);
             b = add2(b, two(M()[o], he[6]));
             m += he[7];
         } else {
@@ -420,9 +422,9 @@ __global__ void __launch_bounds__(G::NT, MINB)
     constexpr int Q = G::Q, N = G::N, R = G::R;
     static_assert(G::S <= 2, "one or two segments per line");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const ConvecShared<G> sm{smem_raw};
     const int tid = threadIdx.x;
     const GroupThread<G> t(tid);
+    const ConvecShared<G> sm{smem_raw, t.el};
     const int r0 = t.seg * R;
     const int e0 = blockIdx.x * G::NE;
     const GroupMetric<G> gm(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);

@@ -109,20 +109,25 @@ constexpr long long diffu_const_points()
 
 // Shared memory of a block.  X1 and X3 hold the xi and eta derivatives of
 // (rho, T, u1, u2), then the fluxes (and divergences) of grad rho, tauU, grad T
-// and tau_1; X2 holds the node fields (rho, T, u1, u2), then the fluxes of
-// tau_2, tau_3 (xi, eta).
+// and tau_1; X2 holds the node fields (rho, T, u1, u2), then (Y1, Y3, eight bytes
+// each) the fluxes of tau_2, tau_3: as halves of 16-byte records, which each direction
+// reads and writes alone, they took twice the wavefronts (porder 4 64^3 0.951 / 0.925
+// ms, 5 51^3 0.904 / 0.886, 7 32^3 0.791 / 0.770).  Not at porder 3, whose rows of four
+// conflict as pairs too (80^3 0.718 / 0.733).
 template <class G>
 struct DiffuShared {
     using real = typename G::real;
+    static constexpr bool kPairs = G::P != 3;
     static constexpr size_t k1 = G::HEB + G::GPB + 16;
     static constexpr size_t k2 = k1 + G::NREC * sizeof(Four<real>);
-    static constexpr size_t k3 = k2 + G::NREC * sizeof(Four<real>);
+    static constexpr size_t k3 = k2 + G::NPR * sizeof(Four<real>);
     static constexpr size_t kU = k3 + G::NREC * sizeof(Four<real>);
-    static constexpr size_t kE1 = kU + G::NREC * sizeof(real);
-    static constexpr size_t kE3 = kE1 + G::NREC * sizeof(real);
-    static constexpr size_t kTab = (kE3 + G::NREC * sizeof(real) + 15) / 16 * 16;
+    static constexpr size_t kE1 = kU + G::NSC * sizeof(real);
+    static constexpr size_t kE3 = kE1 + G::NSC * sizeof(real);
+    static constexpr size_t kTab = (kE3 + G::NSC * sizeof(real) + 15) / 16 * 16;
     static constexpr size_t bytes(bool constd) { return kTab + (constd ? 0 : GroupTables<G, false>::kBytes); }
     unsigned char *base;
+    int el;  // the thread's element
     __device__ __forceinline__ unsigned long long *bar() const
     {
         return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
@@ -131,9 +136,43 @@ struct DiffuShared {
     __device__ __forceinline__ Four<real> *X1() const { return reinterpret_cast<Four<real> *>(base + k1); }
     __device__ __forceinline__ Four<real> *X2() const { return reinterpret_cast<Four<real> *>(base + k2); }
     __device__ __forceinline__ Four<real> *X3() const { return reinterpret_cast<Four<real> *>(base + k3); }
-    __device__ __forceinline__ real *U3() const { return reinterpret_cast<real *>(base + kU); }   // u3
-    __device__ __forceinline__ real *E1() const { return reinterpret_cast<real *>(base + kE1); }  // its xi derivative
-    __device__ __forceinline__ real *E3() const { return reinterpret_cast<real *>(base + kE3); }  // its eta derivative
+    // The flux pair (tau_2, tau_3) of record o along xi and eta.
+    __device__ __forceinline__ Two<real> *Y1() const { return reinterpret_cast<Two<real> *>(base + k2) + el * G::HK; }
+    __device__ __forceinline__ Two<real> *Y3() const { return Y1() + G::NPR; }
+    template <int DIR>
+    __device__ __forceinline__ Two<real> &pair(int o) const
+    {
+        if constexpr (kPairs)
+            return (DIR == 0 ? Y1() : Y3())[o];
+        else
+            return DIR == 0 ? X2()[o].a : X2()[o].b;
+    }
+    __device__ __forceinline__ void put_pairs(int o, const Two<real> &xi, const Two<real> &eta) const
+    {
+        if constexpr (kPairs) {
+            Y1()[o] = xi;
+            Y3()[o] = eta;
+        } else {
+            Four<real> s;
+            s.a = xi;
+            s.b = eta;
+            X2()[o] = s;
+        }
+    }
+    __device__ __forceinline__ Four<real> pairs(int o) const
+    {
+        if constexpr (kPairs) {
+            Four<real> s;
+            s.a = Y1()[o];
+            s.b = Y3()[o];
+            return s;
+        } else {
+            return X2()[o];
+        }
+    }
+    __device__ __forceinline__ real *U3() const { return reinterpret_cast<real *>(base + kU) + el * G::SK; }   // u3
+    __device__ __forceinline__ real *E1() const { return reinterpret_cast<real *>(base + kE1) + el * G::SK; }  // its xi derivative
+    __device__ __forceinline__ real *E3() const { return reinterpret_cast<real *>(base + kE3) + el * G::SK; }  // its eta derivative
 };
 
 // Derivatives of the five fields along the thread's line in direction DIR.
@@ -185,9 +224,8 @@ __device__ __forceinline__ void diffu_div(const GroupThread<G> &t, const DiffuSh
 #pragma unroll
     for (int c = 0; c < Q; ++c) {
         const int o = base + c * G::template step<DIR>();
-        const Four<real> *x2 = sm.X2() + o;
         f[c] = X[o];
-        f2[c] = DIR == 0 ? x2->a : x2->b;
+        f2[c] = sm.template pair<DIR>(o);
     }
     real D[Q][Q];
 #pragma unroll
@@ -205,9 +243,8 @@ __device__ __forceinline__ void diffu_div(const GroupThread<G> &t, const DiffuSh
             s2 = fma2(Dc, f2[c], s2);
         }
         const int o = base + r * G::template step<DIR>();
-        Four<real> *x2 = sm.X2() + o;
         X[o] = s;
-        (DIR == 0 ? x2->a : x2->b) = s2;
+        sm.template pair<DIR>(o) = s2;
     }
 }
 
@@ -227,9 +264,9 @@ __global__ void __launch_bounds__(G::NT, MINB)
     using R2 = Two<real>;
     constexpr int Q = G::Q;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const DiffuShared<G> sm{smem_raw};
     const int tid = threadIdx.x, e0 = blockIdx.x * G::NE;
     const GroupThread<G> t(tid);
+    const DiffuShared<G> sm{smem_raw, t.el};
     const GroupMetric<G> gm(smem_raw, smem_raw + G::HEB, sm.bar(), He, gpvol, e0, nelem, tid);
     const int e = e0 + t.el, base = t.rec0(2);
     const bool in = t.active && e < nelem;
@@ -356,9 +393,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
             s.a = F[1][0];
             s.b = F[1][1];
             sm.X3()[o] = s;
-            s.a = F[0][2];
-            s.b = F[1][2];
-            sm.X2()[o] = s;
+            sm.put_pairs(o, F[0][2], F[1][2]);
 #pragma unroll
             for (int rr = 0; rr < Q; ++rr) {
                 const real D = Dr[rr];
@@ -380,7 +415,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
     for (int k = 0; k < Q; ++k) {
         if (id[k] < 0) continue;
         const int o = base + k * G::template step<2>();
-        const Four<real> x1 = sm.X1()[o], x2 = sm.X2()[o], x3 = sm.X3()[o];
+        const Four<real> x1 = sm.X1()[o], x2 = sm.pairs(o), x3 = sm.X3()[o];
         const R2 s0 = add2(add2(acc[k][0], x1.a), x3.a), s1 = add2(add2(acc[k][1], x1.b), x3.b),
                  s2 = add2(add2(acc[k][2], x2.a), x2.b);
         red_add(Rmass + id[k], nu[k] * s0.x);

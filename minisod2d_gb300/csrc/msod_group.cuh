@@ -102,6 +102,35 @@ constexpr GroupPitch group_pitch(int P, int NE)
     return {RP, Q * RP, Q * Q * RP, false};
 }
 
+// Arrays of 4-byte (8-byte) numbers per record are kept at a pitch per element of
+// that many numbers more than the records', which are placed for 16-byte
+// accesses: fewest conflicts over the three directions (wavefronts per warp and
+// direction without / with: 4-byte porder 5, 4 elements 3.0 / 1.3, 6, 2 elements 2.0
+// / 1.5, 7 2.0 / 1.3, 8 1.8 / 1.3, 2, 16 elements 1.8 / 1.0; 8-byte 5 3.6 / 2.0, 7
+// 4.0 / 2.0).  Without / with, ms: convection porder 7 32^3 0.781 / 0.767, 6 40^3 1.060 /
+// 1.053, 5 51^3 1.130 / 1.128; diffusion 7 0.770 / 0.763, 2 100^3 0.564 / 0.558;
+// estimator 2 0.375 / 0.349.  Groups that are not listed gain nothing (porder 4, 5
+// elements: 2.3 / 2.0) or lose (the estimator at porder 6, 3 elements, 0.484 / 0.491).
+constexpr int group_pad4(int P, int NE)
+{
+    switch (P * 100 + NE) {
+    case 216: return 3;
+    case 504: return 10;
+    case 602: return 20;
+    case 702: return 4;
+    case 802: return 20;
+    default: return 0;
+    }
+}
+constexpr int group_pad8(int P, int NE)
+{
+    switch (P * 100 + NE) {
+    case 504: return 6;
+    case 702: return 12;
+    default: return 0;
+    }
+}
+
 // Q points per line, L lines per direction, N points per element, NE elements
 // per block, S threads per line (each owns R consecutive points; the split is
 // by warp, so that a warp's code and coefficients are uniform).
@@ -116,6 +145,9 @@ struct GroupGeom {
     static constexpr int RP = PITCH.row, PP = PITCH.plane, ES = PITCH.elem;
     static constexpr bool SWAP = PITCH.swap;
     static constexpr int NREC = NE * ES;
+    // Numbers per array of scalars (pairs) and their element pitch beyond ES.
+    static constexpr int SK = sizeof(real) == 4 ? group_pad4(P, NE) : 0, NSC = NREC + NE * SK;
+    static constexpr int HK = sizeof(real) == 4 ? group_pad8(P, NE) : 0, NPR = NREC + NE * HK;
     static constexpr int LT = ((NE * L + 31) / 32) * 32;  // threads of one segment
     static constexpr int NT = S * LT;
     // Pitch of an element's He and gpvol in shared memory.  Where an element's

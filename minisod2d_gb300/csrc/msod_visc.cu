@@ -162,17 +162,18 @@ template <class G, bool LIST>
 struct ViscShared {
     static constexpr size_t kHe = LIST ? 0 : G::HEB + G::GPB + 16;
     static constexpr size_t kR = kHe + G::NREC * sizeof(Four<float>);
-    static constexpr size_t kV = kR + G::NREC * sizeof(float);
+    static constexpr size_t kV = kR + G::NSC * sizeof(float);
     static constexpr size_t kEl = kV + (size_t)G::NE * G::L * sizeof(float);  // per element: max speed, max |R|, nu
     static constexpr size_t kTab = (kEl + 3 * (size_t)G::NE * sizeof(float) + 15) / 16 * 16;
     static constexpr size_t kBytes = kTab + GroupTables<G, false>::kBytes;
     unsigned char *base;
+    int el;  // the thread's element
     __device__ __forceinline__ unsigned long long *bar() const
     {
         return reinterpret_cast<unsigned long long *>(base + G::HEB + G::GPB);
     }
     __device__ __forceinline__ Four<float> *W() const { return reinterpret_cast<Four<float> *>(base + kHe); }  // u, eta
-    __device__ __forceinline__ float *R() const { return reinterpret_cast<float *>(base + kR); }
+    __device__ __forceinline__ float *R() const { return reinterpret_cast<float *>(base + kR) + el * G::SK; }
     __device__ __forceinline__ float *vol() const { return reinterpret_cast<float *>(base + kV); }  // line sums
     __device__ __forceinline__ int *speed() const { return reinterpret_cast<int *>(base + kEl); }
     __device__ __forceinline__ unsigned *res() const { return reinterpret_cast<unsigned *>(speed() + G::NE); }
@@ -234,9 +235,9 @@ __global__ void __launch_bounds__(G::NT, MINB)
 {
     constexpr int Q = G::Q, N = G::N, NE = G::NE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const ViscShared<G, LIST> sm{smem_raw};
     const int tid = threadIdx.x;
     const GroupThread<G> t(tid);
+    const ViscShared<G, LIST> sm{smem_raw, t.el};
     // The block's elements: e0 .. e0+NE-1 (one group per block), or in list mode
     // the entries e0 .. of the compacted list, the blocks striding over the
     // list's groups; -1 beyond the end.
