@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
         convec_pass<G>(ln, t, ip, sm, tab, gm, id, npoin, Rmass, Rmom, Rener);
         if (ip < 2 && __syncthreads_or(!ok)) {
             if (tid == 0) report_wait_fault(tabs);
+            grid_dependency_wait();  // the kernel never ends ahead of the zeroing
             return false;
         }
         return true;

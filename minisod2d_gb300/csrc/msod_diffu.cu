@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
     const bool ok = gm.wait(sm.bar());
     if (__syncthreads_or(!ok)) {
         if (tid == 0) report_wait_fault(tabs);
+        grid_dependency_wait();  // the kernel never ends ahead of the zeroing
         return;
     }
     // Zeta stage: acc[r][0..2] = the zeta divergence at point r of the fluxes of

@@ -348,7 +348,8 @@ __global__ void __launch_bounds__(G::NT, MINB)
         __syncthreads();
         if (tid < NE) {
             const int ee = element(tid);
-            const float neta = normalise ? entropy_norm(&st->norm) : 1.0f;
+            // Waits for the statistics in any case: the kernel never ends ahead of them.
+            const float norm = entropy_norm(&st->norm), neta = normalise ? norm : 1.0f;
             float v = 0.0f;
             for (int l = 0; l < G::L; ++l) v += sm.vol()[l * NE + tid];
             const float h = cbrtf(v) / (float)(Q - 1);

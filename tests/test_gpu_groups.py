@@ -104,3 +104,23 @@ def test_large_meshes_as_small_ones(cuda, P):
     for a, b in zip(large, small):
         err = torch.linalg.vector_norm((a - b).double()) / torch.linalg.vector_norm(b.double().expand_as(a))
         assert float(err) <= 1e-6, (P, float(err))
+
+
+@pytest.mark.parametrize("P,nx", [(4, 12), (2, 5)])
+def test_estimator_without_normalisation(cuda, P, nx):
+    """normalise = 0 takes n_eta = 1, so nu = min(nu_max, nu_E n_eta) of the normalised call: nu_E scales by
+    the same factor in every element that nu_max does not cap (two float roundings of the ratio)."""
+    import torch
+
+    from minisod2d_gb300 import capi, learn, workload
+
+    dev = workload.DeviceCase(workload.HostCase(workload.custom(P, nx, 0.05)))
+    nu = [torch.empty(dev.nelem, device=cuda) for _ in range(2)]
+    cap = torch.empty(dev.nelem, device=cuda)
+    for norm in (1, 0):  # ce small: no element is capped
+        capi.call("msod_entropy_viscosity", *learn._geo(dev), *(learn._p(t) for t in (dev.rho, dev.u, dev.pr)), 1.4,
+                  1e-6, 0.5, norm, None, learn._p(nu[norm]), learn._p(cap), capi.current_stream())
+    live = (nu[0] < 0.9 * cap) & (nu[1] < 0.9 * cap) & (nu[1] > 0)
+    assert int(live.sum()) > dev.nelem // 2
+    ratio = (nu[0][live].double() / nu[1][live].double())
+    assert float((ratio / ratio.median() - 1).abs().max()) < 5e-7
