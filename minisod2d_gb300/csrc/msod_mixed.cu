@@ -156,7 +156,7 @@ struct MixedGeom {
     static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
-    static constexpr size_t half_bytes = (size_t)2 * kNF * PB + plane_guard_bytes<Q>();
+    static constexpr size_t half_bytes = (size_t)2 * kNF * PB;
     static constexpr size_t smem = half_bytes + (size_t)(NBASE + NACC) * NP * sizeof(float) +
                                    (size_t)2 * NP * sizeof(int) + (2 * 32 + 4) * sizeof(float);
     // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
@@ -356,8 +356,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedGeom<P, BF16>::MINB)
                 gp[s] = ldg(gpvol + (size_t)e * N + sPerm[lat[s]]);
             }
         }
-        const unsigned char *rowp =
-            sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
+        const unsigned char *rowp = sHalf + plane_off + operand_row<Q>(d, warp, r8);
 #pragma unroll
         for (int f = 0; f < kNF; f += 2) {
             const unsigned char *src = rowp + 2 * f * G::PB - (f + 1 < kNF ? 0 : alone);

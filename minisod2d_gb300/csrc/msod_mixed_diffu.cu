@@ -59,7 +59,7 @@ struct MixedDiffuGeom {
     static_assert(NTASK <= NT, "one task per thread");
     static constexpr int BITS = BF16 ? 8 : 11;
     static constexpr int PB = plane_bytes<Q>();  // bytes of one field half
-    static constexpr size_t half_bytes = (size_t)2 * kNFX * PB + plane_guard_bytes<Q>();
+    static constexpr size_t half_bytes = (size_t)2 * kNFX * PB;
     static constexpr size_t smem = half_bytes + (size_t)(3 * kNG + 2) * NP * sizeof(float) +
                                    (size_t)2 * NP * sizeof(int) + (3 * 32 + 8) * sizeof(float);
     // Blocks per SM that shared memory allows, as long as a thread keeps kMixedRegs registers.
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
         for (int d = 0; d < 3; ++d) {
             const unsigned bh = d == 0 ? Bgh[0] : (d == 1 ? Bgh[1] : Bgh[2]);
             const unsigned bl = d == 0 ? Bgl[0] : (d == 1 ? Bgl[1] : Bgl[2]);
-            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
+            const unsigned char *rowp = sHalf + plane_off + operand_row<Q>(d, warp, r8);
             int lat[2];
 #pragma unroll
             for (int s = 0; s < 2; ++s) lat[s] = pass_point<Q>(d, s, g, tq, warp);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(32 * (P + 1), MixedDiffuGeom<P, BF16>::MINB)
         for (int d = 0; d < 3; ++d) {
             const unsigned bh = d == 0 ? Bdh[0] : (d == 1 ? Bdh[1] : Bdh[2]);
             const unsigned bl = d == 0 ? Bdl[0] : (d == 1 ? Bdl[1] : Bdl[2]);
-            const unsigned char *rowp = sHalf + plane_off + (d == 2 ? row_pos(r8, warp) : row_pos(warp, r8)) * kRowB;
+            const unsigned char *rowp = sHalf + plane_off + operand_row<Q>(d, warp, r8);
             int lat[2];
             float acc[2][kNX];
 #pragma unroll

@@ -28,9 +28,6 @@ constexpr int mixed_blocks(size_t smem, int threads, int regs)
 constexpr int kRowB = 16;  // bytes per half-plane row: 8 halves along i
 
 // One field half of an element: 8 rows per k-plane of the element, 8 Q rows.
-// The transposed (zeta) reads of input points beyond Q, which meet zero
-// coefficients, reach up to row 63: past the last plane they land in a zero
-// guard of (64 - 8 Q) rows.
 // Measured against 8 x 8-row planes for every order (48^3 hexes): porder-5
 // convection 5.24 -> 4.04 ms and porder-4 diffusion 2.78 -> 2.27 ms (more
 // blocks per SM), the other kernels unchanged (0 selects the full planes).
@@ -41,11 +38,6 @@ template <int Q>
 constexpr int plane_bytes()
 {
     return (MIXED_TRIM_PLANES ? 8 * Q : 64) * kRowB;
-}
-template <int Q>
-constexpr int plane_guard_bytes()
-{
-    return (MIXED_TRIM_PLANES ? 64 - 8 * Q : 0) * kRowB;
 }
 
 // gmsh node of lattice point l = (K Q + J) Q + I, and the 1-D derivative matrices
@@ -100,6 +92,19 @@ __device__ __forceinline__ int pass_point(int d, int s, int g, int tq, int o)
 // Row (k, j) of a half plane sits at position 8k + (j xor k): the eight rows
 // of every ldmatrix phase fall on distinct banks for xi, eta and zeta lines.
 __device__ __forceinline__ int row_pos(int k, int j) { return 8 * k + (j ^ k); }
+
+// Byte offset in a half plane of row r8 of the A operand of direction d, tile w:
+// for xi and eta lines row j = r8 of k-plane w, for zeta lines row j = w of k-plane
+// r8.  There is no k-plane beyond Q: those zeta rows, which meet zero coefficients,
+// are the rows beyond Q of k-plane w, which nothing writes after they are zeroed.
+// They must be zero, not only finite elsewhere: a row of another field, or one that
+// an earlier element left behind, can hold an infinity or a NaN, and zero times that
+// is a NaN.  Same banks as row_pos(r8, w): the eight rows of a phase stay distinct.
+template <int Q>
+__device__ __forceinline__ int operand_row(int d, int w, int r8)
+{
+    return (d == 2 && r8 < Q ? row_pos(r8, w) : row_pos(w, r8)) * kRowB;
+}
 
 template <bool BF16>
 __device__ __forceinline__ unsigned pack2(float a, float b)
