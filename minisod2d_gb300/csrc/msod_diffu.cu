@@ -437,14 +437,20 @@ cudaError_t launch_diffu_pc(const DiffuArgs<real> &a, TableScratch *tabs, cudaSt
     static std::atomic<unsigned long long> allowed{0};
     cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
+    const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
     if constexpr (CONSTD) {
         err = launch_table_prep(P, a, tabs, st);
         if (err == cudaSuccess)
             err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, sizeof(float) * 3 * G::Q * G::Q,
                                           sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
         if (err != cudaSuccess) return err;
+        // An ordinary launch: the kernel reads c_Df from its first pass on, and only its
+        // reductions wait (launch_after).
+        kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK, a.dlxigp_ip, tabs,
+                                        a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
+                                        a.Rmass, a.Rmom, a.Rener);
+        return cudaGetLastError();
     }
-    const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
     return launch_after(kern, grid, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK,
                         a.dlxigp_ip, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
                         a.Rmass, a.Rmom, a.Rener);

@@ -82,7 +82,9 @@ inline cudaError_t allow_smem(std::atomic<unsigned long long> &done, Kernel kern
 
 // Launches kern so that its blocks may start before the kernel ahead of it on
 // the stream has finished (programmatic dependent launch); kern calls
-// grid_dependency_wait() before it touches what that kernel writes.
+// grid_dependency_wait() before it touches what that kernel writes.  Only right
+// behind a kernel: what kern reads earlier has to be complete before that kernel
+// starts, which a copy queued in between is not.
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
                                 A... args)
