@@ -1,4 +1,4 @@
-// msod_diffu.cu -- plain (FP32 / FP64) hex GLL diffusion residual.
+// msod_diffu.cu -- plain FP32 hex GLL diffusion residual (FP64: msod_diffu64.cu).
 //
 // Computes what full_diffusion_ijk computes (elem_diffu.f90:10-197):
 //   pass 1 (per point b): grad rho, grad T, grad u; mu_f = mu_fluid + rho mu_sgs;
@@ -69,38 +69,35 @@ enum { VISC_MU_E = 0, VISC_NU_ELEM = 1 };
 // Whole warps of lines (5 x 25 lines at porder 4: 125 of 128 threads) count
 // most, then the L1 that the blocks' shared memory leaves for the gathers'
 // lines in flight (porder 5: three blocks of 65.6 KB, within a 196 KB carveout,
-// 1.00 ms on 51^3; of 67.7 KB, beyond it, 1.37).  The FP64 kernels, bound by
-// FP64 issue, which a warp pays for its idle lanes too, take the same groups.
-// FP32, ms: porder 4 (64^3) 5 elements at three blocks 1.030, at four (128
+// 1.00 ms on 51^3; of 67.7 KB, beyond it, 1.37).  ms: porder 4 (64^3) 5 elements at three blocks 1.030, at four (128
 // registers, spills) 1.077; before the divisions left the point work, 8
 // elements at two blocks took 1.302, 9 1.284, 4 at four 1.236, where 5 took
 // 1.152.  Porder 5 (51^3) 3 elements at three 0.996, 4 at two 1.053; 6 (40^3) 3
 // 1.094, 2 at two 1.156; 7 (32^3) 2 at two 0.853; 8 (26^3) 1 0.717; 3 (80^3) 8 at
 // the compiler's choice 0.779, at four 0.795; 2 (100^3) 16 at four 0.619, at the
 // compiler's choice 0.717.
-template <typename real, int P>
+template <int P>
 constexpr int diffu_ne()
 {
-    constexpr int nf[9] = {0, 32, 16, 8, 5, 3, 3, 2, 1}, nd[9] = {0, 32, 14, 8, 5, 3, 2, 1, 1};
-    return sizeof(real) == 4 ? nf[P] : nd[P];
+    constexpr int n[9] = {0, 32, 16, 8, 5, 3, 3, 2, 1};
+    return n[P];
 }
-template <typename real, int P>
+template <int P>
 constexpr int diffu_minb()
 {
-    constexpr int nb[9] = {0, 1, 4, 1, 3, 3, 1, 2, 1};
-    return sizeof(real) == 4 ? nb[P] : 1;
+    constexpr int n[9] = {0, 1, 4, 1, 3, 3, 1, 2, 1};
+    return n[P];
 }
-template <typename real, int P>
-using DiffuGeom = GroupGeom<real, P, diffu_ne<real, P>()>;
+template <int P>
+using DiffuGeom = GroupGeom<float, P, diffu_ne<P>()>;
 
-// Element points from which the FP32 kernel takes its matrices from the constant
+// Element points from which the kernel takes its matrices from the constant
 // bank.  That saves it registers and shared-memory loads, and at porders 5 and 6
 // the L1 that the tables' shared memory costs (ms, bank / shared memory: porder
 // 5 51^3 0.996 / 1.327, 6 40^3 1.094 / 1.405, 4 64^3 1.030 / 1.046, 3 80^3 0.779 /
 // 0.854, 2 100^3 0.619 / 0.680, 1 128^3 0.392 / 0.425, 7 32^3 0.853 / 0.882, 8 26^3
 // 0.717 / 0.754), but costs the call the table kernel and a copy to the bank,
-// ~6 us: the lines below are where the two meet.  FP64 stays with shared memory
-// (porder 4 20^3 0.650 against 0.798).
+// ~6 us: the lines below are where the two meet.
 template <int P>
 constexpr long long diffu_const_points()
 {
@@ -427,13 +424,13 @@ __global__ void __launch_bounds__(G::NT, MINB)
     }
 }
 
-template <typename real, int P, int VISC, bool CONSTD>
-cudaError_t launch_diffu_pc(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
+template <int P, int VISC, bool CONSTD>
+cudaError_t launch_diffu_pc(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
 {
-    using G = DiffuGeom<real, P>;
+    using G = DiffuGeom<P>;
     constexpr size_t smem = DiffuShared<G>::bytes(CONSTD);
     static_assert(smem <= 227 * 1024, "shared memory budget");
-    auto kern = diffu_kernel<G, VISC, diffu_minb<real, P>(), CONSTD>;
+    auto kern = diffu_kernel<G, VISC, diffu_minb<P>(), CONSTD>;
     static std::atomic<unsigned long long> allowed{0};
     cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
@@ -455,41 +452,35 @@ cudaError_t launch_diffu_pc(const DiffuArgs<real> &a, TableScratch *tabs, cudaSt
                         a.dlxigp_ip, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
                         a.Rmass, a.Rmom, a.Rener);
 }
-template <typename real, int P, int VISC>
-cudaError_t launch_diffu_pn(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
+template <int P, int VISC>
+cudaError_t launch_diffu_pn(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
 {
-    if constexpr (sizeof(real) == 4)
-        if ((long long)a.nelem * DiffuGeom<real, P>::N >= diffu_const_points<P>())
-            return launch_diffu_pc<real, P, VISC, true>(a, tabs, st);
-    return launch_diffu_pc<real, P, VISC, false>(a, tabs, st);
+    return (long long)a.nelem * DiffuGeom<P>::N >= diffu_const_points<P>() ? launch_diffu_pc<P, VISC, true>(a, tabs, st)
+                                                                           : launch_diffu_pc<P, VISC, false>(a, tabs, st);
 }
 
-template <typename real, int P>
-cudaError_t launch_diffu_p(const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
+template <int P>
+cudaError_t launch_diffu_p(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
 {
-    if (a.nu_elem) return launch_diffu_pn<real, P, VISC_NU_ELEM>(a, tabs, st);
-    return launch_diffu_pn<real, P, VISC_MU_E>(a, tabs, st);
+    return a.nu_elem ? launch_diffu_pn<P, VISC_NU_ELEM>(a, tabs, st) : launch_diffu_pn<P, VISC_MU_E>(a, tabs, st);
 }
 
 }  // namespace
 
-template <typename real>
-cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st)
+template <>
+cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
 {
     switch (porder) {
-    case 1: return launch_diffu_p<real, 1>(a, tabs, st);
-    case 2: return launch_diffu_p<real, 2>(a, tabs, st);
-    case 3: return launch_diffu_p<real, 3>(a, tabs, st);
-    case 4: return launch_diffu_p<real, 4>(a, tabs, st);
-    case 5: return launch_diffu_p<real, 5>(a, tabs, st);
-    case 6: return launch_diffu_p<real, 6>(a, tabs, st);
-    case 7: return launch_diffu_p<real, 7>(a, tabs, st);
-    case 8: return launch_diffu_p<real, 8>(a, tabs, st);
+    case 1: return launch_diffu_p<1>(a, tabs, st);
+    case 2: return launch_diffu_p<2>(a, tabs, st);
+    case 3: return launch_diffu_p<3>(a, tabs, st);
+    case 4: return launch_diffu_p<4>(a, tabs, st);
+    case 5: return launch_diffu_p<5>(a, tabs, st);
+    case 6: return launch_diffu_p<6>(a, tabs, st);
+    case 7: return launch_diffu_p<7>(a, tabs, st);
+    case 8: return launch_diffu_p<8>(a, tabs, st);
     default: return cudaErrorInvalidValue;
     }
 }
-
-template cudaError_t launch_diffu_plain<float>(int, const DiffuArgs<float> &, TableScratch *, cudaStream_t);
-template cudaError_t launch_diffu_plain<double>(int, const DiffuArgs<double> &, TableScratch *, cudaStream_t);
 
 }  // namespace msod

@@ -111,6 +111,10 @@ template <typename real>
 cudaError_t launch_convec_plain(int porder, const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
 template <typename real>
 cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st);
+template <>
+cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st);
+template <>  // msod_diffu64.cu
+cudaError_t launch_diffu_plain<double>(int porder, const DiffuArgs<double> &a, TableScratch *tabs, cudaStream_t st);
 // Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by
 // launch_zero just before).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
 struct MixedConvecArgs : ElementArgs<float> {
