@@ -89,7 +89,7 @@ constexpr int diffu_minb()
     return n[P];
 }
 template <int P>
-using DiffuGeom = GroupGeom<float, P, diffu_ne<P>()>;
+using DiffuGeom = GroupGeom<float, P, diffu_ne<P>(), 1, P == 1>;
 
 // Element points from which the kernel takes its matrices from the constant
 // bank.  That saves it registers and shared-memory loads, and at porders 5 and 6

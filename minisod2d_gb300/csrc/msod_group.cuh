@@ -10,7 +10,12 @@
 //     meshes numbered along x the same local node of consecutive elements, for
 //     neighbouring local nodes, fills whole sectors: a gather or reduction of
 //     a node field touches 1-3 cache lines per warp, where lanes that run over
-//     one element's lattice touch seven or eight;
+//     one element's lattice touch seven or eight.  At porders 1 and 2, whose
+//     warps hold only a line or two of each element, they run along xi ahead of
+//     the elements, so that the nodes of an xi line, neighbours in most
+//     numberings, share sectors whatever the order of the elements (12 M element
+//     points, porder 1, elements first / xi first: convection 0.221 / 0.187 ms,
+//     elements in random order 1.57 / 1.03);
 //   * He and gpvol of a group are contiguous (He(3,3,ngaus,nelem)): one bulk
 //     copy each brings them to shared memory.  Read by the line threads from
 //     global memory, a point's three He values cost one L1 tag lookup per lane
@@ -78,10 +83,11 @@ struct GroupPitch {
     int row, plane, elem;
     bool swap;
 };
-constexpr GroupPitch group_pitch(int P, int NE)
+constexpr GroupPitch group_pitch(int P, int NE, bool ifirst)
 {
+    if (ifirst && P == 2) return {3, 9, 27, true};
     switch (P * 100 + NE) {
-    case 132: return {2, 4, 9, false};
+    case 132: return {2, 5, 10, true};
     case 308: return {4, 16, 67, false};
     case 405: return {5, 25, 125, true};
     case 409: return {5, 25, 129, true};
@@ -106,15 +112,15 @@ constexpr GroupPitch group_pitch(int P, int NE)
 // that many numbers more than the records', which are placed for 16-byte
 // accesses: fewest conflicts over the three directions (wavefronts per warp and
 // direction without / with: 4-byte porder 5, 4 elements 3.0 / 1.3, 6, 2 elements 2.0
-// / 1.5, 7 2.0 / 1.3, 8 1.8 / 1.3, 2, 16 elements 1.8 / 1.0; 8-byte 5 3.6 / 2.0, 7
-// 4.0 / 2.0).  Without / with, ms: convection porder 7 32^3 0.781 / 0.767, 6 40^3 1.060 /
+// / 1.5, 7 2.0 / 1.3, 8 1.8 / 1.3, 2, 16 elements (elements
+// first) 1.8 / 1.0; 8-byte 5 3.6 / 2.0, 7 4.0 / 2.0).  Without / with, ms: convection porder 7 32^3 0.781 / 0.767, 6 40^3 1.060 /
 // 1.053, 5 51^3 1.130 / 1.128; diffusion 7 0.770 / 0.763, 2 100^3 0.564 / 0.558;
 // estimator 2 0.375 / 0.349.  Groups that are not listed gain nothing (porder 4, 5
 // elements: 2.3 / 2.0) or lose (the estimator at porder 6, 3 elements, 0.484 / 0.491).
-constexpr int group_pad4(int P, int NE)
+constexpr int group_pad4(int P, int NE, bool ifirst)
 {
     switch (P * 100 + NE) {
-    case 216: return 3;
+    case 216: return ifirst ? 0 : 3;
     case 504: return 10;
     case 602: return 20;
     case 702: return 4;
@@ -133,20 +139,22 @@ constexpr int group_pad8(int P, int NE)
 
 // Q points per line, L lines per direction, N points per element, NE elements
 // per block, S threads per line (each owns R consecutive points; the split is
-// by warp, so that a warp's code and coefficients are uniform).
-template <typename real_t, int P_, int NE_, int S_ = 1>
+// by warp, so that a warp's code and coefficients are uniform).  IFIRST: lanes
+// along xi ahead of the elements.
+template <typename real_t, int P_, int NE_, int S_ = 1, bool IF_ = (P_ <= 2)>
 struct GroupGeom {
     using real = real_t;
     static constexpr int P = P_, NE = NE_, S = S_;
     static constexpr int Q = P + 1, L = Q * Q, N = Q * Q * Q;
     static constexpr int R = (Q + S - 1) / S;
     // Record of point (I, J, K) of element el: I + RP J + PP K + ES el.
-    static constexpr GroupPitch PITCH = group_pitch(P, NE);
+    static constexpr GroupPitch PITCH = group_pitch(P, NE, IF_);
     static constexpr int RP = PITCH.row, PP = PITCH.plane, ES = PITCH.elem;
     static constexpr bool SWAP = PITCH.swap;
-    static constexpr int NREC = NE * ES;
+    static constexpr int NREC = (NE - 1) * ES + P * (1 + RP + PP) + 1;
+    static constexpr bool IFIRST = IF_;
     // Numbers per array of scalars (pairs) and their element pitch beyond ES.
-    static constexpr int SK = sizeof(real) == 4 ? group_pad4(P, NE) : 0, NSC = NREC + NE * SK;
+    static constexpr int SK = sizeof(real) == 4 ? group_pad4(P, NE, IF_) : 0, NSC = NREC + NE * SK;
     static constexpr int HK = sizeof(real) == 4 ? group_pad8(P, NE) : 0, NPR = NREC + NE * HK;
     static constexpr int LT = ((NE * L + 31) / 32) * 32;  // threads of one segment
     static constexpr int NT = S * LT;
@@ -180,10 +188,17 @@ struct GroupThread {
         seg = G::S == 1 ? 0 : tid / G::LT;
         const int t = tid - seg * G::LT;
         active = t < G::NE * G::L;
-        const int line = active ? t / G::NE : 0;
-        el = active ? t - line * G::NE : 0;
-        q1 = line / G::Q;
-        q0 = line - q1 * G::Q;
+        if constexpr (G::IFIRST) {
+            const int row = active ? t / G::Q : 0;
+            q0 = active ? t - row * G::Q : 0;
+            q1 = row / G::NE;
+            el = row - q1 * G::NE;
+        } else {
+            const int line = active ? t / G::NE : 0;
+            el = active ? t - line * G::NE : 0;
+            q1 = line / G::Q;
+            q0 = line - q1 * G::Q;
+        }
     }
     // Record of the line's first point and its lattice index (K Q + J) Q + I.
     __device__ __forceinline__ int rec0(int dir) const
