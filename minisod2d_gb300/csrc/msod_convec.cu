@@ -107,11 +107,24 @@ constexpr bool convec_rolled()
 }
 // Sums kept in the spent part of the He records (ConvecShared::kSlots): where
 // it makes room for another block (porder 7: 0.786 / 0.860; porder 5 1.143 /
-// 1.155); elsewhere the records' bank conflicts cost more than the room gives.
+// 1.155) or, at porder 3, for 60 instead of 28 KB of L1 beside four blocks (12 M element
+// points, numbered along x 0.256 / 0.258, nodes in random order 1.61 / 2.38, elements in
+// random order 0.752 / 1.015); elsewhere the records' bank conflicts cost more than the
+// room gives.
 template <typename real, int P>
 constexpr bool convec_slots()
 {
-    return sizeof(real) == 4 && (P == 5 || P == 7);
+    return sizeof(real) == 4 && (P == 3 || P == 5 || P == 7);
+}
+// Shared memory that an SM should keep for the blocks (percent, -1: as many blocks as
+// fit).  Porder 1 would take seven blocks in 228 KB and leave 28 KB of L1, where the cache
+// lines of the gathers in flight no longer fit: six in 196 KB take 0.203 instead of 0.187
+// ms on a mesh numbered along x, but 0.557 instead of 0.880 with nodes in random order and
+// 0.574 instead of 1.025 with elements in random order (12 M element points).
+template <typename real, int P>
+constexpr int convec_carveout()
+{
+    return sizeof(real) == 4 && P == 1 ? 80 : -1;
 }
 template <typename real, int P>
 using ConvecGeom = GroupGeom<real, P, convec_ne<real, P>(), convec_s<real, P>()>;
@@ -510,7 +523,7 @@ cudaError_t launch_convec_p(const ConvecArgs<real> &a, const TableScratch *tabs,
     if (!tabs) return cudaErrorInvalidValue;
     auto kern = convec_kernel<G, convec_minb<real, P>()>;
     static std::atomic<unsigned long long> allowed{0};
-    const cudaError_t err = allow_smem(allowed, kern, smem);
+    const cudaError_t err = allow_smem(allowed, kern, smem, convec_carveout<real, P>());
     if (err != cudaSuccess) return err;
     const unsigned ngroups = (unsigned)((a.nelem + G::NE - 1) / G::NE);
     return launch_after(kern, ngroups, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.u, a.q, a.rho,

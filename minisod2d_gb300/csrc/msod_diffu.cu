@@ -88,8 +88,23 @@ constexpr int diffu_minb()
     constexpr int n[9] = {0, 1, 4, 1, 3, 3, 1, 2, 1};
     return n[P];
 }
+// Where a few KB less let the blocks of an SM fit in 196 KB, which leaves 60 KB of L1
+// instead of 28: the eta derivative of u3 is written over u3 (a barrier more), and at
+// porders 3 and 7 the points' gpvol come straight from global memory.  On 12 M element
+// points, staged / so, ms: porder 6 0.588 / 0.461 (gpvol too 0.480), 7 0.594 / 0.480, 3
+// 0.284 / 0.276; with elements in random order 0.938 / 0.726, 0.824 / 0.662, 0.802 / 0.644.
 template <int P>
-using DiffuGeom = GroupGeom<float, P, diffu_ne<P>(), 1, P == 1>;
+constexpr bool diffu_over()
+{
+    return P == 3 || P == 6 || P == 7;
+}
+template <int P>
+constexpr bool diffu_gpvol_staged()
+{
+    return P != 3 && P != 7;
+}
+template <int P>
+using DiffuGeom = GroupGeom<float, P, diffu_ne<P>(), 1, P == 1, diffu_gpvol_staged<P>()>;
 
 // Element points from which the kernel takes its matrices from the constant
 // bank.  That saves it registers and shared-memory loads, and at porders 5 and 6
@@ -120,8 +135,9 @@ struct DiffuShared {
     static constexpr size_t k3 = k2 + G::NPR * sizeof(Four<real>);
     static constexpr size_t kU = k3 + G::NREC * sizeof(Four<real>);
     static constexpr size_t kE1 = kU + G::NSC * sizeof(real);
-    static constexpr size_t kE3 = kE1 + G::NSC * sizeof(real);
-    static constexpr size_t kTab = (kE3 + G::NSC * sizeof(real) + 15) / 16 * 16;
+    static constexpr bool kOver = diffu_over<G::P>();
+    static constexpr size_t kE3 = kOver ? kU : kE1 + G::NSC * sizeof(real);
+    static constexpr size_t kTab = ((kOver ? kE1 : kE3) + G::NSC * sizeof(real) + 15) / 16 * 16;
     static constexpr size_t bytes(bool constd) { return kTab + (constd ? 0 : GroupTables<G, false>::kBytes); }
     unsigned char *base;
     int el;  // the thread's element
@@ -281,6 +297,10 @@ __global__ void __launch_bounds__(G::NT, MINB)
         id[k] = (unsigned)v < (unsigned)npoin ? v : -1;
     }
     if (!CONSTD) sm.tab().build(inv, dlxigp_ip, tid);
+    real gvr[G::GPSTAGED ? 1 : Q];
+    if constexpr (!G::GPSTAGED)
+#pragma unroll
+        for (int k = 0; k < Q; ++k) gvr[k] = in ? ldg_once(gpvol + (size_t)e * G::N + pt[k]) : (real)0;
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const bool ok = id[k] >= 0;
@@ -308,10 +328,9 @@ __global__ void __launch_bounds__(G::NT, MINB)
         }
     __syncthreads();
     const DiffuRows<G, CONSTD> tab(sm.tab());
-    if (t.active) {
-        diffu_grad<G, 0, CONSTD>(t, sm, tab);
-        diffu_grad<G, 1, CONSTD>(t, sm, tab);
-    }
+    if (t.active) diffu_grad<G, 0, CONSTD>(t, sm, tab);
+    if constexpr (DiffuShared<G>::kOver) __syncthreads();
+    if (t.active) diffu_grad<G, 1, CONSTD>(t, sm, tab);
     // Bounded wait for the bulk copies; a wait that ran out is reported and
     // nothing is assembled.
     const bool ok = gm.wait(sm.bar());
@@ -339,7 +358,11 @@ __global__ void __launch_bounds__(G::NT, MINB)
             const real *hp = gm.he(t.el, pt[c]);
 #pragma unroll
             for (int j = 0; j < 9; ++j) H[j] = hp[j];
-            const real gv = *gm.vol(t.el, pt[c]);
+            real gv;
+            if constexpr (G::GPSTAGED)
+                gv = *gm.vol(t.el, pt[c]);
+            else
+                gv = gvr[c];
             const Four<real> gx = sm.X1()[o], ge = sm.X3()[o];
             R2 za = two((real)0, (real)0), zb = za;
             real z3 = (real)0;

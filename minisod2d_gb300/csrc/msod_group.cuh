@@ -16,6 +16,10 @@
 //     numberings, share sectors whatever the order of the elements (12 M element
 //     points, porder 1, elements first / xi first: convection 0.221 / 0.187 ms,
 //     elements in random order 1.57 / 1.03);
+//   * on other numberings the gathers touch more lines (elements with nodes of their own,
+//     porder 4: twelve), and what counts is that the lines in flight fit in the
+//     L1 beside the blocks' shared memory (the choices by the L1's size in the
+//     kernels);
 //   * He and gpvol of a group are contiguous (He(3,3,ngaus,nelem)): one bulk
 //     copy each brings them to shared memory.  Read by the line threads from
 //     global memory, a point's three He values cost one L1 tag lookup per lane
@@ -140,8 +144,8 @@ constexpr int group_pad8(int P, int NE)
 // Q points per line, L lines per direction, N points per element, NE elements
 // per block, S threads per line (each owns R consecutive points; the split is
 // by warp, so that a warp's code and coefficients are uniform).  IFIRST: lanes
-// along xi ahead of the elements.
-template <typename real_t, int P_, int NE_, int S_ = 1, bool IF_ = (P_ <= 2)>
+// along xi ahead of the elements.  GPSTAGED: gpvol in shared memory too.
+template <typename real_t, int P_, int NE_, int S_ = 1, bool IF_ = (P_ <= 2), bool GP_ = true>
 struct GroupGeom {
     using real = real_t;
     static constexpr int P = P_, NE = NE_, S = S_;
@@ -168,7 +172,8 @@ struct GroupGeom {
     static constexpr int pitch(int n) { return SPLIT ? n + (BANKS + OFF - n % BANKS) % BANKS : n; }
     static constexpr int HEP = pitch(9 * N), GPP = pitch(N);
     static constexpr size_t HEB = STAGED ? ((size_t)NE * HEP * sizeof(real) + 31) / 16 * 16 : 0;
-    static constexpr size_t GPB = STAGED ? ((size_t)NE * GPP * sizeof(real) + 31) / 16 * 16 : 0;
+    static constexpr bool GPSTAGED = STAGED && GP_;
+    static constexpr size_t GPB = GPSTAGED ? ((size_t)NE * GPP * sizeof(real) + 31) / 16 * 16 : 0;
     template <int DIR>
     static constexpr int step()
     {
@@ -238,7 +243,7 @@ struct GroupMetric {
     }
     __device__ __forceinline__ const real *vol(int el, int a) const
     {
-        return gp + (G::STAGED ? el : min(el, last)) * G::GPP + a;
+        return gp + (G::GPSTAGED ? el * G::GPP : min(el, last) * G::N) + a;
     }
     // Bounded wait for the bulk copies (false: the limit ran out).
     __device__ __forceinline__ bool wait(unsigned long long *bar) const { return G::STAGED ? mbar_wait(bar, 0) : true; }
@@ -264,23 +269,23 @@ struct GroupMetric {
             const SpanPlan ph(gHe + off * 9, n * 9 * sizeof(real)), pg(ggp + off, n * sizeof(real));
             if (tid == 0) {
                 mbar_init(bar, 1);
-                mbar_arrive_expect_tx(bar, (unsigned)spans * (ph.bulk + pg.bulk));
+                mbar_arrive_expect_tx(bar, (unsigned)spans * (ph.bulk + (G::GPSTAGED ? pg.bulk : 0u)));
             }
             __syncwarp();
             if (tid < spans) {
                 ph.issue(hs + (size_t)k * G::HEP * sizeof(real), bar);
-                pg.issue(gs + (size_t)k * G::GPP * sizeof(real), bar);
+                if (G::GPSTAGED) pg.issue(gs + (size_t)k * G::GPP * sizeof(real), bar);
             }
             if (ph.head + ph.tail + pg.head + pg.tail != 0)
                 for (int s = 0; s < spans; ++s) {
                     const size_t o = ((size_t)e0 + s) * G::N;
                     const SpanPlan qh(gHe + o * 9, n * 9 * sizeof(real)), qg(ggp + o, n * sizeof(real));
                     if (tid >= 8 && tid < 14) qh.plain(hs + (size_t)s * G::HEP * sizeof(real), tid - 8);
-                    if (tid >= 16 && tid < 22) qg.plain(gs + (size_t)s * G::GPP * sizeof(real), tid - 16);
+                    if (G::GPSTAGED && tid >= 16 && tid < 22) qg.plain(gs + (size_t)s * G::GPP * sizeof(real), tid - 16);
                 }
         }
         He = reinterpret_cast<real *>(hs + hsh);
-        gp = reinterpret_cast<const real *>(gs + gsh);
+        gp = G::GPSTAGED ? reinterpret_cast<const real *>(gs + gsh) : ggp + (size_t)e0 * G::N;
     }
 };
 

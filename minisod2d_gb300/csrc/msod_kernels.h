@@ -66,9 +66,10 @@ struct ZeroSpans {
 cudaError_t launch_zero(const ZeroSpans &z, cudaStream_t st);
 
 // Allows kern `smem` bytes of dynamic shared memory on the current device, once
-// per device and kernel (done: one bit per device, owned by the kernel's launcher).
+// per device and kernel (done: one bit per device, owned by the kernel's launcher),
+// and asks for `carveout` percent of an SM's memory for its blocks (-1: no wish).
 template <typename Kernel>
-inline cudaError_t allow_smem(std::atomic<unsigned long long> &done, Kernel kern, size_t smem)
+inline cudaError_t allow_smem(std::atomic<unsigned long long> &done, Kernel kern, size_t smem, int carveout = -1)
 {
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -76,6 +77,8 @@ inline cudaError_t allow_smem(std::atomic<unsigned long long> &done, Kernel kern
     const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
     if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err == cudaSuccess && carveout >= 0)
+        err = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
     if (err == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return err;
 }

@@ -156,6 +156,12 @@ struct ViscGroup {
     using G = GroupGeom<float, P, LIST ? nl[P] : ne[P]>;
     // Blocks per SM that the registers are held to (0: the compiler's choice).
     static constexpr int MINB = LIST && P == 4 ? 6 : 0;
+    // Shared memory that an SM should keep for the blocks (percent, -1: as many blocks
+    // as fit).  Beyond 196 KB 28 KB of L1 are left, too few for the cache lines of the
+    // gathers in flight: one block less (porder 5) takes 0.248 instead of 0.253 ms on a
+    // mesh numbered along x and 0.59 instead of 1.21 with nodes in random order, porder 1
+    // 0.148 / 0.146 and 0.22 / 0.34, 3 0.185 / 0.172 and 0.48 / 0.89 (12 M element points).
+    static constexpr int CARVEOUT = LIST ? -1 : (P == 1 || P == 3 ? 80 : (P == 5 ? 65 : -1));
 };
 
 template <class G, bool LIST>
@@ -381,7 +387,7 @@ cudaError_t visc_pl(const ViscArgs &a, cudaStream_t st)
     static_assert(smem <= 227 * 1024, "shared memory budget");
     auto kern = entropy_visc_kernel<G, LIST, ViscGroup<P, LIST>::MINB>;
     static std::atomic<unsigned long long> allowed{0};
-    const cudaError_t err = allow_smem(allowed, kern, smem);
+    const cudaError_t err = allow_smem(allowed, kern, smem, ViscGroup<P, LIST>::CARVEOUT);
     if (err != cudaSuccess) return err;
     // List mode: resident blocks stride over the list (its length is known on
     // the device only); otherwise one group per block.
