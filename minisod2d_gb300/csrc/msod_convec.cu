@@ -116,6 +116,16 @@ constexpr bool convec_slots()
 {
     return sizeof(real) == 4 && (P == 3 || P == 5 || P == 7);
 }
+// Blocks of closely numbered elements gather through the L1 (group_close): on 12 M
+// element points in elements with nodes of their own, past it / through it, ms: porder 1
+// 0.345 / 0.299, 2 0.425 / 0.329, 3 0.576 / 0.402; on a mesh numbered along x it costs
+// nothing there.  From porder 4 up it would gain as much (4 0.541 / 0.424), but costs up to 1 %
+// on the mesh numbered along x.
+template <typename real, int P>
+constexpr bool convec_close()
+{
+    return sizeof(real) == 4 && P <= 3;
+}
 // Shared memory that an SM should keep for the blocks (percent, -1: as many blocks as
 // fit).  Porder 1 would take seven blocks in 228 KB and leave 28 KB of L1, where the cache
 // lines of the gathers in flight no longer fit: six in 196 KB take 0.203 instead of 0.187
@@ -455,20 +465,26 @@ __global__ void __launch_bounds__(G::NT, MINB)
         }
         sm.tab().build(inv, dlxigp_ip, tid);
         real f[R][9];
+        auto gather = [&](auto load) {
 #pragma unroll
-        for (int k = 0; k < R; ++k) {
-            const bool ok = id[k] >= 0;  // a missing node reads as zeros
-            const size_t p = ok ? (size_t)id[k] : 0;
-            f[k][0] = ok ? ldg_once(u + p) : (real)0;
-            f[k][1] = ok ? ldg_once(u + np + p) : (real)0;
-            f[k][2] = ok ? ldg_once(u + 2 * np + p) : (real)0;
-            f[k][3] = ok ? ldg_once(E + p) : (real)0;
-            f[k][4] = ok ? ldg_once(q + p) : (real)0;
-            f[k][5] = ok ? ldg_once(q + np + p) : (real)0;
-            f[k][6] = ok ? ldg_once(q + 2 * np + p) : (real)0;
-            f[k][7] = ok ? ldg_once(rho + p) : (real)0;
-            f[k][8] = ok ? ldg_once(pr + p) : (real)0;
-        }
+            for (int k = 0; k < R; ++k) {
+                const bool ok = id[k] >= 0;  // a missing node reads as zeros
+                const size_t p = ok ? (size_t)id[k] : 0;
+                f[k][0] = ok ? load(u + p) : (real)0;
+                f[k][1] = ok ? load(u + np + p) : (real)0;
+                f[k][2] = ok ? load(u + 2 * np + p) : (real)0;
+                f[k][3] = ok ? load(E + p) : (real)0;
+                f[k][4] = ok ? load(q + p) : (real)0;
+                f[k][5] = ok ? load(q + np + p) : (real)0;
+                f[k][6] = ok ? load(q + 2 * np + p) : (real)0;
+                f[k][7] = ok ? load(rho + p) : (real)0;
+                f[k][8] = ok ? load(pr + p) : (real)0;
+            }
+        };
+        if (convec_close<real, G::P>() && group_close<G>(id))
+            gather([](const real *x) { return ldg(x); });
+        else
+            gather([](const real *x) { return ldg_once(x); });
         const int base = t.rec0(2);
 #pragma unroll
         for (int k = 0; k < R; ++k) {

@@ -103,6 +103,17 @@ constexpr bool diffu_gpvol_staged()
 {
     return P != 3 && P != 7;
 }
+// Blocks of closely numbered elements gather through the L1 (group_close).  On 12 M
+// element points in elements with nodes of their own, past it / through it, ms: porder 3
+// 0.473 / 0.410, 4 0.523 / 0.420, 6 0.835 / 0.533 (with the smaller shared memory); on a
+// mesh numbered along x the rule costs nothing there (3 0.281 / 0.276, 4 0.364 / 0.349),
+// at the others it costs 1-6 % (7 0.480 / 0.489) and the former line form, for which
+// lanes ran along an element's lattice, was not faster (5 0.580, 7 0.785, 8 0.973).
+template <int P>
+constexpr bool diffu_close()
+{
+    return P == 3 || P == 4 || P == 6;
+}
 template <int P>
 using DiffuGeom = GroupGeom<float, P, diffu_ne<P>(), 1, P == 1, diffu_gpvol_staged<P>()>;
 
@@ -301,17 +312,35 @@ __global__ void __launch_bounds__(G::NT, MINB)
     if constexpr (!G::GPSTAGED)
 #pragma unroll
         for (int k = 0; k < Q; ++k) gvr[k] = in ? ldg_once(gpvol + (size_t)e * G::N + pt[k]) : (real)0;
+    // mu_sgs and mu_e ahead of the node fields, or between them: as measured (porder 4
+    // 0.349 against 0.370 ms, 3 0.286 / 0.301; but 5 0.414 / 0.394, 8 0.599 / 0.576).
+    constexpr bool kEarly = G::P == 3 || G::P == 4;
+    if constexpr (kEarly)
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const bool ok = id[k] >= 0;
-        const size_t p = ok ? (size_t)id[k] : 0, i = in ? (size_t)pt[k] * nelem + e : 0;
-        rT[k] = two(ok ? ldg_once(rho + p) : (real)0, ok ? ldg_once(Tem + p) : (real)0);
-        u12[k] = two(ok ? ldg_once(u + p) : (real)0, ok ? ldg_once(u + np + p) : (real)0);
-        u3[k] = ok ? ldg_once(u + 2 * np + p) : (real)0;
-        muf[k] = ok ? ldg_once(mu_fluid + p) : (real)0;
-        ms[k] = in ? ldg_once(mu_sgs + i) : (real)0;
-        me[k] = (VISC == VISC_MU_E && in) ? ldg_once(mu_e + i) : (real)0;
-    }
+        for (int k = 0; k < Q; ++k) {
+            const size_t i = in ? (size_t)pt[k] * nelem + e : 0;
+            ms[k] = in ? ldg_once(mu_sgs + i) : (real)0;
+            me[k] = (VISC == VISC_MU_E && in) ? ldg_once(mu_e + i) : (real)0;
+        }
+    auto gather = [&](auto load) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const bool ok = id[k] >= 0;
+            const size_t p = ok ? (size_t)id[k] : 0, i = in ? (size_t)pt[k] * nelem + e : 0;
+            rT[k] = two(ok ? load(rho + p) : (real)0, ok ? load(Tem + p) : (real)0);
+            u12[k] = two(ok ? load(u + p) : (real)0, ok ? load(u + np + p) : (real)0);
+            u3[k] = ok ? load(u + 2 * np + p) : (real)0;
+            muf[k] = ok ? load(mu_fluid + p) : (real)0;
+            if constexpr (!kEarly) {
+                ms[k] = in ? ldg_once(mu_sgs + i) : (real)0;
+                me[k] = (VISC == VISC_MU_E && in) ? ldg_once(mu_e + i) : (real)0;
+            }
+        }
+    };
+    if (diffu_close<G::P>() && group_close<G>(id))
+        gather([](const real *x) { return ldg(x); });
+    else
+        gather([](const real *x) { return ldg_once(x); });
     if (VISC == VISC_NU_ELEM) {
         const real nu = in ? ldg(nu_elem + e) : (real)0;
 #pragma unroll

@@ -18,8 +18,8 @@
 //     elements in random order 1.57 / 1.03);
 //   * on other numberings the gathers touch more lines (elements with nodes of their own,
 //     porder 4: twelve), and what counts is that the lines in flight fit in the
-//     L1 beside the blocks' shared memory (the choices by the L1's size in the
-//     kernels);
+//     L1 beside the blocks' shared memory (group_close, and the choices by the L1's size in
+//     the kernels);
 //   * He and gpvol of a group are contiguous (He(3,3,ngaus,nelem)): one bulk
 //     copy each brings them to shared memory.  Read by the line threads from
 //     global memory, a point's three He values cost one L1 tag lookup per lane
@@ -225,6 +225,17 @@ struct GroupThread {
         return lat0(DIR) + r * (DIR == 0 ? 1 : (DIR == 1 ? G::Q : G::L));
     }
 };
+
+// Whether the warp's elements number their nodes closely (within an element's number
+// of nodes along zeta), as a mesh of elements with nodes of their own does.  The lines of
+// such an element share few cache lines, which one warp load after the other comes back
+// to: they are then gathered through the L1, others past it (ldg_once).
+template <class G>
+__device__ __forceinline__ bool group_close(const int (&id)[G::R])
+{
+    static_assert(G::R > 1, "two points of a line");
+    return __all_sync(0xffffffffu, abs(id[1] - id[0]) < G::N);
+}
 
 // Bulk copies of a group's He and gpvol spans into shared memory (one
 // mbarrier phase), a span per lane of the first warp; the unaligned ends, if
