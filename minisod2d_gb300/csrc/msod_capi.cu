@@ -303,18 +303,19 @@ int msod_init(int device)
 int msod_finalize(void)
 {
     std::lock_guard<std::mutex> lk(g_mu);
-    int cur = 0;
-    cudaGetDevice(&cur);
-    for (int d = 0; d < 64; ++d)
-        if (g_flags[d] || g_tables[d]) {
-            cudaSetDevice(d);
-            if (g_flags[d]) cudaFree(g_flags[d]);
-            if (g_tables[d]) cudaFree(g_tables[d]);
-            g_flags[d] = nullptr;
-            g_tables[d] = nullptr;
-        }
-    cudaSetDevice(cur);
+    {
+        DeviceScope scope;
+        for (int d = 0; d < 64; ++d)
+            if (g_flags[d] || g_tables[d]) {
+                scope.select(d);
+                if (g_flags[d]) cudaFree(g_flags[d]);
+                if (g_tables[d]) cudaFree(g_tables[d]);
+                g_flags[d] = nullptr;
+                g_tables[d] = nullptr;
+            }
+    }
     mode_release();
+    learn_release();
     return MSOD_OK;
 }
 

@@ -20,7 +20,29 @@ bool checked_mode();
 // The form chosen by msod_set_mode (msod_mode.cu).
 bool mode_is_default_convec();
 bool mode_is_default_diffusion();
+// msod_finalize's share of the mode's and the estimators' buffers.
 void mode_release();
+void learn_release();
+#ifdef __CUDACC__
+// Selects devices for a while.  A device that is current already is not selected
+// again: cudaSetDevice would replace the caller's context on it by the primary one.
+class DeviceScope {
+    int home_ = 0, now_ = 0;
+
+public:
+    DeviceScope()
+    {
+        cudaGetDevice(&home_);
+        now_ = home_;
+    }
+    ~DeviceScope() { select(home_); }
+    void select(int device)
+    {
+        if (device != now_) cudaSetDevice(device);
+        now_ = device;
+    }
+};
+#endif
 // Convection + diffusion residual in one set of arrays (the default form of both
 // calls; msod_convec_diffusion_ijk's arguments and checks otherwise).
 int residual_sum(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,

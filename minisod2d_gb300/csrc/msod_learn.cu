@@ -106,6 +106,19 @@ struct Rng {
 };
 
 }  // namespace
+
+void learn_release()
+{
+    std::lock_guard<std::mutex> lk(g_mu);
+    DeviceScope scope;
+    for (int d = 0; d < 64; ++d)
+        for (Slot &s : g_slots[d])
+            if (s.p) {
+                scope.select(d);
+                cudaFree(s.p);
+                s = Slot{};
+            }
+}
 }  // namespace msod
 
 using namespace msod;

@@ -132,17 +132,15 @@ bool mode_is_default_diffusion() { return g_prec.load() == MSOD_PREC_FP32 && g_m
 void mode_release()
 {
     std::lock_guard<std::mutex> lk(g_buf_mu);
-    int cur = 0;
-    cudaGetDevice(&cur);
+    DeviceScope scope;
     for (int d = 0; d < 64; ++d)
         for (int s = 0; s < NBUF; ++s)
             if (g_buf[d][s]) {
-                cudaSetDevice(d);
+                scope.select(d);
                 cudaFree(g_buf[d][s]);
                 g_buf[d][s] = nullptr;
                 g_buf_size[d][s] = 0;
             }
-    cudaSetDevice(cur);
 }
 
 int mode_convec(int porder, int nelem, int npoin, const int *connec, const float *He, const float *gpvol,
