@@ -204,14 +204,14 @@ static int diffu_impl(int porder, int nelem, int npoin, const int *connec, const
     }
     TableScratch *tabs = device_tables(porder);
     if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
-    rc = zero_outputs(Rmass, Rmom, Rener, npoin, st);
-    if (rc) return rc;
     DiffuArgs<real> a;
     a.nelem = nelem; a.npoin = npoin; a.connec = connec; a.He = He; a.gpvol = gpvol; a.dlxigp_ip = dlx;
     a.invAtoIJK = inv; a.Cp = Cp; a.Pr = Pr;
     a.rho = rho; a.u = u; a.Tem = Tem; a.mu_fluid = mu_fluid; a.mu_e = mu_e; a.mu_sgs = mu_sgs; a.nu_elem = nu_elem;
     a.Rmass = Rmass; a.Rmom = Rmom; a.Rener = Rener;
-    rc = cuda_status(launch_diffu_plain<real>(porder, a, tabs, st), "diffusion kernel launch");
+    rc = cuda_status(prepare_diffu_plain<real>(porder, a, tabs, st), "derivative matrices of the diffusion");
+    if (!rc) rc = zero_outputs(Rmass, Rmom, Rener, npoin, st);
+    if (!rc) rc = cuda_status(launch_diffu_plain<real>(porder, a, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "diffusion kernel");
     return rc;
 }
@@ -243,11 +243,6 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     }
     TableScratch *tabs = device_tables(porder);
     if (!tabs) return set_error(MSOD_ERR_CUDA, "could not allocate the element-table area");
-    ZeroSpans z;
-    add_outputs(z, Rmass_c, Rmom_c, Rener_c, npoin);
-    if (!joint) add_outputs(z, Rmass_d, Rmom_d, Rener_d, npoin);
-    rc = cuda_status(launch_zero(z, st), "residual zeroing launch");
-    if (rc) return rc;
     ConvecArgs<float> c;
     c.nelem = nelem; c.npoin = npoin; c.connec = connec; c.He = He; c.gpvol = gpvol; c.dlxigp_ip = dlx;
     c.invAtoIJK = inv;
@@ -256,7 +251,12 @@ static int both_impl(int porder, int nelem, int npoin, const int *connec, const 
     static_cast<ElementArgs<float> &>(d) = c;
     d.Cp = Cp; d.Pr = Pr; d.rho = rho; d.u = u; d.Tem = Tem; d.mu_fluid = mu_fluid; d.mu_e = mu_e;
     d.mu_sgs = mu_sgs; d.nu_elem = nullptr; d.Rmass = Rmass_d; d.Rmom = Rmom_d; d.Rener = Rener_d;
-    rc = cuda_status(launch_convec_plain<float>(porder, c, tabs, st), "convection kernel launch");
+    ZeroSpans z;
+    add_outputs(z, Rmass_c, Rmom_c, Rener_c, npoin);
+    if (!joint) add_outputs(z, Rmass_d, Rmom_d, Rener_d, npoin);
+    rc = cuda_status(prepare_diffu_plain<float>(porder, d, tabs, st), "derivative matrices of the diffusion");
+    if (!rc) rc = cuda_status(launch_zero(z, st), "residual zeroing launch");
+    if (!rc) rc = cuda_status(launch_convec_plain<float>(porder, c, tabs, st), "convection kernel launch");
     if (!rc) rc = cuda_status(launch_diffu_plain<float>(porder, d, tabs, st), "diffusion kernel launch");
     if (!rc && checked_mode()) rc = check_wait_fault(tabs, st, "convection + diffusion kernel");
     return rc;

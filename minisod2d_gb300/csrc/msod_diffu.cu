@@ -40,7 +40,7 @@ namespace msod {
 namespace {
 
 // 1-D derivative matrices of the current call, per porder (large meshes: copied
-// from the per-call table area before the launch).
+// from the per-call table area by prepare_diffu_plain, ahead of the zeroing).
 __constant__ float c_Df[MSOD_MAX_PORDER + 1][kTableDMax];
 
 // The matrices' rows: shared-memory tables of the block, or (CONSTD) operands
@@ -476,43 +476,48 @@ __global__ void __launch_bounds__(G::NT, MINB)
     }
 }
 
+// Whether the call reads its matrices from the constant bank.
+template <int P>
+bool diffu_const(const DiffuArgs<float> &a)
+{
+    return (long long)a.nelem * DiffuGeom<P>::N >= diffu_const_points<P>();
+}
+
+template <int P>
+cudaError_t prepare_diffu_p(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+{
+    if (!diffu_const<P>(a)) return cudaSuccess;
+    const cudaError_t err = launch_table_prep(P, a, tabs, st);
+    if (err != cudaSuccess) return err;
+    constexpr size_t row = sizeof(float) * kTableDMax;
+    return cudaMemcpyToSymbolAsync(c_Df, tabs->Df, sizeof(float) * 3 * (P + 1) * (P + 1), row * P,
+                                   cudaMemcpyDeviceToDevice, st);
+}
+
 template <int P, int VISC, bool CONSTD>
-cudaError_t launch_diffu_pc(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_diffu_pc(const DiffuArgs<float> &a, const TableScratch *tabs, cudaStream_t st)
 {
     using G = DiffuGeom<P>;
     constexpr size_t smem = DiffuShared<G>::bytes(CONSTD);
     static_assert(smem <= 227 * 1024, "shared memory budget");
     auto kern = diffu_kernel<G, VISC, diffu_minb<P>(), CONSTD>;
     static std::atomic<unsigned long long> allowed{0};
-    cudaError_t err = allow_smem(allowed, kern, smem);
+    const cudaError_t err = allow_smem(allowed, kern, smem);
     if (err != cudaSuccess) return err;
     const unsigned grid = (unsigned)((a.nelem + G::NE - 1) / G::NE);
-    if constexpr (CONSTD) {
-        err = launch_table_prep(P, a, tabs, st);
-        if (err == cudaSuccess)
-            err = cudaMemcpyToSymbolAsync(c_Df, tabs->Df, sizeof(float) * 3 * G::Q * G::Q,
-                                          sizeof(float) * kTableDMax * P, cudaMemcpyDeviceToDevice, st);
-        if (err != cudaSuccess) return err;
-        // An ordinary launch: the kernel reads c_Df from its first pass on, and only its
-        // reductions wait (launch_after).
-        kern<<<grid, G::NT, smem, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK, a.dlxigp_ip, tabs,
-                                        a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
-                                        a.Rmass, a.Rmom, a.Rener);
-        return cudaGetLastError();
-    }
     return launch_after(kern, grid, G::NT, smem, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK,
                         a.dlxigp_ip, tabs, a.Cp, a.Pr, a.rho, a.u, a.Tem, a.mu_fluid, a.mu_e, a.mu_sgs, a.nu_elem,
                         a.Rmass, a.Rmom, a.Rener);
 }
 template <int P, int VISC>
-cudaError_t launch_diffu_pn(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_diffu_pn(const DiffuArgs<float> &a, const TableScratch *tabs, cudaStream_t st)
 {
-    return (long long)a.nelem * DiffuGeom<P>::N >= diffu_const_points<P>() ? launch_diffu_pc<P, VISC, true>(a, tabs, st)
-                                                                           : launch_diffu_pc<P, VISC, false>(a, tabs, st);
+    return diffu_const<P>(a) ? launch_diffu_pc<P, VISC, true>(a, tabs, st)
+                             : launch_diffu_pc<P, VISC, false>(a, tabs, st);
 }
 
 template <int P>
-cudaError_t launch_diffu_p(const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+cudaError_t launch_diffu_p(const DiffuArgs<float> &a, const TableScratch *tabs, cudaStream_t st)
 {
     return a.nu_elem ? launch_diffu_pn<P, VISC_NU_ELEM>(a, tabs, st) : launch_diffu_pn<P, VISC_MU_E>(a, tabs, st);
 }
@@ -520,7 +525,23 @@ cudaError_t launch_diffu_p(const DiffuArgs<float> &a, TableScratch *tabs, cudaSt
 }  // namespace
 
 template <>
-cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+cudaError_t prepare_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st)
+{
+    switch (porder) {
+    case 1: return prepare_diffu_p<1>(a, tabs, st);
+    case 2: return prepare_diffu_p<2>(a, tabs, st);
+    case 3: return prepare_diffu_p<3>(a, tabs, st);
+    case 4: return prepare_diffu_p<4>(a, tabs, st);
+    case 5: return prepare_diffu_p<5>(a, tabs, st);
+    case 6: return prepare_diffu_p<6>(a, tabs, st);
+    case 7: return prepare_diffu_p<7>(a, tabs, st);
+    case 8: return prepare_diffu_p<8>(a, tabs, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <>
+cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, const TableScratch *tabs, cudaStream_t st)
 {
     switch (porder) {
     case 1: return launch_diffu_p<1>(a, tabs, st);

@@ -184,7 +184,13 @@ cudaError_t launch_diffu64(const DiffuArgs<double> &a, cudaStream_t st)
 }  // namespace
 
 template <>
-cudaError_t launch_diffu_plain<double>(int porder, const DiffuArgs<double> &a, TableScratch *, cudaStream_t st)
+cudaError_t prepare_diffu_plain<double>(int, const DiffuArgs<double> &, TableScratch *, cudaStream_t)
+{
+    return cudaSuccess;
+}
+
+template <>
+cudaError_t launch_diffu_plain<double>(int porder, const DiffuArgs<double> &a, const TableScratch *, cudaStream_t st)
 {
     switch (porder) {
     case 1: return launch_diffu64<1>(a, st);

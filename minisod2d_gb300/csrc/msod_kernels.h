@@ -112,12 +112,22 @@ cudaError_t launch_table_prep(int porder, const ElementArgs<float> &a, TableScra
 // stream; tabs: where a bounded wait that ran out is recorded).
 template <typename real>
 cudaError_t launch_convec_plain(int porder, const ConvecArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
+// Diffusion: prepare_diffu_plain first, ahead of the kernel that launch_diffu_plain's
+// follows on the stream (the zeroing, or the convection behind it): the matrices of a
+// call that reads them from the constant bank are then complete when that kernel starts.
 template <typename real>
-cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st);
+cudaError_t prepare_diffu_plain(int porder, const DiffuArgs<real> &a, TableScratch *tabs, cudaStream_t st);
+template <typename real>
+cudaError_t launch_diffu_plain(int porder, const DiffuArgs<real> &a, const TableScratch *tabs, cudaStream_t st);
 template <>
-cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st);
+cudaError_t prepare_diffu_plain<float>(int porder, const DiffuArgs<float> &a, TableScratch *tabs, cudaStream_t st);
+template <>
+cudaError_t launch_diffu_plain<float>(int porder, const DiffuArgs<float> &a, const TableScratch *tabs, cudaStream_t st);
 template <>  // msod_diffu64.cu
-cudaError_t launch_diffu_plain<double>(int porder, const DiffuArgs<double> &a, TableScratch *tabs, cudaStream_t st);
+cudaError_t prepare_diffu_plain<double>(int porder, const DiffuArgs<double> &a, TableScratch *tabs, cudaStream_t st);
+template <>
+cudaError_t launch_diffu_plain<double>(int porder, const DiffuArgs<double> &a, const TableScratch *tabs,
+                                       cudaStream_t st);
 // Mixed-precision convection: FP32 fields, FP64 residuals (zeroed by
 // launch_zero just before).  precision: MSOD_PREC_FP16 or MSOD_PREC_BF16.
 struct MixedConvecArgs : ElementArgs<float> {

@@ -30,7 +30,7 @@ class Copies:
         f = lambda k: up((1.0 + 0.3 * rng.random(k * self.npn)).astype(np.float32))
         base = dict(con=up(connec), He=up(He), gp=up(gp), rho=f(1), Tem=f(1), mu=f(1), u=f(3) - 1.15,
                     me=up(rng.random(self.ne * self.n).astype(np.float32)), ms=up(rng.random(self.ne * self.n).astype(np.float32)),
-                    nu=up(rng.random(self.ne).astype(np.float32)))
+                    nu=up(rng.random(self.ne).astype(np.float32)), pr=f(1), E=f(1), q=f(3) - 1.15)
         self.tab = [[up(x[k]) for k in ("dlxigp_ip", "invAtoIJK", "AtoI", "AtoJ", "AtoK")]
                     for x in (_tables(P, False), _tables(P, True))]
         self.case = {}
@@ -38,7 +38,7 @@ class Copies:
             rep = lambda x, lead: x.view(lead, 1, -1).expand(lead, copies, -1).reshape(-1).contiguous()
             c = base["con"].view(self.n, 1, self.ne) + (torch.arange(copies, device=cuda, dtype=torch.int32)
                                                         * self.npn).view(1, -1, 1)
-            lead = dict(He=1, gp=1, rho=1, Tem=1, mu=1, u=3, me=self.n, ms=self.n, nu=1)
+            lead = dict(He=1, gp=1, rho=1, Tem=1, mu=1, u=3, me=self.n, ms=self.n, nu=1, pr=1, E=1, q=3)
             d = {k: rep(base[k], v) for k, v in lead.items()}
             d.update(con=c.reshape(-1).contiguous(), copies=copies)
             self.case[copies > 1] = d
@@ -62,6 +62,13 @@ class Copies:
         else:
             kernels.full_diffusion_ijk(ne, npn, d["con"], None, None, d["He"], d["gp"], t[0], None, *t[1:], 1004.5, 0.71,
                                        d["rho"], d["u"], d["Tem"], d["mu"], d["me"], d["ms"], *out)
+
+    def both(self, large, odd, out):
+        """Convection and diffusion in one call."""
+        d, t = self.case[large], self.tab[odd]
+        kernels.full_convec_diffusion_ijk(self.ne * d["copies"], self.npn * d["copies"], d["con"], None, None, d["He"],
+                                          d["gp"], t[0], None, *t[1:], 1004.5, 0.71, d["u"], d["q"], d["rho"], d["pr"],
+                                          d["E"], d["Tem"], d["mu"], d["me"], d["ms"], *out)
 
     def check(self, large, small, what):
         import torch
@@ -121,3 +128,21 @@ def test_bank_in_a_graph(cuda, P):
         torch.cuda.synchronize()
         for k in (0, 1):
             m.check(large[k], small[k], ("replay", odd, k))
+
+
+@pytest.mark.parametrize("P", [1, 4, 5, 7])
+def test_one_call_with_other_tables_back_to_back(cuda, P):
+    import torch
+
+    m = Copies(cuda, P)
+    small = [m.outputs(False) + m.outputs(False) for _ in range(2)]
+    for odd in (0, 1):
+        m.both(False, odd, small[odd])
+    order = [0, 1, 0, 1]
+    large = [m.outputs(True) + m.outputs(True) for _ in order]
+    torch.cuda.synchronize()
+    for odd, out in zip(order, large):
+        m.both(True, odd, out)
+    for odd, out in zip(order, large):
+        m.check(out[:3], small[odd][:3], ("convection", odd))
+        m.check(out[3:], small[odd][3:], ("diffusion", odd))

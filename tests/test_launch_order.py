@@ -50,3 +50,13 @@ def test_finder():
 @pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))))
 def test_no_copy_ahead_of_an_early_start(name):
     assert not _faults(code_only(open(os.path.join(CSRC, name)).read())), name
+
+
+def test_matrices_ahead_of_the_zeroing():
+    code = code_only(open(os.path.join(CSRC, "msod_capi.cu")).read())
+    calls = [b for b in FUNCTION.findall(code) if "launch_diffu_plain" in b]
+    assert calls
+    for body in calls:
+        prepare = body.index("prepare_diffu_plain")
+        zero = re.search(r"\b(launch_zero|zero_outputs)\(", body).start()
+        assert prepare < zero < body.index("launch_diffu_plain")
