@@ -266,11 +266,25 @@ __global__ void __launch_bounds__(32 * feat_warps<P>(), feat_minb<P>())
     if (numax_out) numax_out[e] = cmax * h * spdmax;
 }
 
+// The features start over the statistics, but not with fewer than four blocks per SM:
+// such a grid settles on the first SMs that the statistics leave, five blocks to
+// an SM while others stay empty.  Features with the statistics at 400,000 element points, started early /
+// behind them, us: porder 7 numbered along x 22.9 / 21.6, nodes in random order 68 / 42
+// (52 before they started early), 6 23.4 / 24.7 and 64 / 45, 5 20.1 / 20.0 and 37 / 27;
+// from 2.4 M points on the early start saves 4.
 template <int P>
 cudaError_t features_p(const FeatureArgs &a, cudaStream_t st)
 {
     constexpr int kFeatWarps = feat_warps<P>();
     const unsigned grid = (unsigned)((a.nelem + kFeatWarps - 1) / kFeatWarps);
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (grid < 4u * (unsigned)sms) {
+        features_kernel<P><<<grid, 32 * kFeatWarps, 0, st>>>(a.nelem, a.npoin, a.connec, a.He, a.gpvol, a.invAtoIJK,
+                                                             a.dlxigp_ip, a.rho, a.u, a.p_or_T, a.Rgas, a.gamma,
+                                                             a.cmax, a.stats, a.feat, a.numax);
+        return cudaGetLastError();
+    }
     return launch_after(features_kernel<P>, grid, 32 * kFeatWarps, 0, st, a.nelem, a.npoin, a.connec, a.He, a.gpvol,
                         a.invAtoIJK, a.dlxigp_ip, a.rho, a.u, a.p_or_T, a.Rgas, a.gamma, a.cmax, a.stats, a.feat,
                         a.numax);
