@@ -46,6 +46,13 @@ def algorithmic_bytes(nelem, n, npoin):
     return conv, diff
 
 
+def launches_per_step(porder, points):
+    """Kernels of one convection and one diffusion call: zeroing and residual kernel each, and the table
+    kernel of a diffusion that takes its matrices from the constant bank (diffu_const_points, msod_diffu.cu)."""
+    bank = 500000 if porder in (5, 6) else (12000000 if porder == 4 else 3000000)
+    return 5 if points >= bank else 4
+
+
 def peak_hbm():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
@@ -457,8 +464,7 @@ def run_ours(args, cfg, rank, local, world):
         "kernels": {"convec_ms": conv_ms, "diffu_ms": diff_ms, "convec_gbs": Bc / conv_ms / 1e6,
                     "diffu_gbs": Bd / diff_ms / 1e6,
                     "combined_frac": (Bc + Bd) / ((conv_ms + diff_ms) * 1e-3) / 1e9 / peak},
-        # per step: zeroing + kernel of the convection; zeroing, table preparation and kernel of the diffusion
-        "gpu_launches": 5 * args.steps,
+        "gpu_launches": launches_per_step(cfg.porder, dev.nelem * cfg.nnode) * args.steps,
         "clocks": clocks,
         "e2e": e2e,
     }
