@@ -25,9 +25,9 @@ thread_local char g_err[512] = "";
 std::atomic<int> g_checked{0};
 
 // Per-device library-owned device memory: the 4-byte flag word of
-// msod_check_element_tables and the per-call element tables of the kernels,
-// one table area per porder (calls of different porders on different streams
-// do not share one).
+// msod_check_element_tables, and per porder (calls of different porders on
+// different streams do not share one) the area where a kernel's expired wait is
+// recorded and the constant bank's derivative matrices are formed.
 std::mutex g_mu;
 int *g_flags[64] = {nullptr};
 TableScratch *g_tables[64] = {nullptr};
