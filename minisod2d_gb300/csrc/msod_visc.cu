@@ -153,22 +153,27 @@ __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, c
 template <int P, bool LIST>
 struct ViscGroup {
     static constexpr int ne[8] = {0, 32, 16, 8, 8, 4, 3, 3}, nl[8] = {0, 32, 16, 8, 5, 4, 3, 3};
-    using G = GroupGeom<float, P, LIST ? nl[P] : ne[P]>;
+    // R in the spent zeta columns of He (each read in the zeta pass only, by the thread
+    // that owns the point's zeta line) and gpvol read in place.
+    static constexpr bool SLIM = !LIST && P == 5;
+    using G = GroupGeom<float, P, LIST ? nl[P] : ne[P], 1, (P <= 2), !SLIM>;
     // Blocks per SM that the registers are held to (0: the compiler's choice).
     static constexpr int MINB = LIST && P == 4 ? 6 : 0;
     // Shared memory that an SM should keep for the blocks (percent, -1: as many blocks
     // as fit).  Beyond 196 KB 28 KB of L1 are left, too few for the cache lines of the
-    // gathers in flight: one block less (porder 5) takes 0.248 instead of 0.253 ms on a
-    // mesh numbered along x and 0.59 instead of 1.21 with nodes in random order, porder 1
-    // 0.148 / 0.146 and 0.22 / 0.34, 3 0.185 / 0.172 and 0.48 / 0.89 (12 M element points).
-    static constexpr int CARVEOUT = LIST ? -1 : (P == 1 || P == 3 ? 80 : (P == 5 ? 65 : -1));
+    // gathers in flight: one block less takes, ms, porder 1 0.148 instead of 0.146 on a
+    // mesh numbered along x and 0.22 instead of 0.34 with nodes in random order, 3 0.185 /
+    // 0.172 and 0.48 / 0.89 (12 M element points).  At porder 5 SLIM makes the four
+    // blocks fit: 0.230 against 0.245 and 0.70 against 1.20 (a block less: 0.248, 0.59).
+    static constexpr int CARVEOUT = LIST ? -1 : (P == 1 || P == 3 ? 80 : -1);
 };
 
 template <class G, bool LIST>
 struct ViscShared {
     static constexpr size_t kHe = LIST ? 0 : G::HEB + G::GPB + 16;
     static constexpr size_t kR = kHe + G::NREC * sizeof(Four<float>);
-    static constexpr size_t kV = kR + G::NSC * sizeof(float);
+    static constexpr bool kSlots = !LIST && !G::GPSTAGED;
+    static constexpr size_t kV = kR + (kSlots ? 0 : G::NSC * sizeof(float));
     static constexpr size_t kEl = kV + (size_t)G::NE * G::L * sizeof(float);  // per element: max speed, max |R|, nu
     static constexpr size_t kTab = (kEl + 3 * (size_t)G::NE * sizeof(float) + 15) / 16 * 16;
     static constexpr size_t kBytes = kTab + GroupTables<G, false>::kBytes;
@@ -265,6 +270,13 @@ __global__ void __launch_bounds__(G::NT, MINB)
             else
                 return gm.he(t.el, a);
         };
+        // R of the point with record o and gmsh node a.
+        auto Rat = [&](int o, int a) -> float & {
+            if constexpr (ViscShared<G, LIST>::kSlots)
+                return gm.he(t.el, a)[6];
+            else
+                return sm.R()[o];
+        };
         int pt[Q], id[Q];
 #pragma unroll
         for (int k = 0; k < Q; ++k) pt[k] = GroupTables<G, false>::node(inv, t.template lat<2>(k));
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
         if (t.active) {
 #pragma unroll
             for (int k = 0; k < Q; ++k) {
-                if constexpr (LIST)
+                if constexpr (LIST || !G::GPSTAGED)
                     vol += e >= 0 ? ldg(gpvol + (size_t)e * N + pt[k]) : 0.0f;
                 else
                     vol += *gm.vol(t.el, pt[k]);
@@ -326,7 +338,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
             visc_line<G, 2>(w, t, tab, he, pt, R);
             const int base = t.rec0(2);
 #pragma unroll
-            for (int k = 0; k < Q; ++k) sm.R()[base + k * G::template step<2>()] = R[k];
+            for (int k = 0; k < Q; ++k) Rat(base + k * G::template step<2>(), pt[k]) = R[k];
         }
         __syncthreads();
         if (t.active) {
@@ -336,7 +348,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
             visc_line<G, 0>(w, t, tab, he, lp, R);
             const int base = t.rec0(0);
 #pragma unroll
-            for (int k = 0; k < Q; ++k) sm.R()[base + k] += R[k];
+            for (int k = 0; k < Q; ++k) Rat(base + k, lp[k]) += R[k];
         }
         __syncthreads();
         if (t.active) {
@@ -348,7 +360,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
             unsigned mx = 0u;
 #pragma unroll
             for (int k = 0; k < Q; ++k)
-                mx = max(mx, __float_as_uint(fabsf(sm.R()[base + k * G::template step<1>()] + R[k])));
+                mx = max(mx, __float_as_uint(fabsf(Rat(base + k * G::template step<1>(), lp[k]) + R[k])));
             if (e >= 0) atomicMax(sm.res() + t.el, mx);
         }
         __syncthreads();
