@@ -65,7 +65,10 @@ struct DiffuRows<G, true> {
 // element (mu_e(e, a) = rho(a) nu_elem(e)).
 enum { VISC_MU_E = 0, VISC_NU_ELEM = 1 };
 
-// Elements per block and blocks per SM that the register budget allows for.
+// Elements per block and blocks per SM that the register budget allows for.  The
+// comparisons stand as they were made; a call takes now (ms): porder 1 128^3 0.326,
+// 2 100^3 0.591, 3 80^3 0.743, 4 64^3 0.946, 5 51^3 0.965, 6 40^3 0.875, 7 32^3 0.665, 8
+// 26^3 0.693.
 // Whole warps of lines (5 x 25 lines at porder 4: 125 of 128 threads) count
 // most, then the L1 that the blocks' shared memory leaves for the gathers'
 // lines in flight (porder 5: three blocks of 65.6 KB, within a 196 KB carveout,
@@ -136,7 +139,8 @@ constexpr long long diffu_const_points()
 // each) the fluxes of tau_2, tau_3: as halves of 16-byte records, which each direction
 // reads and writes alone, they took twice the wavefronts (porder 4 64^3 0.951 / 0.925
 // ms, 5 51^3 0.904 / 0.886, 7 32^3 0.791 / 0.770).  Not at porder 3, whose rows of four
-// conflict as pairs too (80^3 0.718 / 0.733).
+// conflict as pairs too (80^3 0.718 / 0.733).  kOver: the eta derivative of u3 takes u3's
+// place (each eta line's thread reads its u3 first; the xi lines are done with it).
 template <class G>
 struct DiffuShared {
     using real = typename G::real;

@@ -132,8 +132,8 @@ __global__ void entropy_stats_kernel(int npoin, const float *__restrict__ rho, c
 //   * He and gpvol come by bulk copy.  In list mode (the per-element fallback)
 //     the group's elements are scattered, and both are read in place.
 // Bound by the gathers' latency and the L1 / shared-memory pipe.  Estimator with
-// its statistics, before / now: porder 4 64^3 0.923 / 0.594 ms, 5 51^3 0.901 /
-// 0.611, 7 32^3 0.772 / 0.412, 2 100^3 0.707 / 0.383, 1 128^3 0.533 / 0.241.
+// its statistics, before / now: porder 4 64^3 0.923 / 0.548 ms, 5 51^3 0.901 /
+// 0.532, 7 32^3 0.772 / 0.374, 2 100^3 0.707 / 0.341, 1 128^3 0.533 / 0.203.
 // The line arithmetic is operation for operation the one that the shipped
 // networks were trained against: on smooth shock fields R is near its rounding
 // floor, and the product-rule defect formed from differences of nodal values
