@@ -100,11 +100,14 @@ __device__ __forceinline__ bool mbar_test(unsigned long long *bar, unsigned pari
 }
 // Waits for the phase of the given parity to complete, for at most about
 // 2^20 polls (~0.1 s with the back-off; a healthy copy of a group's span
-// completes in microseconds).  Returns false if the limit ran out.
+// completes in microseconds).  Returns false if the limit ran out; by then the
+// copies have had as long again, so that a late one does not outlive the block
+// that gives up on it.
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity)
 {
-    for (int it = 0; it < (1 << 20); ++it) {
-        if (mbar_test(bar, parity)) return true;
+    constexpr int limit = 1 << 20;
+    for (int it = 0; it < 2 * limit; ++it) {
+        if (mbar_test(bar, parity)) return it < limit;
         if (it >= 32) __nanosleep(64);
     }
     return false;
