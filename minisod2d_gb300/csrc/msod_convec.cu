@@ -61,8 +61,8 @@ namespace {
 // Elements per block, threads per line, blocks per SM that the register budget
 // allows for, and the form of the passes, measured per porder (FP32, ms).  The
 // comparisons stand as they were made; a call takes now: porder 1 128^3 0.281, 2
-// 100^3 0.521, 3 80^3 0.682, 4 64^3 0.943, 5 51^3 1.132, 6 40^3 1.035, 7 32^3 0.769, 8
-// 26^3 0.907.
+// 100^3 0.520, 3 80^3 0.658, 4 64^3 0.942, 5 51^3 1.130, 6 40^3 1.054, 7 32^3 0.767, 8
+// 26^3 0.903.
 // Whole warps of lines count most (5 x 25 lines at porder 4: 125 of 128
 // threads), then what is left of the L1 beside the blocks' shared memory, where
 // the gathers' lines are in flight: three blocks of 64 KB stay within a 196 KB
@@ -108,16 +108,16 @@ constexpr bool convec_rolled()
 {
     return P >= 6;
 }
-// Sums kept in the spent part of the He records (ConvecShared::kSlots): where
-// it makes room for another block (porder 7: 0.786 / 0.860; porder 5 1.143 /
-// 1.155) or, at porder 3, for 60 instead of 28 KB of L1 beside four blocks (12 M element
-// points, numbered along x 0.256 / 0.258, nodes in random order 1.61 / 2.38, elements in
-// random order 0.752 / 1.015); elsewhere the records' bank conflicts cost more than the
-// room gives.
+// Sums kept in the spent part of the He records (ConvecShared::kSlots): 2, mass and
+// energy and the node, where it makes room for another block (porder 7: 0.786 / 0.860;
+// porder 5 1.143 / 1.155); 1, mass and node, at porder 3, where it makes room for 60
+// instead of 28 KB of L1 beside four blocks (12 M element points, numbered along x
+// 0.248 / 0.257, nodes in random order 1.61 / 2.37, elements in random order 0.75 / 1.01);
+// elsewhere the records' bank conflicts cost more than the room gives.
 template <typename real, int P>
-constexpr bool convec_slots()
+constexpr int convec_slots()
 {
-    return sizeof(real) == 4 && (P == 3 || P == 5 || P == 7);
+    return sizeof(real) == 8 ? 0 : (P == 5 || P == 7 ? 2 : (P == 3 ? 1 : 0));
 }
 // Blocks of closely numbered elements gather through the L1 (group_close): on 12 M
 // element points in elements with nodes of their own, past it / through it, ms: porder 1
@@ -149,10 +149,10 @@ struct ConvecShared {
     static constexpr size_t kW = G::HEB + G::GPB + 16;
     static constexpr size_t kV = kW + G::NREC * sizeof(Four<real>);
     static constexpr size_t kA = kV + G::NREC * sizeof(Four<real>);
-    static constexpr bool kSlots = convec_slots<real, G::P>();
-    static constexpr size_t kZ = kA + (kSlots ? G::NPR * sizeof(Two<real>) : G::NREC * sizeof(Four<real>));
+    static constexpr int kSlots = convec_slots<real, G::P>();
+    static constexpr size_t kZ = kA + (kSlots == 2 ? G::NPR * sizeof(Two<real>) : G::NREC * sizeof(Four<real>));
     static constexpr size_t kM = kZ + G::NSC * sizeof(real);
-    static constexpr size_t kNode = kM + G::NSC * sizeof(real);
+    static constexpr size_t kNode = kM + (kSlots == 1 ? 0 : G::NSC * sizeof(real));
     static constexpr size_t kTab = (kNode + (kSlots ? 0 : G::NSC * sizeof(int)) + 15) / 16 * 16;
     static constexpr size_t kBytes = kTab + GroupTables<G, true>::kBytes;
     unsigned char *base;
@@ -171,10 +171,10 @@ struct ConvecShared {
     // The sums of a point (record o, its He record at he) between the passes.
     // kSlots: the zeta column of a point's He record is read in the zeta pass
     // only, by the thread that owns the point's zeta line; from then on it holds
-    // the mass and energy sums and the point's node.
+    // the mass sum, the energy sum (2) and the point's node.
     __device__ __forceinline__ void put(int o, real *he, const Two<real> &a, const Two<real> &b, real m) const
     {
-        if constexpr (kSlots) {
+        if constexpr (kSlots == 2) {
             A2()[o] = a;
             M()[o] = b.x;
             he[6] = b.y;
@@ -184,12 +184,12 @@ struct ConvecShared {
             p.a = a;
             p.b = b;
             A()[o] = p;
-            M()[o] = m;
+            (kSlots ? he[7] : M()[o]) = m;
         }
     }
     __device__ __forceinline__ void add(int o, const real *he, Two<real> &a, Two<real> &b, real &m) const
     {
-        if constexpr (kSlots) {
+        if constexpr (kSlots == 2) {
             a = add2(a, A2()[o]);
             b = add2(b, two(M()[o], he[6]));
             m += he[7];
@@ -197,12 +197,12 @@ struct ConvecShared {
             const Four<real> p = A()[o];
             a = add2(a, p.a);
             b = add2(b, p.b);
-            m += M()[o];
+            m += kSlots ? he[7] : M()[o];
         }
     }
     __device__ __forceinline__ int node_at(int o, const real *he) const
     {
-        if constexpr (kSlots)
+        if constexpr (kSlots != 0)
             return __float_as_int(he[8]);
         else
             return node()[o];
@@ -255,7 +255,7 @@ __device__ __forceinline__ void convec_finish(const ConvecDir<G> &d, const Conve
     if (!d.first) sm.add(o, he, a, b, m);
     if (!d.last) {
         sm.put(o, he, a, b, m);
-        if constexpr (ConvecShared<G>::kSlots)
+        if constexpr (ConvecShared<G>::kSlots != 0)
             if (d.first) he[8] = __int_as_float(node0);
     } else {
         const int node = sm.node_at(o, he);
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(G::NT, MINB)
                 sm.W()[o] = w;
                 sm.V()[o] = v;
                 sm.Z()[o] = f[k][7];
-                if constexpr (!ConvecShared<G>::kSlots) sm.node()[o] = id[k];
+                if constexpr (ConvecShared<G>::kSlots == 0) sm.node()[o] = id[k];
             }
             if (G::S == 1) ln.set(k, w, v, f[k][7]);
         }

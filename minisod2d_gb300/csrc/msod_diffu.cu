@@ -67,8 +67,8 @@ enum { VISC_MU_E = 0, VISC_NU_ELEM = 1 };
 
 // Elements per block and blocks per SM that the register budget allows for.  The
 // comparisons stand as they were made; a call takes now (ms): porder 1 128^3 0.326,
-// 2 100^3 0.591, 3 80^3 0.743, 4 64^3 0.946, 5 51^3 0.965, 6 40^3 0.875, 7 32^3 0.665, 8
-// 26^3 0.693.
+// 2 100^3 0.592, 3 80^3 0.743, 4 64^3 0.946, 5 51^3 0.933, 6 40^3 0.874, 7 32^3 0.665, 8
+// 26^3 0.691.
 // Whole warps of lines (5 x 25 lines at porder 4: 125 of 128 threads) count
 // most, then the L1 that the blocks' shared memory leaves for the gathers'
 // lines in flight (porder 5: three blocks of 65.6 KB, within a 196 KB carveout,

@@ -33,6 +33,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "msod_device.cuh"
 #include "msod_kernels.h"
 
@@ -171,9 +173,11 @@ struct GroupGeom {
     static constexpr int BANKS = 128 / (int)sizeof(real), OFF = 16 / (int)sizeof(real);
     static constexpr int pitch(int n) { return SPLIT ? n + (BANKS + OFF - n % BANKS) % BANKS : n; }
     static constexpr int HEP = pitch(9 * N), GPP = pitch(N);
-    static constexpr size_t HEB = STAGED ? ((size_t)NE * HEP * sizeof(real) + 31) / 16 * 16 : 0;
+    // Spans of the group with up to 12 bytes of shift (SpanPlan).
+    static constexpr size_t span(int p, int n) { return (((size_t)(NE - 1) * p + n) * sizeof(real) + 12 + 15) / 16 * 16; }
+    static constexpr size_t HEB = STAGED ? span(HEP, 9 * N) : 0;
     static constexpr bool GPSTAGED = STAGED && GP_;
-    static constexpr size_t GPB = GPSTAGED ? ((size_t)NE * GPP * sizeof(real) + 31) / 16 * 16 : 0;
+    static constexpr size_t GPB = GPSTAGED ? span(GPP, N) : 0;
     template <int DIR>
     static constexpr int step()
     {
@@ -320,18 +324,21 @@ struct GroupTables {
     static constexpr int Q = G::Q, N = G::N;
     static constexpr int ROW = (Q + 3) / 4 * 4;  // pitch of a row
     static constexpr size_t kD = (size_t)(FULL ? 6 : 3) * Q * ROW * sizeof(real);
-    static constexpr size_t kBytes = kD + (FULL ? (size_t)(3 * Q) * sizeof(real) + (size_t)N * sizeof(int) : 0);
+    // Permutation entries of two bytes where the block's shared memory is short of 128 (the
+    // porder-3 convection); elsewhere they cost up to 1.6 % (porder 7 32^3).
+    using Node = std::conditional_t<G::P == 3, unsigned short, int>;
+    static constexpr size_t kBytes = kD + (FULL ? (size_t)(3 * Q) * sizeof(real) + (size_t)N * sizeof(Node) : 0);
     unsigned char *base;  // 16-byte aligned
     __device__ __forceinline__ real *D(int dir, int r) const { return reinterpret_cast<real *>(base) + (dir * Q + r) * ROW; }
     __device__ __forceinline__ real *Dt(int dir, int c) const { return D(3 + dir, c); }
     __device__ __forceinline__ real *sums() const { return reinterpret_cast<real *>(base + kD); }  // [dir Q + r]
-    __device__ __forceinline__ int *perm() const { return reinterpret_cast<int *>(sums() + 3 * Q); }
+    __device__ __forceinline__ Node *perm() const { return reinterpret_cast<Node *>(sums() + 3 * Q); }
     static __device__ __forceinline__ int node(const int *inv, int l) { return min(max(ldg(inv + l) - 1, 0), N - 1); }
     // All threads call it; complete after the next barrier.
     __device__ __forceinline__ void build(const int *__restrict__ inv, const real *__restrict__ dlx, int tid) const
     {
         if (FULL)
-            for (int i = tid; i < N; i += G::NT) perm()[i] = node(inv, i);
+            for (int i = tid; i < N; i += G::NT) perm()[i] = (Node)node(inv, i);
         const int i = tid - (G::NT - 32);  // the last warp: one row per lane
         if (i >= 0 && i < 3 * Q) {
             const int d = i / Q, r = i - d * Q;
@@ -365,6 +372,7 @@ __device__ __forceinline__ unsigned after_barrier(const void *p)
     return a;
 }
 __device__ __forceinline__ void lds(int &v, unsigned a) { asm("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_u16(int &v, unsigned a) { asm("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a)); }
 __device__ __forceinline__ void lds(float &v, unsigned a) { asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
 __device__ __forceinline__ void lds(double &v, unsigned a) { asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
 __device__ __forceinline__ void lds(Four<float> &v, unsigned a)
@@ -409,7 +417,11 @@ struct GroupRows {
     __device__ __forceinline__ int node(int l) const
     {
         int v;
-        lds(v, base + (unsigned)(T::kD + 3 * G::Q * sizeof(real) + l * sizeof(int)));
+        const unsigned at = base + (unsigned)(T::kD + 3 * G::Q * sizeof(real) + l * sizeof(typename T::Node));
+        if constexpr (sizeof(typename T::Node) == 2)
+            lds_u16(v, at);
+        else
+            lds(v, at);
         return v;
     }
 };
